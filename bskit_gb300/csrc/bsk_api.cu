@@ -365,6 +365,7 @@ void destroy_plan(bsk_plan* p) {
   if (p->z2d_ok) cufftDestroy(p->z2d);
   if (p->work) cudaFree(p->work);
   if (p->synth_ws) cudaFree(p->synth_ws);
+  for (auto& b : p->tail_scratch) cudaFree(b.first);
   release_stream(p);
   delete p;
 }
@@ -397,7 +398,8 @@ void contract_dispatch(bsk_plan* p, const bsk_triset* set, const float* f1, cons
     case BSK_PREC_BF16X3:
     case BSK_PREC_BF16:
       launch_contract_tc(set->sched, f1, f2, split, split_shells, p->n, K, k0, k1,
-                         precision == BSK_PREC_BF16X3 ? 3 : 1, out, p->num_sms, st);
+                         precision == BSK_PREC_BF16X3 ? 3 : 1, out, p->num_sms, st, 1.0,
+                         set->scratch, set->scratch_bytes);
       break;
     default:
       throw Error{BSK_ERR_ARG, "unknown precision " + std::to_string(precision)};
@@ -698,6 +700,29 @@ void build_levels(bsk_plan* p, bsk_triset* set) {
   }
 }
 
+// The contraction scratch of a set's resident launches (levels run one after the other and
+// share it).  Without room for it, or under a memory budget, the set runs without; it is a
+// triangle set's resource, like its schedule, so the plan's footprint does not count it
+// (callers size budgets from that figure).
+void attach_scratch(bsk_plan* p, bsk_triset* set) {
+  if (p->mem_budget) return;
+  size_t need = set->levels.empty()
+                    ? contract_tc_scratch(set->sched.h_tiles, p->K, p->num_sms) : 0;
+  for (const GridLevel& lv : set->levels)
+    need = std::max(need, contract_tc_scratch(lv.sched.h_tiles, lv.plan->K, p->num_sms));
+  if (!need) return;
+  if (p->tail_scratch.empty() || p->tail_scratch.back().second < need) {
+    void* ptr = nullptr;
+    if (cudaMalloc(&ptr, need) != cudaSuccess) {
+      cudaGetLastError();
+      return;
+    }
+    p->tail_scratch.emplace_back(ptr, need);
+  }
+  set->scratch = p->tail_scratch.back().first;
+  set->scratch_bytes = p->tail_scratch.back().second;
+}
+
 // A point range [k0, k1) of the plan's grid as the matching share of a level's grid
 // (128-point aligned, so that the ranges of consecutive shards tile the level's grid).
 int64_t level_point(int64_t k, int64_t K, int64_t Kq) {
@@ -748,7 +773,7 @@ void measure_levels(bsk_plan* p, const bsk_triset* set, int a, int b, int c, int
       default:
         launch_contract_tc(lv.sched, fa, fb, q->slot[c].split, q->n_alloc(), q->n, q->K, q0,
                            q1, precision == BSK_PREC_BF16X3 ? 3 : 1, out, q->num_sms, st,
-                           scale);
+                           scale, set->scratch, set->scratch_bytes);
         break;
     }
   }
@@ -1088,6 +1113,7 @@ int bsk_triset_create(bsk_plan* p, int64_t n_tri, const int32_t* tri, bsk_triset
     }
     build_schedule(s->u_tri, p->n, s->sched, &s->u_idx);
     if (p->use_levels && !s->u_tri.empty()) build_levels(p, s.get());
+    attach_scratch(p, s.get());
     if (!dups.empty()) {
       s->n_dups = (int)dups.size();
       s->dups = (int2*)dmalloc(dups.size() * sizeof(int2));

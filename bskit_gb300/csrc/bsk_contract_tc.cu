@@ -40,9 +40,19 @@
 // fixed cost of a stage's barrier round trips is spread over 16 MMAs.  Every wait is bounded
 // (globaltimer); on expiry the kernel records an error flag, stops issuing work, drains
 // its own MMAs and frees TMEM.
+//
+// Short grids.  Work items are the unit of the FP32 sums, so a grid of few slices leaves SMs
+// idle: 48^3 points are 7 slices, 7 CTAs of 152, each a chain of 128 stages (110 us).  The
+// items of the last, partly filled wave ("tail items", all items of a short grid) are
+// therefore cut into parts of a few stages spread over all SMs; the drain writes each stage's
+// two accumulator halves (hi*Bhi + lo*Bhi and hi*Blo + lo*Blo) of the bins to a scratch area
+// and tail_sum_kernel adds them in the order the drain's registers would have, so every bin
+// keeps its value bit for bit (tail_plan has the rule and the measured times).
 #include <cuda.h>
 
+#include <algorithm>
 #include <atomic>
+#include <type_traits>
 
 #include "bsk_internal.cuh"
 
@@ -332,17 +342,55 @@ __device__ __forceinline__ void split2(unsigned long long p, uint32_t& hi, uint3
   lo = bf16x2_of(f2_sub(p, g));
 }
 
+// The work of a launch: items [0, n_full) whole, the n_tail items after them in `parts` parts
+// of `part_stages` stages each, whose accumulators go to `scratch` ([tail item][stage of the
+// slice][half][nc_stride columns][128 rows]).
+struct TailPlan {
+  int n_full = 0, n_tail = 0, parts = 1, part_stages = 0, nc_stride = 0;
+  float* scratch = nullptr;
+  __host__ __device__ int units() const { return n_full + n_tail * parts; }
+};
+
+struct Work {
+  int tile;
+  int tail;             // tail item, or -1: a whole item
+  int stage0;           // first stage of the part inside its slice
+  int x_begin, x_end;   // K < 2^31
+};
+
+template <int kSlice, bool kTail>
+__device__ __forceinline__ Work decode(int u, const TailPlan& tp, int n_tiles, int k_begin,
+                                       int k_end) {
+  Work w;
+  int item = u, part = 0;
+  w.tail = -1;
+  if (kTail && u >= tp.n_full) {
+    w.tail = (u - tp.n_full) / tp.parts;
+    part = (u - tp.n_full) - w.tail * tp.parts;
+    item = tp.n_full + w.tail;
+  }
+  const int sl = item / n_tiles;
+  w.tile = item - sl * n_tiles;
+  w.stage0 = part * tp.part_stages;
+  const int first = k_begin + sl * kSlice;
+  const int end = min(k_end - first, kSlice);  // k_end > first: no sum overflows
+  w.x_begin = first + min(end, w.stage0 * KCH);
+  w.x_end = first + min(end, w.tail >= 0 ? (w.stage0 + tp.part_stages) * KCH : kSlice);
+  return w;
+}
+
 // 26 warps: 7 share one SM sub-partition, whose 16K registers allow 73 per thread.
-template <bool kTwoSrc, bool kLongSlice>
+template <bool kTwoSrc, bool kLongSlice, bool kTail>
 __global__ void __launch_bounds__(THREADS, 1)
     contract_tc_kernel(const __grid_constant__ Maps maps, const TileDesc* __restrict__ tiles,
                        const int16_t* __restrict__ row_i, const int16_t* __restrict__ row_j,
                        const int32_t* __restrict__ map, int n_tiles, int same_src,
-                       int64_t k_begin, int64_t k_end, int64_t n_items, int terms, int fused,
+                       int k_begin, int k_end, const TailPlan tp, int terms, int fused,
                        double* __restrict__ out, double scale) {
-  constexpr int64_t slice = kLongSlice ? kSliceLong : kSliceShort;
+  constexpr int slice = (int)(kLongSlice ? kSliceLong : kSliceShort);
   constexpr int STAGE_BYTES = Ring<kTwoSrc>::kStageBytes;
   constexpr int SST = Ring<kTwoSrc>::kStages;
+  const int n_units = tp.units();
   extern __shared__ uint8_t smem_raw[];
   const uint32_t raw = smem_u32(smem_raw);
   const uint32_t pad = (1024u - (raw & 1023u)) & 1023u;
@@ -390,22 +438,21 @@ __global__ void __launch_bounds__(THREADS, 1)
     if (lane == 0) {
       uint32_t chunk = 0;
       bool ok = true;
-      for (int64_t item = blockIdx.x; item < n_items && ok; item += gridDim.x) {
-        const int64_t sl = item / n_tiles;
-        const TileDesc td = tiles[item % n_tiles];
+      for (int u = blockIdx.x; u < n_units && ok; u += gridDim.x) {
+        const Work w = decode<slice, kTail>(u, tp, n_tiles, k_begin, k_end);
+        const TileDesc td = tiles[w.tile];
         const bool one_src = !kTwoSrc || (same_src && td.i0 == td.j0);
-        const int64_t x_begin = k_begin + sl * slice;
-        const int64_t x_end = min(k_end, x_begin + slice);
+        
         // bytes per stage: the four 32-point quarters of each source tile; the column rows
         // of hi and lo in both K blocks
         const uint32_t src_bytes =
             fused ? (uint32_t)(4 * 128 * (td.ni + (one_src ? 0 : td.nj)))
                   : (uint32_t)(4 * 128 * (box_rows(td.ni) + (one_src ? 0 : box_rows(td.nj))));
         const uint32_t b_bytes = (uint32_t)(4 * td.nc * 128);
-        for (int64_t x = x_begin; x < x_end; x += KCH, ++chunk) {
+        for (int x = w.x_begin; x < w.x_end; x += KCH, ++chunk) {
           const int s = chunk % SST;
           const uint32_t st = sbase + s * STAGE_BYTES;
-          const int xi = (int)x;
+          const int xi = x;
           // The source tiles of SMEM stage s were last read by the A-operand warps of stage
           // chunk - SST, its B tiles by that stage's MMAs, which complete ~one A-operand
           // stage later: the sources are refilled as soon as they are free.
@@ -450,18 +497,17 @@ __global__ void __launch_bounds__(THREADS, 1)
     // as one straight run; a loop run by a single lane issued 3-4x slower.
     uint32_t chunk = 0, grp = 0;
     bool ok = true;
-    for (int64_t item = blockIdx.x; item < n_items && ok; item += gridDim.x) {
-      const int64_t sl = item / n_tiles;
-      const TileDesc td = tiles[item % n_tiles];
-      const int64_t x_begin = k_begin + sl * slice;
-      const int64_t x_end = min(k_end, x_begin + slice);
+    for (int u = blockIdx.x; u < n_units && ok; u += gridDim.x) {
+      const Work w = decode<slice, kTail>(u, tp, n_tiles, k_begin, k_end);
+      const TileDesc td = tiles[w.tile];
+      
       // hi x [Bhi; Blo] and lo x [Bhi; Blo] (the lo rows of a block sit right after its nc
       // hi rows; N = 2 nc, a multiple of 16).  bf16 (one term): hi x Bhi, N = nc rounded up
       // to 16 (with nc an odd multiple of 8 the last 8 columns take lo rows, never read).
       const int n16 = (td.nc + 15) & ~15;
       const uint32_t kb_bytes = 2u * td.nc * 128u;
       const uint32_t idesc_stack = idesc_bf16(terms >= 3 ? 2 * td.nc : n16);
-      for (int64_t x = x_begin; x < x_end; x += KCH, ++chunk) {
+      for (int x = w.x_begin; x < w.x_end; x += KCH, ++chunk) {
         // a fresh accumulator per stage, once the drain has emptied it
         const uint32_t b = grp % NACC;
         const int s = chunk % SST;
@@ -507,17 +553,57 @@ __global__ void __launch_bounds__(THREADS, 1)
     const uint32_t taddr = tmem + ((uint32_t)(qd * 32) << 16) + c0;
     uint32_t grp = 0;
     bool ok = true;
-    for (int64_t item = blockIdx.x; item < n_items && ok; item += gridDim.x) {
-      const int64_t sl = item / n_tiles;
-      const TileDesc td = tiles[item % n_tiles];
-      const int64_t x_begin = k_begin + sl * slice;
-      const int64_t x_end = min(k_end, x_begin + slice);
-      const int64_t nch = (x_end - x_begin + KCH - 1) / KCH;
-      const int64_t ngrp = (nch + ACC_CHUNKS - 1) / ACC_CHUNKS;
+    for (int u = blockIdx.x; u < n_units && ok; u += gridDim.x) {
+      const Work w = decode<slice, kTail>(u, tp, n_tiles, k_begin, k_end);
+      const TileDesc td = tiles[w.tile];
+      const int ngrp = (int)((w.x_end - w.x_begin + KCH - 1) / KCH);
+      const int32_t* mp = map + td.map_off + c0 * kTileRows + r;
+      const bool rows = !kTail || qd * 32 < td.nrows;  // else no row of the quadrant is a pair
+      if (kTail && w.tail >= 0) {
+        // a part of a tail item: every stage's sums of the bins to the scratch area
+        uint32_t need = 0;
+#pragma unroll
+        for (int c = 0; c < 32; ++c)
+          if (c0 + c < td.nc && __ldg(mp + c * kTileRows) >= 0) need |= 1u << c;
+        const int64_t half = (int64_t)tp.nc_stride * kTileRows;
+        float* dst = tp.scratch +
+                     ((int64_t)w.tail * (slice / KCH) + w.stage0) * 2 * half + c0 * kTileRows + r;
+        for (int g = 0; g < ngrp; ++g, ++grp, dst += 2 * half) {
+          const uint32_t b = grp % NACC;
+          if (!__all_sync(0xffffffffu,
+                          mbar_wait(&bars->done[grp % DONE_RING], (grp / DONE_RING) & 1))) {
+            ok = false;
+            break;
+          }
+          tc_fence_after();
+#pragma unroll
+          for (int cc = 0; cc < 2; ++cc) {
+            if (rows && c0 + cc * 16 < td.nc) {
+              uint32_t v[16];
+              tmem_ld16(taddr + ACC_COL + b * 128 + cc * 16, v);
+#pragma unroll
+              for (int e = 0; e < 16; ++e)
+                if (need >> (cc * 16 + e) & 1)
+                  dst[(cc * 16 + e) * kTileRows] = __uint_as_float(v[e]);
+              if (terms >= 3) {
+                tmem_ld16(taddr + ACC_COL + b * 128 + td.nc + cc * 16, v);
+#pragma unroll
+                for (int e = 0; e < 16; ++e)
+                  if (need >> (cc * 16 + e) & 1)
+                    dst[half + (cc * 16 + e) * kTileRows] = __uint_as_float(v[e]);
+              }
+            }
+          }
+          tc_fence_before();
+          __syncwarp();
+          if (lane == 0) mbar_arrive(&bars->accempty[b]);
+        }
+        continue;
+      }
       float acc[32];
 #pragma unroll
       for (int c = 0; c < 32; ++c) acc[c] = 0.f;
-      for (int64_t g = 0; g < ngrp; ++g, ++grp) {
+      for (int g = 0; g < ngrp; ++g, ++grp) {
         const uint32_t b = grp % NACC;
         if (!__all_sync(0xffffffffu,
                         mbar_wait(&bars->done[grp % DONE_RING], (grp / DONE_RING) & 1))) {
@@ -527,7 +613,7 @@ __global__ void __launch_bounds__(THREADS, 1)
         tc_fence_after();
 #pragma unroll
         for (int cc = 0; cc < 2; ++cc) {
-          if (c0 + cc * 16 < td.nc) {
+          if (rows && c0 + cc * 16 < td.nc) {
             uint32_t v[16];
             tmem_ld16(taddr + ACC_COL + b * 128 + cc * 16, v);
 #pragma unroll
@@ -544,7 +630,6 @@ __global__ void __launch_bounds__(THREADS, 1)
         if (lane == 0) mbar_arrive(&bars->accempty[b]);
       }
       if (!ok) break;
-      const int32_t* mp = map + td.map_off + c0 * kTileRows + r;
 #pragma unroll
       for (int c = 0; c < 32; ++c) {
         if (c0 + c < td.nc) {
@@ -562,12 +647,15 @@ __global__ void __launch_bounds__(THREADS, 1)
     const uint32_t tlane = (uint32_t)(qd * 32) << 16;
     uint32_t chunk = 0;
     bool ok = true;
-    for (int64_t item = blockIdx.x; item < n_items && ok; item += gridDim.x) {
-      const int64_t sl = item / n_tiles;
-      const TileDesc td = tiles[item % n_tiles];
+    for (int u = blockIdx.x; u < n_units && ok; u += gridDim.x) {
+      const Work w = decode<slice, kTail>(u, tp, n_tiles, k_begin, k_end);
+      const TileDesc td = tiles[w.tile];
       const bool one_src = !kTwoSrc || (same_src && td.i0 == td.j0);
-      const int64_t x_begin = k_begin + sl * slice;
-      const int64_t x_end = min(k_end, x_begin + slice);
+      
+      // a quadrant whose 32 rows are all past the tile's pairs forms nothing: its accumulator
+      // rows depend on its A rows alone and the drain skips them (short grids only: their sets
+      // fill a fraction of one tile, and the test cost the large ones 0.8%)
+      const bool rows = !kTail || qd * 32 < td.nrows;
       const int ri = row_i[td.row_off + r];
       const int rj = row_j[td.row_off + r];
       const bool valid = ri >= 0;
@@ -577,7 +665,7 @@ __global__ void __launch_bounds__(THREADS, 1)
       const int qstride = fused ? td.ni * 128 : A_QUARTER;
       const int src2 = one_src ? 0 : (fused ? 4 * qstride : A_TILE);
       const int qstride2 = one_src ? qstride : (fused ? td.nj * 128 : A_QUARTER);
-      for (int64_t x = x_begin; x < x_end; x += KCH, ++chunk) {
+      for (int x = w.x_begin; x < w.x_end; x += KCH, ++chunk) {
         const int s = chunk % SST;
         const uint32_t ph = (chunk / SST) & 1;
         const int a = chunk % ASTAGES;
@@ -590,6 +678,15 @@ __global__ void __launch_bounds__(THREADS, 1)
           break;
         }
         tc_fence_after();
+        if (!rows) {
+          tc_fence_before();
+          __syncwarp();
+          if (lane == 0) {
+            mbar_arrive(&bars->afull[a]);
+            mbar_arrive(&bars->src_free[s]);
+          }
+          continue;
+        }
         const uint8_t* st = smem + s * STAGE_BYTES;
         const uint32_t a_hi = tmem + tlane + A_COL + a * 128 + part * (PPW / 2);
         // The warp's PPW points in NG groups of 8; the shared-memory loads of group g + 1
@@ -654,6 +751,59 @@ __global__ void __launch_bounds__(THREADS, 1)
                  "r"(TMEM_COLS)
                  : "memory");
   }
+}
+
+// The sums of the tail items: block = (column c, 32 rows) of one item.  Four warps load the
+// two halves of 32 stages each (64 loads a thread in flight: the kernel is bound by their
+// latency) into shared memory, then warp 0, lane = bin, adds them in stage order in FP32 --
+// the drain's own sequence -- and adds the sum to the bin with one FP64 atomic.
+constexpr int kTailChunk = 128;  // stages per round of loads
+__global__ void __launch_bounds__(128)
+    tail_sum_kernel(const TileDesc* __restrict__ tiles, const int32_t* __restrict__ map,
+                    int n_tiles, int64_t slice, int64_t k_begin, int64_t k_end,
+                    const TailPlan tp, int terms, double* __restrict__ out, double scale) {
+  __shared__ float sv[kTailChunk][2][32];
+  const int c = blockIdx.x, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int r = blockIdx.y * 32 + lane;
+  const int item = tp.n_full + blockIdx.z;
+  const int sl = item / n_tiles;
+  const TileDesc td = tiles[item - sl * n_tiles];
+  if (c >= td.nc) return;
+  const int t = __ldg(map + td.map_off + c * kTileRows + r);
+  if (__all_sync(0xffffffffu, t < 0)) return;  // the same rows in every warp of the block
+  const int64_t x_begin = k_begin + sl * slice;
+  const int n = (int)((min(k_end, x_begin + slice) - x_begin + KCH - 1) / KCH);
+  const int64_t half = (int64_t)tp.nc_stride * kTileRows;
+  const float* src = tp.scratch + (int64_t)blockIdx.z * (slice / KCH) * 2 * half +
+                     c * kTileRows + r;
+  float acc = 0.f;
+  for (int g0 = 0; g0 < n; g0 += kTailChunk) {
+    float v[32][2];
+    const int first = g0 + warp * 32;
+#pragma unroll
+    for (int e = 0; e < 32; ++e) {
+      const bool ok = first + e < n && t >= 0;
+      const float* p = src + (int64_t)(first + e) * 2 * half;
+      v[e][0] = ok ? __ldcs(p) : 0.f;
+      v[e][1] = ok && terms >= 3 ? __ldcs(p + half) : 0.f;
+    }
+    if (g0) __syncthreads();  // warp 0 has summed the previous round
+#pragma unroll
+    for (int e = 0; e < 32; ++e) {
+      sv[warp * 32 + e][0][lane] = v[e][0];
+      sv[warp * 32 + e][1][lane] = v[e][1];
+    }
+    __syncthreads();
+    if (warp == 0) {
+      const int m = min(n - g0, kTailChunk);
+#pragma unroll 8
+      for (int e = 0; e < m; ++e) {
+        acc += sv[e][0][lane];
+        if (terms >= 3) acc += sv[e][1][lane];
+      }
+    }
+  }
+  if (warp == 0 && t >= 0) atomicAdd(out + t, (double)acc * scale);
 }
 
 typedef CUresult (*EncodeTiledFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*,
@@ -722,12 +872,74 @@ void make_split_map(CUtensorMap* m, const __nv_bfloat16* split, int S, int64_t K
               "cuTensorMapEncodeTiled (split) failed: " + std::to_string((int)r));
 }
 
+// How the items of a launch are split.  A stage is one unit of time (~0.8 us); without a tail
+// the launch takes ceil(items / SMs) x the stages of a slice.  With one, the last wave's items
+// go out in parts of `ps` stages, in ceil(parts / SMs) rounds, then pay for tail_sum_kernel
+// (~8 units, launch included) and for writing and reading their scratch (~4 units a megabyte
+// over ~5 TB/s: 0.5 unit).  Taken when that saves 3%: the 7 items of 48^3 (110 -> 15 us with
+// the sum kernel) and the 54 of 96^3 do; a last wave that is more than about half full
+// does not.  Scratch above kMaxTailBytes is not considered.
+constexpr double kTailSumStages = 8.0, kTailStagesPerMB = 0.5;
+constexpr size_t kMaxTailBytes = (size_t)128 << 20;
+
+struct Split {
+  int64_t slice = kSliceShort;
+  TailPlan tp;
+  size_t scratch_bytes = 0;
+};
+
+Split make_split(const std::vector<TileDesc>& tiles, int64_t points, int num_sms,
+                 size_t scratch_have) {
+  Split sp;
+  const int n_tiles = (int)tiles.size();
+  const bool long_slice =
+      (points + kSliceLong - 1) / kSliceLong * n_tiles >= kMinItemsPerSm * num_sms;
+  sp.slice = long_slice ? kSliceLong : kSliceShort;
+  const int64_t n_items = (points + sp.slice - 1) / sp.slice * n_tiles;
+  BSK_REQUIRE(n_items < ((int64_t)1 << 30), BSK_ERR_UNSUPPORTED, "too many contraction items");
+  sp.tp.n_full = (int)n_items;
+  const int rem = (int)(n_items % num_sms);
+  if (rem == 0) return sp;
+  const int stages = (int)((std::min(points, sp.slice) + KCH - 1) / KCH);
+  int nc = 0;
+  for (const TileDesc& d : tiles) nc = std::max(nc, d.nc);
+  const size_t bytes =
+      (size_t)rem * (sp.slice / KCH) * 2 * nc * kTileRows * sizeof(float);
+  if (bytes > kMaxTailBytes || bytes > scratch_have) return sp;
+  const double extra = kTailSumStages + kTailStagesPerMB * bytes / 1e6;
+  int best_ps = 0;
+  double best = 0.97 * stages;  // the last wave as it is
+  for (int ps = 2; ps < stages; ++ps) {
+    const int parts = (stages + ps - 1) / ps;
+    const int rounds = (rem * parts + num_sms - 1) / num_sms;
+    const double t = (double)rounds * (ps + 0.5) + extra;
+    if (t < best) {
+      best = t;
+      best_ps = ps;
+    }
+  }
+  if (!best_ps) return sp;
+  sp.tp.n_full = (int)n_items - rem;
+  sp.tp.n_tail = rem;
+  sp.tp.part_stages = best_ps;
+  sp.tp.parts = (stages + best_ps - 1) / best_ps;
+  sp.tp.nc_stride = nc;
+  sp.scratch_bytes = bytes;
+  return sp;
+}
+
 }  // namespace tc
+
+size_t contract_tc_scratch(const std::vector<TileDesc>& tiles, int64_t points, int num_sms) {
+  if (tiles.empty() || points <= 0) return 0;
+  return tc::make_split(tiles, points, num_sms, tc::kMaxTailBytes).scratch_bytes;
+}
 
 void launch_contract_tc(const DeviceSchedule& s, const float* f1, const float* f2,
                         const __nv_bfloat16* f3_split, int split_shells, int n_shells,
                         int64_t K, int64_t k_begin, int64_t k_end, int terms, double* out,
-                        int num_sms, cudaStream_t st, double scale) {
+                        int num_sms, cudaStream_t st, double scale, void* scratch,
+                        size_t scratch_bytes) {
   if (s.n_tiles == 0 || k_end <= k_begin) return;
   BSK_REQUIRE(k_begin % tc::KCH == 0, BSK_ERR_ARG, "k_begin must be a multiple of 128");
   BSK_REQUIRE(k_end % tc::KCH == 0 || k_end == K, BSK_ERR_ARG,
@@ -752,32 +964,41 @@ void launch_contract_tc(const DeviceSchedule& s, const float* f1, const float* f
   }
   bool two_src = f1 != f2;
   for (const TileDesc& d : s.h_tiles) two_src = two_src || d.i0 != d.j0;
-  const bool long_slice = (k_end - k_begin + tc::kSliceLong - 1) / tc::kSliceLong * s.n_tiles >=
-                         tc::kMinItemsPerSm * num_sms;
-  const int64_t slice = long_slice ? tc::kSliceLong : tc::kSliceShort;
-  const int64_t n_slices = (k_end - k_begin + slice - 1) / slice;
-  const int64_t n_items = n_slices * s.n_tiles;
+  tc::Split sp = tc::make_split(s.h_tiles, k_end - k_begin, num_sms,
+                                scratch ? scratch_bytes : 0);
+  sp.tp.scratch = (float*)scratch;
+  const bool long_slice = sp.slice == tc::kSliceLong;
   constexpr int kMaxDev = 64;
-  static std::atomic<bool> attr_set[kMaxDev][4];  // zero-initialised: false
+  static std::atomic<bool> attr_set[kMaxDev][8];  // zero-initialised: false
   int dev = 0;
   BSK_CHECK_CUDA(cudaGetDevice(&dev));
   BSK_REQUIRE(dev < kMaxDev, BSK_ERR_UNSUPPORTED, "device ordinal above 63");
-  auto kern = two_src ? (long_slice ? tc::contract_tc_kernel<true, true>
-                                    : tc::contract_tc_kernel<true, false>)
-                      : (long_slice ? tc::contract_tc_kernel<false, true>
-                                    : tc::contract_tc_kernel<false, false>);
+  const auto pick = [&](auto two, auto tail) {
+    constexpr bool kTwo = decltype(two)::value, kTail = decltype(tail)::value;
+    return long_slice ? tc::contract_tc_kernel<kTwo, true, kTail>
+                      : tc::contract_tc_kernel<kTwo, false, kTail>;
+  };
+  const bool tail = sp.tp.n_tail > 0;
+  const auto yes = std::true_type{};
+  const auto no = std::false_type{};
+  auto kern = two_src ? (tail ? pick(yes, yes) : pick(yes, no))
+                      : (tail ? pick(no, yes) : pick(no, no));
   const int smem = two_src ? tc::smem_bytes<true>() : tc::smem_bytes<false>();
-  const int variant = (two_src ? 2 : 0) + (long_slice ? 1 : 0);
+  const int variant = (two_src ? 4 : 0) + (long_slice ? 2 : 0) + (tail ? 1 : 0);
   if (!attr_set[dev][variant]) {
     BSK_CHECK_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
     attr_set[dev][variant] = true;
   }
-  int64_t grid = num_sms;
-  if (grid > n_items) grid = n_items;
-  kern<<<(unsigned)grid, tc::THREADS, smem, st>>>(
-      m, s.tiles, s.row_i, s.row_j, s.map, s.n_tiles, f1 == f2 ? 1 : 0, k_begin, k_end,
-      n_items, terms, fused ? 1 : 0, out, scale);
+  const int grid = std::min(num_sms, sp.tp.units());
+  kern<<<grid, tc::THREADS, smem, st>>>(m, s.tiles, s.row_i, s.row_j, s.map, s.n_tiles,
+                                        f1 == f2 ? 1 : 0, (int)k_begin, (int)k_end, sp.tp, terms,
+                                        fused ? 1 : 0, out, scale);
   BSK_CHECK_CUDA(cudaGetLastError());
+  if (sp.tp.n_tail) {
+    tc::tail_sum_kernel<<<dim3(sp.tp.nc_stride, kTileRows / 32, sp.tp.n_tail), 128, 0, st>>>(
+        s.tiles, s.map, s.n_tiles, sp.slice, k_begin, k_end, sp.tp, terms, out, scale);
+    BSK_CHECK_CUDA(cudaGetLastError());
+  }
 }
 
 int tc_error_flag(bool reset) {

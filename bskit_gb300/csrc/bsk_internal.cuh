@@ -203,6 +203,9 @@ struct bsk_plan {
   bool use_levels = false;
   bsk_plan* parent = nullptr;
   std::vector<bsk_plan*> levels;
+  // scratch of the tensor-core contraction, grown when a triangle set wants more; earlier
+  // blocks live as long as the plan (captured graphs of earlier sets hold their addresses)
+  std::vector<std::pair<void*, size_t>> tail_scratch;
   int n_alloc() const { return (n + chunk - 1) / chunk * chunk; }  // shells rounded to batches
 };
 
@@ -217,6 +220,8 @@ struct bsk_triset {
   std::vector<bsk::HostTriangle> u_tri;  // first occurrences, in order
   std::vector<int> u_idx;                // their positions in the list
   mutable std::map<int, std::vector<bsk::StreamGroup>> groups;  // per streaming chunk size
+  void* scratch = nullptr;               // of the plan's tail_scratch (null: none wanted)
+  size_t scratch_bytes = 0;
   std::vector<bsk::GridLevel> levels;    // the resident path's grids (empty: the plan's only)
 };
 
@@ -273,7 +278,11 @@ void launch_contract_simt_d64(const DeviceSchedule& s, const double* f1, const d
 void launch_contract_tc(const DeviceSchedule& s, const float* f1, const float* f2,
                         const __nv_bfloat16* f3_split, int split_shells, int n_shells,
                         int64_t K, int64_t k_begin, int64_t k_end, int terms, double* out,
-                        int num_sms, cudaStream_t st, double scale = 1.0);
+                        int num_sms, cudaStream_t st, double scale = 1.0,
+                        void* scratch = nullptr, size_t scratch_bytes = 0);
+// Scratch with which launch_contract_tc spreads the last wave of a schedule's items over all
+// SMs (0: it has no use for any; with less than this it runs without, with the same result).
+size_t contract_tc_scratch(const std::vector<TileDesc>& tiles, int64_t points, int num_sms);
 
 // Bounded-wait error flag of the tcgen05 kernel (1 = a wait expired); optionally reset.
 int tc_error_flag(bool reset);

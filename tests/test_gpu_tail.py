@@ -1,0 +1,54 @@
+"""Contraction of short grids: items cut into parts with a scratch area, against whole items.
+
+bsk_contract gives the triangle set's scratch to the tensor-core launch, which then spreads
+the last wave of work items over all SMs; bsk_contract_noalloc has none and walks whole items.
+Both add the same FP32 slice sums, in FP64 and in any order, so a bin may differ by at most
+(slices) x 2^-52 of the sum of its slices' magnitudes, which sum |f1 f2 f3| bounds.
+"""
+import ctypes
+
+import numpy as np
+import pytest
+import torch
+
+from bskit_gb300 import _lib
+from bskit_gb300 import bins as B
+from bskit_gb300.engine import Plan
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(scope="module")
+def plans(cuda):
+    kf = 2 * np.pi / 100.0
+    out = {}
+    for fields in (1, 2):
+        kw = dict(kmin=kf, kmax=32 * kf, dk=2 * kf)
+        edges = B.generate_bin_edge_list(**kw)
+        tri = np.ascontiguousarray(B.generate_triangle_bin_list(
+            num_fields=fields, return_indices=True, **kw), dtype=np.int32)
+        plan = Plan(128, 100.0, edges)  # 15 shells, 96^3 points
+        out[fields] = plan, plan.triangles(tri), tri
+    return out
+
+
+# one partial stage; whole stages; one slice less / more than full; several slices with a short
+# last one; the plan's grid
+@pytest.mark.parametrize("k", [8, 128, 136, 16384 - 8, 16384 + 8, 5 * 16384 + 1000, 96 ** 3])
+@pytest.mark.parametrize("fields,precision", [(1, "bf16x3"), (2, "bf16x3"), (1, "bf16")])
+def test_parts_equal_whole_items(plans, k, fields, precision):
+    plan, ts, tri = plans[fields]
+    g = torch.Generator(device="cuda")
+    g.manual_seed(k)
+    f = [torch.randn((plan.n_shells, k), generator=g, device="cuda") for _ in range(fields)]
+    fs = [f[0], f[0], f[-1]]
+    got = plan.contract(ts, *fs, precision=precision)
+    whole = torch.full((len(tri),), float("nan"), dtype=torch.float64, device="cuda")
+    stream = ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)
+    _lib.call("bsk_contract_noalloc", plan.n_shells, len(tri), tri.ctypes.data,
+              *[ctypes.c_void_p(x.data_ptr()) for x in fs], k, _lib.PRECISIONS[precision],
+              ctypes.c_void_p(whole.data_ptr()), stream)
+    plan.sync_check()
+    abs_sum = plan.contract(ts, *[x.abs() for x in fs], precision="fp64")
+    slices = -(-k // 16384)
+    assert torch.all((got - whole).abs() <= slices * 2.0 ** -52 * 1.01 * abs_sum)
