@@ -949,6 +949,7 @@ void gridinfo_stream(bsk_plan* p, const bsk_triset* set, double* ntri, double* k
 
 }  // namespace
 
+int64_t device_bytes(const bsk_plan* p) { return footprint(p); }
 void set_error(const std::string& msg) { g_err = msg; }
 const std::string& get_error() { return g_err; }
 
@@ -1372,7 +1373,8 @@ int bsk_gridinfo(bsk_plan* p, const bsk_triset* set, double* ntri, double* kmean
     BSK_REQUIRE(ntri && kmean, BSK_ERR_ARG, "NULL argument");
     if (gridinfo_enum_supported(p)) {  // exact integer enumeration, no FFT
       p->last_stream_C = 0;
-      gridinfo_enum(p, set->tri, ntri, kmean, st);
+      if (!gridinfo_modular(p, set->tri, ntri, kmean, st))
+        gridinfo_enum(p, set->tri, ntri, kmean, st);
       return;
     }
     make_z2d(p);

@@ -47,7 +47,16 @@
 // therefore cut into parts of a few stages spread over all SMs; the drain writes each stage's
 // two accumulator halves (hi*Bhi + lo*Bhi and hi*Blo + lo*Blo) of the bins to a scratch area
 // and tail_sum_kernel adds them in the order the drain's registers would have, so every bin
-// keeps its value bit for bit (tail_plan has the rule and the measured times).
+// keeps its value bit for bit (make_split has the rule and the measured times).
+//
+// Sums modulo a prime (kMod, for the grid information): the fields are residues |f| <= p / 2 of
+// a prime p < kModMaxPrime, kept as FP32 integers.  P = F1_i F2_j (below 2^19, exact) is reduced
+// to its residue before the split, and both splits are by value, not by exponent: hi a
+// multiple of 8 (at most 8 significant bits), lo in [-4, 4].  Every number that the tensor
+// core then adds is an integer of at most 23 bits in units of its last place (hi Bhi: multiples
+// of 64 below 2^26 over a stage's 128 points; lo Bhi: multiples of 8), so a stage's
+// accumulators are exact; the drain reduces them and the slice's sum in FP32 integers below
+// 2^24 and adds it to an int64.
 #include <cuda.h>
 
 #include <algorithm>
@@ -334,6 +343,39 @@ __device__ __forceinline__ unsigned long long f2_sub(unsigned long long a, unsig
 __device__ __forceinline__ uint32_t bf16x2_of(unsigned long long p) {
   return pack_bf16(__uint_as_float((uint32_t)p), __uint_as_float((uint32_t)(p >> 32)));
 }
+__device__ __forceinline__ unsigned long long f2_add(unsigned long long a, unsigned long long b) {
+  unsigned long long d;
+  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
+  return d;
+}
+__device__ __forceinline__ unsigned long long f2_fma(unsigned long long a, unsigned long long b,
+                                                     unsigned long long c) {
+  unsigned long long d;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
+  return d;
+}
+__device__ __forceinline__ unsigned long long f2_pack(uint32_t x, uint32_t y) {
+  return ((unsigned long long)y << 32) | x;
+}
+__device__ __forceinline__ unsigned long long f2_dup(float x) {
+  return f2_pack(__float_as_uint(x), __float_as_uint(x));
+}
+// The residue nearest zero of integers |x| < 2^22 p (x a multiple of any power of two): x - p
+// rint(x / p), the rounding by adding and subtracting 1.5 x 2^23.
+struct ModConst {
+  unsigned long long inv, neg_p;
+};
+__device__ __forceinline__ unsigned long long f2_mod(unsigned long long x, const ModConst& m) {
+  const unsigned long long big = f2_dup(12582912.f), neg_big = f2_dup(-12582912.f);
+  return f2_fma(f2_add(f2_fma(x, m.inv, big), neg_big), m.neg_p, x);
+}
+// Residues -> bf16 hi (multiples of 8) and lo (rest).
+__device__ __forceinline__ void split2_mod(unsigned long long r, uint32_t& hi, uint32_t& lo) {
+  const unsigned long long h =
+      f2_add(f2_add(r, f2_dup(100663296.f)), f2_dup(-100663296.f));  // 1.5 x 2^26: units of 8
+  hi = bf16x2_of(h);
+  lo = bf16x2_of(f2_sub(r, h));
+}
 // hi/lo split of two products held as f32x2: returns (hi bf16x2, lo bf16x2), lo = bf16(p - hi).
 __device__ __forceinline__ void split2(unsigned long long p, uint32_t& hi, uint32_t& lo) {
   hi = bf16x2_of(p);
@@ -347,6 +389,8 @@ __device__ __forceinline__ void split2(unsigned long long p, uint32_t& hi, uint3
 // slice][half][nc_stride columns][128 rows]).
 struct TailPlan {
   int n_full = 0, n_tail = 0, parts = 1, part_stages = 0, nc_stride = 0;
+  int mod_slice = 0;      // kMod: points per item
+  float mod_p = 0.f, mod_inv = 0.f;  // kMod: the prime, 1 / p
   float* scratch = nullptr;
   __host__ __device__ int units() const { return n_full + n_tail * parts; }
 };
@@ -358,9 +402,9 @@ struct Work {
   int x_begin, x_end;   // K < 2^31
 };
 
-template <int kSlice, bool kTail>
-__device__ __forceinline__ Work decode(int u, const TailPlan& tp, int n_tiles, int k_begin,
-                                       int k_end) {
+template <bool kTail>
+__device__ __forceinline__ Work decode(int u, const TailPlan& tp, int kSlice, int n_tiles,
+                                       int k_begin, int k_end) {
   Work w;
   int item = u, part = 0;
   w.tail = -1;
@@ -380,14 +424,14 @@ __device__ __forceinline__ Work decode(int u, const TailPlan& tp, int n_tiles, i
 }
 
 // 26 warps: 7 share one SM sub-partition, whose 16K registers allow 73 per thread.
-template <bool kTwoSrc, bool kLongSlice, bool kTail>
+template <bool kTwoSrc, bool kLongSlice, bool kTail, bool kMod = false>
 __global__ void __launch_bounds__(THREADS, 1)
     contract_tc_kernel(const __grid_constant__ Maps maps, const TileDesc* __restrict__ tiles,
                        const int16_t* __restrict__ row_i, const int16_t* __restrict__ row_j,
                        const int32_t* __restrict__ map, int n_tiles, int same_src,
                        int k_begin, int k_end, const TailPlan tp, int terms, int fused,
                        double* __restrict__ out, double scale) {
-  constexpr int slice = (int)(kLongSlice ? kSliceLong : kSliceShort);
+  const int slice = kMod ? tp.mod_slice : (int)(kLongSlice ? kSliceLong : kSliceShort);
   constexpr int STAGE_BYTES = Ring<kTwoSrc>::kStageBytes;
   constexpr int SST = Ring<kTwoSrc>::kStages;
   const int n_units = tp.units();
@@ -439,7 +483,7 @@ __global__ void __launch_bounds__(THREADS, 1)
       uint32_t chunk = 0;
       bool ok = true;
       for (int u = blockIdx.x; u < n_units && ok; u += gridDim.x) {
-        const Work w = decode<slice, kTail>(u, tp, n_tiles, k_begin, k_end);
+        const Work w = decode<kTail>(u, tp, slice, n_tiles, k_begin, k_end);
         const TileDesc td = tiles[w.tile];
         const bool one_src = !kTwoSrc || (same_src && td.i0 == td.j0);
         
@@ -498,7 +542,7 @@ __global__ void __launch_bounds__(THREADS, 1)
     uint32_t chunk = 0, grp = 0;
     bool ok = true;
     for (int u = blockIdx.x; u < n_units && ok; u += gridDim.x) {
-      const Work w = decode<slice, kTail>(u, tp, n_tiles, k_begin, k_end);
+      const Work w = decode<kTail>(u, tp, slice, n_tiles, k_begin, k_end);
       const TileDesc td = tiles[w.tile];
       
       // hi x [Bhi; Blo] and lo x [Bhi; Blo] (the lo rows of a block sit right after its nc
@@ -554,7 +598,7 @@ __global__ void __launch_bounds__(THREADS, 1)
     uint32_t grp = 0;
     bool ok = true;
     for (int u = blockIdx.x; u < n_units && ok; u += gridDim.x) {
-      const Work w = decode<slice, kTail>(u, tp, n_tiles, k_begin, k_end);
+      const Work w = decode<kTail>(u, tp, slice, n_tiles, k_begin, k_end);
       const TileDesc td = tiles[w.tile];
       const int ngrp = (int)((w.x_end - w.x_begin + KCH - 1) / KCH);
       const int32_t* mp = map + td.map_off + c0 * kTileRows + r;
@@ -597,6 +641,53 @@ __global__ void __launch_bounds__(THREADS, 1)
           tc_fence_before();
           __syncwarp();
           if (lane == 0) mbar_arrive(&bars->accempty[b]);
+        }
+        continue;
+      }
+      if constexpr (kMod) {
+        const ModConst mc = {f2_dup(tp.mod_inv), f2_dup(-tp.mod_p)};
+        unsigned long long acc[16];  // columns c0 + 2 e, c0 + 2 e + 1
+#pragma unroll
+        for (int e = 0; e < 16; ++e) acc[e] = 0ull;
+        for (int g = 0; g < ngrp; ++g, ++grp) {
+          const uint32_t b = grp % NACC;
+          if (!__all_sync(0xffffffffu,
+                          mbar_wait(&bars->done[grp % DONE_RING], (grp / DONE_RING) & 1))) {
+            ok = false;
+            break;
+          }
+          tc_fence_after();
+#pragma unroll
+          for (int cc = 0; cc < 2; ++cc) {
+            if (c0 + cc * 16 < td.nc) {
+              uint32_t v[16];
+              tmem_ld16(taddr + ACC_COL + b * 128 + cc * 16, v);
+#pragma unroll
+              for (int e = 0; e < 8; ++e)
+                acc[cc * 8 + e] = f2_add(acc[cc * 8 + e], f2_mod(f2_pack(v[2 * e], v[2 * e + 1]), mc));
+              tmem_ld16(taddr + ACC_COL + b * 128 + td.nc + cc * 16, v);
+#pragma unroll
+              for (int e = 0; e < 8; ++e)
+                acc[cc * 8 + e] = f2_add(acc[cc * 8 + e], f2_pack(v[2 * e], v[2 * e + 1]));
+            }
+          }
+          if ((g & 15) == 15) {  // a stage adds less than 2^19.3 + p / 2: 16 of them stay exact
+#pragma unroll
+            for (int e = 0; e < 16; ++e) acc[e] = f2_mod(acc[e], mc);
+          }
+          tc_fence_before();
+          __syncwarp();
+          if (lane == 0) mbar_arrive(&bars->accempty[b]);
+        }
+        if (!ok) break;
+        unsigned long long* out64 = reinterpret_cast<unsigned long long*>(out);
+#pragma unroll
+        for (int c = 0; c < 32; ++c) {
+          if (c0 + c < td.nc) {
+            const int t = __ldg(mp + c * kTileRows);
+            const float v = __uint_as_float((uint32_t)(acc[c / 2] >> (c & 1 ? 32 : 0)));
+            if (t >= 0) atomicAdd(out64 + t, (unsigned long long)(long long)__float2int_rn(v));
+          }
         }
         continue;
       }
@@ -648,7 +739,7 @@ __global__ void __launch_bounds__(THREADS, 1)
     uint32_t chunk = 0;
     bool ok = true;
     for (int u = blockIdx.x; u < n_units && ok; u += gridDim.x) {
-      const Work w = decode<slice, kTail>(u, tp, n_tiles, k_begin, k_end);
+      const Work w = decode<kTail>(u, tp, slice, n_tiles, k_begin, k_end);
       const TileDesc td = tiles[w.tile];
       const bool one_src = !kTwoSrc || (same_src && td.i0 == td.j0);
       
@@ -715,6 +806,12 @@ __global__ void __launch_bounds__(THREADS, 1)
 #pragma unroll
           for (int e = 0; e < 2; ++e) {
             const int c4 = (g & 1) * 2 + e;
+            if constexpr (kMod) {
+              const ModConst mc = {f2_dup(tp.mod_inv), f2_dup(-tp.mod_p)};
+              split2_mod(f2_mod(f2_mul(ca[e].x, cb[e].x), mc), hi[2 * c4], lo[2 * c4]);
+              split2_mod(f2_mod(f2_mul(ca[e].y, cb[e].y), mc), hi[2 * c4 + 1], lo[2 * c4 + 1]);
+              continue;
+            }
             split2(f2_mul(ca[e].x, cb[e].x), hi[2 * c4], lo[2 * c4]);
             split2(f2_mul(ca[e].y, cb[e].y), hi[2 * c4 + 1], lo[2 * c4 + 1]);
           }
@@ -999,6 +1096,41 @@ void launch_contract_tc(const DeviceSchedule& s, const float* f1, const float* f
         s.tiles, s.map, s.n_tiles, sp.slice, k_begin, k_end, sp.tp, terms, out, scale);
     BSK_CHECK_CUDA(cudaGetLastError());
   }
+}
+
+void launch_contract_mod(const DeviceSchedule& s, const float* f, const __nv_bfloat16* f3_split,
+                         int n_shells, int64_t K, int p, unsigned long long* out, int num_sms,
+                         cudaStream_t st) {
+  if (s.n_tiles == 0) return;
+  BSK_REQUIRE(K > 0 && K % tc::KCH == 0 && K < (int64_t)1 << 31, BSK_ERR_STATE,
+              "internal: bad modular contraction size");
+  BSK_REQUIRE(p < kModMaxPrime, BSK_ERR_STATE, "internal: modulus too large");
+  for (const TileDesc& d : s.h_tiles)
+    BSK_REQUIRE(d.i0 == d.j0, BSK_ERR_STATE, "internal: a modular tile wants one source range");
+  tc::Maps m;
+  for (int i = 0; i < tc::kRowSizes; ++i) {
+    tc::make_split_map(&m.b[i], f3_split, n_shells, K, 8 * (i + 1));
+    BSK_REQUIRE(tc::make_block_map(&m.a1[i], CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 4, f, K, n_shells,
+                                   32, 8 * (i + 1), 4),
+                BSK_ERR_CUDA, "cuTensorMapEncodeTiled (residues) failed");
+  }
+  // any split of the sums is exact: the slice that spreads the items most evenly, about four
+  // to an SM (shorter items pay their epilogue's atomics more often)
+  tc::TailPlan tp;
+  const int stages = (int)(K / tc::KCH);
+  const int want = std::max(1, 4 * num_sms / s.n_tiles);
+  const int slice = std::max(4, (stages + want - 1) / want);
+  tp.mod_slice = slice * tc::KCH;
+  tp.mod_p = (float)p;
+  tp.mod_inv = 1.f / (float)p;
+  tp.n_full = (stages + slice - 1) / slice * s.n_tiles;
+  auto kern = tc::contract_tc_kernel<false, false, false, true>;
+  const int smem = tc::smem_bytes<false>();
+  BSK_CHECK_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+  kern<<<std::min(num_sms, tp.n_full), tc::THREADS, smem, st>>>(
+      m, s.tiles, s.row_i, s.row_j, s.map, s.n_tiles, 1, 0, (int)K, tp, 3, 1,
+      reinterpret_cast<double*>(out), 1.0);
+  BSK_CHECK_CUDA(cudaGetLastError());
 }
 
 int tc_error_flag(bool reset) {

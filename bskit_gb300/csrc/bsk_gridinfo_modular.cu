@@ -1,0 +1,614 @@
+// Grid information (triangle counts and mean |k| per bin) from residues modulo small primes.
+//
+// The sums that bsk_gridinfo_enum.cu evaluates by enumeration,
+//   N_tri(a, b, c) = #{q1 in a, q2 in b, q3 in c : q1 + q2 + q3 = 0}
+//   S(a; b, c)     = sum over those triangles of w(q1),  w(q) = |q| 2^44 rounded to an integer,
+// are cyclic convolutions at zero of integer arrays, and no triangle wraps around a grid of side
+// N > 3 qmax.  So in any field that has an N-th root of unity omega
+//   N^3 N_tri(a, b, c) = sum_x n_a(x) n_b(x) n_c(x),  n_s(x) = sum_{q in s} omega^(q . x),
+// and likewise for S with k_s(x) = sum_{q in s} w(q) omega^(q . x).  In the integers modulo a
+// prime p = 1 (mod N) everything is exact; a handful of primes below 1448 determines the
+// values (the Chinese remainder theorem) because they are non-negative and bounded by the
+// mode counts.  The whole evaluation is then three small dense transforms per shell and the
+// triple-product contraction of the tensor-core kernel (launch_contract_mod), instead of a
+// visit to every pair of modes: ~qmax^6 pairs against ~qmax^3 points times bins.  At 512^3 (63
+// shells to |q| = 127) 1.81 s -> 0.127 s, at 256^3 (31 shells to 63) 41 -> 7.7 ms, at |q| <= 40
+// (14 shells) 3.9 -> 2.2 ms; the enumeration's two launches are kept below that (kMinQ).
+//
+// Symmetry.  Membership and w do not change under sign flips of a component or the x <-> y swap
+// (bsk_gridinfo_enum.cu), so n_s and k_s are even in every coordinate and symmetric in (x, y):
+// they are evaluated at 0 <= y <= x, z <= N / 2 only (1/16 of the grid), a point's weight
+// (1 or 2 per coordinate, 2 for x != y) multiplied into the column fields.  An even transform
+// is E[x][q] = omega^(q x) + omega^(-q x) (1 for q = 0).
+//
+// Arithmetic.  Residues are kept as FP32 integers of magnitude at most (p - 1) / 2 <= 723; a
+// product is below 2^19.1, so 32 of them add exactly in FP32 before a reduction.
+#include <algorithm>
+#include <cmath>
+#include <cstring>
+
+#include "bsk_internal.cuh"
+
+namespace bsk {
+namespace gmod {
+
+constexpr int kMaxPrimes = 16;
+constexpr int kFrac = 44;       // fractional bits of w, as in the enumeration
+constexpr int kMinQ = 40, kMaxQ = 159;  // kMaxQ: shared memory of the transforms
+constexpr int kRun = 32;        // products added between reductions
+
+struct Prime {
+  int p, N, h, hz;      // h = N / 2 + 1 points an axis, hz = h rounded up to even
+  int np;               // (x, y) pairs, h (h + 1) / 2
+  int64_t K;            // np hz rounded up to 128
+  int inv_n3;           // N^-3 mod p
+};
+
+struct Garner {         // inv[j][k] = p_j^-1 mod p_k (j < k)
+  int n;
+  int p[kMaxPrimes], inv_n3[kMaxPrimes];
+  int inv[kMaxPrimes][kMaxPrimes];
+};
+
+int pow_mod(int64_t b, int64_t e, int p) {
+  int64_t r = 1;
+  for (b %= p; e; e >>= 1, b = b * b % p)
+    if (e & 1) r = r * b % p;
+  return (int)r;
+}
+
+bool is_prime(int n) {
+  for (int d = 2; d * d <= n; ++d)
+    if (n % d == 0) return false;
+  return n > 1;
+}
+
+// Primes p = 1 (mod N) below kModMaxPrime with the smallest N > 3 qmax each has, cheapest first
+// (points per bit), until their product exceeds 2^bits.
+std::vector<Prime> choose_primes(int qmax, double bits) {
+  std::vector<Prime> all;
+  for (int p = 3; p < kModMaxPrime; p += 2) {
+    if (!is_prime(p)) continue;
+    for (int N = 3 * qmax + 1; N < p; ++N)
+      if ((p - 1) % N == 0) {
+        Prime q{};
+        q.p = p;
+        q.N = N;
+        all.push_back(q);
+        break;
+      }
+  }
+  auto cost = [](const Prime& q) { return std::pow((double)q.N, 3) / std::log2((double)q.p); };
+  std::sort(all.begin(), all.end(), [&](const Prime& a, const Prime& b) {
+    const double ca = cost(a), cb = cost(b);
+    return ca != cb ? ca < cb : a.p > b.p;
+  });
+  std::vector<Prime> out;
+  double have = 0;
+  for (Prime q : all) {
+    if (have > bits) break;
+    if ((int)out.size() == kMaxPrimes) return {};
+    q.h = q.N / 2 + 1;
+    q.hz = (q.h + 1) & ~1;
+    q.np = q.h * (q.h + 1) / 2;
+    q.K = ((int64_t)q.np * q.hz + 127) / 128 * 128;
+    q.inv_n3 = pow_mod(pow_mod(q.N, 3, q.p), q.p - 2, q.p);
+    have += std::log2((double)q.p);
+    out.push_back(q);
+  }
+  if (have <= bits) return {};
+  return out;
+}
+
+float centred(int64_t v, int p) {
+  v %= p;
+  if (v < 0) v += p;
+  return (float)(2 * v > p ? v - p : v);
+}
+
+__device__ __forceinline__ float mod_red(float v, float p, float inv) {
+  return fmaf(-rintf(v * inv), p, v);
+}
+
+// The modes (q_a >= 0) of shell s on the line (q_b, q_c) are one interval of q_a (|k| grows with
+// q_a): range[s][b][c] = first | last << 8, 0x00FF when empty (never with first = 255).
+// flag is set when a mode lies in more than two shells.
+__global__ void range_kernel(const uint16_t* __restrict__ table, int Ng, int n_shells, int q1,
+                             uint16_t* __restrict__ range, int* __restrict__ flag) {
+  const int c = blockIdx.x * blockDim.x + threadIdx.x, b = blockIdx.y;
+  if (c >= q1) return;
+  const int64_t plane = (int64_t)q1 * q1, at = (int64_t)b * q1 + c;
+  for (int s = 0; s < n_shells; ++s) range[s * plane + at] = 0x00FF;
+  for (int a = 0; a < q1; ++a) {
+    const uint16_t code = __ldg(table + ((int64_t)a * Ng + b) * (Ng / 2 + 1) + c);
+    const int first = code & 0xFF, extra = code >> 8;
+    if (first == 0xFF) continue;
+    if (extra > 1) atomicOr(flag, 1);
+    for (int s = first; s <= first + min(extra, 1); ++s) {
+      uint16_t* r = range + s * plane + at;
+      const uint16_t v = *r;
+      *r = (uint16_t)((v == 0x00FF ? a : (v & 0xFF)) | (a << 8));
+    }
+  }
+}
+
+// w(q) mod p, centred, for 0 <= q_a, q_b, q_c <= qmax: the correctly rounded |q| 2^44.
+__global__ void weight_kernel(int q1, int p, int16_t* __restrict__ w) {
+  const int c = blockIdx.x * blockDim.x + threadIdx.x, b = blockIdx.y, a = blockIdx.z;
+  if (c >= q1) return;
+  const double v = __dsqrt_rn((double)(a * a + b * b + c * c)) * 17592186044416.0;  // 2^44
+  int r = (int)(llround(v) % p);
+  if (2 * r > p) r -= p;
+  w[((int64_t)a * q1 + b) * q1 + c] = (int16_t)r;
+}
+
+// First two axes: block = (x, shell).  The plane A[b][c] = sum over the shell's q_a of
+// E[x][q_a] (times w for the |k| field) goes to shared memory, for the count field as a
+// difference of E's prefix sums; then out[pair(x, y)][c] = sum_b E[y][b] A[b][c], y <= x: a
+// warp takes 8 y, a lane 4 c (32 FMAs for one 16-byte shared-memory load and two broadcast
+// loads of E).  Bound by FMA issue; its output is written once.
+constexpr int kXyThreads = 256;
+template <bool kWeighted>
+__global__ void __launch_bounds__(kXyThreads)
+    xy_kernel(const uint16_t* __restrict__ range, const int16_t* __restrict__ w,
+              const float* __restrict__ E /*[q][ep]*/, const float* __restrict__ prefix, int ep,
+              int q1, const int* __restrict__ radius, int np, int cp, float p, float inv,
+              float* __restrict__ out) {
+  extern __shared__ __align__(16) float sA[];  // [R + 1][cp]
+  __shared__ float sE[kMaxQ + 2];
+  const int x = (int)gridDim.x - 1 - (int)blockIdx.x;  // the longest blocks first
+  const int s = blockIdx.y;
+  const int R = radius[s], nb = R + 1;
+  const float* src = kWeighted ? E : prefix;
+  for (int a = threadIdx.x; a < q1 + 1; a += kXyThreads)
+    sE[a] = (!kWeighted || a < q1) ? src[(int64_t)a * ep + x] : 0.f;
+  __syncthreads();
+  const uint16_t* rg = range + (int64_t)s * q1 * q1;
+  for (int i = threadIdx.x; i < nb * cp; i += kXyThreads) {
+    const int b = i / cp, c = i - b * cp;
+    float v = 0.f;
+    const uint16_t r = c < nb ? rg[b * q1 + c] : (uint16_t)0x00FF;
+    if (r != 0x00FF) {
+      const int a0 = r & 0xFF, a1 = r >> 8;
+      if (kWeighted) {
+        int run = 0;
+        for (int a = a0; a <= a1; ++a) {
+          v = fmaf(sE[a], (float)w[((int64_t)a * q1 + b) * q1 + c], v);
+          if (++run == kRun) {
+            v = mod_red(v, p, inv);
+            run = 1;
+          }
+        }
+        v = mod_red(v, p, inv);
+      } else {
+        v = mod_red(sE[a1 + 1] - sE[a0], p, inv);
+      }
+    }
+    sA[i] = v;
+  }
+  __syncthreads();
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  float* o = out + ((int64_t)s * np + (int64_t)x * (x + 1) / 2) * cp;
+  for (int y0 = warp * 8; y0 <= x; y0 += (kXyThreads / 32) * 8) {
+    for (int c = lane * 4; c < cp; c += 128) {
+      float acc[8][4];
+#pragma unroll
+      for (int y = 0; y < 8; ++y)
+#pragma unroll
+        for (int e = 0; e < 4; ++e) acc[y][e] = 0.f;
+      for (int b0 = 0; b0 < nb; b0 += kRun - 1) {
+        const int b1 = min(nb, b0 + kRun - 1);
+#pragma unroll 4
+        for (int b = b0; b < b1; ++b) {
+          const float4 av = *reinterpret_cast<const float4*>(sA + b * cp + c);
+          const float4 e0 = __ldg(reinterpret_cast<const float4*>(E + (int64_t)b * ep + y0));
+          const float4 e1 = __ldg(reinterpret_cast<const float4*>(E + (int64_t)b * ep + y0 + 4));
+          const float ev[8] = {e0.x, e0.y, e0.z, e0.w, e1.x, e1.y, e1.z, e1.w};
+#pragma unroll
+          for (int y = 0; y < 8; ++y) {
+            acc[y][0] = fmaf(ev[y], av.x, acc[y][0]);
+            acc[y][1] = fmaf(ev[y], av.y, acc[y][1]);
+            acc[y][2] = fmaf(ev[y], av.z, acc[y][2]);
+            acc[y][3] = fmaf(ev[y], av.w, acc[y][3]);
+          }
+        }
+#pragma unroll
+        for (int y = 0; y < 8; ++y)
+#pragma unroll
+          for (int e = 0; e < 4; ++e) acc[y][e] = mod_red(acc[y][e], p, inv);
+      }
+#pragma unroll
+      for (int y = 0; y < 8; ++y)
+        if (y0 + y <= x)
+          *reinterpret_cast<float4*>(o + (int64_t)(y0 + y) * cp + c) =
+              make_float4(acc[y][0], acc[y][1], acc[y][2], acc[y][3]);
+    }
+  }
+}
+
+// Last axis: out[pair][z] = sum_c H[pair][c] E[z][c] for 64 pairs at a time, persistent blocks
+// (E stays in shared memory).  A warp takes 32 pairs x 64 z, a thread 8 x 8: 8 rows of H (16
+// bytes each per 4 c, broadcast in a quarter warp) and 4 x 8 bytes of E per c and 64 FMAs, 16
+// shared-memory wavefronts per 64 warp-wide FMAs, which is also their issue time.  Writes the
+// FP32 field (pair factors) and / or the weighted field's split (columns).
+constexpr int kZThreads = 256, kZPairs = 64;
+__global__ void __launch_bounds__(kZThreads, 1)
+    z_kernel(const float* __restrict__ H, const float* __restrict__ E, int ep, int q1,
+             const int* __restrict__ radius, int n_shells, Prime pr, int cp, float p, float inv,
+             float* __restrict__ field, __nv_bfloat16* __restrict__ split) {
+  extern __shared__ __align__(16) float smz[];
+  const int zp = (pr.hz + 63) / 64 * 64;
+  float* sE = smz;                    // [q1][zp]
+  float* sH = sE + (size_t)q1 * zp;   // [64][cp + 4]
+  const int hp = cp + 4;
+  for (int i = threadIdx.x; i < q1 * zp; i += kZThreads) {
+    const int c = i / zp, z = i - c * zp;
+    sE[i] = z < pr.h ? E[(int64_t)c * ep + z] : 0.f;
+  }
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int pg = (warp & 1) * 32 + (lane >> 3) * 8;  // this thread's 8 pairs of the block's 64
+  const int zl = (lane & 7) * 2;                     // its z: zl + {0, 1} + 16 j of each 64
+  const int tiles = (pr.np + kZPairs - 1) / kZPairs;
+  for (int u = blockIdx.x; u < tiles * n_shells; u += gridDim.x) {
+    const int s = u / tiles, t0 = (u - s * tiles) * kZPairs;
+    const int nc = radius[s] + 1, nc4 = (nc + 3) & ~3;
+    __syncthreads();  // the previous tile's reads of sH (and the stores of sE)
+    for (int i = threadIdx.x; i < kZPairs * (nc4 / 4); i += kZThreads) {
+      const int r = i / (nc4 / 4), c = (i - r * (nc4 / 4)) * 4;
+      float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
+      if (t0 + r < pr.np)
+        v = *reinterpret_cast<const float4*>(H + ((int64_t)s * pr.np + t0 + r) * cp + c);
+      *reinterpret_cast<float4*>(sH + r * hp + c) = v;
+    }
+    __syncthreads();
+    for (int z0 = (warp >> 1) * 64; z0 < pr.hz; z0 += (kZThreads / 64) * 64) {
+      float acc[8][8];
+#pragma unroll
+      for (int a = 0; a < 8; ++a)
+#pragma unroll
+        for (int e = 0; e < 8; ++e) acc[a][e] = 0.f;
+      for (int c0 = 0; c0 < nc; c0 += 28) {  // 28 products and a residue between reductions
+        const int c1 = min(nc4, c0 + 28);
+        for (int c = c0; c < c1; c += 4) {
+          float4 hv[8];
+#pragma unroll
+          for (int a = 0; a < 8; ++a)
+            hv[a] = *reinterpret_cast<const float4*>(sH + (pg + a) * hp + c);
+#pragma unroll
+          for (int k = 0; k < 4; ++k) {
+            if (c + k >= q1) break;  // H is zero there and E has no row
+            float2 ev[4];
+#pragma unroll
+            for (int j = 0; j < 4; ++j)
+              ev[j] = *reinterpret_cast<const float2*>(sE + (c + k) * zp + z0 + zl + 16 * j);
+#pragma unroll
+            for (int a = 0; a < 8; ++a) {
+              const float h = k == 0 ? hv[a].x : k == 1 ? hv[a].y : k == 2 ? hv[a].z : hv[a].w;
+#pragma unroll
+              for (int j = 0; j < 4; ++j) {
+                acc[a][2 * j] = fmaf(h, ev[j].x, acc[a][2 * j]);
+                acc[a][2 * j + 1] = fmaf(h, ev[j].y, acc[a][2 * j + 1]);
+              }
+            }
+          }
+        }
+#pragma unroll
+        for (int a = 0; a < 8; ++a)
+#pragma unroll
+          for (int e = 0; e < 8; ++e) acc[a][e] = mod_red(acc[a][e], p, inv);
+      }
+#pragma unroll
+      for (int a = 0; a < 8; ++a) {
+        const int pair = t0 + pg + a;
+        if (pair >= pr.np) break;
+        int x = (int)((sqrtf(8.f * pair + 1.f) - 1.f) * 0.5f);
+        while ((x + 1) * (x + 2) / 2 <= pair) ++x;
+        while (x * (x + 1) / 2 > pair) --x;
+        const int y = pair - x * (x + 1) / 2;
+        const float wxy = (x == 0 || 2 * x == pr.N ? 1.f : 2.f) *
+                          (y == 0 || 2 * y == pr.N ? 1.f : 2.f) * (x != y ? 2.f : 1.f);
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+          const int z = z0 + zl + 16 * j;
+          if (z >= pr.hz) continue;
+          const float v0 = acc[a][2 * j], v1 = acc[a][2 * j + 1];
+          const int64_t pt = (int64_t)pair * pr.hz + z;
+          if (field) *reinterpret_cast<float2*>(field + (int64_t)s * pr.K + pt) = make_float2(v0, v1);
+          if (split) {
+            const float w0 = wxy * (z == 0 || 2 * z == pr.N ? 1.f : 2.f);
+            const float w1 = wxy * (2 * (z + 1) == pr.N ? 1.f : 2.f);
+            const float u0 = mod_red(v0 * w0, p, inv), u1 = mod_red(v1 * w1, p, inv);
+            const float h0 = 8.f * rintf(u0 * 0.125f), h1 = 8.f * rintf(u1 * 0.125f);
+            *reinterpret_cast<__nv_bfloat162*>(split + split_index(0, s, pt, n_shells)) =
+                __floats2bfloat162_rn(h0, h1);
+            *reinterpret_cast<__nv_bfloat162*>(split + split_index(1, s, pt, n_shells)) =
+                __floats2bfloat162_rn(u0 - h0, u1 - h1);
+          }
+        }
+      }
+    }
+  }
+}
+
+// The non-negative integer below the product of the first n primes with the given residues.
+__device__ unsigned __int128 crt(const Garner& g, int n, const int* r) {
+  int d[kMaxPrimes];  // mixed-radix digits
+  for (int k = 0; k < n; ++k) {
+    int v = r[k];
+    for (int j = 0; j < k; ++j) {
+      v = (v - d[j]) % g.p[k];
+      if (v < 0) v += g.p[k];
+      v = (int)((int64_t)v * g.inv[j][k] % g.p[k]);
+    }
+    d[k] = v;
+  }
+  unsigned __int128 x = 0;
+  for (int k = n - 1; k >= 0; --k) x = x * (unsigned)g.p[k] + (unsigned)d[k];
+  return x;
+}
+
+// Per triangle: its count and three |k| sums from their residues (cnt [n_cnt][ne], sum
+// [g.n][ns]: integers congruent to N^3 times them).
+__global__ void modular_finish_kernel(int64_t T, const int4* __restrict__ idx, Garner g,
+                                      int n_cnt, int ne, int ns,
+                                      const long long* __restrict__ cnt,
+                                      const long long* __restrict__ sum, double kf,
+                                      double* __restrict__ ntri, double* __restrict__ kmean) {
+  const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= 4 * T) return;
+  const int64_t t = i >> 2;
+  const int role = (int)(i & 3);  // 0: the count, 1 .. 3: the |k| sums (lanes of one triangle)
+  const int4 id = idx[t];
+  int r[kMaxPrimes];
+  const int n = role ? g.n : n_cnt;
+  const int e = role == 0 ? id.x : role == 1 ? id.y : role == 2 ? id.z : id.w;
+  for (int k = 0; k < n; ++k) {
+    long long v = (role ? sum[(int64_t)k * ns + e] : cnt[(int64_t)k * ne + e]) % g.p[k];
+    if (v < 0) v += g.p[k];
+    r[k] = (int)(v * g.inv_n3[k] % g.p[k]);
+  }
+  const unsigned __int128 x = crt(g, n, r);
+  const double value = (double)(unsigned long long)(x >> 64) * 18446744073709551616.0 +
+                       (double)(unsigned long long)x;
+  // 4 T is a multiple of 4, so a triangle's four lanes are all here
+  const unsigned lanes = 0xFu << (threadIdx.x & 28);
+  const double count = __shfl_sync(lanes, value, 0, 4);
+  if (role == 0) {
+    ntri[t] = value;
+  } else {
+    kmean[3 * t + role - 1] =
+        count != 0.0 ? value * (1.0 / (double)(1ull << kFrac)) / count * kf : nan("");
+  }
+}
+
+struct Upload {  // host arrays gathered into one device block
+  std::vector<unsigned char> host;
+  size_t add(const void* src, size_t bytes) {
+    const size_t at = (host.size() + 255) / 256 * 256;
+    host.resize(at + bytes);
+    if (bytes) memcpy(host.data() + at, src, bytes);
+    return at;
+  }
+};
+
+struct UploadedSchedule {
+  size_t tiles, ri, rj, map;
+  HostSchedule h;
+  void add(Upload& up) {
+    tiles = up.add(h.tiles.data(), h.tiles.size() * sizeof(TileDesc));
+    ri = up.add(h.ri.data(), h.ri.size() * sizeof(int16_t));
+    rj = up.add(h.rj.data(), h.rj.size() * sizeof(int16_t));
+    map = up.add(h.map.data(), h.map.size() * sizeof(int32_t));
+  }
+  void bind(unsigned char* base, DeviceSchedule& s) const {
+    s.n_tiles = (int)h.tiles.size();
+    s.tiles = (TileDesc*)(base + tiles);
+    s.row_i = (int16_t*)(base + ri);
+    s.row_j = (int16_t*)(base + rj);
+    s.map = (int32_t*)(base + map);
+    s.h_tiles = h.tiles;
+  }
+};
+
+size_t z_smem(const Prime& q, int q1, int cp) {
+  return ((size_t)q1 * ((q.hz + 63) / 64 * 64) + (size_t)kZPairs * (cp + 4)) * sizeof(float);
+}
+
+}  // namespace gmod
+
+bool gridinfo_modular(bsk_plan* p, const std::vector<HostTriangle>& tri, double* ntri,
+                      double* kmean, cudaStream_t st) {
+  using namespace gmod;
+  if (!gridinfo_enum_supported(p) || p->qmax < kMinQ || p->qmax > kMaxQ) return false;
+  const int n = p->n, q1 = p->qmax + 1;
+  const int64_t T = (int64_t)tri.size();
+  if (T > (int64_t)1 << 28) return false;
+
+  // distinct counts (shells sorted) and distinct |k| sums (pair (y >= z), the weighted shell x)
+  std::vector<HostTriangle> ec, es;
+  std::vector<int> at_c((size_t)n * n * n, -1), at_s(at_c);
+  std::vector<int4> idx(T);
+  auto entry = [&](std::vector<int>& at, std::vector<HostTriangle>& list, int i, int j, int l) {
+    int& e = at[((size_t)i * n + j) * n + l];
+    if (e < 0) {
+      e = (int)list.size();
+      list.push_back(HostTriangle{i, j, l});
+    }
+    return e;
+  };
+  double bound = 1.0;  // on any count: the product of a bin's two smallest mode counts
+  double kmax = 1.0;
+  for (int64_t t = 0; t < T; ++t) {
+    int a[3] = {tri[t].i, tri[t].j, tri[t].l};
+    int id[3];
+    for (int role = 0; role < 3; ++role) {
+      const int y = a[(role + 1) % 3], z = a[(role + 2) % 3];
+      id[role] = entry(at_s, es, std::max(y, z), std::min(y, z), a[role]);
+    }
+    std::sort(a, a + 3);
+    const int c = entry(at_c, ec, a[2], a[1], a[0]);
+    idx[t] = make_int4(c, id[0], id[1], id[2]);
+    double m[3] = {(double)p->counts[a[0]], (double)p->counts[a[1]], (double)p->counts[a[2]]};
+    std::sort(m, m + 3);
+    bound = std::max(bound, m[0] * m[1]);
+  }
+  kmax = (p->qmax + 1) * std::ldexp(1.0, kFrac);
+  const std::vector<Prime> primes = choose_primes(p->qmax, std::log2(bound * kmax) + 1.0);
+  if (primes.empty()) return false;
+  const int n_pr = (int)primes.size();
+  int n_cnt = 0;
+  double have = 0;
+  while (n_cnt < n_pr && have <= std::log2(bound) + 1.0) have += std::log2((double)primes[n_cnt++].p);
+  const int cp = (q1 + 3) / 4 * 4;
+  int64_t max_k = 0, max_np = 0;
+  for (const Prime& q : primes) {
+    if (z_smem(q, q1, cp) > 227 * 1024) return false;
+    max_k = std::max(max_k, q.K);
+    max_np = std::max<int64_t>(max_np, q.np);
+  }
+
+  // host tables: schedules, shell radii, triangle entries, E and its prefix sums per prime
+  Upload up;
+  UploadedSchedule sc, ss;
+  tile_schedule(ec, n, nullptr, sc.h);
+  tile_schedule(es, n, nullptr, ss.h);
+  sc.add(up);
+  ss.add(up);
+  const size_t o_idx = up.add(idx.data(), T * sizeof(int4));
+  const size_t o_rad = up.add(p->shell_r.data(), n * sizeof(int));
+  std::vector<size_t> o_e(n_pr), o_pre(n_pr);
+  std::vector<int> ep(n_pr);
+  Garner g{};
+  g.n = n_pr;
+  for (int k = 0; k < n_pr; ++k) {
+    const Prime& q = primes[k];
+    g.p[k] = q.p;
+    g.inv_n3[k] = q.inv_n3;
+    for (int j = 0; j < k; ++j) g.inv[j][k] = pow_mod(primes[j].p, q.p - 2, q.p);
+    int gen = 2;  // a generator of the field: its (p - 1) / f powers differ from 1 for every prime f
+    for (;; ++gen) {
+      bool ok = true;
+      for (int f = 2, m = q.p - 1; m > 1; ++f)
+        if (m % f == 0) {
+          while (m % f == 0) m /= f;
+          ok = ok && pow_mod(gen, (q.p - 1) / f, q.p) != 1;
+        }
+      if (ok) break;
+    }
+    std::vector<int> om(q.N);  // powers of omega
+    const int omega = pow_mod(gen, (q.p - 1) / q.N, q.p);
+    om[0] = 1;
+    for (int i = 1; i < q.N; ++i) om[i] = (int)((int64_t)om[i - 1] * omega % q.p);
+    ep[k] = (q.h + 7) / 8 * 8;
+    std::vector<float> e((size_t)q1 * ep[k], 0.f), pre((size_t)(q1 + 1) * ep[k], 0.f);
+    for (int x = 0; x < q.h; ++x) {
+      int64_t sum = 0;
+      for (int a = 0; a < q1; ++a) {
+        const int r = (int)((int64_t)a * x % q.N);
+        const int64_t v = a == 0 ? 1 : (int64_t)om[r] + om[(q.N - r) % q.N];
+        e[(size_t)a * ep[k] + x] = centred(v, q.p);
+        sum += v;
+        pre[(size_t)(a + 1) * ep[k] + x] = centred(sum, q.p);
+      }
+    }
+    o_e[k] = up.add(e.data(), e.size() * sizeof(float));
+    o_pre[k] = up.add(pre.data(), pre.size() * sizeof(float));
+  }
+
+  // device scratch in one stream-ordered block
+  const int ne = (int)ec.size(), ns = (int)es.size();
+  size_t total = 0;
+  auto take = [&](size_t bytes) {
+    const size_t at = total;
+    total += (bytes + 1023) / 1024 * 1024;
+    return at;
+  };
+  const size_t a_up = take(up.host.size());
+  const size_t a_range = take((size_t)n * q1 * q1 * sizeof(uint16_t));
+  const size_t a_w = take((size_t)q1 * q1 * q1 * sizeof(int16_t));
+  const size_t a_out = take(((size_t)n_cnt * ne + (size_t)n_pr * ns) * sizeof(long long) + 8);
+  const size_t a_h = take((size_t)n * max_np * cp * sizeof(float));
+  const size_t a_f = take((size_t)n * max_k * sizeof(float));
+  const size_t a_s = take(split_elems(n, max_k) * sizeof(__nv_bfloat16));
+  if (p->mem_budget && device_bytes(p) + (int64_t)total > (int64_t)p->mem_budget) return false;
+  unsigned char* base = nullptr;
+  if (cudaMallocAsync((void**)&base, total, st) != cudaSuccess) {
+    cudaGetLastError();
+    return false;
+  }
+  struct Free {
+    void* w;
+    cudaStream_t s;
+    ~Free() { cudaFreeAsync(w, s); }
+  } free_base{base, st};
+  BSK_CHECK_CUDA(cudaMemcpyAsync(base + a_up, up.host.data(), up.host.size(),
+                                 cudaMemcpyHostToDevice, st));
+  uint16_t* range = (uint16_t*)(base + a_range);
+  int16_t* w = (int16_t*)(base + a_w);
+  long long* cnt = (long long*)(base + a_out);
+  long long* sum = cnt + (size_t)n_cnt * ne;
+  int* flag = (int*)(sum + (size_t)n_pr * ns);
+  float* H = (float*)(base + a_h);
+  float* field = (float*)(base + a_f);
+  __nv_bfloat16* split = (__nv_bfloat16*)(base + a_s);
+  const int* radius = (const int*)(base + a_up + o_rad);
+  BSK_CHECK_CUDA(cudaMemsetAsync(cnt, 0, (char*)(flag + 2) - (char*)cnt, st));
+  range_kernel<<<dim3((q1 + 63) / 64, q1), 64, 0, st>>>(p->table, p->Ng, n, q1, range, flag);
+  BSK_CHECK_CUDA(cudaGetLastError());
+  int hflag = 0;
+  BSK_CHECK_CUDA(cudaMemcpyAsync(&hflag, flag, sizeof(int), cudaMemcpyDeviceToHost, st));
+  BSK_CHECK_CUDA(cudaStreamSynchronize(st));
+  BSK_REQUIRE(hflag == 0, BSK_ERR_STATE, "internal: a mode lies in more than two shells");
+
+  DeviceSchedule dc, ds;
+  sc.bind(base + a_up, dc);
+  ss.bind(base + a_up, ds);
+  const size_t xy_smem = (size_t)q1 * cp * sizeof(float);
+  BSK_CHECK_CUDA(cudaFuncSetAttribute(xy_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                      (int)xy_smem));
+  BSK_CHECK_CUDA(cudaFuncSetAttribute(xy_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                      (int)xy_smem));
+  BSK_CHECK_CUDA(cudaFuncSetAttribute(z_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                      227 * 1024));
+  for (int k = 0; k < n_pr; ++k) {
+    const Prime& q = primes[k];
+    const float* E = (const float*)(base + a_up + o_e[k]);
+    const float* pre = (const float*)(base + a_up + o_pre[k]);
+    const float pf = (float)q.p, inv = 1.f / pf;
+    const int64_t points = (int64_t)q.np * q.hz;
+    // the points past the last pair: zero in the fields, and so is the last chunk's split
+    if (q.K > points)
+      BSK_CHECK_CUDA(cudaMemset2DAsync(field + points, q.K * sizeof(float), 0,
+                                       (q.K - points) * sizeof(float), n, st));
+    BSK_CHECK_CUDA(cudaMemsetAsync(split + split_elems(n, q.K - 128), 0,
+                                   (split_elems(n, q.K) - split_elems(n, q.K - 128)) *
+                                       sizeof(__nv_bfloat16), st));
+    const size_t zs = z_smem(q, q1, cp);
+    const int z_grid = std::min(p->num_sms, (q.np + kZPairs - 1) / kZPairs * n);
+    xy_kernel<false><<<dim3(q.h, n), kXyThreads, xy_smem, st>>>(range, w, E, pre, ep[k], q1, radius,
+                                                               q.np, cp, pf, inv, H);
+    z_kernel<<<z_grid, kZThreads, zs, st>>>(H, E, ep[k], q1, radius, n, q, cp, pf, inv, field,
+                                            k < n_cnt ? split : nullptr);
+    BSK_CHECK_CUDA(cudaGetLastError());
+    if (k < n_cnt)
+      launch_contract_mod(dc, field, split, n, q.K, q.p,
+                          (unsigned long long*)cnt + (size_t)k * ne, p->num_sms, st);
+    weight_kernel<<<dim3((q1 + 63) / 64, q1, q1), 64, 0, st>>>(q1, q.p, w);
+    xy_kernel<true><<<dim3(q.h, n), kXyThreads, xy_smem, st>>>(range, w, E, pre, ep[k], q1, radius,
+                                                              q.np, cp, pf, inv, H);
+    z_kernel<<<z_grid, kZThreads, zs, st>>>(H, E, ep[k], q1, radius, n, q, cp, pf, inv, nullptr,
+                                            split);
+    BSK_CHECK_CUDA(cudaGetLastError());
+    launch_contract_mod(ds, field, split, n, q.K, q.p,
+                        (unsigned long long*)sum + (size_t)k * ns, p->num_sms, st);
+  }
+  const double kf = 2.0 * 3.14159265358979323846 / p->L;
+  modular_finish_kernel<<<(unsigned)((4 * T + 127) / 128), 128, 0, st>>>(
+      T, (const int4*)(base + a_up + o_idx), g, n_cnt, ne, ns, cnt, sum, kf, ntri, kmean);
+  BSK_CHECK_CUDA(cudaGetLastError());
+  dc.tiles = ds.tiles = nullptr;  // in the scratch block: nothing to release
+  BSK_CHECK_CUDA(cudaStreamSynchronize(st));  // the host tables must outlive their copy
+  return true;
+}
+
+}  // namespace bsk

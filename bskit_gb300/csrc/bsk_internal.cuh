@@ -227,6 +227,9 @@ struct bsk_triset {
 
 namespace bsk {
 
+// Device bytes the plan holds (BSK_INFO_FOOTPRINT).
+int64_t device_bytes(const bsk_plan* p);
+
 // ---------------------------------------------------------------- kernels
 // Shell table + exact mode counts (FP64 predicate, Hermitian weights).
 void launch_shell_table(const bsk_plan* p, unsigned long long* d_counts, int* d_flag,
@@ -284,6 +287,15 @@ void launch_contract_tc(const DeviceSchedule& s, const float* f1, const float* f
 // SMs (0: it has no use for any; with less than this it runs without, with the same result).
 size_t contract_tc_scratch(const std::vector<TileDesc>& tiles, int64_t points, int num_sms);
 
+// The contraction modulo a prime p < kModMaxPrime: out[t] += the sum over K of f[i] f[j] f3[l],
+// as some integer congruent to it (f: residues of magnitude at most p / 2 as FP32 integers;
+// f3_split: residues split into multiples of 8 and the rest).  K a multiple of 128, f's tail
+// zero.
+constexpr int kModMaxPrime = 1448;  // residues below 724: products of two below 2^19.1
+void launch_contract_mod(const DeviceSchedule& s, const float* f, const __nv_bfloat16* f3_split,
+                         int n_shells, int64_t K, int p, unsigned long long* out, int num_sms,
+                         cudaStream_t st);
+
 // Bounded-wait error flag of the tcgen05 kernel (1 = a wait expired); optionally reset.
 int tc_error_flag(bool reset);
 
@@ -291,6 +303,11 @@ int tc_error_flag(bool reset);
 // plans whose shell modes cannot form a triangle that wraps around the grid and that have
 // at most 64 shells; ntri[T], kmean[T][3] (device).  Synchronises `st`.
 bool gridinfo_enum_supported(const bsk_plan* p);
+// The same sums from residues of the shells' count and |k| fields modulo small primes
+// (bsk_gridinfo_modular.cu): faster for large |q|.  False, with nothing done, when the plan's
+// |q| range is below or above what it is for or its scratch does not fit.
+bool gridinfo_modular(bsk_plan* p, const std::vector<HostTriangle>& tri, double* ntri,
+                      double* kmean, cudaStream_t st);
 void gridinfo_enum(bsk_plan* p, const std::vector<HostTriangle>& tri, double* ntri,
                    double* kmean, cudaStream_t st);
 

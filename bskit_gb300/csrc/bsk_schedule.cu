@@ -15,7 +15,6 @@
 // are not bins).
 #include <algorithm>
 #include <cmath>
-#include <map>
 
 #include "bsk_internal.cuh"
 
@@ -49,22 +48,17 @@ inline int round_up(int v, int m) { return (v + m - 1) / m * m; }
 
 void tile_schedule(const std::vector<HostTriangle>& tri, int n_shells,
                    const std::vector<int>* map_index, HostSchedule& out) {
-  std::map<std::pair<int, int>, int> index;
+  std::vector<int> index((size_t)n_shells * n_shells, -1);  // (i, j) -> row
   std::vector<Row> rows;
   for (size_t t = 0; t < tri.size(); ++t) {
     const HostTriangle& h = tri[t];
     BSK_REQUIRE(h.i >= 0 && h.j >= 0 && h.l >= 0 && h.i < n_shells && h.j < n_shells &&
                     h.l < n_shells,
                 BSK_ERR_ARG, "triangle shell index out of range");
-    auto key = std::make_pair(h.i, h.j);
-    auto it = index.find(key);
-    int r;
-    if (it == index.end()) {
+    int& r = index[(size_t)h.i * n_shells + h.j];
+    if (r < 0) {
       r = (int)rows.size();
-      index.emplace(key, r);
       rows.push_back(Row{h.i, h.j, h.l, h.l, {}});
-    } else {
-      r = it->second;
     }
     Row& R = rows[r];
     R.lmin = std::min(R.lmin, h.l);
