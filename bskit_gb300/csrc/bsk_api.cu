@@ -192,6 +192,14 @@ void check_budget(const bsk_plan* p, size_t bytes, const char* what) {
                                  std::to_string(root->mem_budget)};
 }
 
+// The shells' |q_a| intervals that the field synthesis masks by (a few MB, not counted in the
+// footprint, like the shell edges).
+void make_range(bsk_plan* p) {
+  const size_t q1 = p->qmax + 1;
+  p->range = (uint32_t*)dmalloc((size_t)p->n * q1 * q1 * sizeof(uint32_t));
+  launch_shell_range(p, p->range, nullptr, 0);
+}
+
 void release_stream(bsk_plan* p) {
   for (auto& b : p->stream_f) {
     if (b.ptr) cudaFree(b.ptr);
@@ -243,7 +251,7 @@ void ensure_fields(bsk_plan* p, int s, cudaStream_t st, bool with_split = false,
       const int ns = std::min(p->chunk, p->n - s0);
       int R = 0;
       for (int k = s0; k < s0 + ns; ++k) R = std::max(R, p->shell_r[k]);
-      launch_synth(p->Ng, f.spec, p->table, s0, ns, R, p->synth_ws, f.fields,
+      launch_synth(p->Ng, f.spec, p->table, p->range, p->qmax + 1, s0, ns, R, p->synth_ws, f.fields,
                    with_split ? f.split : nullptr, p->n_alloc(), st);
       done = s0 + ns;
     }
@@ -316,8 +324,8 @@ void ensure_level_fields(bsk_plan* q, int s, cudaStream_t st, int nn, int fp_fro
     const int ns = std::min(q->chunk, q->n - s0);
     int R = 0;
     for (int k = s0; k < s0 + ns; ++k) R = std::max(R, q->shell_r[k]);
-    launch_synth(q->Ng, f.spec, q->table, s0, ns, R, q->synth_ws, f.fields,
-                 need_split ? f.split : nullptr, q->n_alloc(), st, 0, fp_from);
+    launch_synth(q->Ng, f.spec, q->table, q->range, q->qmax + 1, s0, ns, R, q->synth_ws,
+                 f.fields, need_split ? f.split : nullptr, q->n_alloc(), st, 0, fp_from);
     done = s0 + ns;
   }
   // what this pass wrote replaces what the slot held
@@ -356,6 +364,7 @@ void destroy_plan(bsk_plan* p) {
   p->levels.clear();
   for (auto& s : p->slot) free_slot(s);
   if (p->table) cudaFree(p->table);
+  if (p->range) cudaFree(p->range);
   if (p->d_edges) cudaFree(p->d_edges);
   if (p->chunk_spec) cudaFree(p->chunk_spec);
   if (p->cic_w) cudaFree(p->cic_w);
@@ -457,8 +466,8 @@ void chunk_fields(bsk_plan* p, int slot, int s0, int C, float* dst, cudaStream_t
       }
       int R = 0;
       for (int k = first; k < first + ns; ++k) R = std::max(R, p->shell_r[k]);
-      launch_synth(p->Ng, f.spec, p->table, first, ns, R, p->synth_ws, dst, nullptr, 0, st,
-                   s0);
+      launch_synth(p->Ng, f.spec, p->table, p->range, p->qmax + 1, first, ns, R, p->synth_ws,
+                   dst, nullptr, 0, st, s0);
       if (ns < p->chunk)
         BSK_CHECK_CUDA(cudaMemsetAsync(dst + (size_t)(b + ns) * p->K, 0,
                                        (size_t)(p->chunk - ns) * p->K * sizeof(float), st));
@@ -629,6 +638,7 @@ bsk_plan* level_plan(bsk_plan* p, int Ng, int n) {
   q->use_synth = synth_supported(Ng);
   BSK_REQUIRE(q->use_synth, BSK_ERR_STATE, "internal: no field synthesis for a grid level");
   q->synth_ws_bytes = synth_workspace_bytes(Ng, q->qmax, q->chunk);
+  make_range(q.get());
   p->levels.push_back(q.get());
   return q.release();
 }
@@ -1039,7 +1049,10 @@ int bsk_plan_create(int nmesh, double box_size, int n_shells, const double* shel
       p->shell_r[s] = (int)std::min<double>(std::max(q, 0.0), qmax);
     }
     p->use_synth = synth_supported(p->Ng);
-    if (p->use_synth) p->synth_ws_bytes = synth_workspace_bytes(p->Ng, qmax, p->chunk);
+    if (p->use_synth) {
+      p->synth_ws_bytes = synth_workspace_bytes(p->Ng, qmax, p->chunk);
+      make_range(p.get());
+    }
     p->use_levels = grid_mode == BSK_GRID_REDUCED && p->Ng != p->N && p->use_synth;
     make_r2c(p.get());
     make_c2r(p.get());

@@ -110,28 +110,6 @@ __device__ __forceinline__ float mod_red(float v, float p, float inv) {
   return fmaf(-rintf(v * inv), p, v);
 }
 
-// The modes (q_a >= 0) of shell s on the line (q_b, q_c) are one interval of q_a (|k| grows with
-// q_a): range[s][b][c] = first | last << 8, 0x00FF when empty (never with first = 255).
-// flag is set when a mode lies in more than two shells.
-__global__ void range_kernel(const uint16_t* __restrict__ table, int Ng, int n_shells, int q1,
-                             uint16_t* __restrict__ range, int* __restrict__ flag) {
-  const int c = blockIdx.x * blockDim.x + threadIdx.x, b = blockIdx.y;
-  if (c >= q1) return;
-  const int64_t plane = (int64_t)q1 * q1, at = (int64_t)b * q1 + c;
-  for (int s = 0; s < n_shells; ++s) range[s * plane + at] = 0x00FF;
-  for (int a = 0; a < q1; ++a) {
-    const uint16_t code = __ldg(table + ((int64_t)a * Ng + b) * (Ng / 2 + 1) + c);
-    const int first = code & 0xFF, extra = code >> 8;
-    if (first == 0xFF) continue;
-    if (extra > 1) atomicOr(flag, 1);
-    for (int s = first; s <= first + min(extra, 1); ++s) {
-      uint16_t* r = range + s * plane + at;
-      const uint16_t v = *r;
-      *r = (uint16_t)((v == 0x00FF ? a : (v & 0xFF)) | (a << 8));
-    }
-  }
-}
-
 // w(q) mod p, centred, for 0 <= q_a, q_b, q_c <= qmax: the correctly rounded |q| 2^44.
 __global__ void weight_kernel(int q1, int p, int16_t* __restrict__ w) {
   const int c = blockIdx.x * blockDim.x + threadIdx.x, b = blockIdx.y, a = blockIdx.z;
@@ -150,7 +128,7 @@ __global__ void weight_kernel(int q1, int p, int16_t* __restrict__ w) {
 constexpr int kXyThreads = 256;
 template <bool kWeighted>
 __global__ void __launch_bounds__(kXyThreads)
-    xy_kernel(const uint16_t* __restrict__ range, const int16_t* __restrict__ w,
+    xy_kernel(const uint32_t* __restrict__ range, const int16_t* __restrict__ w,
               const float* __restrict__ E /*[q][ep]*/, const float* __restrict__ prefix, int ep,
               int q1, const int* __restrict__ radius, int np, int cp, float p, float inv,
               float* __restrict__ out) {
@@ -163,13 +141,13 @@ __global__ void __launch_bounds__(kXyThreads)
   for (int a = threadIdx.x; a < q1 + 1; a += kXyThreads)
     sE[a] = (!kWeighted || a < q1) ? src[(int64_t)a * ep + x] : 0.f;
   __syncthreads();
-  const uint16_t* rg = range + (int64_t)s * q1 * q1;
+  const uint32_t* rg = range + (int64_t)s * q1 * q1;
   for (int i = threadIdx.x; i < nb * cp; i += kXyThreads) {
     const int b = i / cp, c = i - b * cp;
     float v = 0.f;
-    const uint16_t r = c < nb ? rg[b * q1 + c] : (uint16_t)0x00FF;
-    if (r != 0x00FF) {
-      const int a0 = r & 0xFF, a1 = r >> 8;
+    const uint32_t r = c < nb ? rg[b * q1 + c] : kEmptyRange;
+    if (r != kEmptyRange) {
+      const int a0 = (int)(r & 0xFFFF), a1 = (int)(r >> 16);
       if (kWeighted) {
         int run = 0;
         for (int a = a0; a <= a1; ++a) {
@@ -524,7 +502,7 @@ bool gridinfo_modular(bsk_plan* p, const std::vector<HostTriangle>& tri, double*
     return at;
   };
   const size_t a_up = take(up.host.size());
-  const size_t a_range = take((size_t)n * q1 * q1 * sizeof(uint16_t));
+  const size_t a_range = take((size_t)n * q1 * q1 * sizeof(uint32_t));
   const size_t a_w = take((size_t)q1 * q1 * q1 * sizeof(int16_t));
   const size_t a_out = take(((size_t)n_cnt * ne + (size_t)n_pr * ns) * sizeof(long long) + 8);
   const size_t a_h = take((size_t)n * max_np * cp * sizeof(float));
@@ -543,7 +521,7 @@ bool gridinfo_modular(bsk_plan* p, const std::vector<HostTriangle>& tri, double*
   } free_base{base, st};
   BSK_CHECK_CUDA(cudaMemcpyAsync(base + a_up, up.host.data(), up.host.size(),
                                  cudaMemcpyHostToDevice, st));
-  uint16_t* range = (uint16_t*)(base + a_range);
+  uint32_t* range = (uint32_t*)(base + a_range);
   int16_t* w = (int16_t*)(base + a_w);
   long long* cnt = (long long*)(base + a_out);
   long long* sum = cnt + (size_t)n_cnt * ne;
@@ -553,8 +531,7 @@ bool gridinfo_modular(bsk_plan* p, const std::vector<HostTriangle>& tri, double*
   __nv_bfloat16* split = (__nv_bfloat16*)(base + a_s);
   const int* radius = (const int*)(base + a_up + o_rad);
   BSK_CHECK_CUDA(cudaMemsetAsync(cnt, 0, (char*)(flag + 2) - (char*)cnt, st));
-  range_kernel<<<dim3((q1 + 63) / 64, q1), 64, 0, st>>>(p->table, p->Ng, n, q1, range, flag);
-  BSK_CHECK_CUDA(cudaGetLastError());
+  launch_shell_range(p, range, flag, st);
   int hflag = 0;
   BSK_CHECK_CUDA(cudaMemcpyAsync(&hflag, flag, sizeof(int), cudaMemcpyDeviceToHost, st));
   BSK_CHECK_CUDA(cudaStreamSynchronize(st));

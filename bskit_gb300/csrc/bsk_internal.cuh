@@ -170,6 +170,7 @@ struct bsk_plan {
   int64_t K = 0;        // Ng^3
   int64_t Mh = 0;       // Ng*Ng*(Ng/2+1) half-complex modes
   uint16_t* table = nullptr;  // device [Mh] shell code
+  uint32_t* range = nullptr;  // device [n][qmax + 1]^2, the shells' |q_a| intervals
   double* d_edges = nullptr;  // device [2n]
   cufftHandle r2c = 0;        // N^3 R2C
   bool r2c_ok = false;
@@ -234,6 +235,11 @@ int64_t device_bytes(const bsk_plan* p);
 // Shell table + exact mode counts (FP64 predicate, Hermitian weights).
 void launch_shell_table(const bsk_plan* p, unsigned long long* d_counts, int* d_flag,
                         cudaStream_t st);
+// The modes of shell s on a line (|q_b|, q_c) are those of one interval of |q_a| (|k| grows with
+// |q_a|): range[s][|q_b|][q_c] = first | last << 16, q1 = qmax + 1 values an axis, kEmptyRange
+// when none.  flag (optional) is set when a mode lies in more than two shells.
+constexpr uint32_t kEmptyRange = 0x0000FFFFu;
+void launch_shell_range(const bsk_plan* p, uint32_t* range, int* flag, cudaStream_t st);
 // Copy the |q_c| < Ng/2 modes of an N^3 half spectrum into the Ng half grid,
 // scaled by 1/N^3.
 // axis_w: optional per-axis window factors indexed by q + N/2 (NULL = none).
@@ -249,15 +255,17 @@ void launch_filter_indicator(const bsk_plan* p, int s0, int ns, int kweight,
 void launch_window(int N, float scale, cufftComplex* spec, const float* axis_w, int num_sms,
                    cudaStream_t st);
 // Field synthesis: fields (and optionally the hi / lo planes) of shells [s0, s0 + ns)
-// from the slot spectrum by three pruned FFT passes; R = largest |q_c| of those shells.
+// from the slot spectrum by three pruned FFT passes; R = largest |q_c| of those shells; the
+// FP32 fields of shells >= fields_from and the planes of shells < split_to are written.
 // Shell s is written at fields[(s - out_s0) K].
 bool synth_supported(int n);
 size_t synth_workspace_bytes(int n, int max_r, int batch);
 // Twiddle table at the start of the workspace (synchronous; once, after allocation).
 void synth_init_workspace(int n, void* work);
-void launch_synth(int N, const cufftComplex* spec, const uint16_t* table, int s0, int ns, int R,
-                  void* work, float* fields, __nv_bfloat16* split, int split_shells,
-                  cudaStream_t st, int out_s0 = 0, int fields_from = 0);
+void launch_synth(int N, const cufftComplex* spec, const uint16_t* table, const uint32_t* range,
+                  int q1, int s0, int ns, int R, void* work, float* fields,
+                  __nv_bfloat16* split, int split_shells, cudaStream_t st, int out_s0 = 0,
+                  int fields_from = 0, int split_to = 1 << 30);
 // FP32 fields [S][K] -> their chunk-major bf16 hi / lo split (split_elems(S, K) values,
 // the tail of the last chunk zeroed).
 void launch_split(const float* in, int S, int64_t K, __nv_bfloat16* split, cudaStream_t st);

@@ -68,6 +68,26 @@ __global__ void shell_table_kernel(int Ng, int reduced, double kf, int n,
     if (s_counts[i]) atomicAdd(&counts[i], s_counts[i]);
 }
 
+// Thread = line (b, c); see launch_shell_range.  The codes are read coalesced along c.
+__global__ void shell_range_kernel(const uint16_t* __restrict__ table, int Ng, int n_shells,
+                                   int q1, uint32_t* __restrict__ range, int* __restrict__ flag) {
+  const int c = blockIdx.x * blockDim.x + threadIdx.x, b = blockIdx.y;
+  if (c >= q1) return;
+  const int64_t plane = (int64_t)q1 * q1, at = (int64_t)b * q1 + c;
+  for (int s = 0; s < n_shells; ++s) range[s * plane + at] = kEmptyRange;
+  for (int a = 0; a < q1; ++a) {
+    const uint16_t code = __ldg(table + ((int64_t)a * Ng + b) * (Ng / 2 + 1) + c);
+    const int first = code & 0xFF, extra = code >> 8;
+    if (first == 0xFF) continue;
+    if (flag && extra > 1) atomicOr(flag, 1);
+    for (int s = first; s <= first + extra; ++s) {
+      uint32_t* r = range + s * plane + at;
+      const uint32_t v = *r;
+      *r = (v == kEmptyRange ? (uint32_t)a : (v & 0xFFFFu)) | ((uint32_t)a << 16);
+    }
+  }
+}
+
 // coarse[a][b][c] = fine[qa mod N][qb mod N][c] / N^3 for modes strictly below the coarse
 // Nyquist frequency; zero elsewhere.  When Ng == N it is a scaled copy.
 // Optional window compensation: per-axis factor table w[q + N/2], the mode's value
@@ -245,6 +265,13 @@ void launch_shell_table(const bsk_plan* p, unsigned long long* d_counts, int* d_
   size_t shm = sizeof(unsigned long long) * (size_t)p->n;
   shell_table_kernel<<<grid_for(p->Mh, 256, p->num_sms * 8), 256, shm, st>>>(
       p->Ng, reduced, kf, p->n, p->d_edges, p->table, d_counts, d_flag);
+  BSK_CHECK_CUDA(cudaGetLastError());
+}
+
+void launch_shell_range(const bsk_plan* p, uint32_t* range, int* flag, cudaStream_t st) {
+  const int q1 = p->qmax + 1;
+  shell_range_kernel<<<dim3((q1 + 63) / 64, q1), 64, 0, st>>>(p->table, p->Ng, p->n, q1, range,
+                                                              flag);
   BSK_CHECK_CUDA(cudaGetLastError());
 }
 

@@ -14,12 +14,12 @@
 // runs of it.
 // The FFTs are radix-16/24/12/8/6/4/2/3/5 Stockham passes in shared memory (twiddles from a
 // table computed in double precision on the host); unnormalised, sign +1, as cuFFT's C2R.
-#include <atomic>
-#include <cmath>
-
-#include "bsk_internal.cuh"
+// Lengths of two or three radices are compiled (bsk_synth_warp.cuh); this file has the same
+// passes for the other lengths, with the radix plan at run time.
+#include "bsk_synth_warp.cuh"
 
 namespace bsk {
+namespace synth {
 namespace {
 
 constexpr int kLines = 16;   // lines (one 16-wide q_c run) per block of the Y pass
@@ -28,174 +28,16 @@ constexpr int kXLines = 8;   // X pass: half a q_c run per block (its staged spe
 constexpr int kZLines = 16;  // lines (two output rows each) per block of the Z pass
 constexpr int kThreads = 256;
 
-__device__ __forceinline__ int fft_freq(int a, int n) { return a < (n + 1) / 2 ? a : a - n; }
-
 __device__ __forceinline__ bool in_shell(uint16_t code, int s) {
   const int first = code & 0xFF;
   const int cnt = (code >> 8) + 1;
   return first != 0xFF && s >= first && s < first + cnt;
 }
 
-__device__ __forceinline__ float2 cmul(float2 a, float2 b) {
-  return make_float2(a.x * b.x - a.y * b.y, a.x * b.y + a.y * b.x);
-}
-__device__ __forceinline__ float2 cadd(float2 a, float2 b) { return make_float2(a.x + b.x, a.y + b.y); }
-__device__ __forceinline__ float2 csub(float2 a, float2 b) { return make_float2(a.x - b.x, a.y - b.y); }
-// multiply by +i
-__device__ __forceinline__ float2 mul_i(float2 a) { return make_float2(-a.y, a.x); }
-
-// Unnormalised R-point DFT with sign +1 in registers: v[q] <- sum_r v[r] e^{+2 pi i r q / R}.
-// roots[R][k] = e^{+2 pi i k / R}.
-__device__ __forceinline__ void dft2(float2* v) {
-  const float2 a = v[0], b = v[1];
-  v[0] = cadd(a, b);
-  v[1] = csub(a, b);
-}
-__device__ __forceinline__ void dft4(float2* v) {
-  const float2 s02 = cadd(v[0], v[2]), d02 = csub(v[0], v[2]);
-  const float2 s13 = cadd(v[1], v[3]), d13 = mul_i(csub(v[1], v[3]));
-  v[0] = cadd(s02, s13);
-  v[2] = csub(s02, s13);
-  v[1] = cadd(d02, d13);
-  v[3] = csub(d02, d13);
-}
-__device__ __forceinline__ void dft8(float2* v) {
-  // two 4-point DFTs of the even and odd samples, combined with e^{+2 pi i k / 8}
-  float2 e[4] = {v[0], v[2], v[4], v[6]};
-  float2 o[4] = {v[1], v[3], v[5], v[7]};
-  dft4(e);
-  dft4(o);
-  const float h = 0.70710678118654752f;
-  const float2 w1 = make_float2(h, h), w3 = make_float2(-h, h);
-  const float2 t0 = o[0], t1 = cmul(o[1], w1), t2 = mul_i(o[2]), t3 = cmul(o[3], w3);
-  v[0] = cadd(e[0], t0);
-  v[4] = csub(e[0], t0);
-  v[1] = cadd(e[1], t1);
-  v[5] = csub(e[1], t1);
-  v[2] = cadd(e[2], t2);
-  v[6] = csub(e[2], t2);
-  v[3] = cadd(e[3], t3);
-  v[7] = csub(e[3], t3);
-}
-__device__ __forceinline__ void dft16(float2* v) {
-  // 16 = 4 x 4: DFT4 over a of v[4a + b], twiddle e^{2 pi i b c / 16}, DFT4 over b
-  float2 y[4][4];
-#pragma unroll
-  for (int b = 0; b < 4; ++b) {
-    float2 t[4] = {v[b], v[4 + b], v[8 + b], v[12 + b]};
-    dft4(t);
-#pragma unroll
-    for (int c = 0; c < 4; ++c) y[b][c] = t[c];
-  }
-  const float c1 = 0.92387953251128676f, s1 = 0.38268343236508977f;  // cos, sin(pi/8)
-  const float h = 0.70710678118654752f;
-  // e^{2 pi i k / 16} for k = b c: k = 1, 2, 3, 4, 6, 9
-  y[1][1] = cmul(y[1][1], make_float2(c1, s1));
-  y[1][2] = cmul(y[1][2], make_float2(h, h));
-  y[1][3] = cmul(y[1][3], make_float2(s1, c1));
-  y[2][1] = cmul(y[2][1], make_float2(h, h));
-  y[2][2] = mul_i(y[2][2]);
-  y[2][3] = cmul(y[2][3], make_float2(-h, h));
-  y[3][1] = cmul(y[3][1], make_float2(s1, c1));
-  y[3][2] = cmul(y[3][2], make_float2(-h, h));
-  y[3][3] = cmul(y[3][3], make_float2(-c1, -s1));
-#pragma unroll
-  for (int c = 0; c < 4; ++c) {
-    float2 t[4] = {y[0][c], y[1][c], y[2][c], y[3][c]};
-    dft4(t);
-#pragma unroll
-    for (int d = 0; d < 4; ++d) v[c + 4 * d] = t[d];
-  }
-}
-template <int R>
-__device__ __forceinline__ void dft_generic(float2* v, const float2* roots) {
-  float2 out[R];
-#pragma unroll
-  for (int q = 0; q < R; ++q) {
-    float2 acc = v[0];
-#pragma unroll
-    for (int r = 1; r < R; ++r) acc = cadd(acc, cmul(v[r], roots[(r * q) % R]));
-    out[q] = acc;
-  }
-#pragma unroll
-  for (int q = 0; q < R; ++q) v[q] = out[q];
-}
-
-struct FftPlan {
-  int n;
-  int np;
-  int radix[8];  // 16, 24, 12, 8, 6, 4, 2, 3 or 5
-  float2 root3[3];
-  float2 root5[5];
-  float2 rootc[24];  // e^{+2 pi i k / Rc} of the plan's composite radix Rc (24, 12 or 6)
-};
-
-template <int R>
-__device__ __forceinline__ void dft_small(float2* v, const FftPlan& pl) {
-  if (R == 8) dft8(v);
-  else if (R == 4) dft4(v);
-  else if (R == 2) dft2(v);
-  else if (R == 3) dft_generic<3>(v, pl.root3);
-  else dft_generic<5>(v, pl.root5);
-}
-
-// R = R1 R2 point DFT: input r = R2 a + b, output q = c + R1 d:
-// X[c + R1 d] = sum_b e^{2 pi i b d / R2} e^{2 pi i b c / R} sum_a v[R2 a + b] e^{2 pi i a c / R1}.
-template <int R1, int R2>
-__device__ __forceinline__ void dft_comp(float2* v, const FftPlan& pl) {
-  float2 y[R2][R1];
-#pragma unroll
-  for (int b = 0; b < R2; ++b) {
-    float2 t[R1];
-#pragma unroll
-    for (int a = 0; a < R1; ++a) t[a] = v[R2 * a + b];
-    dft_small<R1>(t, pl);
-#pragma unroll
-    for (int c = 0; c < R1; ++c) y[b][c] = b && c ? cmul(t[c], pl.rootc[b * c]) : t[c];
-  }
-#pragma unroll
-  for (int c = 0; c < R1; ++c) {
-    float2 t[R2];
-#pragma unroll
-    for (int b = 0; b < R2; ++b) t[b] = y[b][c];
-    dft_small<R2>(t, pl);
-#pragma unroll
-    for (int d = 0; d < R2; ++d) v[c + R1 * d] = t[d];
-  }
-}
-
-// Radix plan of a length: 16s, then one of 24 / 12 / 8 / 6 / 4 / 2, then 3s and 5s (constexpr, so that a
-// compile-time length gets a fully unrolled pass sequence).
-// The p-th radix of a length's plan (0 past the end, -1 when the length does not factor).
-__host__ __device__ constexpr int plan_radix(int n, int p) {
-  int k = 0;
-  while (n % 16 == 0) { n /= 16; if (k++ == p) return 16; }
-  const int comp[6] = {24, 12, 8, 6, 4, 2};  // at most one of these, 2^a 3 first
-  for (int c : comp)
-    if (n % c == 0) { n /= c; if (k++ == p) return c; break; }
-  while (n % 3 == 0) { n /= 3; if (k++ == p) return 3; }
-  while (n % 5 == 0) { n /= 5; if (k++ == p) return 5; }
-  return n == 1 ? 0 : -1;
-}
-__host__ __device__ constexpr int plan_np(int n) {
-  int p = 0;
-  while (plan_radix(n, p) > 0) ++p;
-  return plan_radix(n, p) == 0 ? p : -1;
-}
-
 // Lines are kept in shared memory with a stride of n + 1 complex values, and consecutive
 // threads take the same butterfly of consecutive lines: both keep the Stockham reads and
 // writes of a warp on distinct banks.
 __host__ __device__ constexpr int line_stride(int n) { return n + 1; }
-
-template <int R>
-__device__ __forceinline__ void dft_radix(float2* v, const FftPlan& pl) {
-  if (R == 16) dft16(v);
-  else if (R == 24) dft_comp<8, 3>(v, pl);
-  else if (R == 12) dft_comp<4, 3>(v, pl);
-  else if (R == 6) dft_comp<2, 3>(v, pl);
-  else dft_small<R>(v, pl);
-}
 
 // One Stockham pass of radix R over `lines` sequences of length n (src -> dst).  Input
 // positions zlo .. zhi are known to be zero: they are neither read nor need to be written
@@ -230,52 +72,15 @@ __device__ __forceinline__ void fft_pass(const float2* __restrict__ src, float2*
   }
 }
 
-// Compile-time length: the pass sequence unrolled, every divisor a constant.
-template <int N, int L, int P, int Ns>
-__device__ __forceinline__ void run_passes(float2*& src, float2*& dst,
-                                           const float2* __restrict__ tw, const FftPlan& pl,
-                                           int zlo = 1 << 30, int zhi = -1) {
-  if constexpr (P < plan_np(N)) {
-    constexpr int R = plan_radix(N, P);
-    if (P == 0) fft_pass<R>(src, dst, L, N, Ns, tw, pl, zlo, zhi);
-    else fft_pass<R>(src, dst, L, N, Ns, tw, pl);
-    __syncthreads();
-    float2* t2 = src;
-    src = dst;
-    dst = t2;
-    run_passes<N, L, P + 1, Ns * R>(src, dst, tw, pl);
-  }
-}
-
-// All passes but the last (the Z pass fuses the last one with its stores).
-template <int N, int L, int P, int Ns>
-__device__ __forceinline__ void run_passes_but_last(float2*& src, float2*& dst,
-                                                    const float2* __restrict__ tw,
-                                                    const FftPlan& pl, int zlo = 1 << 30,
-                                                    int zhi = -1) {
-  if constexpr (P + 1 < plan_np(N)) {
-    constexpr int R = plan_radix(N, P);
-    if (P == 0) fft_pass<R>(src, dst, L, N, Ns, tw, pl, zlo, zhi);
-    else fft_pass<R>(src, dst, L, N, Ns, tw, pl);
-    __syncthreads();
-    float2* t2 = src;
-    src = dst;
-    dst = t2;
-    run_passes_but_last<N, L, P + 1, Ns * R>(src, dst, tw, pl);
-  }
-}
-
 // Inverse FFT (sign +1, unnormalised) of L sequences of length n stored with line
 // stride n + 1 in `a`; `b` is scratch of the same size.  Returns the buffer holding the
-// result.  NC = n at compile time, or 0.
-template <int NC, int L>
+// result.
+template <int L>
 __device__ float2* fft_lines(float2* a, float2* b, const FftPlan& pl,
                              const float2* __restrict__ tw, int zlo = 1 << 30, int zhi = -1) {
   float2* src = a;
   float2* dst = b;
-  if constexpr (NC != 0) {
-    run_passes<NC, L, 0, 1>(src, dst, tw, pl, zlo, zhi);
-  } else {
+  {
     const int n = pl.n;
     int Ns = 1;
     for (int p = 0; p < pl.np; ++p) {
@@ -302,31 +107,10 @@ __device__ float2* fft_lines(float2* a, float2* b, const FftPlan& pl,
   return src;
 }
 
-// Index of the i-th kept frequency of an axis: the `nk` frequencies |q| <= R around 0
-// (all n of them when 2R + 1 >= n).
-__device__ __forceinline__ int kept_index(int i, int nk, int R, int n) {
-  return nk == n ? i : (i - R + n) % n;
-}
-
-struct SynthArgs {
-  int N, H, R, nk, Cp, s0, ns;
-  int out0;                // shell written at fields[0] (and hi/lo[0])
-  int fields_from;         // the FP32 field is written for shells s0 + s >= fields_from only
-  const float2* spec;      // [a][b][c] slot spectrum
-  const uint16_t* table;   // [a][b][c] shell codes
-  float2* G;               // [s][x][bk][c]   (c < Cp)
-  float2* Hh;              // [s][x][y][c]
-  float* fields;           // [shell][N^3], shell index s0 + s
-  __nv_bfloat16* split;    // optional chunk-major hi / lo split of split_shells shells
-  int split_shells;
-  const float2* tw;        // [N] e^{+2 pi i k / N}
-};
-
 // X pass: block (bk, c-run).  Spectrum and table columns are read once for all shells.
-template <int NC>
 __global__ void __launch_bounds__(kThreads) synth_x_kernel(SynthArgs A, FftPlan pl) {
   extern __shared__ float2 sm[];
-  const int N = NC ? NC : A.N, nk = A.nk;
+  const int N = A.N, nk = A.nk;
   const int ls = line_stride(N);
   float2* buf0 = sm;                       // kXLines lines
   float2* buf1 = buf0 + kXLines * ls;       // kXLines lines
@@ -364,7 +148,7 @@ __global__ void __launch_bounds__(kThreads) synth_x_kernel(SynthArgs A, FftPlan 
       buf0[l * ls + a] = v;
     }
     __syncthreads();
-    const float2* res = fft_lines<NC, kXLines>(buf0, buf1, pl, tw, zlo, zhi);
+    const float2* res = fft_lines<kXLines>(buf0, buf1, pl, tw, zlo, zhi);
     // G[s][x][bk][c0 + l]
     float2* g = A.G + (((int64_t)s * N) * nk + bk) * A.Cp + c0;
     for (int i = threadIdx.x; i < kXLines * N; i += blockDim.x) {
@@ -383,10 +167,9 @@ constexpr int kYPf = 16;  // Y pass: kYPf * kThreads / kLines kept q_b per line
 constexpr int kZPf = 8;   // Z pass: kZPf * kThreads / kZLines nonzero q_c per line
 
 // Y pass: unit (x, c-run, shell).
-template <int NC>
 __global__ void __launch_bounds__(kThreads, 2) synth_y_kernel(SynthArgs A, FftPlan pl, int units) {
   extern __shared__ float2 sm[];
-  const int N = NC ? NC : A.N, nk = A.nk;
+  const int N = A.N, nk = A.nk;
   const int ls = line_stride(N);
   float2* buf0 = sm;
   float2* buf1 = buf0 + kLines * ls;
@@ -427,8 +210,8 @@ __global__ void __launch_bounds__(kThreads, 2) synth_y_kernel(SynthArgs A, FftPl
     // positions R + 1 .. N - R - 1 (|q_b| > R) are zero: not written, not read
     __syncthreads();
     if (u + (int)gridDim.x < units) fetch(u + gridDim.x);
-    const float2* res = nk < N ? fft_lines<NC, kLines>(buf0, buf1, pl, tw, A.R + 1, N - A.R - 1)
-                               : fft_lines<NC, kLines>(buf0, buf1, pl, tw);
+    const float2* res = nk < N ? fft_lines<kLines>(buf0, buf1, pl, tw, A.R + 1, N - A.R - 1)
+                               : fft_lines<kLines>(buf0, buf1, pl, tw);
     const int s = u / (N * nrun), r = u - s * (N * nrun);
     const int x = r / nrun, c0 = (r - x * nrun) * kLines;
     float2* h = A.Hh + (((int64_t)s * N + x) * N) * A.Cp + c0;
@@ -440,79 +223,16 @@ __global__ void __launch_bounds__(kThreads, 2) synth_y_kernel(SynthArgs A, FftPl
   }
 }
 
-// Radix of the last pass of a compile-time length, and the size of its twiddle table twl.
-template <int NC>
-__host__ __device__ constexpr int z_last_radix() { return plan_radix(NC, plan_np(NC) - 1); }
-template <int NC>
-__host__ __device__ constexpr int z_twl_size() { return NC - NC / z_last_radix<NC>(); }
-
-// Last FFT pass of the Z pass fused with its stores.  Butterfly j of a line yields the
-// outputs z = j + M r (M = n / R); lanes j (even) and j + 1 hold z and z + 1, so one
-// exchange gives the even lane row y1's pair (z, z + 1) (real parts) and the odd lane row
-// y2's (imaginary parts): 8-byte field stores, 4-byte hi / lo stores, 32-byte sectors.
-// Consecutive lanes take consecutive j, so the twiddles come from a table twl[(r - 1) M + j]
-// = e^{+2 pi i r j / n}: a warp reads consecutive entries (tw[r j] would be r apart, a
-// gcd(r, 16)-way bank conflict).
-template <int NC>
-__device__ __forceinline__ void z_last_pass(const float2* __restrict__ src,
-                                            const float2* __restrict__ twl, const FftPlan& pl,
-                                            const SynthArgs& A, int sh, int64_t row0, int y0,
-                                            bool fp32) {
-  constexpr int np = plan_np(NC);
-  constexpr int R = z_last_radix<NC>();
-  constexpr int M = NC / R;
-  static_assert(np >= 2 && M % 2 == 0 && (kZLines * M) % kThreads == 0,
-                "the fused last pass wants full warps of line-ordered butterfly pairs");
-  constexpr int ls = line_stride(NC);
-  for (int t = threadIdx.x; t < kZLines * M; t += kThreads) {
-    const int line = t / M, j = t - line * M;
-    const float2* in = src + line * ls;
-    float2 v[R];
-#pragma unroll
-    for (int r = 0; r < R; ++r) v[r] = in[j + r * M];
-#pragma unroll
-    for (int r = 1; r < R; ++r) v[r] = cmul(v[r], twl[(r - 1) * M + j]);
-    dft_radix<R>(v, pl);
-    const bool odd = j & 1;
-    const int y = y0 + 2 * line + (odd ? 1 : 0);
-    const int64_t K = (int64_t)NC * NC * NC;
-    const int64_t o = row0 + (int64_t)y * NC + (j & ~1);  // point index within the shell
-#pragma unroll
-    for (int r = 0; r < R; ++r) {
-      const float got = __shfl_xor_sync(0xffffffffu, odd ? v[r].x : v[r].y, 1);
-      const float2 f = odd ? make_float2(got, v[r].y) : make_float2(v[r].x, got);
-      if (y < NC) {
-        const int64_t pt = o + (int64_t)M * r;
-        if (fp32) *reinterpret_cast<float2*>(A.fields + (int64_t)sh * K + pt) = f;
-        if (A.split) {
-          const __nv_bfloat162 h = __floats2bfloat162_rn(f.x, f.y);
-          const float2 fb = __bfloat1622float2(h);
-          const __nv_bfloat162 lw = __floats2bfloat162_rn(f.x - fb.x, f.y - fb.y);
-          *reinterpret_cast<__nv_bfloat162*>(A.split + split_index(0, sh, pt, A.split_shells)) = h;
-          *reinterpret_cast<__nv_bfloat162*>(A.split + split_index(1, sh, pt, A.split_shells)) = lw;
-        }
-      }
-    }
-  }
-}
-
 // Z pass: unit (x, run of 2 kZLines rows y, shell).  Line l packs rows y0 + 2l, y0 + 2l + 1.
-template <int NC>
 __global__ void __launch_bounds__(kThreads, 2) synth_z_kernel(SynthArgs A, FftPlan pl, int units) {
   extern __shared__ float2 sm[];
-  const int N = NC ? NC : A.N;
+  const int N = A.N;
   const int ls = line_stride(N);
   float2* buf0 = sm;
   float2* buf1 = buf0 + kZLines * ls;
   float2* tw = buf1 + kZLines * ls;
-  float2* twl = tw + N;  // the last pass's twiddles (compile-time lengths)
   const int ny = (N + 2 * kZLines - 1) / (2 * kZLines);
   for (int i = threadIdx.x; i < N; i += blockDim.x) tw[i] = A.tw[i];
-  if constexpr (NC != 0) {
-    constexpr int M = NC / z_last_radix<NC>();
-    for (int i = threadIdx.x; i < z_twl_size<NC>(); i += blockDim.x)
-      twl[i] = A.tw[(i / M + 1) * (i % M)];  // r j < R M = n
-  }
   const int cn = min(A.R, N / 2) + 1;  // q_c = 0 .. cn - 1 can be nonzero
   // kThreads / kZLines threads per line, q_c strided by that
   constexpr int tpl = kThreads / kZLines;
@@ -564,13 +284,8 @@ __global__ void __launch_bounds__(kThreads, 2) synth_z_kernel(SynthArgs A, FftPl
     const int64_t K = (int64_t)N * N * N;
     const int sh = A.s0 + s - A.out0;  // shell index in the output arrays
     const int64_t row0 = ((int64_t)x * N) * N;
-    if constexpr (NC != 0) {
-      float2* src = buf0;
-      float2* dst = buf1;
-      run_passes_but_last<NC, kZLines, 0, 1>(src, dst, tw, pl, cn, N - cn);
-      z_last_pass<NC>(src, twl, pl, A, sh, row0, y0, A.s0 + s >= A.fields_from);
-    } else {
-      const float2* res = fft_lines<NC, kZLines>(buf0, buf1, pl, tw, cn, N - cn);
+    {
+      const float2* res = fft_lines<kZLines>(buf0, buf1, pl, tw, cn, N - cn);
       // four consecutive z per thread: 16-byte field stores, 8-byte hi / lo stores (N % 4 == 0)
       const int nq = N / 4;
       for (int i = threadIdx.x; i < 2 * kZLines * nq; i += kThreads) {
@@ -584,7 +299,7 @@ __global__ void __launch_bounds__(kThreads, 2) synth_z_kernel(SynthArgs A, FftPl
         const int64_t pt = row0 + (int64_t)y * N + z;
         if (A.s0 + s >= A.fields_from)
           *reinterpret_cast<float4*>(A.fields + (int64_t)sh * K + pt) = v;
-        if (A.split) {
+        if (A.split && A.s0 + s < A.split_to) {
           const __nv_bfloat162 h01 = __floats2bfloat162_rn(v.x, v.y);
           const __nv_bfloat162 h23 = __floats2bfloat162_rn(v.z, v.w);
           const float2 f01 = __bfloat1622float2(h01), f23 = __bfloat1622float2(h23);
@@ -604,41 +319,42 @@ __global__ void __launch_bounds__(kThreads, 2) synth_z_kernel(SynthArgs A, FftPl
   }
 }
 
-template <int NC>
-void run_synth(const SynthArgs& A, const FftPlan& pl, int nk, int Cp, int ns, size_t fft_smem,
-               size_t x_smem, cudaStream_t st) {
+void run_synth(const SynthArgs& A, const FftPlan& pl, int nk, int Cp, int ns, cudaStream_t st) {
+  const int N = A.N;
+  const size_t fft_smem = (2 * (size_t)kLines * (N + 1) + N) * sizeof(float2);
+  const size_t x_smem = (2 * (size_t)kXLines * (N + 1) + N) * sizeof(float2) +
+                        (size_t)nk * kXLines * (sizeof(float2) + sizeof(uint16_t));
+  BSK_REQUIRE(x_smem <= 227 * 1024, BSK_ERR_UNSUPPORTED, "grid too large for the field synthesis");
   static std::atomic<bool> attr_done[64];  // zero-initialised: false
   int dev = 0;
   BSK_CHECK_CUDA(cudaGetDevice(&dev));
   if (dev < 64 && !attr_done[dev]) {
     const int maxs = 227 * 1024;
-    BSK_CHECK_CUDA(cudaFuncSetAttribute(synth_x_kernel<NC>,
+    BSK_CHECK_CUDA(cudaFuncSetAttribute(synth_x_kernel,
                                         cudaFuncAttributeMaxDynamicSharedMemorySize, maxs));
-    BSK_CHECK_CUDA(cudaFuncSetAttribute(synth_y_kernel<NC>,
+    BSK_CHECK_CUDA(cudaFuncSetAttribute(synth_y_kernel,
                                         cudaFuncAttributeMaxDynamicSharedMemorySize, maxs));
-    BSK_CHECK_CUDA(cudaFuncSetAttribute(synth_z_kernel<NC>,
+    BSK_CHECK_CUDA(cudaFuncSetAttribute(synth_z_kernel,
                                         cudaFuncAttributeMaxDynamicSharedMemorySize, maxs));
     attr_done[dev] = true;
   }
-  const int N = A.N;
-  synth_x_kernel<NC><<<dim3(nk, Cp / kXLines), kThreads, x_smem, st>>>(A, pl);
+  synth_x_kernel<<<dim3(nk, Cp / kXLines), kThreads, x_smem, st>>>(A, pl);
   BSK_CHECK_CUDA(cudaGetLastError());
   // persistent Y and Z passes: as many blocks as are resident at once
   int nsm = 0, by = 0, bz = 0;
   BSK_CHECK_CUDA(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev));
-  size_t z_smem = (2 * (size_t)kZLines * (N + 1) + N) * sizeof(float2);
-  if constexpr (NC != 0) z_smem += z_twl_size<NC>() * sizeof(float2);
-  BSK_CHECK_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&by, synth_y_kernel<NC>, kThreads,
+  const size_t z_smem = (2 * (size_t)kZLines * (N + 1) + N) * sizeof(float2);
+  BSK_CHECK_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&by, synth_y_kernel, kThreads,
                                                                fft_smem));
-  BSK_CHECK_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&bz, synth_z_kernel<NC>, kThreads,
+  BSK_CHECK_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&bz, synth_z_kernel, kThreads,
                                                                z_smem));
   const int y_units = N * (Cp / kLines) * ns;
   const int z_units = N * ((N + 2 * kZLines - 1) / (2 * kZLines)) * ns;
   const int y_grid = std::max(1, std::min(y_units, std::max(by, 1) * nsm));
   const int z_grid = std::max(1, std::min(z_units, std::max(bz, 1) * nsm));
-  synth_y_kernel<NC><<<y_grid, kThreads, fft_smem, st>>>(A, pl, y_units);
+  synth_y_kernel<<<y_grid, kThreads, fft_smem, st>>>(A, pl, y_units);
   BSK_CHECK_CUDA(cudaGetLastError());
-  synth_z_kernel<NC><<<z_grid, kThreads, z_smem, st>>>(A, pl, z_units);
+  synth_z_kernel<<<z_grid, kThreads, z_smem, st>>>(A, pl, z_units);
   BSK_CHECK_CUDA(cudaGetLastError());
 }
 
@@ -661,8 +377,18 @@ bool make_plan(int n, FftPlan& pl) {
   return true;
 }
 
-}  // namespace
+bool run_compiled(int N, const SynthArgs& A, const FftPlan& pl, cudaStream_t st) {
+  return run_compiled_a(N, A, pl, st) || run_compiled_b(N, A, pl, st) ||
+         run_compiled_c(N, A, pl, st) || run_compiled_d(N, A, pl, st) ||
+         run_compiled_e(N, A, pl, st) || run_compiled_f(N, A, pl, st);
+}
 
+}  // namespace
+}  // namespace synth
+
+using namespace synth;
+
+// The sides a grid level may have.
 bool synth_fast_size(int n) {
   switch (n) {
     case 48: case 96: case 128: case 160: case 192: case 240: case 256: case 288: case 320:
@@ -692,9 +418,10 @@ void synth_init_workspace(int N, void* work) {
   BSK_CHECK_CUDA(cudaMemcpy(work, htw.data(), N * sizeof(float2), cudaMemcpyHostToDevice));
 }
 
-void launch_synth(int N, const cufftComplex* spec, const uint16_t* table, int s0, int ns, int R,
-                  void* work, float* fields, __nv_bfloat16* split, int split_shells,
-                  cudaStream_t st, int out_s0, int fields_from) {
+void launch_synth(int N, const cufftComplex* spec, const uint16_t* table, const uint32_t* range,
+                  int q1, int s0, int ns, int R, void* work, float* fields,
+                  __nv_bfloat16* split, int split_shells, cudaStream_t st, int out_s0,
+                  int fields_from, int split_to) {
   FftPlan pl;
   BSK_REQUIRE(make_plan(N, pl), BSK_ERR_UNSUPPORTED, "no FFT plan for this grid size");
   R = std::min(R, N / 2);
@@ -710,8 +437,11 @@ void launch_synth(int N, const cufftComplex* spec, const uint16_t* table, int s0
   A.ns = ns;
   A.out0 = out_s0;
   A.fields_from = fields_from;
+  A.split_to = split_to;
   A.spec = reinterpret_cast<const float2*>(spec);
   A.table = table;
+  A.range = range;
+  A.q1 = q1;
   float2* tw = reinterpret_cast<float2*>(work);
   A.G = tw + N;
   A.Hh = A.G + (size_t)ns * N * nk * Cp;
@@ -719,24 +449,7 @@ void launch_synth(int N, const cufftComplex* spec, const uint16_t* table, int s0
   A.split = split;
   A.split_shells = split_shells;
   A.tw = tw;
-  const size_t fft_smem = (2 * (size_t)kLines * (N + 1) + N) * sizeof(float2);
-  const size_t x_smem = (2 * (size_t)kXLines * (N + 1) + N) * sizeof(float2) +
-                        (size_t)nk * kXLines * (sizeof(float2) + sizeof(uint16_t));
-  BSK_REQUIRE(x_smem <= 227 * 1024, BSK_ERR_UNSUPPORTED, "grid too large for the field synthesis");
-  switch (N) {
-    case 48: run_synth<48>(A, pl, nk, Cp, ns, fft_smem, x_smem, st); break;
-    case 96: run_synth<96>(A, pl, nk, Cp, ns, fft_smem, x_smem, st); break;
-    case 128: run_synth<128>(A, pl, nk, Cp, ns, fft_smem, x_smem, st); break;
-    case 160: run_synth<160>(A, pl, nk, Cp, ns, fft_smem, x_smem, st); break;
-    case 192: run_synth<192>(A, pl, nk, Cp, ns, fft_smem, x_smem, st); break;
-    case 240: run_synth<240>(A, pl, nk, Cp, ns, fft_smem, x_smem, st); break;
-    case 256: run_synth<256>(A, pl, nk, Cp, ns, fft_smem, x_smem, st); break;
-    case 288: run_synth<288>(A, pl, nk, Cp, ns, fft_smem, x_smem, st); break;
-    case 320: run_synth<320>(A, pl, nk, Cp, ns, fft_smem, x_smem, st); break;
-    case 384: run_synth<384>(A, pl, nk, Cp, ns, fft_smem, x_smem, st); break;
-    case 480: run_synth<480>(A, pl, nk, Cp, ns, fft_smem, x_smem, st); break;
-    default: run_synth<0>(A, pl, nk, Cp, ns, fft_smem, x_smem, st); break;
-  }
+  if (!run_compiled(N, A, pl, st)) run_synth(A, pl, nk, Cp, ns, st);
 }
 
 }  // namespace bsk

@@ -1,0 +1,12 @@
+// Field synthesis passes of some compiled lengths (one translation unit of several).
+#include "bsk_synth_warp.cuh"
+
+namespace bsk {
+namespace synth {
+
+bool run_compiled_c(int N, const SynthArgs& A, const FftPlan& pl, cudaStream_t st) {
+  return run_one_of<400, 36, 128, 200, 216>(N, A, pl, st);
+}
+
+}  // namespace synth
+}  // namespace bsk
