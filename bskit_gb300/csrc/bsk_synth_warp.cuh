@@ -244,11 +244,11 @@ __device__ __forceinline__ void fill_twiddles(float2* t, const float2* __restric
 }
 
 // L lines: load(line, r, j, v) -> v[r] = input j + RB r of the line for every r; store(line, k, v):
-// outputs k + RA q in v[q].  Each lane's butterflies are numbered with the line fastest or
+// outputs k + RA q in v[q]; mid() runs between the stages, when every input has been read.  Each lane's butterflies are numbered with the line fastest or
 // slowest (the layout of the global arrays decides which coalesces).
-template <int N, int L, bool kLineFast, class Load, class Store>
+template <int N, int L, bool kLineFast, class Load, class Mid, class Store>
 __device__ __forceinline__ void warp_fft(float2* __restrict__ buf, const float2* __restrict__ tw,
-                                         const FftPlan& pl, Load load, Store store) {
+                                         const FftPlan& pl, Load load, Mid mid, Store store) {
   using P = Len<N>;
   constexpr int LP = line_pitch<N, L, kLineFast>();
   const int lane = threadIdx.x & 31;
@@ -263,6 +263,7 @@ __device__ __forceinline__ void warp_fft(float2* __restrict__ buf, const float2*
     for (int r = 0; r < P::RA; ++r) o[r] = v[r];
   }
   __syncwarp();
+  mid();
   constexpr int rounds = (L * P::RA + 31) / 32;
 #pragma unroll 1
   for (int i = 0; i < rounds; ++i) {
@@ -308,16 +309,23 @@ __device__ __forceinline__ void warp_fft(float2* __restrict__ buf, const float2*
   __syncwarp();  // the next unit's stage A rewrites the buffer
 }
 
+__device__ __forceinline__ void cp_async16(void* dst, const void* src) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(
+                   (uint32_t)__cvta_generic_to_shared(dst)),
+               "l"(src)
+               : "memory");
+}
+
 constexpr int kWarps = 4;                      // warps a block
 template <int N>
 constexpr int lines_xy() { return N <= 192 ? 8 : 4; }  // 64- or 32-byte runs of q_c
 template <int N>
-constexpr int lines_z() { return N <= 192 ? 8 : 4; }
+constexpr int lines_z() { return N <= 64 ? 8 : N > 400 ? 2 : 4; }
 template <int N>
 constexpr int min_blocks() { return Len<N>::RB > 25 ? 3 : 4; }  // 168 or 128 registers
 template <int N, int L, bool kLineFast>
 constexpr size_t pass_smem() {
-  return ((size_t)kWarps * L * line_pitch<N, L, kLineFast>() + Len<N>::TW) * sizeof(float2);
+  return ((size_t)kWarps * L * line_pitch<N, L, kLineFast>() + Len<N>::TW + 1) / 2 * 2 * sizeof(float2);
 }
 
 // X pass: unit = L columns q_c of (shell, q_b); the masked spectrum along q_a (the shell's modes
@@ -354,10 +362,12 @@ __global__ void __launch_bounds__(32 * kWarps, min_blocks<N>())
         [&](int, int j, float2* in) {
 #pragma unroll
           for (int r = 0; r < Len<N>::RA; ++r) {
-            const int q = j + r * Len<N>::M, aq = q <= N / 2 ? q : N - q;
-            in[r] = aq >= a0 && aq <= a1 ? spec[(int64_t)q * N * A.H] : make_float2(0.f, 0.f);
+            const int q = j + r * Len<N>::M, aq = 2 * r < Len<N>::RA ? q : N - q;  // |q_a|
+            in[r] = aq >= a0 && aq <= a1 ? spec[(int64_t)q * (N * (N / 2 + 1))]
+                                         : make_float2(0.f, 0.f);
           }
         },
+        [] {},
         [&](bool on, int, int k, const float2* out) {
           if (!on) return;
 #pragma unroll
@@ -366,7 +376,8 @@ __global__ void __launch_bounds__(32 * kWarps, min_blocks<N>())
   }
 }
 
-// Y pass: unit = L columns q_c of (shell, x); G along q_b -> Hh[s][x][y][c].
+// Y pass: unit = L columns q_c of (shell, x); G along q_b -> Hh[s][x][y][c].  The unit's kept
+// rows (nk runs of 8 L bytes) are copied to shared memory during the previous unit's stage B.
 template <int N>
 __global__ void __launch_bounds__(32 * kWarps, min_blocks<N>())
     y_kernel(SynthArgs A, FftPlan pl, int runs, int units) {
@@ -379,26 +390,42 @@ __global__ void __launch_bounds__(32 * kWarps, min_blocks<N>())
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   float2* buf = sm + warp * L * LP;
   const int nk = A.nk, R = A.R;
+  float2* stage = sm + pass_smem<N, L, true>() / sizeof(float2) + warp * L * nk;
+  auto fetch = [&](int u) {
+    if (u < units) {
+      const int run = u % runs, sx = u / runs;
+      const float2* src = A.G + (int64_t)sx * nk * A.Cp + run * L;
+      for (int i = lane; i < nk * (L / 2); i += 32) {
+        const int bk = i / (L / 2), e = i % (L / 2) * 2;
+        cp_async16(stage + bk * L + e, src + bk * A.Cp + e);
+      }
+    }
+    asm volatile("cp.async.commit_group;" ::: "memory");
+  };
+  fetch(blockIdx.x * kWarps + warp);
   for (int u = blockIdx.x * kWarps + warp; u < units; u += gridDim.x * kWarps) {
     const int run = u % runs, sx = u / runs;  // sx = s N + x
     const int c = run * L + lane % L;
-    const float2* g = A.G + (int64_t)sx * nk * A.Cp + c;
     float2* h = A.Hh + (int64_t)sx * N * A.Cp + c;
+    asm volatile("cp.async.wait_group 0;" ::: "memory");
+    __syncwarp();
     warp_fft<N, L, true>(
         buf, tw, pl,
         [&](int, int j, float2* in) {
 #pragma unroll
           for (int r = 0; r < Len<N>::RA; ++r) {
+            // the first half of the inputs are q_b >= 0, the second q_b = q - N < 0
             const int q = j + r * Len<N>::M;
-            const int bk = nk == N ? q : q <= R ? q + R : q - N + R;
-            in[r] = nk == N || q <= R || q >= N - R ? g[(int64_t)bk * A.Cp]
-                                                    : make_float2(0.f, 0.f);
+            const bool kept = nk == N || (2 * r < Len<N>::RA ? q <= R : q >= N - R);
+            const int bk = nk == N ? q : 2 * r < Len<N>::RA ? q + R : q - N + R;
+            in[r] = kept ? stage[bk * L + lane % L] : make_float2(0.f, 0.f);
           }
         },
+        [&] { fetch(u + gridDim.x * kWarps); },
         [&](bool on, int, int k, const float2* out) {
           if (!on) return;
 #pragma unroll
-          for (int q = 0; q < Len<N>::RB; ++q) h[(int64_t)(k + Len<N>::RA * q) * A.Cp] = out[q];
+          for (int q = 0; q < Len<N>::RB; ++q) h[(k + Len<N>::RA * q) * A.Cp] = out[q];
         });
   }
 }
@@ -407,6 +434,9 @@ __global__ void __launch_bounds__(32 * kWarps, min_blocks<N>())
 // Hermitian extension along q_c of each), so that one complex transform gives both real rows.
 // Lanes k, k + 1 (even k) hold points z, z + 1 of a line and exchange one value: the even lane
 // stores row y's pair, the odd lane row y + 1's: 8-byte field and 4-byte hi / lo stores.
+// The unit's 2 L rows are one contiguous block of Hh: it is copied to shared memory with
+// cp.async while the previous unit is in stage B, so that stage A, which reads each value twice
+// (at q_c and at N - q_c), waits for no load.
 template <int N>
 __global__ void __launch_bounds__(32 * kWarps, min_blocks<N>())
     z_kernel(SynthArgs A, FftPlan pl, int runs, int units) {
@@ -416,61 +446,83 @@ __global__ void __launch_bounds__(32 * kWarps, min_blocks<N>())
   float2* tw = sm + kWarps * L * LP;
   fill_twiddles<N>(tw, A.tw);
   __syncthreads();
-  const int warp = threadIdx.x >> 5;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   float2* buf = sm + warp * L * LP;
+  const int Cp = A.Cp;
+  float2* stage = sm + pass_smem<N, L, false>() / sizeof(float2) + warp * 2 * L * Cp;
+  auto fetch = [&](int u) {
+    if (u < units) {
+      // rows y0 .. y0 + 2 L - 1 of (shell, x); a ragged last unit has fewer
+      const int run = u % runs, sx = u / runs;
+      const int rows = min(2 * L, N - run * 2 * L);
+      const float2* src = A.Hh + ((int64_t)sx * N + run * 2 * L) * Cp;
+      for (int i = lane * 2; i < rows * Cp; i += 64) cp_async16(stage + i, src + i);
+    }
+    asm volatile("cp.async.commit_group;" ::: "memory");
+  };
+  fetch(blockIdx.x * kWarps + warp);
   const int cn = min(A.R, N / 2) + 1;  // q_c = 0 .. cn - 1 can be nonzero
   constexpr int64_t K = (int64_t)N * N * N;
   for (int u = blockIdx.x * kWarps + warp; u < units; u += gridDim.x * kWarps) {
     const int run = u % runs, sx = u / runs;
     const int s = sx / N, x = sx - s * N;
     const int y0 = run * 2 * L;  // first of the unit's 2 L rows
-    const float2* h = A.Hh + ((int64_t)sx * N + y0) * A.Cp;
     const int sh = A.s0 + s - A.out0;  // shell index in the output arrays
     const bool fp32 = A.s0 + s >= A.fields_from;
     const bool planes = A.split && A.s0 + s < A.split_to;
     float* field = A.fields + (int64_t)sh * K;
     const int64_t row0 = ((int64_t)x * N + y0) * N;
+    asm volatile("cp.async.wait_group 0;" ::: "memory");
+    __syncwarp();
     warp_fft<N, L, false>(
         buf, tw, pl,
         [&](int line, int j, float2* in) {
-          const float2* h1 = h + (int64_t)2 * line * A.Cp;
+          const float2* h1 = stage + 2 * line * Cp;
           const bool row = (N / 2) % L == 0 || y0 + 2 * line < N;
           float2 z1[Len<N>::RA], z2[Len<N>::RA];
 #pragma unroll
           for (int r = 0; r < Len<N>::RA; ++r) {
-            const int q = j + r * Len<N>::M, c = q <= N / 2 ? q : N - q;
+            // inputs q < N / 2, then N / 2 and the mirror images q_c = N - q
+            const int q = j + r * Len<N>::M, c = 2 * r < Len<N>::RA ? q : N - q;
             const bool in_r = c < cn && row;
             z1[r] = in_r ? h1[c] : make_float2(0.f, 0.f);
-            z2[r] = in_r ? h1[A.Cp + c] : make_float2(0.f, 0.f);
+            z2[r] = in_r ? h1[Cp + c] : make_float2(0.f, 0.f);
           }
 #pragma unroll
           for (int r = 0; r < Len<N>::RA; ++r) {
-            const int q = j + r * Len<N>::M;
-            if (q == 0 || 2 * q == N)
-              in[r] = make_float2(z1[r].x, z2[r].x);
-            else if (2 * q < N)
+            if (2 * r < Len<N>::RA)
               in[r] = make_float2(z1[r].x - z2[r].y, z1[r].y + z2[r].x);   // Z1 + i Z2
             else
               in[r] = make_float2(z1[r].x + z2[r].y, -z1[r].y + z2[r].x);  // conj(Z1) + i conj(Z2)
+            if ((r == 0 || 2 * r == Len<N>::RA) && j == 0)                 // q = 0 or N / 2: real
+              in[r] = make_float2(z1[r].x, z2[r].x);
           }
         },
+        [&] { fetch(u + gridDim.x * kWarps); },
         [&](bool on, int line, int k, const float2* v) {
           const bool odd = k & 1;
           const int y = 2 * line + (odd ? 1 : 0);
           on = on && ((N / 2) % L == 0 || y0 + y < N);
+          // point o = z & ~1 of the row at chunk o >> 7; the row's later points are RA q further
           const int64_t o = row0 + (int64_t)y * N + (k & ~1);
+          float* fp = field + o;
+          const int o127 = (int)(o & 127), cs = 256 * A.split_shells, lo_plane = 128 * A.split_shells;
+          __nv_bfloat16* hp = A.split + (o >> 7) * (int64_t)cs + sh * 128;
 #pragma unroll
           for (int q = 0; q < Len<N>::RB; ++q) {
             const float got = __shfl_xor_sync(0xffffffffu, odd ? v[q].x : v[q].y, 1);
             const float2 f = odd ? make_float2(got, v[q].y) : make_float2(v[q].x, got);
-            const int64_t pt = o + Len<N>::RA * q;
-            if (on && fp32) *reinterpret_cast<float2*>(field + pt) = f;
+            if (on && fp32) *reinterpret_cast<float2*>(fp + Len<N>::RA * q) = f;
             if (on && planes) {
               const __nv_bfloat162 hi = __floats2bfloat162_rn(f.x, f.y);
               const float2 fb = __bfloat1622float2(hi);
               const __nv_bfloat162 lo = __floats2bfloat162_rn(f.x - fb.x, f.y - fb.y);
-              *reinterpret_cast<__nv_bfloat162*>(A.split + split_index(0, sh, pt, A.split_shells)) = hi;
-              *reinterpret_cast<__nv_bfloat162*>(A.split + split_index(1, sh, pt, A.split_shells)) = lo;
+              // rows of a multiple of 128 points start a chunk: which one z is in is a constant
+              const int e = N % 128 == 0 && 128 % Len<N>::RA == 0
+                                ? (Len<N>::RA * q >> 7) * cs + (Len<N>::RA * q & 127) + o127
+                                : (o127 + Len<N>::RA * q >> 7) * cs + (o127 + Len<N>::RA * q & 127);
+              *reinterpret_cast<__nv_bfloat162*>(hp + e) = hi;
+              *reinterpret_cast<__nv_bfloat162*>(hp + e + lo_plane) = lo;
             }
           }
         });
@@ -481,35 +533,42 @@ __global__ void __launch_bounds__(32 * kWarps, min_blocks<N>())
 template <int N>
 void run_passes(const SynthArgs& A, const FftPlan& pl, cudaStream_t st) {
   constexpr int LX = lines_xy<N>(), LZ = lines_z<N>();
-  constexpr size_t sxy = pass_smem<N, LX, true>(), sz = pass_smem<N, LZ, false>();
-  static std::atomic<int> per_sm[64][3];  // resident blocks an SM (0: not asked yet)
-  int dev = 0, nsm = 0;
+  const size_t smem[3] = {
+      pass_smem<N, LX, true>(),
+      pass_smem<N, LX, true>() + (size_t)kWarps * LX * A.nk * sizeof(float2),
+      pass_smem<N, LZ, false>() + (size_t)kWarps * 2 * LZ * A.Cp * sizeof(float2)};
+  int dev = 0, nsm = 0, sm_bytes = 0, reserved = 0;
   BSK_CHECK_CUDA(cudaGetDevice(&dev));
   BSK_REQUIRE(dev < 64, BSK_ERR_UNSUPPORTED, "device ordinal above 63");
   BSK_CHECK_CUDA(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev));
+  BSK_CHECK_CUDA(cudaDeviceGetAttribute(&sm_bytes, cudaDevAttrMaxSharedMemoryPerMultiprocessor, dev));
+  BSK_CHECK_CUDA(cudaDeviceGetAttribute(&reserved, cudaDevAttrReservedSharedMemoryPerBlock, dev));
   const void* kern[3] = {(const void*)x_kernel<N>, (const void*)y_kernel<N>,
                          (const void*)z_kernel<N>};
-  if (!per_sm[dev][2]) {
+  // blocks an SM holds by registers (0: not asked yet)
+  static std::atomic<int> by_regs[64][3];
+  if (!by_regs[dev][2])
     for (int k = 0; k < 3; ++k) {
-      const size_t smem = k == 2 ? sz : sxy;
       BSK_CHECK_CUDA(cudaFuncSetAttribute(kern[k], cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                          (int)smem));
+                                          227 * 1024));
       int n = 0;
-      BSK_CHECK_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, kern[k], 32 * kWarps, smem));
-      per_sm[dev][k] = std::max(n, 1);
+      BSK_CHECK_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, kern[k], 32 * kWarps, 0));
+      by_regs[dev][k] = n;
     }
-  }
+  // persistent passes: as many blocks as are resident at once
   const auto grid = [&](int k, int units) {
-    return std::max(1, std::min((units + kWarps - 1) / kWarps, per_sm[dev][k] * nsm));
+    const int fit = std::min<int>(by_regs[dev][k], sm_bytes / (int)(smem[k] + reserved));
+    BSK_REQUIRE(fit > 0, BSK_ERR_STATE, "internal: a synthesis pass does not fit an SM");
+    return std::max(1, std::min((units + kWarps - 1) / kWarps, fit * nsm));
   };
   const int runs = (A.R + LX) / LX;  // q_c = 0 .. R
   const int xu = A.ns * A.nk * runs, yu = A.ns * N * runs;
   const int zruns = (N / 2 + LZ - 1) / LZ, zu = A.ns * N * zruns;
-  x_kernel<N><<<grid(0, xu), 32 * kWarps, sxy, st>>>(A, pl, runs, xu);
+  x_kernel<N><<<grid(0, xu), 32 * kWarps, smem[0], st>>>(A, pl, runs, xu);
   BSK_CHECK_CUDA(cudaGetLastError());
-  y_kernel<N><<<grid(1, yu), 32 * kWarps, sxy, st>>>(A, pl, runs, yu);
+  y_kernel<N><<<grid(1, yu), 32 * kWarps, smem[1], st>>>(A, pl, runs, yu);
   BSK_CHECK_CUDA(cudaGetLastError());
-  z_kernel<N><<<grid(2, zu), 32 * kWarps, sz, st>>>(A, pl, zruns, zu);
+  z_kernel<N><<<grid(2, zu), 32 * kWarps, smem[2], st>>>(A, pl, zruns, zu);
   BSK_CHECK_CUDA(cudaGetLastError());
 }
 
