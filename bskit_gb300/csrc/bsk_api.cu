@@ -198,6 +198,21 @@ void make_range(bsk_plan* p) {
   const size_t q1 = p->qmax + 1;
   p->range = (uint32_t*)dmalloc((size_t)p->n * q1 * q1 * sizeof(uint32_t));
   launch_shell_range(p, p->range, nullptr, 0);
+  p->d_radius = (int*)dmalloc((size_t)p->n * sizeof(int));
+  BSK_CHECK_CUDA(cudaMemcpy(p->d_radius, p->shell_r.data(), (size_t)p->n * sizeof(int),
+                            cudaMemcpyHostToDevice));
+}
+
+// Shells per synthesis launch: the FFT batch, or more on a small grid, as long as the workspace
+// stays within kSmallWorkspace (96^3, 15 shells: one launch a pass instead of two that half
+// fill the GPU).  Under a memory budget the batch, whose workspace the budget was sized for.
+constexpr size_t kSmallWorkspace = (size_t)256 << 20;
+void size_synth(bsk_plan* p, size_t mem_budget) {
+  p->synth_batch = p->chunk;
+  while (!mem_budget && p->synth_batch < p->n &&
+         synth_workspace_bytes(p->Ng, p->qmax, p->synth_batch + 1) <= kSmallWorkspace)
+    ++p->synth_batch;
+  p->synth_ws_bytes = synth_workspace_bytes(p->Ng, p->qmax, p->synth_batch);
 }
 
 void release_stream(bsk_plan* p) {
@@ -247,11 +262,11 @@ void ensure_fields(bsk_plan* p, int s, cudaStream_t st, bool with_split = false,
     }
     if (with_split) alloc_split(p, f);
     int done = 0;
-    for (int s0 = 0; s0 < need; s0 += p->chunk) {
-      const int ns = std::min(p->chunk, p->n - s0);
+    for (int s0 = 0; s0 < need; s0 += p->synth_batch) {
+      const int ns = std::min(p->synth_batch, p->n - s0);
       int R = 0;
       for (int k = s0; k < s0 + ns; ++k) R = std::max(R, p->shell_r[k]);
-      launch_synth(p->Ng, f.spec, p->table, p->range, p->qmax + 1, s0, ns, R, p->synth_ws, f.fields,
+      launch_synth(p->Ng, f.spec, p->table, p->range, p->d_radius, p->qmax + 1, s0, ns, R, p->synth_ws, f.fields,
                    with_split ? f.split : nullptr, p->n_alloc(), st);
       done = s0 + ns;
     }
@@ -261,6 +276,7 @@ void ensure_fields(bsk_plan* p, int s, cudaStream_t st, bool with_split = false,
     if (with_split) {
       f.split_ok = true;
       f.split_n = done;
+      f.split_from = 0;
     }
     return;
   }
@@ -284,26 +300,31 @@ void ensure_split(bsk_plan* p, int s, cudaStream_t st, int n_need = -1) {
   FieldSlot& f = p->slot[s];
   const int need = n_need < 0 ? p->n : std::min(n_need, p->n);
   ensure_fields(p, s, st, true, n_need);
-  if (f.split_ok && f.split_n >= need) return;
+  if (f.split_ok && f.split_n >= need && f.split_from == 0) return;
   alloc_split(p, f);
   launch_split(f.fields, p->n_alloc(), p->K, f.split, st);  // FP32 valid from shell 0
   f.split_ok = true;
   f.split_n = p->n;
+  f.split_from = 0;
 }
 
 // A grid level's slot for shells [0, nn): the FP32 fields of shells >= fp_from (the pair
-// factors of its bins; nn when the slot is not a pair factor) and, when `need_split`, the
-// bf16 split of all of them (the column operand), in one synthesis pass per batch; batches
-// that hold neither are skipped.
-void ensure_level_fields(bsk_plan* q, int s, cudaStream_t st, int nn, int fp_from,
-                         bool need_split) {
+// factors of its bins; nn when the slot is not a pair factor) and the bf16 split of shells
+// [col_from, col_to) (its third shells; an empty range when the slot is no column operand), in
+// one synthesis pass per batch; batches that hold neither are skipped.  (On the 512^3 headline
+// the 384^3 level's bins use no shell below 16 and the 288^3 level's no third shell above 46:
+// two batches less of 384^3 and a quarter of the 288^3 planes.)
+void ensure_level_fields(bsk_plan* q, int s, cudaStream_t st, int nn, int fp_from, int col_from,
+                         int col_to) {
   FieldSlot& f = q->slot[s];
   BSK_REQUIRE(f.painted, BSK_ERR_STATE, "field slot " + std::to_string(s) + " was not painted");
   nn = std::min(nn, q->n);
   fp_from = std::min(fp_from, nn);
+  const bool need_split = col_from < col_to;
   const bool fp_ok = fp_from >= nn || (f.fields_ok && f.fields_from <= fp_from &&
                                        f.fields_n >= nn);
-  const bool split_ok = !need_split || (f.split_ok && f.split_n >= nn);
+  const bool split_ok = !need_split ||
+                        (f.split_ok && f.split_from <= col_from && f.split_n >= col_to);
   if (fp_ok && split_ok) return;
   if (!f.fields && fp_from < nn) {  // a column-only slot needs no FP32 fields
     check_budget(q, (size_t)q->n_alloc() * q->K * sizeof(float), "the shell fields");
@@ -318,23 +339,25 @@ void ensure_level_fields(bsk_plan* q, int s, cudaStream_t st, int nn, int fp_fro
     synth_init_workspace(q->Ng, q->synth_ws);
   }
   if (need_split) alloc_split(q, f);
-  const int from = need_split ? 0 : fp_from / q->chunk * q->chunk;
-  int done = from;
-  for (int s0 = from; s0 < nn; s0 += q->chunk) {
-    const int ns = std::min(q->chunk, q->n - s0);
+  const int first = need_split ? std::min(fp_from, col_from) : fp_from;
+  for (int s0 = first / q->chunk * q->chunk; s0 < nn; s0 += q->synth_batch) {
+    const int ns = std::min(q->synth_batch, q->n - s0);
+    const bool cols = s0 < col_to && s0 + ns > col_from;
+    if (!cols && s0 + ns <= fp_from) continue;
     int R = 0;
     for (int k = s0; k < s0 + ns; ++k) R = std::max(R, q->shell_r[k]);
-    launch_synth(q->Ng, f.spec, q->table, q->range, q->qmax + 1, s0, ns, R, q->synth_ws,
-                 f.fields, need_split ? f.split : nullptr, q->n_alloc(), st, 0, fp_from);
-    done = s0 + ns;
+    launch_synth(q->Ng, f.spec, q->table, q->range, q->d_radius, q->qmax + 1, s0, ns, R,
+                 q->synth_ws, f.fields, cols ? f.split : nullptr, q->n_alloc(), st, 0, fp_from,
+                 col_to);
   }
   // what this pass wrote replaces what the slot held
   f.fields_ok = fp_from < nn;
   f.fields_from = fp_from;
-  f.fields_n = done;
+  f.fields_n = nn;
   if (need_split) {
     f.split_ok = true;
-    f.split_n = done;
+    f.split_from = col_from;
+    f.split_n = col_to;
   }
 }
 
@@ -365,6 +388,7 @@ void destroy_plan(bsk_plan* p) {
   for (auto& s : p->slot) free_slot(s);
   if (p->table) cudaFree(p->table);
   if (p->range) cudaFree(p->range);
+  if (p->d_radius) cudaFree(p->d_radius);
   if (p->d_edges) cudaFree(p->d_edges);
   if (p->chunk_spec) cudaFree(p->chunk_spec);
   if (p->cic_w) cudaFree(p->cic_w);
@@ -466,7 +490,7 @@ void chunk_fields(bsk_plan* p, int slot, int s0, int C, float* dst, cudaStream_t
       }
       int R = 0;
       for (int k = first; k < first + ns; ++k) R = std::max(R, p->shell_r[k]);
-      launch_synth(p->Ng, f.spec, p->table, p->range, p->qmax + 1, first, ns, R, p->synth_ws,
+      launch_synth(p->Ng, f.spec, p->table, p->range, p->d_radius, p->qmax + 1, first, ns, R, p->synth_ws,
                    dst, nullptr, 0, st, s0);
       if (ns < p->chunk)
         BSK_CHECK_CUDA(cudaMemsetAsync(dst + (size_t)(b + ns) * p->K, 0,
@@ -637,7 +661,7 @@ bsk_plan* level_plan(bsk_plan* p, int Ng, int n) {
               "internal: a grid level's shell table disagrees with its plan");
   q->use_synth = synth_supported(Ng);
   BSK_REQUIRE(q->use_synth, BSK_ERR_STATE, "internal: no field synthesis for a grid level");
-  q->synth_ws_bytes = synth_workspace_bytes(Ng, q->qmax, q->chunk);
+  size_synth(q.get(), p->mem_budget);
   make_range(q.get());
   p->levels.push_back(q.get());
   return q.release();
@@ -658,7 +682,7 @@ void sync_level(bsk_plan* p, bsk_plan* q, int s, cudaStream_t st) {
   qf.gen = pf.gen;
   qf.fields_ok = false;
   qf.split_ok = false;
-  qf.fields_n = qf.split_n = qf.fields_from = 0;
+  qf.fields_n = qf.split_n = qf.fields_from = qf.split_from = 0;
 }
 
 // Grid sides the levels may take (below the plan's own): the sizes whose field synthesis is
@@ -702,7 +726,12 @@ void build_levels(bsk_plan* p, bsk_triset* set) {
     GridLevel lv;
     lv.n_shells = top + 1;
     lv.src_min = top + 1;
-    for (const HostTriangle& h : tk) lv.src_min = std::min(lv.src_min, std::min(h.i, h.j));
+    lv.col_min = top + 1;
+    for (const HostTriangle& h : tk) {
+      lv.src_min = std::min(lv.src_min, std::min(h.i, h.j));
+      lv.col_min = std::min(lv.col_min, h.l);
+      lv.col_end = std::max(lv.col_end, h.l + 1);
+    }
     lv.bins = (int64_t)tk.size();
     lv.plan = j == m - 1 ? p : level_plan(p, sides[j], top + 1);
     set->levels.push_back(lv);
@@ -755,14 +784,16 @@ void measure_levels(bsk_plan* p, const bsk_triset* set, int a, int b, int c, int
       if (c != a && c != b) sync_level(p, q, c, st);
     }
     // tensor-core paths read FP32 fields only as pair factors (shells >= the level's smallest
-    // i or j) and the split of slot c; the SIMT paths read FP32 fields of every shell
+    // i or j) and the split of slot c; the SIMT paths read FP32 fields of every shell they use
     const int sls[3] = {a, b, c};
     for (int k = 0; k < 3; ++k) {
       const int sl = sls[k];
       if ((k >= 1 && sl == sls[0]) || (k == 2 && sl == sls[1])) continue;  // done already
       const bool factor = sl == a || sl == b;
-      const int fp_from = !tc ? 0 : factor ? lv.src_min : nn;
-      ensure_level_fields(q, sl, st, nn, fp_from, tc && sl == c);
+      const int fp_from = !tc ? std::min(lv.src_min, lv.col_min) : factor ? lv.src_min : nn;
+      const bool column = tc && sl == c;
+      ensure_level_fields(q, sl, st, nn, fp_from, column ? lv.col_min : nn,
+                          column ? lv.col_end : nn);
     }
     BSK_REQUIRE(q->slot[a].fields && q->slot[b].fields &&
                     (tc ? q->slot[c].split != nullptr : q->slot[c].fields != nullptr),
@@ -1050,7 +1081,7 @@ int bsk_plan_create(int nmesh, double box_size, int n_shells, const double* shel
     }
     p->use_synth = synth_supported(p->Ng);
     if (p->use_synth) {
-      p->synth_ws_bytes = synth_workspace_bytes(p->Ng, qmax, p->chunk);
+      size_synth(p.get(), mem_budget);
       make_range(p.get());
     }
     p->use_levels = grid_mode == BSK_GRID_REDUCED && p->Ng != p->N && p->use_synth;

@@ -138,7 +138,8 @@ struct FieldSlot {
   bool split_ok = false;
   int fields_n = 0;               // the FP32 fields of shells [fields_from, fields_n) are valid
   int fields_from = 0;            // (0 unless a grid level only needed the later shells)
-  int split_n = 0;                // the split of shells [0, split_n) is valid
+  int split_n = 0;                // the split of shells [split_from, split_n) is valid
+  int split_from = 0;             // (0 unless a grid level only needed the later shells)
   int64_t gen = 0;                // bumped by every paint (keys of streamed fields); on a grid
                                   // level's plan: the parent paint its spectrum was taken from
 };
@@ -151,6 +152,7 @@ struct GridLevel {
   DeviceSchedule sched;   // map entries are positions in the set's output
   int n_shells = 0;       // shells [0, n_shells) the level's bins use
   int src_min = 0;        // smallest shell of the level's bins used as a pair factor (i or j)
+  int col_min = 0, col_end = 0;  // the third shells l lie in [col_min, col_end)
   int64_t bins = 0;
 };
 
@@ -171,6 +173,7 @@ struct bsk_plan {
   int64_t Mh = 0;       // Ng*Ng*(Ng/2+1) half-complex modes
   uint16_t* table = nullptr;  // device [Mh] shell code
   uint32_t* range = nullptr;  // device [n][qmax + 1]^2, the shells' |q_a| intervals
+  int* d_radius = nullptr;    // device [n], shell_r
   double* d_edges = nullptr;  // device [2n]
   cufftHandle r2c = 0;        // N^3 R2C
   bool r2c_ok = false;
@@ -196,6 +199,7 @@ struct bsk_plan {
   // field synthesis (pruned FFT passes) instead of filter + cuFFT C2R
   bool use_synth = false;
   std::vector<int> shell_r;             // largest |q_c| of a mode in each shell
+  int synth_batch = 0;                  // shells per synthesis launch (>= chunk)
   void* synth_ws = nullptr;             // twiddles + X / Y pass intermediates of one batch
   size_t synth_ws_bytes = 0;
   // grid levels: smaller contraction grids for bins of small shells (owned by the plan);
@@ -263,7 +267,7 @@ size_t synth_workspace_bytes(int n, int max_r, int batch);
 // Twiddle table at the start of the workspace (synchronous; once, after allocation).
 void synth_init_workspace(int n, void* work);
 void launch_synth(int N, const cufftComplex* spec, const uint16_t* table, const uint32_t* range,
-                  int q1, int s0, int ns, int R, void* work, float* fields,
+                  const int* radius, int q1, int s0, int ns, int R, void* work, float* fields,
                   __nv_bfloat16* split, int split_shells, cudaStream_t st, int out_s0 = 0,
                   int fields_from = 0, int split_to = 1 << 30);
 // FP32 fields [S][K] -> their chunk-major bf16 hi / lo split (split_elems(S, K) values,

@@ -419,7 +419,7 @@ void synth_init_workspace(int N, void* work) {
 }
 
 void launch_synth(int N, const cufftComplex* spec, const uint16_t* table, const uint32_t* range,
-                  int q1, int s0, int ns, int R, void* work, float* fields,
+                  const int* radius, int q1, int s0, int ns, int R, void* work, float* fields,
                   __nv_bfloat16* split, int split_shells, cudaStream_t st, int out_s0,
                   int fields_from, int split_to) {
   FftPlan pl;
@@ -441,6 +441,7 @@ void launch_synth(int N, const cufftComplex* spec, const uint16_t* table, const 
   A.spec = reinterpret_cast<const float2*>(spec);
   A.table = table;
   A.range = range;
+  A.radius = radius;
   A.q1 = q1;
   float2* tw = reinterpret_cast<float2*>(work);
   A.G = tw + N;

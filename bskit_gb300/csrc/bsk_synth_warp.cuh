@@ -194,6 +194,7 @@ struct SynthArgs {
   int fields_from;         // the FP32 field is written for shells s0 + s >= fields_from only
   const float2* spec;      // [a][b][c] slot spectrum
   const uint16_t* table;   // [a][b][c] shell codes (run-time lengths)
+  const int* radius;       // [shell] largest |q_c| of each shell, at most R of the batch's
   const uint32_t* range;   // [shell][|b|][c] |q_a| interval (compiled lengths), q1 values an axis
   int q1;
   float2* G;               // [s][x][bk][c]   (c < Cp)
@@ -317,6 +318,7 @@ __device__ __forceinline__ void cp_async16(void* dst, const void* src) {
 }
 
 constexpr int kWarps = 4;                      // warps a block
+constexpr int kStagePad = 8;                   // staged rows of the Z pass fall on both bank halves
 template <int N>
 constexpr int lines_xy() { return N <= 192 ? 8 : 4; }  // 64- or 32-byte runs of q_c
 template <int N>
@@ -346,9 +348,10 @@ __global__ void __launch_bounds__(32 * kWarps, min_blocks<N>())
     const int run = u % runs, v = u / runs, bk = v % nk, s = v / nk;
     const int b = kept_index(bk, nk, A.R, N);
     const int c = run * L + lane % L;  // this lane's column in both stages (32 is a multiple of L)
-    const int ab = b <= N / 2 ? b : N - b;
+    const int ab = b <= N / 2 ? b : N - b, R = A.radius[A.s0 + s];
+    if (ab > R || run * L > R) continue;  // the Y pass does not read it
     uint32_t rg = kEmptyRange;
-    if (c <= A.R && c < A.H) rg = A.range[((int64_t)(A.s0 + s) * A.q1 + ab) * A.q1 + c];
+    if (c <= R) rg = A.range[((int64_t)(A.s0 + s) * A.q1 + ab) * A.q1 + c];
     const int a0 = (int)(rg & 0xFFFF), a1 = (int)(rg >> 16);
     float2* g = A.G + (((int64_t)s * N) * nk + bk) * A.Cp + c;
     const int64_t xs = (int64_t)nk * A.Cp;
@@ -389,14 +392,18 @@ __global__ void __launch_bounds__(32 * kWarps, min_blocks<N>())
   __syncthreads();
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   float2* buf = sm + warp * L * LP;
-  const int nk = A.nk, R = A.R;
+  const int nk = A.nk;
   float2* stage = sm + pass_smem<N, L, true>() / sizeof(float2) + warp * L * nk;
   auto fetch = [&](int u) {
     if (u < units) {
-      const int run = u % runs, sx = u / runs;
+      const int run = u % runs, sx = u / runs, R = A.radius[A.s0 + sx / N];
       const float2* src = A.G + (int64_t)sx * nk * A.Cp + run * L;
-      for (int i = lane; i < nk * (L / 2); i += 32) {
-        const int bk = i / (L / 2), e = i % (L / 2) * 2;
+      // rows |q_b| <= R of the shell (in an array of all N frequencies, q_b < 0 comes last)
+      const int lo = nk == N ? 0 : A.R - R, n_rows = run * L > R ? 0 : min(2 * R + 1, nk);
+      for (int i = lane; i < n_rows * (L / 2); i += 32) {
+        int bk = lo + i / (L / 2);
+        const int e = i % (L / 2) * 2;
+        if (nk == N && bk > R) bk += N - n_rows;
         cp_async16(stage + bk * L + e, src + bk * A.Cp + e);
       }
     }
@@ -405,7 +412,12 @@ __global__ void __launch_bounds__(32 * kWarps, min_blocks<N>())
   fetch(blockIdx.x * kWarps + warp);
   for (int u = blockIdx.x * kWarps + warp; u < units; u += gridDim.x * kWarps) {
     const int run = u % runs, sx = u / runs;  // sx = s N + x
-    const int c = run * L + lane % L;
+    const int c = run * L + lane % L, R = A.radius[A.s0 + sx / N], RB = A.R;
+    if (run * L > R) {  // columns past the shell: the Z pass does not read them
+      __syncwarp();
+      fetch(u + gridDim.x * kWarps);
+      continue;
+    }
     float2* h = A.Hh + (int64_t)sx * N * A.Cp + c;
     asm volatile("cp.async.wait_group 0;" ::: "memory");
     __syncwarp();
@@ -416,8 +428,8 @@ __global__ void __launch_bounds__(32 * kWarps, min_blocks<N>())
           for (int r = 0; r < Len<N>::RA; ++r) {
             // the first half of the inputs are q_b >= 0, the second q_b = q - N < 0
             const int q = j + r * Len<N>::M;
-            const bool kept = nk == N || (2 * r < Len<N>::RA ? q <= R : q >= N - R);
-            const int bk = nk == N ? q : 2 * r < Len<N>::RA ? q + R : q - N + R;
+            const bool kept = 2 * r < Len<N>::RA ? q <= R : q >= N - R;
+            const int bk = nk == N ? q : 2 * r < Len<N>::RA ? q + RB : q - N + RB;
             in[r] = kept ? stage[bk * L + lane % L] : make_float2(0.f, 0.f);
           }
         },
@@ -448,25 +460,29 @@ __global__ void __launch_bounds__(32 * kWarps, min_blocks<N>())
   __syncthreads();
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   float2* buf = sm + warp * L * LP;
-  const int Cp = A.Cp;
-  float2* stage = sm + pass_smem<N, L, false>() / sizeof(float2) + warp * 2 * L * Cp;
+  const int Cp = A.Cp, sp = Cp + kStagePad;
+  float2* stage = sm + pass_smem<N, L, false>() / sizeof(float2) + warp * 2 * L * sp;
   auto fetch = [&](int u) {
     if (u < units) {
       // rows y0 .. y0 + 2 L - 1 of (shell, x); a ragged last unit has fewer
       const int run = u % runs, sx = u / runs;
       const int rows = min(2 * L, N - run * 2 * L);
       const float2* src = A.Hh + ((int64_t)sx * N + run * 2 * L) * Cp;
-      for (int i = lane * 2; i < rows * Cp; i += 64) cp_async16(stage + i, src + i);
+      constexpr int per_row = 32 / (2 * L);  // lanes a row, 16 bytes each
+      const int r = lane / per_row, R = A.radius[A.s0 + sx / N];
+      if (r < rows)
+        for (int c = lane % per_row * 2; c <= R; c += 2 * per_row)
+          cp_async16(stage + r * sp + c, src + r * Cp + c);
     }
     asm volatile("cp.async.commit_group;" ::: "memory");
   };
   fetch(blockIdx.x * kWarps + warp);
-  const int cn = min(A.R, N / 2) + 1;  // q_c = 0 .. cn - 1 can be nonzero
   constexpr int64_t K = (int64_t)N * N * N;
   for (int u = blockIdx.x * kWarps + warp; u < units; u += gridDim.x * kWarps) {
     const int run = u % runs, sx = u / runs;
     const int s = sx / N, x = sx - s * N;
     const int y0 = run * 2 * L;  // first of the unit's 2 L rows
+    const int cn = min(A.radius[A.s0 + s], N / 2) + 1;  // q_c = 0 .. cn - 1 can be nonzero
     const int sh = A.s0 + s - A.out0;  // shell index in the output arrays
     const bool fp32 = A.s0 + s >= A.fields_from;
     const bool planes = A.split && A.s0 + s < A.split_to;
@@ -477,7 +493,7 @@ __global__ void __launch_bounds__(32 * kWarps, min_blocks<N>())
     warp_fft<N, L, false>(
         buf, tw, pl,
         [&](int line, int j, float2* in) {
-          const float2* h1 = stage + 2 * line * Cp;
+          const float2* h1 = stage + 2 * line * sp;
           const bool row = (N / 2) % L == 0 || y0 + 2 * line < N;
           float2 z1[Len<N>::RA], z2[Len<N>::RA];
 #pragma unroll
@@ -486,7 +502,7 @@ __global__ void __launch_bounds__(32 * kWarps, min_blocks<N>())
             const int q = j + r * Len<N>::M, c = 2 * r < Len<N>::RA ? q : N - q;
             const bool in_r = c < cn && row;
             z1[r] = in_r ? h1[c] : make_float2(0.f, 0.f);
-            z2[r] = in_r ? h1[Cp + c] : make_float2(0.f, 0.f);
+            z2[r] = in_r ? h1[sp + c] : make_float2(0.f, 0.f);
           }
 #pragma unroll
           for (int r = 0; r < Len<N>::RA; ++r) {
@@ -536,7 +552,7 @@ void run_passes(const SynthArgs& A, const FftPlan& pl, cudaStream_t st) {
   const size_t smem[3] = {
       pass_smem<N, LX, true>(),
       pass_smem<N, LX, true>() + (size_t)kWarps * LX * A.nk * sizeof(float2),
-      pass_smem<N, LZ, false>() + (size_t)kWarps * 2 * LZ * A.Cp * sizeof(float2)};
+      pass_smem<N, LZ, false>() + (size_t)kWarps * 2 * LZ * (A.Cp + kStagePad) * sizeof(float2)};
   int dev = 0, nsm = 0, sm_bytes = 0, reserved = 0;
   BSK_CHECK_CUDA(cudaGetDevice(&dev));
   BSK_REQUIRE(dev < 64, BSK_ERR_UNSUPPORTED, "device ordinal above 63");

@@ -1,0 +1,54 @@
+"""Grid levels synthesise only the shells their bins use: sets that use different shells of one
+painted mesh, measured in any order on one plan, give what each gives on a plan of its own.
+
+The contractions are the same ones on the same fields, so only the FP64 order of the slices'
+sums may differ: relative to the largest bin, a few thousand slices x 2^-53.
+"""
+import itertools
+
+import numpy as np
+import pytest
+import torch
+
+from bskit_gb300 import bins as B
+from bskit_gb300.engine import Plan
+from bskit_gb300 import synthetic
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("precision", ["bf16x3", "fp32"])
+def test_sets_of_different_shells(cuda, monkeypatch, precision):
+    monkeypatch.setenv("BSK_LEVEL_MIN_POINTS", "0.2")  # at least two levels on 256^3
+    n, box = 256, 500.0
+    kf = 2 * np.pi / box
+    kw = dict(kmin=kf, kmax=64 * kf, dk=2 * kf)
+    edges = B.generate_bin_edge_list(**kw)
+    tri = B.generate_triangle_bin_list(return_indices=True, **kw)
+    high = tri[tri[:, 2] >= 18]                       # no small shell at all
+    equal = B.generate_equilateral_triangle_bin_list(return_indices=True, **kw)
+    d = synthetic.lognormal_mesh_torch(n, box, seed=3, device=cuda).contiguous()
+    e = (1.5 * d + 0.3 * torch.randn_like(d)).contiguous()
+    sets = {"all": (tri, (0, 0, 0)), "high": (high, (0, 0, 0)), "equal": (equal, (0, 0, 1)),
+            "cross": (high, (1, 0, 1))}
+
+    def paint(p):
+        p.paint(0, d)
+        p.paint(1, e)
+
+    want = {}
+    for k, (t, slots) in sets.items():
+        p = Plan(n, box, edges)
+        paint(p)
+        want[k] = p.measure_b(p.triangles(t), slots=slots, precision=precision)
+        p.close()
+    p = Plan(n, box, edges)
+    made = {k: p.triangles(t) for k, (t, _) in sets.items()}
+    assert len(made["all"].levels()) >= 2
+    for order in itertools.permutations(sets):
+        paint(p)
+        for k in order + order[:1]:
+            got = p.measure_b(made[k], slots=sets[k][1], precision=precision)
+            assert torch.all((got - want[k]).abs() <= 4096 * 2.0 ** -53 * want[k].abs().max()), \
+                (order, k)
+    p.sync_check()
