@@ -10,6 +10,9 @@
 // atomics (only entries that are triangle bins); warps whose 16 x 32 entries hold
 // no bin skip the multiply-adds.  Items are ordered slice-major
 // so that blocks running at the same time share field data in L2.
+#include <algorithm>
+#include <type_traits>
+
 #include "bsk_internal.cuh"
 
 namespace bsk {
@@ -140,40 +143,53 @@ __global__ void __launch_bounds__(THREADS) contract_simt_kernel(
 }
 
 // ---------------------------------------------------------------- plain FP32 path
-// Work item = (tile of 128 pair rows x up to 64 column shells, 8192-point slice).  Per
-// 32-point chunk the block copies the tile's source rows (coalesced) and its column rows
-// into shared memory, forms the 128 x 32 pair products P = F1_i F2_j there, and each warp
-// runs a 32-row x 32-column block of the outer product, 8 rows x 4 columns per thread
-// (two 16-byte loads of P and one of F3 per 32 FMAs).  Warps whose 32 columns lie past the
-// tile's nc skip their multiply-adds.  FP32 sums over the slice, FP64 atomics across slices.
+// FP32 pair products P = F1_i F2_j, FP32 multiply-adds in point order over 8192-point slices,
+// FP64 atomics across slices; one warp per (8 TR rows x 4 TC columns of a tile, slice).  No
+// block barriers: a block is one warp.  Source and column rows of the next chunks are copied
+// with cp.async (16 bytes; 4 where a shard's range starts off a 16-byte boundary) while the
+// current chunk is formed and multiplied.
+//
+// Long grids (TR = 16: all 128 rows x up to 32 columns).  Operand loads bound the outer
+// product: a float delivered to a warp costs a shared-memory wavefront whatever is broadcast,
+// so a thread tile of R rows x C columns costs (R + C) / (R C) wavefronts a multiply-add: 0.19
+// for 16 x 8, 0.375 for the 8 x 4 that four warps sharing the tile have.  Columns come in the
+// tile's own width, multiply-adds packed by two rows (fma.rn.f32x2).  250 registers, eight
+// warps an SM (168 or 200 of them spill: +60%).  256^3 (31 shells, 3 tiles): 4.15 ms, where a
+// block of four warps a tile took 6.5.
+//
+// Short grids (TR = 4: 32 rows x up to 16 columns).  A slice is a chain of 8192 dependent
+// multiply-adds an entry, so with few items the chain's pace is the time (48^3, 14 items: 144
+// cycles a point with four warps and three barriers a chunk, 623 us): more, smaller items, and
+// copies three chunks ahead (250 us).  Forming the next chunk's products before the current
+// chunk's multiply-adds, to save a barrier, was 7% slower.
 namespace f32 {
-// The plain-FP32 path: work item = (tile of 128 pair rows x nc <= 64 columns, 8192-point
-// slice), one block of 128 threads.  Per 32-point chunk the block forms the 128 x 32 pair
-// products once in shared memory and runs a register-tiled outer product
-// C[r][c] += P[r][x] F3[c][x]; each thread holds 8 rows x CB columns, CB = 4, 6 or 8 chosen
-// per tile (tile widths 32, 48, 64).  The operand loads of the outer product, not the
-// multiply-adds, bound this kernel: a warp's 128-bit shared-memory load costs four wavefronts
-// whatever its broadcast, so the 8 x 8 thread tile (16 values loaded per 64 multiply-adds)
-// is what raises the arithmetic per wavefront.  The next chunk's source and column rows are
-// copied global -> shared with cp.async into the other half of a double buffer while the
-// current chunk is computed.
-constexpr int KC = 32;
-constexpr int THREADS = 128;
-constexpr int ROWS = 128, COLS = 64, SRC = 64;
-constexpr int APITCH = ROWS + 4;    // A[x][r]
-constexpr int BPITCH = COLS + 4;    // B[x][c]
-constexpr int SPITCH = KC + 1;      // S[row][x]
+constexpr int ROWS = 128, COLS = 32, SRC = 64;
 constexpr int64_t SLICE = 8192;
-constexpr int STAGE = SRC * KC / THREADS;  // values per thread and array of one chunk (16)
-static_assert(COLS == SRC, "one staging pattern for sources and columns");
 
-struct Smem {
-  float A[KC][APITCH];
-  float B[2][KC][BPITCH];
-  float S1[2][SRC][SPITCH];
-  float S2[2][SRC][SPITCH];
+template <int TR_, int KC_, int ST_, int COLS_, bool kTwoSrc_, bool kAligned_>
+struct Cfg {
+  static constexpr int TR = TR_, KC = KC_, ST = ST_;  // rows a thread, points a chunk, chunks held
+  static constexpr int COLS = COLS_;                  // columns of an item at most
+  static constexpr bool kTwoSrc = kTwoSrc_, kAligned = kAligned_;
+  static constexpr int PITCH = KC + 4;                // 16-byte pieces of 8 rows on distinct banks
+  static constexpr int APITCH = 8 * TR + 4;
+  // A[KC][APITCH] pair products of the chunk, B[ST][COLS][PITCH] column rows, then S1 and S2
+  // [ST][src][PITCH] source rows (src: the widest source range of the launch's tiles)
+  static constexpr int A_FLOATS = KC * APITCH, B_FLOATS = ST * COLS * PITCH;
+  static size_t smem(int src) {
+    return (A_FLOATS + B_FLOATS + (kTwoSrc ? 2 : 1) * ST * src * PITCH) * sizeof(float);
+  }
 };
+template <bool kTwoSrc, bool kAligned>
+using Long = Cfg<16, 8, 2, 32, kTwoSrc, kAligned>;
+template <bool kTwoSrc, bool kAligned>
+using Short = Cfg<4, 16, 4, 16, kTwoSrc, kAligned>;
 
+__device__ __forceinline__ void cp_async16(float* dst, const float* src, int bytes) {
+  const uint32_t d = (uint32_t)__cvta_generic_to_shared(dst);
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(d), "l"(src), "r"(bytes)
+               : "memory");
+}
 __device__ __forceinline__ void cp_async4(float* dst, const float* src, bool ok) {
   const uint32_t d = (uint32_t)__cvta_generic_to_shared(dst);
   asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"(d), "l"(src),
@@ -187,137 +203,191 @@ template <int N>
 __device__ __forceinline__ void cp_async_wait() {
   asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory");
 }
-
-// The outer product of one chunk: thread rows r0 .. r0 + 7, columns c0 .. c0 + CB - 1.
-template <int CB>
-__device__ __forceinline__ void fma_chunk(const float (&A)[KC][APITCH],
-                                          const float (&B)[KC][BPITCH], int r0, int c0,
-                                          float (&acc)[8][8]) {
-#pragma unroll 4
-  for (int k = 0; k < KC; ++k) {
-    const float4 a0 = *reinterpret_cast<const float4*>(&A[k][r0]);
-    const float4 a1 = *reinterpret_cast<const float4*>(&A[k][r0 + 4]);
-    const float av[8] = {a0.x, a0.y, a0.z, a0.w, a1.x, a1.y, a1.z, a1.w};
-    float bv[8];
-    if (CB == 8) {
-      const float4 b0 = *reinterpret_cast<const float4*>(&B[k][c0]);
-      const float4 b1 = *reinterpret_cast<const float4*>(&B[k][c0 + 4]);
-      bv[0] = b0.x; bv[1] = b0.y; bv[2] = b0.z; bv[3] = b0.w;
-      bv[4] = b1.x; bv[5] = b1.y; bv[6] = b1.z; bv[7] = b1.w;
-    } else if (CB == 6) {  // c0 = 6 m: 8-byte aligned
-#pragma unroll
-      for (int q = 0; q < 3; ++q) {
-        const float2 b = *reinterpret_cast<const float2*>(&B[k][c0 + 2 * q]);
-        bv[2 * q] = b.x;
-        bv[2 * q + 1] = b.y;
-      }
-      bv[6] = bv[7] = 0.f;
-    } else {
-      const float4 b0 = *reinterpret_cast<const float4*>(&B[k][c0]);
-      bv[0] = b0.x; bv[1] = b0.y; bv[2] = b0.z; bv[3] = b0.w;
-      bv[4] = bv[5] = bv[6] = bv[7] = 0.f;
-    }
-#pragma unroll
-    for (int p = 0; p < 8; ++p)
-#pragma unroll
-      for (int q = 0; q < CB; ++q) acc[p][q] = fmaf(av[p], bv[q], acc[p][q]);
-  }
+__device__ __forceinline__ unsigned long long dup2(float x) {
+  unsigned long long d;
+  asm("mov.b64 %0, {%1, %1};" : "=l"(d) : "f"(x));
+  return d;
+}
+__device__ __forceinline__ void fma2(unsigned long long& acc, unsigned long long a,
+                                     unsigned long long b) {
+  asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(acc) : "l"(a), "l"(b));
 }
 
-template <int CB>
-__device__ __forceinline__ void run_item(Smem& sm, const TileDesc& td, const int16_t* row_i,
-                                         const int16_t* row_j, const int32_t* map,
-                                         const float* f1, const float* f2, const float* f3,
-                                         int n_shells, int64_t K, int64_t x_begin, int64_t x_end,
-                                         bool one_src, double* out, double scale) {
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  // outer-product block of this warp: rows [32 warp, +32), all 8 CB columns
-  const int r0 = 32 * warp + 8 * (lane >> 3);
-  const int c0 = CB * (lane & 7);
-  // pair-product formation: row tid, all points of the chunk
-  const int ri = row_i[td.row_off + tid], rj = row_j[td.row_off + tid];
-  const int pi = ri >= 0 ? ri - td.i0 : -1, pj = ri >= 0 ? rj - td.j0 : -1;
-  // staging: value k of a thread is row (tid >> 5) + 4 k, point tid & 31 of the chunk
-  const int sx = tid & 31, srow = tid >> 5;
-  auto stage = [&](int buf, int64_t x0) {
-    const bool xin = x0 + sx < x_end;
+// Columns c0 + 4 e + (lane & 3), e < TC; rows r0 + TR (lane >> 2) .. + TR - 1.
+template <class C, int TC>
+__device__ __forceinline__ void run_item(float* sm, int src, const TileDesc& td, int r0, int c0,
+                                         const int16_t* row_i, const int16_t* row_j,
+                                         const int32_t* map, const float* f1, const float* f2,
+                                         const float* f3, int n_shells, int64_t K,
+                                         int64_t x_begin, int64_t x_end, bool one_src,
+                                         double* out, double scale) {
+  constexpr int TR = C::TR, KC = C::KC, ST = C::ST, PITCH = C::PITCH, AP = C::APITCH;
+  float* sA = sm;
+  float* sB = sA + C::A_FLOATS;
+  float* s1 = sB + C::B_FLOATS;
+  float* s2 = C::kTwoSrc && !one_src ? s1 + ST * src * PITCH : s1;
+  const int lane = threadIdx.x, cg = lane & 3, rg = lane >> 2;
+  // pair products: rows r0 + lane + 32 g
+  int p1[TR / 4], p2[TR / 4];
 #pragma unroll
-    for (int k = 0; k < STAGE; ++k) {
-      const int row = srow + 4 * k;
-      const int s1 = td.i0 + row, s2 = td.j0 + row, l = td.l0 + row;
-      const bool ok1 = row < td.ni && s1 < n_shells && xin;
-      cp_async4(&sm.S1[buf][row][sx], f1 + (ok1 ? (int64_t)s1 * K + x0 + sx : 0), ok1);
-      if (!one_src) {
-        const bool ok2 = row < td.nj && s2 < n_shells && xin;
-        cp_async4(&sm.S2[buf][row][sx], f2 + (ok2 ? (int64_t)s2 * K + x0 + sx : 0), ok2);
-      }
-      const bool okb = row < td.nc && l < n_shells && xin;
-      cp_async4(&sm.B[buf][sx][row], f3 + (okb ? (int64_t)l * K + x0 + sx : 0), okb);
+  for (int g = 0; g < TR / 4; ++g) {
+    const int at = td.row_off + r0 + lane + 32 * g;
+    const int ri = row_i[at], rj = row_j[at];
+    p1[g] = ri >= 0 ? ri - td.i0 : 0;  // rows past the tile's pairs: any (their sums are not read)
+    p2[g] = ri >= 0 ? rj - td.j0 : 0;
+  }
+  // copies of one chunk in 16-byte pieces, lanes on consecutive ones; points past the slice zero
+  auto copy_rows = [&](float* dst, const float* f, int s0, int rows, int64_t x0) {
+    constexpr int W = C::kAligned ? 4 : 1;  // points a copy
+    for (int i = lane; i < KC / W * rows; i += 32) {
+      const int row = i / (KC / W), k = i % (KC / W) * W, s = s0 + row;
+      const int64_t left = s < n_shells ? (x_end - (x0 + k)) * 4 : 0;
+      const int bytes = (int)min((int64_t)(4 * W), max((int64_t)0, left));
+      const float* p = bytes ? f + (int64_t)s * K + x0 + k : f;
+      if constexpr (C::kAligned) cp_async16(dst + row * PITCH + k, p, bytes);
+      else cp_async4(dst + row * PITCH + k, p, bytes != 0);
+    }
+  };
+  auto stage = [&](int buf, int64_t x0) {
+    if (x0 < x_end) {
+      copy_rows(s1 + buf * src * PITCH, f1, td.i0, td.ni, x0);
+      if (C::kTwoSrc && !one_src) copy_rows(s2 + buf * src * PITCH, f2, td.j0, td.nj, x0);
+      copy_rows(sB + buf * C::COLS * PITCH, f3, td.l0 + c0, 4 * TC, x0);
     }
     cp_async_commit();
   };
-  float acc[8][8];
+  unsigned long long acc[TR / 2][TC];  // rows 2 m, 2 m + 1
 #pragma unroll
-  for (int a = 0; a < 8; ++a)
+  for (int m = 0; m < TR / 2; ++m)
 #pragma unroll
-    for (int b = 0; b < 8; ++b) acc[a][b] = 0.f;
-  stage(0, x_begin);
+    for (int e = 0; e < TC; ++e) acc[m][e] = 0ull;
+#pragma unroll
+  for (int q = 0; q < ST - 1; ++q) stage(q, x_begin + q * KC);
   int buf = 0;
-  for (int64_t x0 = x_begin; x0 < x_end; x0 += KC) {
-    if (x0 + KC < x_end) {
-      stage(buf ^ 1, x0 + KC);
-      cp_async_wait<1>();  // this chunk's copies are complete, the next chunk's in flight
-    } else {
-      cp_async_wait<0>();
-    }
-    __syncthreads();
-    {
-      const float(*S1)[SPITCH] = sm.S1[buf];
-      const float(*S2)[SPITCH] = one_src ? sm.S1[buf] : sm.S2[buf];
-#pragma unroll 8
-      for (int xx = 0; xx < KC; ++xx) sm.A[xx][tid] = pi >= 0 ? S1[pi][xx] * S2[pj][xx] : 0.f;
-    }
-    __syncthreads();
-    fma_chunk<CB>(sm.A, sm.B[buf], r0, c0, acc);
-    __syncthreads();  // A and this buffer are rewritten next
-    buf ^= 1;
-  }
+  for (int64_t x0 = x_begin; x0 < x_end; x0 += KC, buf = (buf + 1) % ST) {
+    cp_async_wait<ST - 2>();
+    __syncwarp();  // the chunk has landed; the previous one and its products have been used
+    stage((buf + ST - 1) % ST, x0 + (ST - 1) * KC);
+    const float* S1 = s1 + buf * src * PITCH;
+    const float* S2 = s2 + buf * src * PITCH;
 #pragma unroll
-  for (int p = 0; p < 8; ++p) {
+    for (int g = 0; g < TR / 4; ++g)
 #pragma unroll
-    for (int q = 0; q < CB; ++q) {
-      const int c = c0 + q;
-      if (c < td.nc) {
-        const int t = __ldg(map + td.map_off + c * kTileRows + r0 + p);
-        if (t >= 0) atomicAdd(out + t, (double)acc[p][q] * scale);
+      for (int k = 0; k < KC; k += 4) {
+        const float4 a = *reinterpret_cast<const float4*>(S1 + p1[g] * PITCH + k);
+        const float4 b = *reinterpret_cast<const float4*>(S2 + p2[g] * PITCH + k);
+        float* A = sA + k * AP + lane + 32 * g;
+        A[0] = a.x * b.x;
+        A[AP] = a.y * b.y;
+        A[2 * AP] = a.z * b.z;
+        A[3 * AP] = a.w * b.w;
       }
+    __syncwarp();
+    const float* A = sA + TR * rg;
+    const float* B = sB + buf * C::COLS * PITCH + cg * PITCH;
+#pragma unroll
+    for (int k0 = 0; k0 < KC; k0 += 2) {
+      float2 bv[TC];
+#pragma unroll
+      for (int e = 0; e < TC; ++e)
+        bv[e] = *reinterpret_cast<const float2*>(B + 4 * e * PITCH + k0);
+#pragma unroll
+      for (int k = 0; k < 2; ++k) {
+        ulonglong2 av[TR / 4];
+#pragma unroll
+        for (int m = 0; m < TR / 4; ++m)
+          av[m] = *reinterpret_cast<const ulonglong2*>(A + (k0 + k) * AP + 4 * m);
+#pragma unroll
+        for (int e = 0; e < TC; ++e) {
+          const unsigned long long b = dup2(k ? bv[e].y : bv[e].x);
+#pragma unroll
+          for (int m = 0; m < TR / 4; ++m) {
+            fma2(acc[2 * m][e], av[m].x, b);
+            fma2(acc[2 * m + 1][e], av[m].y, b);
+          }
+        }
+      }
+    }
+  }
+  cp_async_wait<0>();
+  __syncwarp();  // the next item's copies overwrite the buffers
+#pragma unroll
+  for (int e = 0; e < TC; ++e)
+#pragma unroll
+    for (int r = 0; r < TR; ++r) {
+      const int t = __ldg(map + td.map_off + (c0 + 4 * e + cg) * kTileRows + r0 + TR * rg + r);
+      const uint32_t bits = (uint32_t)(acc[r / 2][e] >> (r & 1 ? 32 : 0));
+      if (t >= 0) atomicAdd(out + t, (double)__uint_as_float(bits) * scale);
+    }
+}
+
+// Item = (slice, sub-tile of 32 columns, part of the sub-tile): `parts` of them, rows in 128 / (8
+// TR) parts and, for short grids, columns in two.
+template <class C>
+constexpr int parts() { return C::TR == 16 ? 1 : 2 * ROWS / (8 * C::TR); }
+
+template <class C>
+__global__ void __launch_bounds__(32)
+    contract_f32_kernel(const TileDesc* __restrict__ tiles, const int2* __restrict__ subs,
+                        int n_sub, const int16_t* __restrict__ row_i,
+                        const int16_t* __restrict__ row_j, const int32_t* __restrict__ map,
+                        const float* __restrict__ f1, const float* __restrict__ f2,
+                        const float* __restrict__ f3, int n_shells, int64_t K, int64_t k_begin,
+                        int64_t k_end, int64_t n_slices, int src, double* __restrict__ out,
+                        double scale) {
+  extern __shared__ __align__(16) float f32_smem[];
+  float* sm = f32_smem;
+  constexpr int P = parts<C>();
+  for (int64_t item = blockIdx.x; item < n_slices * n_sub * P; item += gridDim.x) {
+    const int64_t sl = item / (n_sub * P);
+    const int in_slice = (int)(item - sl * (n_sub * P));
+    const int part = in_slice % P;
+    const int2 sub = subs[in_slice / P];
+    const TileDesc td = tiles[sub.x];
+    // the tile's columns in as many equal runs, multiples of 8, as it has 32-column sub-tiles
+    const int runs = (td.nc + COLS - 1) / COLS, width = ((td.nc + runs - 1) / runs + 7) / 8 * 8;
+    int c0 = sub.y / COLS * width, nc = min(width, td.nc - c0), r0 = 0;
+    if (P > 1) {
+      const int half = (nc + 15) / 16 * 8;  // columns [c0, c0 + half) and the rest
+      r0 = (part >> 1) * 8 * C::TR;
+      c0 += part & 1 ? half : 0;
+      nc = part & 1 ? nc - half : half;
+      if (nc <= 0 || r0 >= td.nrows) continue;
+    }
+    const bool one_src = !C::kTwoSrc || (f1 == f2 && td.i0 == td.j0);
+    const int64_t x_begin = k_begin + sl * SLICE;
+    const int64_t x_end = min(k_end, x_begin + SLICE);
+    if (nc <= 8)
+      run_item<C, 2>(sm, src, td, r0, c0, row_i, row_j, map, f1, f2, f3, n_shells, K, x_begin, x_end, one_src, out, scale);
+    else if (nc <= 16)
+      run_item<C, 4>(sm, src, td, r0, c0, row_i, row_j, map, f1, f2, f3, n_shells, K, x_begin, x_end, one_src, out, scale);
+    else if constexpr (P == 1) {
+      if (nc <= 24)
+        run_item<C, 6>(sm, src, td, r0, c0, row_i, row_j, map, f1, f2, f3, n_shells, K, x_begin, x_end, one_src, out, scale);
+      else
+        run_item<C, 8>(sm, src, td, r0, c0, row_i, row_j, map, f1, f2, f3, n_shells, K, x_begin, x_end, one_src, out, scale);
     }
   }
 }
 
-__global__ void __launch_bounds__(THREADS, 3)
-    contract_f32_kernel(const TileDesc* __restrict__ tiles, int n_tiles,
-                        const int16_t* __restrict__ row_i, const int16_t* __restrict__ row_j,
-                        const int32_t* __restrict__ map, const float* __restrict__ f1,
-                        const float* __restrict__ f2, const float* __restrict__ f3,
-                        int n_shells, int64_t K, int64_t k_begin, int64_t k_end,
-                        int64_t n_slices, double* __restrict__ out, double scale) {
-  extern __shared__ __align__(16) unsigned char f32_smem[];
-  Smem& sm = *reinterpret_cast<Smem*>(f32_smem);
-  const int64_t n_items = (int64_t)n_tiles * n_slices;
-  for (int64_t item = blockIdx.x; item < n_items; item += gridDim.x) {
-    const int64_t sl = item / n_tiles;
-    const TileDesc td = tiles[item % n_tiles];
-    const bool one_src = f1 == f2 && td.i0 == td.j0;
-    const int64_t x_begin = k_begin + sl * SLICE;
-    const int64_t x_end = min(k_end, x_begin + SLICE);
-    if (td.nc <= 32)
-      run_item<4>(sm, td, row_i, row_j, map, f1, f2, f3, n_shells, K, x_begin, x_end, one_src, out, scale);
-    else if (td.nc <= 48)
-      run_item<6>(sm, td, row_i, row_j, map, f1, f2, f3, n_shells, K, x_begin, x_end, one_src, out, scale);
-    else
-      run_item<8>(sm, td, row_i, row_j, map, f1, f2, f3, n_shells, K, x_begin, x_end, one_src, out, scale);
-  }
+template <class C>
+void launch(const DeviceSchedule& s, const float* f1, const float* f2, const float* f3,
+            int n_shells, int64_t K, int64_t k_begin, int64_t k_end, double* out, int num_sms,
+            cudaStream_t st, double scale) {
+  const int64_t n_slices = (k_end - k_begin + SLICE - 1) / SLICE;
+  int src = 8;
+  for (const TileDesc& d : s.h_tiles) src = std::max(src, std::max(d.ni, d.nj));
+  const size_t smem = C::smem(src);
+  auto kern = contract_f32_kernel<C>;
+  BSK_CHECK_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                      (int)C::smem(SRC)));
+  int per_sm = 0;
+  BSK_CHECK_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, 32, smem));
+  const int64_t grid =
+      std::min<int64_t>((int64_t)num_sms * std::max(per_sm, 1), n_slices * s.n_sub * parts<C>());
+  kern<<<(unsigned)grid, 32, smem, st>>>(s.tiles, s.subs, s.n_sub, s.row_i, s.row_j, s.map, f1, f2,
+                                         f3, n_shells, K, k_begin, k_end, n_slices, src, out, scale);
+  BSK_CHECK_CUDA(cudaGetLastError());
 }
 }  // namespace f32
 
@@ -345,27 +415,31 @@ void launch_simt(const DeviceSchedule& s, const Tin* f1, const Tin* f2, const Ti
 
 }  // namespace
 
+// Whole-tile items from four an SM on (both sides measured, us): 335 items 848 short / 845 long,
+// 670 items 1522 .. 1917 / 1613 .. 1727, 824 items 2218 / 1610; 211 items 682 / 1180.
+constexpr int64_t kLongItemsPerSm = 4;
+
 // FP32 products and tile sums (8192-point slices), FP64 cross-slice sum.
 void launch_contract_simt_f32(const DeviceSchedule& s, const float* f1, const float* f2,
                               const float* f3, int n_shells, int64_t K, int64_t k_begin,
                               int64_t k_end, double* out, int num_sms, cudaStream_t st,
                               double scale) {
   if (s.n_tiles == 0 || k_end <= k_begin) return;
-  const size_t smem = sizeof(f32::Smem);
-  BSK_CHECK_CUDA(cudaFuncSetAttribute(f32::contract_f32_kernel,
-                                      cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-  int per_sm = 0;
-  BSK_CHECK_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(
-      &per_sm, f32::contract_f32_kernel, f32::THREADS, smem));
-  if (per_sm < 1) per_sm = 1;
   const int64_t n_slices = (k_end - k_begin + f32::SLICE - 1) / f32::SLICE;
-  const int64_t n_items = n_slices * s.n_tiles;
-  int64_t grid = (int64_t)num_sms * per_sm;
-  if (grid > n_items) grid = n_items;
-  f32::contract_f32_kernel<<<(unsigned)grid, f32::THREADS, smem, st>>>(
-      s.tiles, s.n_tiles, s.row_i, s.row_j, s.map, f1, f2, f3, n_shells, K, k_begin, k_end,
-      n_slices, out, scale);
-  BSK_CHECK_CUDA(cudaGetLastError());
+  const bool is_long = n_slices * s.n_sub >= kLongItemsPerSm * num_sms;
+  bool two_src = f1 != f2;
+  for (const TileDesc& d : s.h_tiles) two_src = two_src || d.i0 != d.j0;
+  const bool aligned = k_begin % 4 == 0 && K % 4 == 0 &&
+                       ((uintptr_t)f1 | (uintptr_t)f2 | (uintptr_t)f3) % 16 == 0;
+  const auto pick = [&](auto two, auto al) {
+    constexpr bool kTwo = decltype(two)::value, kAl = decltype(al)::value;
+    return is_long ? f32::launch<f32::Long<kTwo, kAl>> : f32::launch<f32::Short<kTwo, kAl>>;
+  };
+  const auto yes = std::true_type{};
+  const auto no = std::false_type{};
+  auto run = aligned ? (two_src ? pick(yes, yes) : pick(no, yes))
+                     : (two_src ? pick(yes, no) : pick(no, no));
+  run(s, f1, f2, f3, n_shells, K, k_begin, k_end, out, num_sms, st, scale);
 }
 
 // FP64 products and sums of FP32 fields (the yardstick of the precision study).
