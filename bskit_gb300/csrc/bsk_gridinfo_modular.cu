@@ -12,8 +12,9 @@
 // mode counts.  The whole evaluation is then three small dense transforms per shell and the
 // triple-product contraction of the tensor-core kernel (launch_contract_mod), instead of a
 // visit to every pair of modes: ~qmax^6 pairs against ~qmax^3 points times bins.  At 512^3 (63
-// shells to |q| = 127) 1.81 s -> 0.127 s, at 256^3 (31 shells to 63) 41 -> 7.7 ms, at |q| <= 40
-// (14 shells) 3.9 -> 2.2 ms; the enumeration's two launches are kept below that (kMinQ).
+// shells to |q| = 127) 1.81 s -> 90 ms (contraction 41, last axis 23, first two 17), at 256^3 (31
+// shells to 63) 41 -> 5.9 ms, at |q| <= 40 (14 shells) 3.9 -> 1.8 ms; the enumeration's two
+// launches are kept below that (kMinQ).
 //
 // Symmetry.  Membership and w do not change under sign flips of a component or the x <-> y swap
 // (bsk_gridinfo_enum.cu), so n_s and k_s are even in every coordinate and symmetric in (x, y):
@@ -97,17 +98,63 @@ std::vector<Prime> choose_primes(int qmax, double bits) {
     out.push_back(q);
   }
   if (have <= bits) return {};
+  // without the smallest prime that the others do not need
+  std::sort(out.begin(), out.end(), [](const Prime& a, const Prime& b) { return a.p > b.p; });
+  while (!out.empty() && have - std::log2((double)out.back().p) > bits) {
+    have -= std::log2((double)out.back().p);
+    out.pop_back();
+  }
   return out;
-}
-
-float centred(int64_t v, int p) {
-  v %= p;
-  if (v < 0) v += p;
-  return (float)(2 * v > p ? v - p : v);
 }
 
 __device__ __forceinline__ float mod_red(float v, float p, float inv) {
   return fmaf(-rintf(v * inv), p, v);
+}
+
+__device__ __forceinline__ float centred(int v, int p) {  // 0 <= v < p
+  return (float)(2 * v > p ? v - p : v);
+}
+__device__ __forceinline__ unsigned long long fma2(unsigned long long a, unsigned long long b,
+                                                   unsigned long long c) {
+  unsigned long long d;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
+  return d;
+}
+__device__ __forceinline__ unsigned long long pack2(float x, float y) {
+  unsigned long long d;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(d) : "f"(x), "f"(y));
+  return d;
+}
+__device__ __forceinline__ float2 unpack2(unsigned long long v) {
+  float2 f;
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(f.x), "=f"(f.y) : "l"(v));
+  return f;
+}
+__device__ __forceinline__ unsigned long long mod_red2(unsigned long long v, float p, float inv) {
+  const float2 f = unpack2(v);
+  return pack2(mod_red(f.x, p, inv), mod_red(f.y, p, inv));
+}
+
+// E[q][x] (rows of ep, zero past h) and its prefix sums over q, thread = x; om: omega's powers.
+__global__ void table_kernel(const int* __restrict__ om, int N, int h, int ep, int q1, int p,
+                             float* __restrict__ E, float* __restrict__ prefix) {
+  const int x = blockIdx.x * blockDim.x + threadIdx.x;
+  if (x >= ep) return;
+  int sum = 0, r = 0;
+  prefix[x] = 0.f;
+  for (int a = 0; a < q1; ++a) {
+    int v = 0;
+    if (x < h) {
+      v = a == 0 ? 1 : om[r] + om[r ? N - r : 0];
+      if (v >= p) v -= p;
+      sum += v;
+      if (sum >= p) sum -= p;
+      r += x;  // a x mod N
+      if (r >= N) r -= N;
+    }
+    E[(int64_t)a * ep + x] = centred(v, p);
+    prefix[(int64_t)(a + 1) * ep + x] = centred(sum, p);
+  }
 }
 
 // w(q) mod p, centred, for 0 <= q_a, q_b, q_c <= qmax: the correctly rounded |q| 2^44.
@@ -120,189 +167,243 @@ __global__ void weight_kernel(int q1, int p, int16_t* __restrict__ w) {
   w[((int64_t)a * q1 + b) * q1 + c] = (int16_t)r;
 }
 
-// First two axes: block = (x, shell).  The plane A[b][c] = sum over the shell's q_a of
-// E[x][q_a] (times w for the |k| field) goes to shared memory, for the count field as a
-// difference of E's prefix sums; then out[pair(x, y)][c] = sum_b E[y][b] A[b][c], y <= x: a
-// warp takes 8 y, a lane 4 c (32 FMAs for one 16-byte shared-memory load and two broadcast
-// loads of E).  Bound by FMA issue; its output is written once.
+// First axis of the |k| fields: out[s][x][b][c] = sum over the shell's q_a of E[x][q_a] w(q_a, b,
+// c), rows of cp; thread = column (b, c) of a shell, eight x at a time, so that a column's
+// weights are read once for eight x (a block per x read them from L2 for each: 1.1 of 2.1 ms).
+__global__ void __launch_bounds__(128)
+    column_kernel(const uint32_t* __restrict__ range, const int16_t* __restrict__ w,
+                  const float* __restrict__ E, int ep, int q1, int h, int cp,
+                  const int* __restrict__ radius, float p, float inv, int16_t* __restrict__ out) {
+  const int c = blockIdx.z * blockDim.x + threadIdx.x, b = blockIdx.x, s = blockIdx.y;
+  if (b > radius[s] || c >= cp) return;
+  const uint32_t r = c < q1 ? range[((int64_t)s * q1 + b) * q1 + c] : kEmptyRange;
+  const int a0 = (int)(r & 0xFFFF), a1 = (int)(r >> 16);
+  int16_t* o = out + ((int64_t)s * h * q1 + b) * cp + c;
+  for (int x0 = 0; x0 < h; x0 += 8) {
+    float v[8];
+#pragma unroll
+    for (int e = 0; e < 8; ++e) v[e] = 0.f;
+    int run = 0;
+    for (int a = a0; a <= a1; ++a) {
+      const float wa = (float)w[((int64_t)a * q1 + b) * q1 + c];
+      const float4 e0 = __ldg(reinterpret_cast<const float4*>(E + (int64_t)a * ep + x0));
+      const float4 e1 = __ldg(reinterpret_cast<const float4*>(E + (int64_t)a * ep + x0 + 4));
+      const float ev[8] = {e0.x, e0.y, e0.z, e0.w, e1.x, e1.y, e1.z, e1.w};
+#pragma unroll
+      for (int e = 0; e < 8; ++e) v[e] = fmaf(ev[e], wa, v[e]);
+      if (++run == kRun - 1) {  // with the residue carried on, kRun terms at most
+#pragma unroll
+        for (int e = 0; e < 8; ++e) v[e] = mod_red(v[e], p, inv);
+        run = 0;
+      }
+    }
+#pragma unroll
+    for (int e = 0; e < 8; ++e)
+      if (x0 + e < h) o[(int64_t)(x0 + e) * q1 * cp] = (int16_t)mod_red(v[e], p, inv);
+  }
+}
+
+// First two axes: block = (x, shell).  The plane A[b][c] (first axis done) goes to shared memory:
+// for the count fields sum_{q_a in s} E[x][q_a], a difference of E's prefix sums, for the |k|
+// fields column_kernel's.  Then out[pair(x, y)][c] = sum_b E[y][b] A[b][c], y <= x: a warp takes
+// 8 y, a lane 4 c, 16 packed multiply-adds (by two y) for one 16-byte shared-memory load and
+// two broadcast loads of E.
 constexpr int kXyThreads = 256;
 template <bool kWeighted>
 __global__ void __launch_bounds__(kXyThreads)
-    xy_kernel(const uint32_t* __restrict__ range, const int16_t* __restrict__ w,
+    xy_kernel(const uint32_t* __restrict__ range, const int16_t* __restrict__ plane,
               const float* __restrict__ E /*[q][ep]*/, const float* __restrict__ prefix, int ep,
               int q1, const int* __restrict__ radius, int np, int cp, float p, float inv,
               float* __restrict__ out) {
   extern __shared__ __align__(16) float sA[];  // [R + 1][cp]
   __shared__ float sE[kMaxQ + 2];
-  const int x = (int)gridDim.x - 1 - (int)blockIdx.x;  // the longest blocks first
+  const int h = (int)gridDim.x;
+  const int x = h - 1 - (int)blockIdx.x;  // the longest blocks first
   const int s = blockIdx.y;
   const int R = radius[s], nb = R + 1;
-  const float* src = kWeighted ? E : prefix;
-  for (int a = threadIdx.x; a < q1 + 1; a += kXyThreads)
-    sE[a] = (!kWeighted || a < q1) ? src[(int64_t)a * ep + x] : 0.f;
-  __syncthreads();
-  const uint32_t* rg = range + (int64_t)s * q1 * q1;
-  for (int i = threadIdx.x; i < nb * cp; i += kXyThreads) {
-    const int b = i / cp, c = i - b * cp;
-    float v = 0.f;
-    const uint32_t r = c < nb ? rg[b * q1 + c] : kEmptyRange;
-    if (r != kEmptyRange) {
-      const int a0 = (int)(r & 0xFFFF), a1 = (int)(r >> 16);
-      if (kWeighted) {
-        int run = 0;
-        for (int a = a0; a <= a1; ++a) {
-          v = fmaf(sE[a], (float)w[((int64_t)a * q1 + b) * q1 + c], v);
-          if (++run == kRun) {
-            v = mod_red(v, p, inv);
-            run = 1;
-          }
-        }
-        v = mod_red(v, p, inv);
-      } else {
-        v = mod_red(sE[a1 + 1] - sE[a0], p, inv);
-      }
+  if (kWeighted) {
+    const int16_t* src = plane + ((int64_t)s * h + x) * q1 * cp;
+    for (int i = threadIdx.x * 4; i < nb * cp; i += kXyThreads * 4) {
+      const short4 v = *reinterpret_cast<const short4*>(src + i);
+      *reinterpret_cast<float4*>(sA + i) = make_float4(v.x, v.y, v.z, v.w);
     }
-    sA[i] = v;
+  } else {
+    for (int a = threadIdx.x; a < q1 + 1; a += kXyThreads) sE[a] = prefix[(int64_t)a * ep + x];
+    __syncthreads();
+    const uint32_t* rg = range + (int64_t)s * q1 * q1;
+    for (int b = threadIdx.x >> 5; b < nb; b += kXyThreads / 32)
+      for (int c = threadIdx.x & 31; c < cp; c += 32) {
+        const uint32_t r = c < nb ? rg[b * q1 + c] : kEmptyRange;
+        sA[b * cp + c] = r == kEmptyRange
+                             ? 0.f
+                             : mod_red(sE[(int)(r >> 16) + 1] - sE[(int)(r & 0xFFFF)], p, inv);
+      }
   }
   __syncthreads();
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   float* o = out + ((int64_t)s * np + (int64_t)x * (x + 1) / 2) * cp;
   for (int y0 = warp * 8; y0 <= x; y0 += (kXyThreads / 32) * 8) {
     for (int c = lane * 4; c < cp; c += 128) {
-      float acc[8][4];
+      unsigned long long acc[4][4];  // y pair, c
 #pragma unroll
-      for (int y = 0; y < 8; ++y)
+      for (int y = 0; y < 4; ++y)
 #pragma unroll
-        for (int e = 0; e < 4; ++e) acc[y][e] = 0.f;
+        for (int e = 0; e < 4; ++e) acc[y][e] = 0ull;
       for (int b0 = 0; b0 < nb; b0 += kRun - 1) {
         const int b1 = min(nb, b0 + kRun - 1);
 #pragma unroll 4
         for (int b = b0; b < b1; ++b) {
           const float4 av = *reinterpret_cast<const float4*>(sA + b * cp + c);
-          const float4 e0 = __ldg(reinterpret_cast<const float4*>(E + (int64_t)b * ep + y0));
-          const float4 e1 = __ldg(reinterpret_cast<const float4*>(E + (int64_t)b * ep + y0 + 4));
-          const float ev[8] = {e0.x, e0.y, e0.z, e0.w, e1.x, e1.y, e1.z, e1.w};
+          const ulonglong2 e0 = __ldg(reinterpret_cast<const ulonglong2*>(E + (int64_t)b * ep + y0));
+          const ulonglong2 e1 =
+              __ldg(reinterpret_cast<const ulonglong2*>(E + (int64_t)b * ep + y0 + 4));
+          const unsigned long long ev[4] = {e0.x, e0.y, e1.x, e1.y};
+          const unsigned long long ad[4] = {pack2(av.x, av.x), pack2(av.y, av.y),
+                                            pack2(av.z, av.z), pack2(av.w, av.w)};
 #pragma unroll
-          for (int y = 0; y < 8; ++y) {
-            acc[y][0] = fmaf(ev[y], av.x, acc[y][0]);
-            acc[y][1] = fmaf(ev[y], av.y, acc[y][1]);
-            acc[y][2] = fmaf(ev[y], av.z, acc[y][2]);
-            acc[y][3] = fmaf(ev[y], av.w, acc[y][3]);
-          }
+          for (int y = 0; y < 4; ++y)
+#pragma unroll
+            for (int e = 0; e < 4; ++e) acc[y][e] = fma2(ev[y], ad[e], acc[y][e]);
         }
 #pragma unroll
-        for (int y = 0; y < 8; ++y)
+        for (int y = 0; y < 4; ++y)
 #pragma unroll
-          for (int e = 0; e < 4; ++e) acc[y][e] = mod_red(acc[y][e], p, inv);
+          for (int e = 0; e < 4; ++e) acc[y][e] = mod_red2(acc[y][e], p, inv);
       }
 #pragma unroll
-      for (int y = 0; y < 8; ++y)
-        if (y0 + y <= x)
-          *reinterpret_cast<float4*>(o + (int64_t)(y0 + y) * cp + c) =
-              make_float4(acc[y][0], acc[y][1], acc[y][2], acc[y][3]);
+      for (int y = 0; y < 4; ++y) {
+        const float2 v[4] = {unpack2(acc[y][0]), unpack2(acc[y][1]), unpack2(acc[y][2]),
+                             unpack2(acc[y][3])};
+        float* oy = o + (int64_t)(y0 + 2 * y) * cp + c;
+        if (y0 + 2 * y <= x)
+          *reinterpret_cast<float4*>(oy) = make_float4(v[0].x, v[1].x, v[2].x, v[3].x);
+        if (y0 + 2 * y + 1 <= x)
+          *reinterpret_cast<float4*>(oy + cp) = make_float4(v[0].y, v[1].y, v[2].y, v[3].y);
+      }
     }
   }
 }
 
-// Last axis: out[pair][z] = sum_c H[pair][c] E[z][c] for 64 pairs at a time, persistent blocks
-// (E stays in shared memory).  A warp takes 32 pairs x 64 z, a thread 8 x 8: 8 rows of H (16
-// bytes each per 4 c, broadcast in a quarter warp) and 4 x 8 bytes of E per c and 64 FMAs, 16
-// shared-memory wavefronts per 64 warp-wide FMAs, which is also their issue time.  Writes the
-// FP32 field (pair factors) and / or the weighted field's split (columns).
-constexpr int kZThreads = 256, kZPairs = 64;
-__global__ void __launch_bounds__(kZThreads, 1)
+// Last axis: out[pair][z] = sum_c H[pair][c] E[z][c] for kPairs pairs at a time, persistent blocks
+// (E stays in shared memory).  A warp takes 32 pairs x 64 z, a thread 8 x 8, as 32 multiply-adds
+// packed by two z: per c 8 values of H (broadcast in a quarter warp) and 4 x 8 bytes of E, 16
+// shared-memory wavefronts.  Writes the FP32 field (pair factors) and / or the weighted
+// field's split (columns).
+template <int kPairs>
+__global__ void __launch_bounds__(4 * kPairs, 1)
     z_kernel(const float* __restrict__ H, const float* __restrict__ E, int ep, int q1,
              const int* __restrict__ radius, int n_shells, Prime pr, int cp, float p, float inv,
              float* __restrict__ field, __nv_bfloat16* __restrict__ split) {
   extern __shared__ __align__(16) float smz[];
+  constexpr int kThreads = 4 * kPairs, kWarpRows = kPairs / 32;
   const int zp = (pr.hz + 63) / 64 * 64;
-  float* sE = smz;                    // [q1][zp]
-  float* sH = sE + (size_t)q1 * zp;   // [64][cp + 4]
+  float* sE = smz;                    // [q1 + 1][zp], the last row zero (an odd count's second c)
+  float* sH = sE + (size_t)(q1 + 1) * zp;   // [kPairs][cp + 4]
   const int hp = cp + 4;
-  for (int i = threadIdx.x; i < q1 * zp; i += kZThreads) {
+  for (int i = threadIdx.x; i < (q1 + 1) * zp; i += kThreads) {
     const int c = i / zp, z = i - c * zp;
-    sE[i] = z < pr.h ? E[(int64_t)c * ep + z] : 0.f;
+    sE[i] = z < pr.h && c < q1 ? E[(int64_t)c * ep + z] : 0.f;
   }
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int pg = (warp & 1) * 32 + (lane >> 3) * 8;  // this thread's 8 pairs of the block's 64
+  const int pg = warp % kWarpRows * 32 + (lane >> 3) * 8;  // this thread's 8 pairs
   const int zl = (lane & 7) * 2;                     // its z: zl + {0, 1} + 16 j of each 64
-  const int tiles = (pr.np + kZPairs - 1) / kZPairs;
-  for (int u = blockIdx.x; u < tiles * n_shells; u += gridDim.x) {
-    const int s = u / tiles, t0 = (u - s * tiles) * kZPairs;
-    const int nc = radius[s] + 1, nc4 = (nc + 3) & ~3;
-    __syncthreads();  // the previous tile's reads of sH (and the stores of sE)
-    for (int i = threadIdx.x; i < kZPairs * (nc4 / 4); i += kZThreads) {
-      const int r = i / (nc4 / 4), c = (i - r * (nc4 / 4)) * 4;
-      float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
-      if (t0 + r < pr.np)
-        v = *reinterpret_cast<const float4*>(H + ((int64_t)s * pr.np + t0 + r) * cp + c);
-      *reinterpret_cast<float4*>(sH + r * hp + c) = v;
+  const int tiles = (pr.np + kPairs - 1) / kPairs;
+  // the next tile's rows are copied while the current one is reduced and stored
+  auto fetch = [&](int u) {
+    if (u >= tiles * n_shells) return;
+    const int s = u / tiles, t0 = (u - s * tiles) * kPairs;
+    const int nc4 = (radius[s] + 4) & ~3;
+    for (int r = threadIdx.x >> 2; r < kPairs; r += kThreads / 4) {
+      const int pair = min(t0 + r, pr.np - 1);  // past the last pair: any (not stored)
+      const float* src = H + ((int64_t)s * pr.np + pair) * cp;
+      for (int c = (threadIdx.x & 3) * 4; c < nc4; c += 16)
+        asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(
+                         (uint32_t)__cvta_generic_to_shared(sH + r * hp + c)),
+                     "l"(src + c)
+                     : "memory");
     }
-    __syncthreads();
-    for (int z0 = (warp >> 1) * 64; z0 < pr.hz; z0 += (kZThreads / 64) * 64) {
-      float acc[8][8];
+  };
+  fetch(blockIdx.x);
+  for (int u = blockIdx.x; u < tiles * n_shells; u += gridDim.x) {
+    const int s = u / tiles, t0 = (u - s * tiles) * kPairs;
+    const int nc = radius[s] + 1, nc2 = (nc + 1) & ~1;
+    asm volatile("cp.async.wait_all;" ::: "memory");
+    __syncthreads();  // the rows have landed (and E, the first time)
+    const int z0 = warp / kWarpRows * 64;  // 4 x 64 points cover hz (at most 256)
+    unsigned long long acc[8][4];  // pair, z pair
+#pragma unroll
+    for (int a = 0; a < 8; ++a)
+#pragma unroll
+      for (int j = 0; j < 4; ++j) acc[a][j] = 0ull;
+    // 28 products and a residue between reductions
+    for (int c0 = 0; c0 < nc && z0 < pr.hz; c0 += 28) {
+      const int c1 = min(nc2, c0 + 28);
+      for (int c = c0; c < c1; c += 2) {
+        float2 hv[8];
+#pragma unroll
+        for (int a = 0; a < 8; ++a)
+          hv[a] = *reinterpret_cast<const float2*>(sH + (pg + a) * hp + c);
+#pragma unroll
+        for (int k = 0; k < 2; ++k) {
+          unsigned long long ev[4];
+#pragma unroll
+          for (int j = 0; j < 4; ++j)
+            ev[j] = *reinterpret_cast<const unsigned long long*>(sE + (c + k) * zp + z0 + zl +
+                                                                 16 * j);
+#pragma unroll
+          for (int a = 0; a < 8; ++a) {
+            const float h = k == 0 ? hv[a].x : hv[a].y;
+            const unsigned long long hd = pack2(h, h);
+#pragma unroll
+            for (int j = 0; j < 4; ++j) acc[a][j] = fma2(hd, ev[j], acc[a][j]);
+          }
+        }
+      }
 #pragma unroll
       for (int a = 0; a < 8; ++a)
 #pragma unroll
-        for (int e = 0; e < 8; ++e) acc[a][e] = 0.f;
-      for (int c0 = 0; c0 < nc; c0 += 28) {  // 28 products and a residue between reductions
-        const int c1 = min(nc4, c0 + 28);
-        for (int c = c0; c < c1; c += 4) {
-          float4 hv[8];
+        for (int j = 0; j < 4; ++j) acc[a][j] = mod_red2(acc[a][j], p, inv);
+    }
+    __syncthreads();  // every warp has read the rows
+    fetch(u + gridDim.x);
+    // (x, y) of the thread's first pair
+    int x, y;
+    {
+      const int pair = min(t0 + pg, pr.np - 1);
+      x = (int)((sqrtf(8.f * pair + 1.f) - 1.f) * 0.5f);
+      while ((x + 1) * (x + 2) / 2 <= pair) ++x;
+      while (x * (x + 1) / 2 > pair) --x;
+      y = pair - x * (x + 1) / 2;
+    }
 #pragma unroll
-          for (int a = 0; a < 8; ++a)
-            hv[a] = *reinterpret_cast<const float4*>(sH + (pg + a) * hp + c);
+    for (int a = 0; a < 8; ++a) {
+      const int pair = t0 + pg + a;
+      if (pair >= pr.np) break;
+      const float wxy = (x == 0 || 2 * x == pr.N ? 1.f : 2.f) *
+                        (y == 0 || 2 * y == pr.N ? 1.f : 2.f) * (x != y ? 2.f : 1.f);
 #pragma unroll
-          for (int k = 0; k < 4; ++k) {
-            if (c + k >= q1) break;  // H is zero there and E has no row
-            float2 ev[4];
-#pragma unroll
-            for (int j = 0; j < 4; ++j)
-              ev[j] = *reinterpret_cast<const float2*>(sE + (c + k) * zp + z0 + zl + 16 * j);
-#pragma unroll
-            for (int a = 0; a < 8; ++a) {
-              const float h = k == 0 ? hv[a].x : k == 1 ? hv[a].y : k == 2 ? hv[a].z : hv[a].w;
-#pragma unroll
-              for (int j = 0; j < 4; ++j) {
-                acc[a][2 * j] = fmaf(h, ev[j].x, acc[a][2 * j]);
-                acc[a][2 * j + 1] = fmaf(h, ev[j].y, acc[a][2 * j + 1]);
-              }
-            }
-          }
+      for (int j = 0; j < 4; ++j) {
+        const int z = z0 + zl + 16 * j;
+        if (z >= pr.hz) continue;
+        const float2 v = unpack2(acc[a][j]);
+        const float v0 = v.x, v1 = v.y;
+        const int64_t pt = (int64_t)pair * pr.hz + z;
+        if (field)
+          *reinterpret_cast<float2*>(field + (int64_t)s * pr.K + pt) = make_float2(v0, v1);
+        if (split) {
+          const float w0 = wxy * (z == 0 || 2 * z == pr.N ? 1.f : 2.f);
+          const float w1 = wxy * (2 * (z + 1) == pr.N ? 1.f : 2.f);
+          const float u0 = mod_red(v0 * w0, p, inv), u1 = mod_red(v1 * w1, p, inv);
+          const float h0 = 8.f * rintf(u0 * 0.125f), h1 = 8.f * rintf(u1 * 0.125f);
+          *reinterpret_cast<__nv_bfloat162*>(split + split_index(0, s, pt, n_shells)) =
+              __floats2bfloat162_rn(h0, h1);
+          *reinterpret_cast<__nv_bfloat162*>(split + split_index(1, s, pt, n_shells)) =
+              __floats2bfloat162_rn(u0 - h0, u1 - h1);
         }
-#pragma unroll
-        for (int a = 0; a < 8; ++a)
-#pragma unroll
-          for (int e = 0; e < 8; ++e) acc[a][e] = mod_red(acc[a][e], p, inv);
       }
-#pragma unroll
-      for (int a = 0; a < 8; ++a) {
-        const int pair = t0 + pg + a;
-        if (pair >= pr.np) break;
-        int x = (int)((sqrtf(8.f * pair + 1.f) - 1.f) * 0.5f);
-        while ((x + 1) * (x + 2) / 2 <= pair) ++x;
-        while (x * (x + 1) / 2 > pair) --x;
-        const int y = pair - x * (x + 1) / 2;
-        const float wxy = (x == 0 || 2 * x == pr.N ? 1.f : 2.f) *
-                          (y == 0 || 2 * y == pr.N ? 1.f : 2.f) * (x != y ? 2.f : 1.f);
-#pragma unroll
-        for (int j = 0; j < 4; ++j) {
-          const int z = z0 + zl + 16 * j;
-          if (z >= pr.hz) continue;
-          const float v0 = acc[a][2 * j], v1 = acc[a][2 * j + 1];
-          const int64_t pt = (int64_t)pair * pr.hz + z;
-          if (field) *reinterpret_cast<float2*>(field + (int64_t)s * pr.K + pt) = make_float2(v0, v1);
-          if (split) {
-            const float w0 = wxy * (z == 0 || 2 * z == pr.N ? 1.f : 2.f);
-            const float w1 = wxy * (2 * (z + 1) == pr.N ? 1.f : 2.f);
-            const float u0 = mod_red(v0 * w0, p, inv), u1 = mod_red(v1 * w1, p, inv);
-            const float h0 = 8.f * rintf(u0 * 0.125f), h1 = 8.f * rintf(u1 * 0.125f);
-            *reinterpret_cast<__nv_bfloat162*>(split + split_index(0, s, pt, n_shells)) =
-                __floats2bfloat162_rn(h0, h1);
-            *reinterpret_cast<__nv_bfloat162*>(split + split_index(1, s, pt, n_shells)) =
-                __floats2bfloat162_rn(u0 - h0, u1 - h1);
-          }
-        }
+      if (++y > x) {
+        ++x;
+        y = 0;
       }
     }
   }
@@ -388,9 +489,10 @@ struct UploadedSchedule {
   }
 };
 
-size_t z_smem(const Prime& q, int q1, int cp) {
-  return ((size_t)q1 * ((q.hz + 63) / 64 * 64) + (size_t)kZPairs * (cp + 4)) * sizeof(float);
+size_t z_smem(const Prime& q, int q1, int cp, int pairs) {
+  return ((size_t)(q1 + 1) * ((q.hz + 63) / 64 * 64) + (size_t)pairs * (cp + 4)) * sizeof(float);
 }
+constexpr size_t kMaxSmem = 227 * 1024;
 
 }  // namespace gmod
 
@@ -440,12 +542,12 @@ bool gridinfo_modular(bsk_plan* p, const std::vector<HostTriangle>& tri, double*
   const int cp = (q1 + 3) / 4 * 4;
   int64_t max_k = 0, max_np = 0;
   for (const Prime& q : primes) {
-    if (z_smem(q, q1, cp) > 227 * 1024) return false;
+    if (q.hz > 256 || z_smem(q, q1, cp, 64) > kMaxSmem) return false;
     max_k = std::max(max_k, q.K);
     max_np = std::max<int64_t>(max_np, q.np);
   }
 
-  // host tables: schedules, shell radii, triangle entries, E and its prefix sums per prime
+  // host tables: schedules, shell radii, triangle entries, powers of omega per prime
   Upload up;
   UploadedSchedule sc, ss;
   tile_schedule(ec, n, nullptr, sc.h);
@@ -454,7 +556,7 @@ bool gridinfo_modular(bsk_plan* p, const std::vector<HostTriangle>& tri, double*
   ss.add(up);
   const size_t o_idx = up.add(idx.data(), T * sizeof(int4));
   const size_t o_rad = up.add(p->shell_r.data(), n * sizeof(int));
-  std::vector<size_t> o_e(n_pr), o_pre(n_pr);
+  std::vector<size_t> o_om(n_pr);
   std::vector<int> ep(n_pr);
   Garner g{};
   g.n = n_pr;
@@ -478,19 +580,7 @@ bool gridinfo_modular(bsk_plan* p, const std::vector<HostTriangle>& tri, double*
     om[0] = 1;
     for (int i = 1; i < q.N; ++i) om[i] = (int)((int64_t)om[i - 1] * omega % q.p);
     ep[k] = (q.h + 7) / 8 * 8;
-    std::vector<float> e((size_t)q1 * ep[k], 0.f), pre((size_t)(q1 + 1) * ep[k], 0.f);
-    for (int x = 0; x < q.h; ++x) {
-      int64_t sum = 0;
-      for (int a = 0; a < q1; ++a) {
-        const int r = (int)((int64_t)a * x % q.N);
-        const int64_t v = a == 0 ? 1 : (int64_t)om[r] + om[(q.N - r) % q.N];
-        e[(size_t)a * ep[k] + x] = centred(v, q.p);
-        sum += v;
-        pre[(size_t)(a + 1) * ep[k] + x] = centred(sum, q.p);
-      }
-    }
-    o_e[k] = up.add(e.data(), e.size() * sizeof(float));
-    o_pre[k] = up.add(pre.data(), pre.size() * sizeof(float));
+    o_om[k] = up.add(om.data(), om.size() * sizeof(int));
   }
 
   // device scratch in one stream-ordered block
@@ -505,9 +595,16 @@ bool gridinfo_modular(bsk_plan* p, const std::vector<HostTriangle>& tri, double*
   const size_t a_range = take((size_t)n * q1 * q1 * sizeof(uint32_t));
   const size_t a_w = take((size_t)q1 * q1 * q1 * sizeof(int16_t));
   const size_t a_out = take(((size_t)n_cnt * ne + (size_t)n_pr * ns) * sizeof(long long) + 8);
+  int max_ep = 0;
+  for (int e : ep) max_ep = std::max(max_ep, e);
+  const size_t a_e = take((size_t)(2 * q1 + 1) * max_ep * sizeof(float));
   const size_t a_h = take((size_t)n * max_np * cp * sizeof(float));
   const size_t a_f = take((size_t)n * max_k * sizeof(float));
-  const size_t a_s = take(split_elems(n, max_k) * sizeof(__nv_bfloat16));
+  // column_kernel's planes lie where the split of the same prime's |k| field goes later
+  size_t planes = 0;
+  for (const Prime& q : primes) planes = std::max(planes, (size_t)n * q.h * q1 * cp);
+  const size_t a_s = take(std::max(split_elems(n, max_k) * sizeof(__nv_bfloat16),
+                                   planes * sizeof(int16_t)));
   if (p->mem_budget && device_bytes(p) + (int64_t)total > (int64_t)p->mem_budget) return false;
   unsigned char* base = nullptr;
   if (cudaMallocAsync((void**)&base, total, st) != cudaSuccess) {
@@ -540,42 +637,54 @@ bool gridinfo_modular(bsk_plan* p, const std::vector<HostTriangle>& tri, double*
   DeviceSchedule dc, ds;
   sc.bind(base + a_up, dc);
   ss.bind(base + a_up, ds);
+  float* E = (float*)(base + a_e);
+  float* pre = E + (size_t)q1 * max_ep;
   const size_t xy_smem = (size_t)q1 * cp * sizeof(float);
   BSK_CHECK_CUDA(cudaFuncSetAttribute(xy_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                       (int)xy_smem));
   BSK_CHECK_CUDA(cudaFuncSetAttribute(xy_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                       (int)xy_smem));
-  BSK_CHECK_CUDA(cudaFuncSetAttribute(z_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                      227 * 1024));
+  for (auto z : {z_kernel<64>, z_kernel<128>})
+    BSK_CHECK_CUDA(cudaFuncSetAttribute(z, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                        (int)kMaxSmem));
   for (int k = 0; k < n_pr; ++k) {
     const Prime& q = primes[k];
-    const float* E = (const float*)(base + a_up + o_e[k]);
-    const float* pre = (const float*)(base + a_up + o_pre[k]);
+    table_kernel<<<(ep[k] + 31) / 32, 32, 0, st>>>((const int*)(base + a_up + o_om[k]), q.N, q.h,
+                                                   ep[k], q1, q.p, E, pre);
+    BSK_CHECK_CUDA(cudaGetLastError());
     const float pf = (float)q.p, inv = 1.f / pf;
     const int64_t points = (int64_t)q.np * q.hz;
     // the points past the last pair: zero in the fields, and so is the last chunk's split
     if (q.K > points)
       BSK_CHECK_CUDA(cudaMemset2DAsync(field + points, q.K * sizeof(float), 0,
                                        (q.K - points) * sizeof(float), n, st));
-    BSK_CHECK_CUDA(cudaMemsetAsync(split + split_elems(n, q.K - 128), 0,
-                                   (split_elems(n, q.K) - split_elems(n, q.K - 128)) *
-                                       sizeof(__nv_bfloat16), st));
-    const size_t zs = z_smem(q, q1, cp);
-    const int z_grid = std::min(p->num_sms, (q.np + kZPairs - 1) / kZPairs * n);
-    xy_kernel<false><<<dim3(q.h, n), kXyThreads, xy_smem, st>>>(range, w, E, pre, ep[k], q1, radius,
-                                                               q.np, cp, pf, inv, H);
-    z_kernel<<<z_grid, kZThreads, zs, st>>>(H, E, ep[k], q1, radius, n, q, cp, pf, inv, field,
-                                            k < n_cnt ? split : nullptr);
+    const int pairs = z_smem(q, q1, cp, 128) <= kMaxSmem ? 128 : 64;
+    const size_t zs = z_smem(q, q1, cp, pairs);
+    const int z_grid = std::min(p->num_sms, (q.np + pairs - 1) / pairs * n);
+    const auto last_axis = [&](float* f, __nv_bfloat16* planes_out) {
+      if (planes_out)
+        BSK_CHECK_CUDA(cudaMemsetAsync(split + split_elems(n, q.K - 128), 0,
+                                       (split_elems(n, q.K) - split_elems(n, q.K - 128)) *
+                                           sizeof(__nv_bfloat16), st));
+      auto z = pairs == 128 ? z_kernel<128> : z_kernel<64>;
+      z<<<z_grid, 4 * pairs, zs, st>>>(H, E, ep[k], q1, radius, n, q, cp, pf, inv, f, planes_out);
+      BSK_CHECK_CUDA(cudaGetLastError());
+    };
+    xy_kernel<false><<<dim3(q.h, n), kXyThreads, xy_smem, st>>>(range, nullptr, E, pre, ep[k], q1,
+                                                               radius, q.np, cp, pf, inv, H);
     BSK_CHECK_CUDA(cudaGetLastError());
+    last_axis(field, k < n_cnt ? split : nullptr);
     if (k < n_cnt)
       launch_contract_mod(dc, field, split, n, q.K, q.p,
                           (unsigned long long*)cnt + (size_t)k * ne, p->num_sms, st);
     weight_kernel<<<dim3((q1 + 63) / 64, q1, q1), 64, 0, st>>>(q1, q.p, w);
-    xy_kernel<true><<<dim3(q.h, n), kXyThreads, xy_smem, st>>>(range, w, E, pre, ep[k], q1, radius,
-                                                              q.np, cp, pf, inv, H);
-    z_kernel<<<z_grid, kZThreads, zs, st>>>(H, E, ep[k], q1, radius, n, q, cp, pf, inv, nullptr,
-                                            split);
+    int16_t* plane = (int16_t*)split;
+    column_kernel<<<dim3(q1, n, (cp + 127) / 128), 128, 0, st>>>(range, w, E, ep[k], q1, q.h, cp,
+                                                                 radius, pf, inv, plane);
+    xy_kernel<true><<<dim3(q.h, n), kXyThreads, xy_smem, st>>>(range, plane, E, pre, ep[k], q1,
+                                                              radius, q.np, cp, pf, inv, H);
     BSK_CHECK_CUDA(cudaGetLastError());
+    last_axis(nullptr, split);
     launch_contract_mod(ds, field, split, n, q.K, q.p,
                         (unsigned long long*)sum + (size_t)k * ns, p->num_sms, st);
   }
