@@ -192,17 +192,6 @@ void check_budget(const bsk_plan* p, size_t bytes, const char* what) {
                                  std::to_string(root->mem_budget)};
 }
 
-// The shells' |q_a| intervals that the field synthesis masks by (a few MB, not counted in the
-// footprint, like the shell edges).
-void make_range(bsk_plan* p) {
-  const size_t q1 = p->qmax + 1;
-  p->range = (uint32_t*)dmalloc((size_t)p->n * q1 * q1 * sizeof(uint32_t));
-  launch_shell_range(p, p->range, nullptr, 0);
-  p->d_radius = (int*)dmalloc((size_t)p->n * sizeof(int));
-  BSK_CHECK_CUDA(cudaMemcpy(p->d_radius, p->shell_r.data(), (size_t)p->n * sizeof(int),
-                            cudaMemcpyHostToDevice));
-}
-
 // Shells per synthesis launch: the FFT batch, or more on a small grid, as long as the workspace
 // stays within kSmallWorkspace (96^3, 15 shells: one launch a pass instead of two that half
 // fill the GPU).  Under a memory budget the batch, whose workspace the budget was sized for.
@@ -213,6 +202,25 @@ void size_synth(bsk_plan* p, size_t mem_budget) {
          synth_workspace_bytes(p->Ng, p->qmax, p->synth_batch + 1) <= kSmallWorkspace)
     ++p->synth_batch;
   p->synth_ws_bytes = synth_workspace_bytes(p->Ng, p->qmax, p->synth_batch);
+}
+
+// The synthesis workspace, with the twiddles, and (not counted in the footprint, like the shell
+// edges) the shells' |q_a| intervals and radii that its passes mask by.
+void ensure_synth(bsk_plan* p, bool against_budget = true) {
+  if (p->synth_ws) return;
+  if (against_budget) check_budget(p, p->synth_ws_bytes, "the field-synthesis workspace");
+  const size_t q1 = p->qmax + 1, n_range = (size_t)p->n * q1 * q1;
+  if (!p->range) {
+    p->range = (uint32_t*)dmalloc((n_range + p->n) * sizeof(uint32_t));
+    p->d_radius = (int*)(p->range + n_range);
+    launch_shell_range(p, p->range, nullptr, 0);
+    BSK_CHECK_CUDA(cudaMemcpy(p->d_radius, p->shell_r.data(), (size_t)p->n * sizeof(int),
+                              cudaMemcpyHostToDevice));
+  }
+  p->synth_ws = dmalloc(p->synth_ws_bytes);
+  synth_init_workspace(p->Ng, p->synth_ws);
+  // the passes may run on a stream that does not wait for the default one
+  BSK_CHECK_CUDA(cudaStreamSynchronize(nullptr));
 }
 
 void release_stream(bsk_plan* p) {
@@ -255,11 +263,7 @@ void ensure_fields(bsk_plan* p, int s, cudaStream_t st, bool with_split = false,
       BSK_CHECK_CUDA(cudaMemset(f.fields + (size_t)p->n * p->K, 0, pad * sizeof(float)));
   }
   if (p->use_synth) {
-    if (!p->synth_ws) {
-      check_budget(p, p->synth_ws_bytes, "the field-synthesis workspace");
-      p->synth_ws = dmalloc(p->synth_ws_bytes);
-      synth_init_workspace(p->Ng, p->synth_ws);
-    }
+    ensure_synth(p);
     if (with_split) alloc_split(p, f);
     int done = 0;
     for (int s0 = 0; s0 < need; s0 += p->synth_batch) {
@@ -333,11 +337,7 @@ void ensure_level_fields(bsk_plan* q, int s, cudaStream_t st, int nn, int fp_fro
     if (pad)
       BSK_CHECK_CUDA(cudaMemset(f.fields + (size_t)q->n * q->K, 0, pad * sizeof(float)));
   }
-  if (!q->synth_ws) {
-    check_budget(q, q->synth_ws_bytes, "the field-synthesis workspace");
-    q->synth_ws = dmalloc(q->synth_ws_bytes);
-    synth_init_workspace(q->Ng, q->synth_ws);
-  }
+  ensure_synth(q);
   if (need_split) alloc_split(q, f);
   const int first = need_split ? std::min(fp_from, col_from) : fp_from;
   for (int s0 = first / q->chunk * q->chunk; s0 < nn; s0 += q->synth_batch) {
@@ -363,6 +363,7 @@ void ensure_level_fields(bsk_plan* q, int s, cudaStream_t st, int nn, int fp_fro
 
 void free_slot(FieldSlot& f) {
   if (f.spec) cudaFree(f.spec);
+  if (f.fine) cudaFree(f.fine);
   if (f.fields) cudaFree(f.fields);
   if (f.split) cudaFree(f.split);
   f = FieldSlot{};
@@ -388,7 +389,6 @@ void destroy_plan(bsk_plan* p) {
   for (auto& s : p->slot) free_slot(s);
   if (p->table) cudaFree(p->table);
   if (p->range) cudaFree(p->range);
-  if (p->d_radius) cudaFree(p->d_radius);
   if (p->d_edges) cudaFree(p->d_edges);
   if (p->chunk_spec) cudaFree(p->chunk_spec);
   if (p->cic_w) cudaFree(p->cic_w);
@@ -476,10 +476,7 @@ void chunk_fields(bsk_plan* p, int slot, int s0, int C, float* dst, cudaStream_t
   const bool ws_fits = p->synth_ws || p->mem_budget == 0 ||
                        footprint(p) + (int64_t)p->synth_ws_bytes <= (int64_t)p->mem_budget;
   if (p->use_synth && ws_fits) {
-    if (!p->synth_ws) {
-      p->synth_ws = dmalloc(p->synth_ws_bytes);
-      synth_init_workspace(p->Ng, p->synth_ws);
-    }
+    ensure_synth(p, false);
     for (int b = 0; b < C; b += p->chunk) {
       const int first = s0 + b;
       const int ns = std::max(0, std::min(p->chunk, p->n - first));
@@ -662,7 +659,6 @@ bsk_plan* level_plan(bsk_plan* p, int Ng, int n) {
   q->use_synth = synth_supported(Ng);
   BSK_REQUIRE(q->use_synth, BSK_ERR_STATE, "internal: no field synthesis for a grid level");
   size_synth(q.get(), p->mem_budget);
-  make_range(q.get());
   p->levels.push_back(q.get());
   return q.release();
 }
@@ -739,24 +735,33 @@ void build_levels(bsk_plan* p, bsk_triset* set) {
   }
 }
 
-// The contraction scratch of a set's resident launches (levels run one after the other and
-// share it).  Without room for it, or under a memory budget, the set runs without; it is a
-// triangle set's resource, like its schedule, so the plan's footprint does not count it
-// (callers size budgets from that figure).
-void attach_scratch(bsk_plan* p, bsk_triset* set) {
-  if (p->mem_budget) return;
-  size_t need = set->levels.empty()
-                    ? contract_tc_scratch(set->sched.h_tiles, p->K, p->num_sms) : 0;
+// The contraction scratch that a set's resident launches want (levels run one after the other
+// and share it); none under a memory budget.
+size_t scratch_need(const bsk_plan* p, const bsk_triset* set) {
+  if (p->mem_budget) return 0;
+  if (set->levels.empty()) return contract_tc_scratch(set->sched.h_tiles, p->K, p->num_sms);
+  size_t need = 0;
   for (const GridLevel& lv : set->levels)
     need = std::max(need, contract_tc_scratch(lv.sched.h_tiles, lv.plan->K, p->num_sms));
-  if (!need) return;
-  if (p->tail_scratch.empty() || p->tail_scratch.back().second < need) {
+  return need;
+}
+
+// Taken with the set's first tensor-core measurement (not when that is being captured, where
+// nothing can be allocated).  Without room for it the set runs without.  It is a triangle
+// set's resource, like its schedule, so the plan's footprint does not count it (callers size
+// budgets from that figure).
+void attach_scratch(bsk_plan* p, const bsk_triset* set, cudaStream_t st) {
+  if (set->scratch || !set->scratch_need) return;
+  if (p->tail_scratch.empty() || p->tail_scratch.back().second < set->scratch_need) {
+    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+    BSK_CHECK_CUDA(cudaStreamIsCapturing(st, &cap));
+    if (cap != cudaStreamCaptureStatusNone) return;
     void* ptr = nullptr;
-    if (cudaMalloc(&ptr, need) != cudaSuccess) {
+    if (cudaMalloc(&ptr, set->scratch_need) != cudaSuccess) {
       cudaGetLastError();
       return;
     }
-    p->tail_scratch.emplace_back(ptr, need);
+    p->tail_scratch.emplace_back(ptr, set->scratch_need);
   }
   set->scratch = p->tail_scratch.back().first;
   set->scratch_bytes = p->tail_scratch.back().second;
@@ -879,6 +884,7 @@ void measure_b(bsk_plan* p, const bsk_triset* set, int a, int b, int c, int prec
     release_stream(p);
   }
   p->last_stream_C = 0;
+  if (tc) attach_scratch(p, set, st);
   if (!set->levels.empty()) {
     measure_levels(p, set, a, b, c, precision, k0, k1, out, st);
     return;
@@ -1080,10 +1086,7 @@ int bsk_plan_create(int nmesh, double box_size, int n_shells, const double* shel
       p->shell_r[s] = (int)std::min<double>(std::max(q, 0.0), qmax);
     }
     p->use_synth = synth_supported(p->Ng);
-    if (p->use_synth) {
-      size_synth(p.get(), mem_budget);
-      make_range(p.get());
-    }
+    if (p->use_synth) size_synth(p.get(), mem_budget);
     p->use_levels = grid_mode == BSK_GRID_REDUCED && p->Ng != p->N && p->use_synth;
     make_r2c(p.get());
     make_c2r(p.get());
@@ -1158,7 +1161,7 @@ int bsk_triset_create(bsk_plan* p, int64_t n_tri, const int32_t* tri, bsk_triset
     }
     build_schedule(s->u_tri, p->n, s->sched, &s->u_idx);
     if (p->use_levels && !s->u_tri.empty()) build_levels(p, s.get());
-    attach_scratch(p, s.get());
+    s->scratch_need = scratch_need(p, s.get());
     if (!dups.empty()) {
       s->n_dups = (int)dups.size();
       s->dups = (int2*)dmalloc(dups.size() * sizeof(int2));
@@ -1250,6 +1253,8 @@ void make_r2c_sub(bsk_plan* p, int nfull) {
   grow_work(p, ws);
 }
 
+constexpr size_t kKeptFine = (size_t)80 << 20;  // 256^3 and below
+
 void paint(bsk_plan* p, int slot, const float* mesh, int nmesh_cic, cudaStream_t st,
            int nfull = 0) {
   BSK_REQUIRE(p && mesh, BSK_ERR_ARG, "NULL argument");
@@ -1262,14 +1267,23 @@ void paint(bsk_plan* p, int slot, const float* mesh, int nmesh_cic, cudaStream_t
   }
   if (nfull) make_r2c_sub(p, nfull);
   cufftHandle h = nfull ? p->r2c_sub : p->r2c;
-  size_t fine_elems = (size_t)p->N * p->N * (p->N / 2 + 1);
-  AsyncTemp fine_t(fine_elems * sizeof(cufftComplex), st);
-  cufftComplex* fine = (cufftComplex*)fine_t.ptr;
+  const size_t fine_bytes = (size_t)p->N * p->N * (p->N / 2 + 1) * sizeof(cufftComplex);
+  // A small mesh's slot keeps the scratch of its transform: allocating it from the stream's pool
+  // takes longer than a 64^3 paint, and after a synchronisation, which empties the pool, 60 us
+  // more.  Without room, and for large meshes and under a memory budget, it is taken per call.
+  if (!f.spec && !p->mem_budget && fine_bytes <= kKeptFine &&
+      cudaMalloc(&f.fine, fine_bytes) != cudaSuccess) {
+    cudaGetLastError();
+    f.fine = nullptr;
+  }
+  std::unique_ptr<AsyncTemp> fine_t;
+  if (!f.fine) fine_t.reset(new AsyncTemp(fine_bytes, st));
+  cufftComplex* fine = f.fine ? f.fine : (cufftComplex*)fine_t->ptr;
   bind_work(p, h, st);
   BSK_CHECK_CUFFT(cufftExecR2C(h, const_cast<float*>(mesh), fine));
   if (!f.spec) f.spec = (cufftComplex*)dmalloc((size_t)p->Mh * sizeof(cufftComplex));
   launch_extract(p, fine, f.spec, axis_w, st);
-  fine_t.release();
+  if (fine_t) fine_t->release();
   f.painted = true;
   ++f.gen;
   f.fields_ok = false;
@@ -1400,6 +1414,7 @@ int bsk_contract(bsk_plan* p, const bsk_triset* set, const float* f1, const floa
       split_t.reset(new AsyncTemp(split_elems(p->n, K) * sizeof(__nv_bfloat16), st));
       split = (__nv_bfloat16*)split_t->ptr;
       launch_split(f3, p->n, K, split, st);
+      attach_scratch(p, set, st);
     }
     contract_dispatch(p, set, f1, f2, f3, split, p->n, K, 0, K, precision, out, st);
     if (split_t) split_t->release();

@@ -45,6 +45,7 @@
 #include <algorithm>
 #include <climits>
 #include <cmath>
+#include <cstring>
 
 #include "bsk_internal.cuh"
 
@@ -403,28 +404,30 @@ void gridinfo_enum(bsk_plan* p, const std::vector<HostTriangle>& tri, double* nt
   const size_t n_cube = (size_t)S * S * S;
   // byte codes of the cube [-r, r]^3, kept on the device for the enumeration; the octant
   // part is read back to list the q1 modes
-  // [pad][cube][pad][cube_rev][pad][flag]: the pads hold the few bytes that the 4-byte reads
-  // of a line's first and last points take from before and after the cube
+  // [pad][cube][pad][cube_rev][pad]: the pads hold the few bytes that the 8-byte reads of a line's
+  // first and last points take from before and after the cube (not counted, whatever they
+  // are); the flag sits in the middle pad, so that one copy reads it back with the cube
   const size_t pad = 64, span = (n_cube + 15) / 16 * 16;
   char* cube_mem = nullptr;
-  BSK_CHECK_CUDA(cudaMallocAsync((void**)&cube_mem, 3 * pad + 2 * span + 16, st));
+  BSK_CHECK_CUDA(cudaMallocAsync((void**)&cube_mem, 3 * pad + 2 * span, st));
   struct FreeCube {
     char* w;
     cudaStream_t s;
     ~FreeCube() { cudaFreeAsync(w, s); }
   } free_cube{cube_mem, st};
-  BSK_CHECK_CUDA(cudaMemsetAsync(cube_mem, 0, 3 * pad + 2 * span + 16, st));
+  BSK_CHECK_CUDA(cudaMemsetAsync(cube_mem, 0, 3 * pad + 2 * span, st));
   uint8_t* d_cube = (uint8_t*)cube_mem + pad;
   uint8_t* d_cube_rev = d_cube + span + pad;
-  int* d_flag = (int*)(d_cube_rev + span + pad);
-  std::vector<uint8_t> cube(n_cube);
+  const size_t flag_at = span + 32;
+  int* d_flag = (int*)(d_cube + flag_at);
+  std::vector<uint8_t> cube(flag_at + sizeof(int));
   int flag = 0;
   cube_codes_kernel<<<p->num_sms * 8, 256, 0, st>>>(p->table, p->Ng, r, R2, d_cube, d_cube_rev,
                                                     d_flag);
   BSK_CHECK_CUDA(cudaGetLastError());
-  BSK_CHECK_CUDA(cudaMemcpyAsync(cube.data(), d_cube, n_cube, cudaMemcpyDeviceToHost, st));
-  BSK_CHECK_CUDA(cudaMemcpyAsync(&flag, d_flag, sizeof(int), cudaMemcpyDeviceToHost, st));
+  BSK_CHECK_CUDA(cudaMemcpyAsync(cube.data(), d_cube, cube.size(), cudaMemcpyDeviceToHost, st));
   BSK_CHECK_CUDA(cudaStreamSynchronize(st));
+  std::memcpy(&flag, cube.data() + flag_at, sizeof(int));
   BSK_REQUIRE(flag == 0, BSK_ERR_STATE, "internal: a mode lies in more than two shells");
   std::vector<Mode> modes;
   for (int x = 0; x <= r; ++x)

@@ -132,6 +132,7 @@ __host__ __device__ __forceinline__ int64_t split_index(int plane, int s, int64_
 struct FieldSlot {
   bool painted = false;
   cufftComplex* spec = nullptr;   // coarse half spectrum, scaled 1/N^3 (Ng*Ng*(Ng/2+1))
+  cufftComplex* fine = nullptr;   // small meshes: the mesh's own half spectrum, a paint's scratch
   float* fields = nullptr;        // [n][K] FP32 shell fields (nullptr until built)
   __nv_bfloat16* split = nullptr; // bf16 split of the n_alloc shells, chunk-major (above)
   bool fields_ok = false;
@@ -172,8 +173,8 @@ struct bsk_plan {
   int64_t K = 0;        // Ng^3
   int64_t Mh = 0;       // Ng*Ng*(Ng/2+1) half-complex modes
   uint16_t* table = nullptr;  // device [Mh] shell code
-  uint32_t* range = nullptr;  // device [n][qmax + 1]^2, the shells' |q_a| intervals
-  int* d_radius = nullptr;    // device [n], shell_r
+  uint32_t* range = nullptr;  // device [n][qmax + 1]^2, the shells' |q_a| intervals, then
+  int* d_radius = nullptr;    // [n], shell_r (same allocation; with the synthesis workspace)
   double* d_edges = nullptr;  // device [2n]
   cufftHandle r2c = 0;        // N^3 R2C
   bool r2c_ok = false;
@@ -225,8 +226,9 @@ struct bsk_triset {
   std::vector<bsk::HostTriangle> u_tri;  // first occurrences, in order
   std::vector<int> u_idx;                // their positions in the list
   mutable std::map<int, std::vector<bsk::StreamGroup>> groups;  // per streaming chunk size
-  void* scratch = nullptr;               // of the plan's tail_scratch (null: none wanted)
-  size_t scratch_bytes = 0;
+  size_t scratch_need = 0;               // contraction scratch wanted (0: none)
+  mutable void* scratch = nullptr;       // of the plan's tail_scratch, from the first measurement
+  mutable size_t scratch_bytes = 0;
   std::vector<bsk::GridLevel> levels;    // the resident path's grids (empty: the plan's only)
 };
 
