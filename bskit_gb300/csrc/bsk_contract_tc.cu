@@ -476,6 +476,8 @@ __global__ void __launch_bounds__(THREADS, 1)
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem = bars->tmem_base;
+  pdl_trigger();
+  pdl_wait();
 
   if (warp == 0) {
     // ------------------------------------------------------------ TMA producer
@@ -860,6 +862,7 @@ __global__ void __launch_bounds__(128)
                     int n_tiles, int64_t slice, int64_t k_begin, int64_t k_end,
                     const TailPlan tp, int terms, double* __restrict__ out, double scale) {
   __shared__ float sv[kTailChunk][2][32];
+  pdl_wait();
   const int c = blockIdx.x, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int r = blockIdx.y * 32 + lane;
   const int item = tp.n_full + blockIdx.z;
@@ -1095,15 +1098,12 @@ void launch_contract_tc(const DeviceSchedule& s, const float* f1, const float* f
     attr_set[dev][variant] = true;
   }
   const int grid = std::min(num_sms, sp.tp.units());
-  kern<<<grid, tc::THREADS, smem, st>>>(m, s.tiles, s.row_i, s.row_j, s.map, s.n_tiles,
-                                        f1 == f2 ? 1 : 0, (int)k_begin, (int)k_end, sp.tp, terms,
-                                        fused ? 1 : 0, out, scale);
-  BSK_CHECK_CUDA(cudaGetLastError());
-  if (sp.tp.n_tail) {
-    tc::tail_sum_kernel<<<dim3(sp.tp.nc_stride, kTileRows / 32, sp.tp.n_tail), 128, 0, st>>>(
-        s.tiles, s.map, s.n_tiles, sp.slice, k_begin, k_end, sp.tp, terms, out, scale);
-    BSK_CHECK_CUDA(cudaGetLastError());
-  }
+  const bool pdl = k_end - k_begin <= (int64_t)kPdlSide * kPdlSide * kPdlSide;
+  launch_pdl(pdl, kern, grid, tc::THREADS, smem, st, m, s.tiles, s.row_i, s.row_j, s.map, s.n_tiles,
+             f1 == f2 ? 1 : 0, (int)k_begin, (int)k_end, sp.tp, terms, fused ? 1 : 0, out, scale);
+  if (sp.tp.n_tail)
+    launch_pdl(pdl, tc::tail_sum_kernel, dim3(sp.tp.nc_stride, kTileRows / 32, sp.tp.n_tail), 128, 0, st,
+               s.tiles, s.map, s.n_tiles, sp.slice, k_begin, k_end, sp.tp, terms, out, scale);
 }
 
 void launch_contract_mod(const DeviceSchedule& s, const float* f, const __nv_bfloat16* f3_split,

@@ -94,6 +94,8 @@ __global__ void shell_range_kernel(const uint16_t* __restrict__ table, int Ng, i
 // is multiplied by w[qa] w[qb] w[qc].
 __global__ void extract_kernel(int N, int Ng, float scale, const float2* __restrict__ fine,
                                float2* __restrict__ coarse, const float* __restrict__ axis_w) {
+  pdl_trigger();
+  pdl_wait();
   const int H = Ng / 2 + 1, HN = N / 2 + 1;
   const int64_t Mh = (int64_t)Ng * Ng * H;
   for (int64_t m = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; m < Mh;
@@ -278,10 +280,9 @@ void launch_shell_range(const bsk_plan* p, uint32_t* range, int* flag, cudaStrea
 void launch_extract(const bsk_plan* p, const cufftComplex* fine, cufftComplex* coarse,
                     const float* axis_w, cudaStream_t st) {
   float scale = (float)(1.0 / ((double)p->N * p->N * p->N));
-  extract_kernel<<<grid_for(p->Mh, 256, p->num_sms * 16), 256, 0, st>>>(
-      p->N, p->Ng, scale, reinterpret_cast<const float2*>(fine), reinterpret_cast<float2*>(coarse),
-      axis_w);
-  BSK_CHECK_CUDA(cudaGetLastError());
+  launch_pdl(p->Ng <= kPdlSide, extract_kernel, grid_for(p->Mh, 256, p->num_sms * 16), 256, 0, st,
+             p->N, p->Ng, scale,
+             reinterpret_cast<const float2*>(fine), reinterpret_cast<float2*>(coarse), axis_w);
 }
 
 // A grid level's coarse spectrum from its parent's: sub[a][b][c] = parent[qa mod Ngp][qb mod

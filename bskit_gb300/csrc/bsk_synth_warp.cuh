@@ -339,8 +339,10 @@ __global__ void __launch_bounds__(32 * kWarps, min_blocks<N>())
   constexpr int L = lines_xy<N>();
   constexpr int LP = line_pitch<N, L, true>();
   float2* tw = sm + kWarps * L * LP;
-  fill_twiddles<N>(tw, A.tw);
+  pdl_trigger();
+  fill_twiddles<N>(tw, A.tw);  // written with the workspace, long before
   __syncthreads();
+  pdl_wait();
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   float2* buf = sm + warp * L * LP;
   const int nk = A.nk;
@@ -388,8 +390,10 @@ __global__ void __launch_bounds__(32 * kWarps, min_blocks<N>())
   constexpr int L = lines_xy<N>();
   constexpr int LP = line_pitch<N, L, true>();
   float2* tw = sm + kWarps * L * LP;
-  fill_twiddles<N>(tw, A.tw);
+  pdl_trigger();
+  fill_twiddles<N>(tw, A.tw);  // written with the workspace, long before
   __syncthreads();
+  pdl_wait();
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   float2* buf = sm + warp * L * LP;
   const int nk = A.nk;
@@ -456,8 +460,10 @@ __global__ void __launch_bounds__(32 * kWarps, min_blocks<N>())
   constexpr int L = lines_z<N>();
   constexpr int LP = line_pitch<N, L, false>();
   float2* tw = sm + kWarps * L * LP;
-  fill_twiddles<N>(tw, A.tw);
+  pdl_trigger();
+  fill_twiddles<N>(tw, A.tw);  // written with the workspace, long before
   __syncthreads();
+  pdl_wait();
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   float2* buf = sm + warp * L * LP;
   const int Cp = A.Cp, sp = Cp + kStagePad;
@@ -580,12 +586,9 @@ void run_passes(const SynthArgs& A, const FftPlan& pl, cudaStream_t st) {
   const int runs = (A.R + LX) / LX;  // q_c = 0 .. R
   const int xu = A.ns * A.nk * runs, yu = A.ns * N * runs;
   const int zruns = (N / 2 + LZ - 1) / LZ, zu = A.ns * N * zruns;
-  x_kernel<N><<<grid(0, xu), 32 * kWarps, smem[0], st>>>(A, pl, runs, xu);
-  BSK_CHECK_CUDA(cudaGetLastError());
-  y_kernel<N><<<grid(1, yu), 32 * kWarps, smem[1], st>>>(A, pl, runs, yu);
-  BSK_CHECK_CUDA(cudaGetLastError());
-  z_kernel<N><<<grid(2, zu), 32 * kWarps, smem[2], st>>>(A, pl, zruns, zu);
-  BSK_CHECK_CUDA(cudaGetLastError());
+  launch_pdl(N <= kPdlSide, x_kernel<N>, grid(0, xu), 32 * kWarps, smem[0], st, A, pl, runs, xu);
+  launch_pdl(N <= kPdlSide, y_kernel<N>, grid(1, yu), 32 * kWarps, smem[1], st, A, pl, runs, yu);
+  launch_pdl(N <= kPdlSide, z_kernel<N>, grid(2, zu), 32 * kWarps, smem[2], st, A, pl, zruns, zu);
 }
 
 // Compiled lengths, spread over translation units; false when N is not one of a unit's.
