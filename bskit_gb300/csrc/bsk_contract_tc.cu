@@ -81,8 +81,12 @@ constexpr int A_TILE = 4 * A_QUARTER;         // 32 KB: one source tile of a sta
 // shared-memory loads are latency-bound: 4 per quadrant ran 3.5% faster than 2, with 72
 // registers a thread instead of 96.
 constexpr int AGW = 4;
-constexpr int NUM_WARPS = 10 + 4 * AGW;       // producer, MMA, 8 drain, 4 AGW A-operand
-constexpr int THREADS = NUM_WARPS * 32;
+// Drain warps: one per TMEM lane quadrant and 32 columns.  A launch whose tiles all have at most
+// 32 columns runs four (kNarrow): four warps fewer to poll a barrier and 80 registers a thread
+// instead of 72.
+template <bool kNarrow> constexpr int kDrain = kNarrow ? 4 : 8;
+// producer, MMA, drain, 4 AGW A-operand
+template <bool kNarrow> constexpr int kThreads = (2 + kDrain<kNarrow> + 4 * AGW) * 32;
 constexpr uint32_t TMEM_COLS = 512;
 constexpr uint32_t ACC_COL = 0;               // accumulator b at 128 b: [0,nc) hi*Bhi+lo*Bhi, [nc,2nc) hi*Blo+lo*Blo
 constexpr uint32_t A_COL = 256;               // A stage a at 256 + 128 a: hi +0..63, lo +64..127
@@ -423,9 +427,9 @@ __device__ __forceinline__ Work decode(int u, const TailPlan& tp, int kSlice, in
   return w;
 }
 
-// 26 warps: 7 share one SM sub-partition, whose 16K registers allow 73 per thread.
-template <bool kTwoSrc, bool kLongSlice, bool kTail, bool kMod = false>
-__global__ void __launch_bounds__(THREADS, 1)
+// 26 warps: 7 share one SM sub-partition, whose 16K registers allow 73 per thread (22: 85).
+template <bool kTwoSrc, bool kLongSlice, bool kTail, bool kNarrow, bool kMod = false>
+__global__ void __launch_bounds__(kThreads<kNarrow>, 1)
     contract_tc_kernel(const __grid_constant__ Maps maps, const TileDesc* __restrict__ tiles,
                        const int16_t* __restrict__ row_i, const int16_t* __restrict__ row_j,
                        const int32_t* __restrict__ map, int n_tiles, int same_src,
@@ -450,15 +454,12 @@ __global__ void __launch_bounds__(THREADS, 1)
       mbar_init(&bars->full[s], 1);
       mbar_init(&bars->full_b[s], 1);
       mbar_init(&bars->src_free[s], 4 * AGW);
-
     }
     for (int a = 0; a < ASTAGES; ++a) {
       mbar_init(&bars->afull[a], 4 * AGW);
-
     }
     for (int b = 0; b < NACC; ++b) {
-
-      mbar_init(&bars->accempty[b], 8);
+      mbar_init(&bars->accempty[b], kDrain<kNarrow>);
     }
     for (int d = 0; d < DONE_RING; ++d) mbar_init(&bars->done[d], 1);
     mbar_init(&bars->all_done, 1);
@@ -488,7 +489,6 @@ __global__ void __launch_bounds__(THREADS, 1)
         const Work w = decode<kTail>(u, tp, slice, n_tiles, k_begin, k_end);
         const TileDesc td = tiles[w.tile];
         const bool one_src = !kTwoSrc || (same_src && td.i0 == td.j0);
-        
         // bytes per stage: the four 32-point quarters of each source tile; the column rows
         // of hi and lo in both K blocks
         const uint32_t src_bytes =
@@ -546,7 +546,6 @@ __global__ void __launch_bounds__(THREADS, 1)
     for (int u = blockIdx.x; u < n_units && ok; u += gridDim.x) {
       const Work w = decode<kTail>(u, tp, slice, n_tiles, k_begin, k_end);
       const TileDesc td = tiles[w.tile];
-      
       // hi x [Bhi; Blo] and lo x [Bhi; Blo] (the lo rows of a block sit right after its nc
       // hi rows; N = 2 nc, a multiple of 16).  bf16 (one term): hi x Bhi, N = nc rounded up
       // to 16 (with nc an odd multiple of 8 the last 8 columns take lo rows, never read).
@@ -591,7 +590,7 @@ __global__ void __launch_bounds__(THREADS, 1)
     if (elect_one()) tc_commit(&bars->all_done);
     __syncwarp();
     mbar_wait(&bars->all_done, 0);
-  } else if (warp < 10) {
+  } else if (warp < 2 + kDrain<kNarrow>) {
     // ------------------------------------------------------------ accumulator drain
     const int qd = warp & 3;
     const int c0 = ((warp - 2) >> 2) * 32;  // this warp's 32 accumulator columns
@@ -735,7 +734,7 @@ __global__ void __launch_bounds__(THREADS, 1)
     // ------------------------------------------------------------ A-operand producers
     const int qd = warp & 3;
     constexpr int PPW = KCH / AGW, NG = PPW / 8;  // points per warp, 8-point groups
-    const int part = (warp - 10) >> 2;  // points [PPW part, PPW part + PPW) of a stage
+    const int part = (warp - 2 - kDrain<kNarrow>) >> 2;  // points [PPW part, PPW part + PPW) of a stage
     const int r = qd * 32 + lane;
     const uint32_t tlane = (uint32_t)(qd * 32) << 16;
     uint32_t chunk = 0;
@@ -744,7 +743,6 @@ __global__ void __launch_bounds__(THREADS, 1)
       const Work w = decode<kTail>(u, tp, slice, n_tiles, k_begin, k_end);
       const TileDesc td = tiles[w.tile];
       const bool one_src = !kTwoSrc || (same_src && td.i0 == td.j0);
-      
       // a quadrant whose 32 rows are all past the tile's pairs forms nothing: its accumulator
       // rows depend on its A rows alone and the drain skips them (short grids only: their sets
       // fill a fraction of one tile, and the test cost the large ones 0.8%)
@@ -1077,14 +1075,18 @@ void launch_contract_tc(const DeviceSchedule& s, const float* f1, const float* f
   sp.tp.scratch = (float*)scratch;
   const bool long_slice = sp.slice == tc::kSliceLong;
   constexpr int kMaxDev = 64;
-  static std::atomic<bool> attr_set[kMaxDev][8];  // zero-initialised: false
+  static std::atomic<bool> attr_set[kMaxDev][16];  // zero-initialised: false
   int dev = 0;
   BSK_CHECK_CUDA(cudaGetDevice(&dev));
   BSK_REQUIRE(dev < kMaxDev, BSK_ERR_UNSUPPORTED, "device ordinal above 63");
+  bool narrow = true;
+  for (const TileDesc& d : s.h_tiles) narrow = narrow && d.nc <= 32;
   const auto pick = [&](auto two, auto tail) {
     constexpr bool kTwo = decltype(two)::value, kTail = decltype(tail)::value;
-    return long_slice ? tc::contract_tc_kernel<kTwo, true, kTail>
-                      : tc::contract_tc_kernel<kTwo, false, kTail>;
+    return narrow ? (long_slice ? tc::contract_tc_kernel<kTwo, true, kTail, true>
+                                : tc::contract_tc_kernel<kTwo, false, kTail, true>)
+                  : (long_slice ? tc::contract_tc_kernel<kTwo, true, kTail, false>
+                                : tc::contract_tc_kernel<kTwo, false, kTail, false>);
   };
   const bool tail = sp.tp.n_tail > 0;
   const auto yes = std::true_type{};
@@ -1092,15 +1094,16 @@ void launch_contract_tc(const DeviceSchedule& s, const float* f1, const float* f
   auto kern = two_src ? (tail ? pick(yes, yes) : pick(yes, no))
                       : (tail ? pick(no, yes) : pick(no, no));
   const int smem = two_src ? tc::smem_bytes<true>() : tc::smem_bytes<false>();
-  const int variant = (two_src ? 4 : 0) + (long_slice ? 2 : 0) + (tail ? 1 : 0);
+  const int variant = (narrow ? 8 : 0) + (two_src ? 4 : 0) + (long_slice ? 2 : 0) + (tail ? 1 : 0);
   if (!attr_set[dev][variant]) {
     BSK_CHECK_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
     attr_set[dev][variant] = true;
   }
   const int grid = std::min(num_sms, sp.tp.units());
   const bool pdl = k_end - k_begin <= (int64_t)kPdlSide * kPdlSide * kPdlSide;
-  launch_pdl(pdl, kern, grid, tc::THREADS, smem, st, m, s.tiles, s.row_i, s.row_j, s.map, s.n_tiles,
-             f1 == f2 ? 1 : 0, (int)k_begin, (int)k_end, sp.tp, terms, fused ? 1 : 0, out, scale);
+  launch_pdl(pdl, kern, grid, narrow ? tc::kThreads<true> : tc::kThreads<false>, smem, st, m, s.tiles,
+             s.row_i, s.row_j, s.map, s.n_tiles, f1 == f2 ? 1 : 0, (int)k_begin, (int)k_end, sp.tp,
+             terms, fused ? 1 : 0, out, scale);
   if (sp.tp.n_tail)
     launch_pdl(pdl, tc::tail_sum_kernel, dim3(sp.tp.nc_stride, kTileRows / 32, sp.tp.n_tail), 128, 0, st,
                s.tiles, s.map, s.n_tiles, sp.slice, k_begin, k_end, sp.tp, terms, out, scale);
@@ -1132,10 +1135,13 @@ void launch_contract_mod(const DeviceSchedule& s, const float* f, const __nv_bfl
   tp.mod_p = (float)p;
   tp.mod_inv = 1.f / (float)p;
   tp.n_full = (stages + slice - 1) / slice * s.n_tiles;
-  auto kern = tc::contract_tc_kernel<false, false, false, true>;
+  bool narrow = true;
+  for (const TileDesc& d : s.h_tiles) narrow = narrow && d.nc <= 32;
+  auto kern = narrow ? tc::contract_tc_kernel<false, false, false, true, true>
+                     : tc::contract_tc_kernel<false, false, false, false, true>;
   const int smem = tc::smem_bytes<false>();
   BSK_CHECK_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
-  kern<<<std::min(num_sms, tp.n_full), tc::THREADS, smem, st>>>(
+  kern<<<std::min(num_sms, tp.n_full), narrow ? tc::kThreads<true> : tc::kThreads<false>, smem, st>>>(
       m, s.tiles, s.row_i, s.row_j, s.map, s.n_tiles, 1, 0, (int)K, tp, 3, 1,
       reinterpret_cast<double*>(out), 1.0);
   BSK_CHECK_CUDA(cudaGetLastError());
