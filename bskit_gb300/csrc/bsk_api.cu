@@ -341,7 +341,9 @@ void ensure_level_fields(bsk_plan* q, int s, cudaStream_t st, int nn, int fp_fro
   if (need_split) alloc_split(q, f);
   const int first = need_split ? std::min(fp_from, col_from) : fp_from;
   for (int s0 = first / q->chunk * q->chunk; s0 < nn; s0 += q->synth_batch) {
-    const int ns = std::min(q->synth_batch, q->n - s0);
+    // up to nn only: a column-only slot has no FP32 fields, and a shell past nn >= fp_from of a
+    // batch cut at the level plan's n (every shell that fits its side) would be written to them
+    const int ns = std::min(q->synth_batch, nn - s0);
     const bool cols = s0 < col_to && s0 + ns > col_from;
     if (!cols && s0 + ns <= fp_from) continue;
     int R = 0;
@@ -1430,7 +1432,7 @@ int bsk_gridinfo(bsk_plan* p, const bsk_triset* set, double* ntri, double* kmean
     cudaStream_t st = (cudaStream_t)stream;
     if (set->T == 0) return;  // nothing to write: ntri and kmean may be NULL
     BSK_REQUIRE(ntri && kmean, BSK_ERR_ARG, "NULL argument");
-    if (gridinfo_enum_supported(p)) {  // exact integer enumeration, no FFT
+    if (gridinfo_enum_supported(p)) {  // exact, in integers: no floating-point FFT
       p->last_stream_C = 0;
       if (!gridinfo_modular(p, set->tri, ntri, kmean, st))
         gridinfo_enum(p, set->tri, ntri, kmean, st);

@@ -424,6 +424,8 @@ void launch_synth(int N, const cufftComplex* spec, const uint16_t* table, const 
                   int fields_from, int split_to) {
   FftPlan pl;
   BSK_REQUIRE(make_plan(N, pl), BSK_ERR_UNSUPPORTED, "no FFT plan for this grid size");
+  BSK_REQUIRE(fields || s0 + ns <= fields_from, BSK_ERR_STATE,
+              "internal: no FP32 fields to write a shell to");
   R = std::min(R, N / 2);
   const int nk = std::min(2 * R + 1, N);
   const int Cp = (R + 1 + kLines - 1) / kLines * kLines;

@@ -52,3 +52,32 @@ def test_sets_of_different_shells(cuda, monkeypatch, precision):
             assert torch.all((got - want[k]).abs() <= 4096 * 2.0 ** -53 * want[k].abs().max()), \
                 (order, k)
     p.sync_check()
+
+
+@pytest.mark.parametrize("low", [11, 21, 29])
+def test_column_slot_without_fields(cuda, monkeypatch, low):
+    """A slot that is only a third shell has no FP32 fields, and its level stops inside a batch
+    of the level plan, which holds every shell that fits the side: none of the batch's further
+    shells is written.  Same contraction as on a plan whose slot has them."""
+    monkeypatch.setenv("BSK_LEVEL_MIN_POINTS", "0.01")
+    n, box = 256, 500.0
+    kf = 2 * np.pi / box
+    kw = dict(kmin=kf, kmax=64 * kf, dk=2 * kf)
+    edges = B.generate_bin_edge_list(**kw)
+    tri = B.generate_triangle_bin_list(return_indices=True, **kw)
+    tri = tri[tri.max(1) < low]
+    d = synthetic.lognormal_mesh_torch(n, box, seed=4, device=cuda).contiguous()
+    e = (1.5 * d + 0.3 * torch.randn_like(d)).contiguous()
+    got = []
+    for first in ((), ((1, 1, 0),)):
+        p = Plan(n, box, edges)
+        p.paint(0, d)
+        p.paint(1, e)
+        t = p.triangles(tri)
+        assert max(lv["shells"] for lv in t.levels()) == low
+        for slots in first:
+            p.measure_b(t, slots=slots, precision="bf16x3")
+        got.append(p.measure_b(t, slots=(0, 0, 1), precision="bf16x3"))
+        p.sync_check()
+        p.close()
+    assert torch.all((got[0] - got[1]).abs() <= 4096 * 2.0 ** -53 * got[1].abs().max())
