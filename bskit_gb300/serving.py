@@ -191,7 +191,11 @@ class Scheduler(object):
                 and (pinned_too or not getattr(g, "pinned", False))]
         if self.used - sum(g.footprint for g in idle) + need > self.mem_budget:
             return False  # would not fit even with all of them gone: destroy nothing
-        idle.sort(key=lambda g: self.last_used.get(g, 0.0))
+        # with prepared groups among them, those of shell sets that keep another group go
+        # first: the only 512^3 group is not given up for what one of four 256^3 groups frees
+        def shared(g):
+            return sum(1 for o in self.groups if o.shell_key == g.shell_key) > 1
+        idle.sort(key=lambda g: (pinned_too and not shared(g), self.last_used.get(g, 0.0)))
         while self.used + need > self.mem_budget and idle:
             g = idle.pop(0)
             self.backend.destroy_group(g)

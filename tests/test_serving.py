@@ -118,6 +118,18 @@ def test_prepared_groups_are_kept_unless_a_shell_set_has_no_group():
     assert sorted(be.destroyed) == [32, 32, 64]
 
 
+def test_a_first_group_takes_the_place_of_one_of_several():
+    be = FakeBackend()
+    # one 64^3 group (1280) and two 32^3 groups (640 each) leave 40: the first 16^3 group (320)
+    # takes a 32^3 group's place, not that of the only 64^3 group, although that is older
+    sch = serving.Scheduler(be, mem_budget=2600, max_batch=2, max_groups=2, clock=FakeClock())
+    sch.prepare([_req(0, 64)], groups=1)
+    sch.prepare([_req(1, 32)])
+    sch.prepare([_req(2, 16)], groups=1)
+    assert be.created == [(64, 2), (32, 2), (32, 2), (16, 2)] and be.destroyed == [32]
+    assert sorted(g.shell_key[0] for g in sch.groups) == [16, 32, 64]
+
+
 def test_no_eviction_for_a_group_that_cannot_fit_and_smaller_groups_tried_first():
     be = FakeBackend()
     # a 64^3 group of 4 (2560) cannot fit a 2000 budget even in an empty server; a group of
