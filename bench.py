@@ -238,16 +238,29 @@ class ClockSampler(object):
 def kernel_launches_per_step(plan, ts, slots=(0, 0, 0)):
     """Kernels of libbskit_gb300 launched by one step (cuFFT's R2C kernels excluded): the
     spectrum extraction of each painted slot; per grid level the level's spectrum (levels
-    below the plan's grid), the field synthesis (X, Y, Z passes per batch of 8 shells, the
-    bf16 split written by the Z pass) and one contraction; the normalisation."""
+    below the plan's grid), the field synthesis (X, Y, Z passes per batch of 8 shells from the
+    first that the level's bins use, the bf16 split written by the Z pass) and one
+    contraction; the normalisation.  (The sums of a contraction's last wave, on some sizes,
+    are one launch more.)"""
+    import numpy as np
     nslot = len(set(slots))
     levels = ts.levels()
     n = nslot
     if levels:
+        # a level holds the bins that fit its side and no smaller level's; batches below its
+        # bins' first shell are not synthesised
+        kf = 2 * np.pi / plan.box_size
+        r = np.floor(np.asarray(plan.shell_edges).reshape(-1, 2)[:, 1] / kf * (1 + 1e-9))
+        tri = ts.indices
+        need = np.maximum(r[tri].sum(1), 2 * r[tri].max(1))
+        done = np.zeros(len(tri), bool)
         for lv in levels:
             if lv["ngrid"] != plan.ngrid:
                 n += nslot
-            n += 3 * ((lv["shells"] + 7) // 8) * nslot + 1
+            mine = ~done & ((need < lv["ngrid"]) | (lv is levels[-1]))
+            done |= mine
+            first = int(tri[mine].min()) // 8 if mine.any() else 0
+            n += 3 * ((lv["shells"] + 7) // 8 - first) * nslot + 1
     else:
         n += 3 * ((plan.n_shells + 7) // 8) * nslot + 1 + 1  # synthesis, contraction, scale
     return n + 1

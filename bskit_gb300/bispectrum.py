@@ -48,8 +48,8 @@ class FFTBispectrum(object):
 
     Extra keyword arguments beyond bskit's:
     precision : 'bf16x3' (default), 'fp32', 'bf16' or 'fp64' -- arithmetic of the
-        triple-product contraction of B (grid information is exact: integer lattice
-        enumeration, or FP64 fields where that does not apply);
+        triple-product contraction of B (grid information is exact: integer sums over the
+        lattice triangles, or FP64 fields where those do not apply);
     grid : 'reduced' (default: each bin on the smallest exact grid its shells allow),
         'single' (the reduced grid for every bin) or 'native' -- see ``engine.Plan``;
     device : CUDA device of the computation;

@@ -13,7 +13,7 @@
 // triple-product contraction of the tensor-core kernel (launch_contract_mod), instead of a
 // visit to every pair of modes: ~qmax^6 pairs against ~qmax^3 points times bins.  At 512^3 (63
 // shells to |q| = 127) 1.81 s -> 90 ms (contraction 41, last axis 23, first two 17), at 256^3 (31
-// shells to 63) 41 -> 5.9 ms, at |q| <= 40 (14 shells) 3.9 -> 1.8 ms; the enumeration's two
+// shells to 63) 41 -> 5.3 ms, at |q| <= 40 (14 shells) 3.9 -> 1.8 ms; the enumeration's two
 // launches are kept below that (kMinQ).
 //
 // Symmetry.  Membership and w do not change under sign flips of a component or the x <-> y swap

@@ -16,7 +16,7 @@
  *  - `stream` is a cudaStream_t passed as void* (NULL = legacy default).
  *    Work is enqueued on that stream; the host does not synchronise except
  *    in bsk_plan_create / bsk_triset_create / bsk_shell_mode_counts /
- *    bsk_compensate_cic / bsk_sync_check / bsk_gridinfo (enumeration path) /
+ *    bsk_compensate_cic / bsk_sync_check / bsk_gridinfo (exact routes) /
  *    bsk_contract_noalloc (which waits for its own schedule copies on `stream`
  *    and so cannot be captured).
  *  - A plan is bound to the CUDA device that was current at creation.
@@ -220,10 +220,11 @@ int bsk_measure_b_range(bsk_plan* plan, const bsk_triset* set, int slot_a, int s
  * kmean[3t+a] = mean |k_a| over the bin's triangles (NaN when ntri == 0).
  * When no triangle of shell modes can wrap around the grid (grid side above
  * three times the largest |q_c| of a shell mode: every reduced plan) and the
- * plan has at most 64 shells, the sums are evaluated exactly by enumerating
- * the lattice triangles q1 + q2 + q3 = 0 (integer counts, fixed-point |q|
- * sums); otherwise from FP64 indicator / |k| fields and an FP64 contraction
- * (counts are the rounded FP64 sums).  The enumeration synchronises `stream`.
+ * plan has at most 64 shells, the sums over the lattice triangles q1 + q2 + q3
+ * = 0 are evaluated exactly (integer counts, fixed-point |q| sums): from
+ * residues modulo small primes when 40 <= qmax <= 159 and the temporary memory
+ * (3.4 GB for 63 shells at 512^3) fits, else by enumeration; otherwise from FP64 indicator / |k| fields and an FP64 contraction
+ * (counts are the rounded FP64 sums).  The exact routes synchronise `stream`.
  * Replaces: FFTBispectrum.measure_gridinfo_faster, bskit/main.py:1941-2132,
  *           compute_Nbin / compute_k_means_on_grid, main.py:431-567.
  */
