@@ -400,7 +400,8 @@ void destroy_plan(bsk_plan* p) {
   if (p->z2d_ok) cufftDestroy(p->z2d);
   if (p->work) cudaFree(p->work);
   if (p->synth_ws) cudaFree(p->synth_ws);
-  for (auto& b : p->tail_scratch) cudaFree(b.first);
+  if (p->tail_scratch) cudaFree(p->tail_scratch);
+  if (p->tail_done) cudaEventDestroy(p->tail_done);
   release_stream(p);
   delete p;
 }
@@ -418,6 +419,59 @@ void copy_dups(const bsk_triset* set, double* v, cudaStream_t st) {
   BSK_CHECK_CUDA(cudaGetLastError());
 }
 
+// The contraction scratch of one measurement (set->scratch_need).  Eager calls share the plan's,
+// taken with the first that wants it; as calls may come on several streams, each waits for
+// the last one's use of it on another.  A captured call takes its own from the
+// stream's pool (an allocation node of its graph), as graphs replay on any streams.  Without room
+// a set runs without.  The scratch is a triangle set's resource, like its schedule, so the
+// plan's footprint does not count it (callers size budgets from that figure).
+struct TailScratch {
+  bsk_plan* p;
+  cudaStream_t st;
+  void* ptr = nullptr;
+  size_t bytes = 0;
+  std::unique_ptr<AsyncTemp> own;
+  TailScratch(bsk_plan* plan, const bsk_triset* set, int precision, cudaStream_t s)
+      : p(plan), st(s) {
+    const size_t need = set->scratch_need;
+    if (!need || (precision != BSK_PREC_BF16X3 && precision != BSK_PREC_BF16)) return;
+    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+    BSK_CHECK_CUDA(cudaStreamIsCapturing(st, &cap));
+    if (cap != cudaStreamCaptureStatusNone) {
+      own.reset(new AsyncTemp(need, st));
+      ptr = own->ptr;
+      bytes = need;
+      return;
+    }
+    if (!p->tail_done)
+      BSK_CHECK_CUDA(cudaEventCreateWithFlags(&p->tail_done, cudaEventDisableTiming));
+    if (p->tail_bytes < need) {
+      if (p->tail_scratch) cudaFree(p->tail_scratch);  // waits for the work that uses it
+      p->tail_scratch = nullptr;
+      p->tail_bytes = 0;
+      if (cudaMalloc(&p->tail_scratch, need) != cudaSuccess) {
+        cudaGetLastError();
+        p->tail_scratch = nullptr;
+        return;
+      }
+      p->tail_bytes = need;
+    }
+    unsigned long long id = 0;  // unlike the handle, never used again
+    BSK_CHECK_CUDA(cudaStreamGetId(st, &id));
+    if (id != p->tail_stream) BSK_CHECK_CUDA(cudaStreamWaitEvent(st, p->tail_done, 0));
+    p->tail_stream = id;
+    ptr = p->tail_scratch;
+    bytes = p->tail_bytes;
+  }
+  void release() {  // everything that uses it is enqueued
+    if (own) {
+      own->release();
+    } else if (ptr) {
+      BSK_CHECK_CUDA(cudaEventRecord(p->tail_done, st));
+    }
+  }
+};
+
 void contract_dispatch(bsk_plan* p, const bsk_triset* set, const float* f1, const float* f2,
                        const float* f3, const __nv_bfloat16* split, int split_shells,
                        int64_t K, int64_t k0, int64_t k1, int precision, double* out,
@@ -431,11 +485,14 @@ void contract_dispatch(bsk_plan* p, const bsk_triset* set, const float* f1, cons
       launch_contract_simt_f32(set->sched, f1, f2, f3, p->n, K, k0, k1, out, p->num_sms, st);
       break;
     case BSK_PREC_BF16X3:
-    case BSK_PREC_BF16:
+    case BSK_PREC_BF16: {
+      TailScratch ts(p, set, precision, st);
       launch_contract_tc(set->sched, f1, f2, split, split_shells, p->n, K, k0, k1,
-                         precision == BSK_PREC_BF16X3 ? 3 : 1, out, p->num_sms, st, 1.0,
-                         set->scratch, set->scratch_bytes);
+                         precision == BSK_PREC_BF16X3 ? 3 : 1, out, p->num_sms, st, 1.0, ts.ptr,
+                         ts.bytes);
+      ts.release();
       break;
+    }
     default:
       throw Error{BSK_ERR_ARG, "unknown precision " + std::to_string(precision)};
   }
@@ -748,27 +805,6 @@ size_t scratch_need(const bsk_plan* p, const bsk_triset* set) {
   return need;
 }
 
-// Taken with the set's first tensor-core measurement (not when that is being captured, where
-// nothing can be allocated).  Without room for it the set runs without.  It is a triangle
-// set's resource, like its schedule, so the plan's footprint does not count it (callers size
-// budgets from that figure).
-void attach_scratch(bsk_plan* p, const bsk_triset* set, cudaStream_t st) {
-  if (set->scratch || !set->scratch_need) return;
-  if (p->tail_scratch.empty() || p->tail_scratch.back().second < set->scratch_need) {
-    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
-    BSK_CHECK_CUDA(cudaStreamIsCapturing(st, &cap));
-    if (cap != cudaStreamCaptureStatusNone) return;
-    void* ptr = nullptr;
-    if (cudaMalloc(&ptr, set->scratch_need) != cudaSuccess) {
-      cudaGetLastError();
-      return;
-    }
-    p->tail_scratch.emplace_back(ptr, set->scratch_need);
-  }
-  set->scratch = p->tail_scratch.back().first;
-  set->scratch_bytes = p->tail_scratch.back().second;
-}
-
 // A point range [k0, k1) of the plan's grid as the matching share of a level's grid
 // (128-point aligned, so that the ranges of consecutive shards tile the level's grid).
 int64_t level_point(int64_t k, int64_t K, int64_t Kq) {
@@ -782,6 +818,7 @@ void measure_levels(bsk_plan* p, const bsk_triset* set, int a, int b, int c, int
                     int64_t k0, int64_t k1, double* out, cudaStream_t st) {
   const bool tc = precision == BSK_PREC_BF16X3 || precision == BSK_PREC_BF16;
   BSK_CHECK_CUDA(cudaMemsetAsync(out, 0, (size_t)set->T * sizeof(double), st));
+  TailScratch ts(p, set, precision, st);
   for (const GridLevel& lv : set->levels) {
     bsk_plan* q = lv.plan;
     const int nn = lv.n_shells;
@@ -821,10 +858,11 @@ void measure_levels(bsk_plan* p, const bsk_triset* set, int a, int b, int c, int
       default:
         launch_contract_tc(lv.sched, fa, fb, q->slot[c].split, q->n_alloc(), q->n, q->K, q0,
                            q1, precision == BSK_PREC_BF16X3 ? 3 : 1, out, q->num_sms, st,
-                           scale, set->scratch, set->scratch_bytes);
+                           scale, ts.ptr, ts.bytes);
         break;
     }
   }
+  ts.release();
   copy_dups(set, out, st);
 }
 
@@ -886,7 +924,6 @@ void measure_b(bsk_plan* p, const bsk_triset* set, int a, int b, int c, int prec
     release_stream(p);
   }
   p->last_stream_C = 0;
-  if (tc) attach_scratch(p, set, st);
   if (!set->levels.empty()) {
     measure_levels(p, set, a, b, c, precision, k0, k1, out, st);
     return;
@@ -1416,7 +1453,6 @@ int bsk_contract(bsk_plan* p, const bsk_triset* set, const float* f1, const floa
       split_t.reset(new AsyncTemp(split_elems(p->n, K) * sizeof(__nv_bfloat16), st));
       split = (__nv_bfloat16*)split_t->ptr;
       launch_split(f3, p->n, K, split, st);
-      attach_scratch(p, set, st);
     }
     contract_dispatch(p, set, f1, f2, f3, split, p->n, K, 0, K, precision, out, st);
     if (split_t) split_t->release();

@@ -209,9 +209,11 @@ struct bsk_plan {
   bool use_levels = false;
   bsk_plan* parent = nullptr;
   std::vector<bsk_plan*> levels;
-  // scratch of the tensor-core contraction, grown when a triangle set wants more; earlier
-  // blocks live as long as the plan (captured graphs of earlier sets hold their addresses)
-  std::vector<std::pair<void*, size_t>> tail_scratch;
+  // scratch of the eager tensor-core contractions, grown when a triangle set wants more
+  void* tail_scratch = nullptr;
+  size_t tail_bytes = 0;
+  cudaEvent_t tail_done = nullptr;  // the last use of it (TailScratch), on stream tail_stream
+  unsigned long long tail_stream = ~0ull;
   int n_alloc() const { return (n + chunk - 1) / chunk * chunk; }  // shells rounded to batches
 };
 
@@ -227,8 +229,6 @@ struct bsk_triset {
   std::vector<int> u_idx;                // their positions in the list
   mutable std::map<int, std::vector<bsk::StreamGroup>> groups;  // per streaming chunk size
   size_t scratch_need = 0;               // contraction scratch wanted (0: none)
-  mutable void* scratch = nullptr;       // of the plan's tail_scratch, from the first measurement
-  mutable size_t scratch_bytes = 0;
   std::vector<bsk::GridLevel> levels;    // the resident path's grids (empty: the plan's only)
 };
 

@@ -52,3 +52,36 @@ def test_parts_equal_whole_items(plans, k, fields, precision):
     abs_sum = plan.contract(ts, *[x.abs() for x in fs], precision="fp64")
     slices = -(-k // 16384)
     assert torch.all((got - whole).abs() <= slices * 2.0 ** -52 * 1.01 * abs_sum)
+
+
+def test_streams_and_graphs_share_no_scratch_unordered(plans):
+    """Contractions of one plan on several streams, eager and captured, overlapping as they may:
+    each gives what it gives alone (bins within the FP64 order bound above)."""
+    plan, ts, tri = plans[1]
+    k = 96 ** 3
+    g = torch.Generator(device="cuda")
+    g.manual_seed(7)
+    f = [torch.randn((plan.n_shells, k), generator=g, device="cuda") for _ in range(4)]
+    want = [plan.contract(ts, x, x, x) for x in f]
+    bound = [-(-k // 16384) * 2.0 ** -52 * 1.01 * plan.contract(ts, *[x.abs()] * 3, precision="fp64")
+             for x in f]
+    streams = [torch.cuda.Stream() for _ in f]
+    graphs, outs = [], []
+    for x, s in zip(f[:2], streams[:2]):
+        torch.cuda.synchronize()
+        gr = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(gr, stream=s):
+            outs.append(plan.contract(ts, x, x, x))
+        graphs.append(gr)
+    torch.cuda.synchronize()
+    for _ in range(5):
+        for gr, s in zip(graphs, streams[:2]):
+            with torch.cuda.stream(s):
+                gr.replay()
+        eager = []
+        for x, s in zip(f[2:], streams[2:]):
+            with torch.cuda.stream(s):
+                eager.append(plan.contract(ts, x, x, x))
+        torch.cuda.synchronize()
+        for got, w, b in zip(outs + eager, want, bound):
+            assert torch.all((got - w).abs() <= b)
