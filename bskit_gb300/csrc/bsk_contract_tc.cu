@@ -1158,4 +1158,9 @@ int tc_error_flag(bool reset) {
   return v;
 }
 
+void tc_error_flag_async(int* out, cudaStream_t st) {
+  BSK_CHECK_CUDA(cudaMemcpyFromSymbolAsync(out, tc::g_tc_error, sizeof(int), 0,
+                                           cudaMemcpyDeviceToHost, st));
+}
+
 }  // namespace bsk

@@ -629,10 +629,12 @@ bool gridinfo_modular(bsk_plan* p, const std::vector<HostTriangle>& tri, double*
   const int* radius = (const int*)(base + a_up + o_rad);
   BSK_CHECK_CUDA(cudaMemsetAsync(cnt, 0, (char*)(flag + 2) - (char*)cnt, st));
   launch_shell_range(p, range, flag, st);
-  int hflag = 0;
+  int hflag = 0, gave_up = 0;
   BSK_CHECK_CUDA(cudaMemcpyAsync(&hflag, flag, sizeof(int), cudaMemcpyDeviceToHost, st));
+  tc_error_flag_async(&gave_up, st);
   BSK_CHECK_CUDA(cudaStreamSynchronize(st));
   BSK_REQUIRE(hflag == 0, BSK_ERR_STATE, "internal: a mode lies in more than two shells");
+  if (gave_up) return false;  // set by an earlier launch: it cuts the waits of later ones short
 
   DeviceSchedule dc, ds;
   sc.bind(base + a_up, dc);
@@ -693,8 +695,10 @@ bool gridinfo_modular(bsk_plan* p, const std::vector<HostTriangle>& tri, double*
       T, (const int4*)(base + a_up + o_idx), g, n_cnt, ne, ns, cnt, sum, kf, ntri, kmean);
   BSK_CHECK_CUDA(cudaGetLastError());
   dc.tiles = ds.tiles = nullptr;  // in the scratch block: nothing to release
+  // a contraction that gave up has left sums out, and any residues make a count of some kind
+  tc_error_flag_async(&gave_up, st);
   BSK_CHECK_CUDA(cudaStreamSynchronize(st));  // the host tables must outlive their copy
-  return true;
+  return !gave_up;
 }
 
 }  // namespace bsk

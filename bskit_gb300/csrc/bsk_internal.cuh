@@ -340,14 +340,17 @@ void launch_contract_mod(const DeviceSchedule& s, const float* f, const __nv_bfl
 
 // Bounded-wait error flag of the tcgen05 kernel (1 = a wait expired); optionally reset.
 int tc_error_flag(bool reset);
+// The same, as the work before it on `st` leaves it; valid once `st` has been synchronised.
+void tc_error_flag_async(int* out, cudaStream_t st);
 
 // Grid information by exact lattice enumeration (counts and |k| sums in integers) for
 // plans whose shell modes cannot form a triangle that wraps around the grid and that have
 // at most 64 shells; ntri[T], kmean[T][3] (device).  Synchronises `st`.
 bool gridinfo_enum_supported(const bsk_plan* p);
 // The same sums from residues of the shells' count and |k| fields modulo small primes
-// (bsk_gridinfo_modular.cu): faster for large |q|.  False, with nothing done, when the plan's
-// |q| range is below or above what it is for or its scratch does not fit.
+// (bsk_gridinfo_modular.cu): faster for large |q|.  False when the plan's |q| range is below or
+// above what it is for, its scratch does not fit, or a contraction gave up waiting (the error
+// flag, which stays set): the outputs are then to be computed another way.
 bool gridinfo_modular(bsk_plan* p, const std::vector<HostTriangle>& tri, double* ntri,
                       double* kmean, cudaStream_t st);
 void gridinfo_enum(bsk_plan* p, const std::vector<HostTriangle>& tri, double* ntri,

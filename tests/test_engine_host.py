@@ -1,0 +1,68 @@
+"""Host side of the library on a CUDA runtime without a device (tests/engine_fake.py): what it
+allocates and reports, and which kernels a call enqueues."""
+import ctypes
+
+import numpy as np
+import pytest
+
+import engine_fake
+from bskit_gb300 import _lib
+from bskit_gb300 import bins as B
+
+TWO_PI = 2 * np.pi
+
+
+@pytest.fixture(scope="module")
+def eng(tmp_path_factory):
+    return engine_fake.Engine(engine_fake.link(str(tmp_path_factory.mktemp("fake"))))
+
+
+@pytest.fixture(autouse=True)
+def clean(eng):
+    eng.lib.fake_set_limit(0)
+    eng.lib.fake_set_capturing(0)
+    eng.lib.fake_set_symbol(0, -1)
+    eng.lib.fake_reset_counts()
+    yield
+
+
+def binning(box, kmax, dk, fields=1):
+    kf = TWO_PI / box
+    kw = dict(kmin=kf, kmax=kmax * kf, dk=dk * kf)
+    return (np.asarray(B.generate_bin_edge_list(**kw)),
+            np.asarray(B.generate_triangle_bin_list(num_fields=fields, return_indices=True, **kw)))
+
+
+def test_everything_is_given_back(eng):
+    """Plans, their levels, sets and what measurements kept of them."""
+    before = eng.live()
+    for n, kmax, grid in ((64, 16, _lib.GRID_REDUCED), (128, 32, _lib.GRID_REDUCED),
+                          (96, 40, _lib.GRID_NATIVE), (70, 16, _lib.GRID_NATIVE)):
+        edges, tri = binning(100.0, kmax, 2.0)
+        p = eng.plan(n, 100.0, edges, grid=grid)
+        ts = eng.triangles(p, tri)
+        eng.paint(p)
+        eng.paint(p, 1)
+        for prec in (_lib.PREC_BF16X3, _lib.PREC_FP32):
+            eng.measure(p, ts, (0, 0, 1), prec)
+        eng.ok(eng.lib.bsk_gridinfo(p, ts, engine_fake.OUT, engine_fake.OUT, None))
+        eng.close(p, ts)
+    assert eng.live() == before
+
+
+# the flag that an expired wait of a contraction sets: never, left by an earlier launch, set by
+# the route's own launches (second and later reads)
+@pytest.mark.parametrize("at", [-1, 0, 1])
+def test_gridinfo_does_not_trust_a_contraction_that_gave_up(eng, at):
+    edges, tri = binning(100.0, 45, 5.0)
+    p = eng.plan(192, 100.0, edges, grid=_lib.GRID_REDUCED_SINGLE)
+    assert eng.info(p, _lib.INFO_QMAX) >= 40
+    ts = eng.triangles(p, tri)
+    eng.lib.fake_reset_counts()
+    eng.lib.fake_set_symbol(1, at)
+    eng.ok(eng.lib.bsk_gridinfo(p, ts, engine_fake.OUT, engine_fake.OUT, None))
+    # the enumeration gives the answer instead, and the flag stays for bsk_sync_check
+    assert (eng.launches("enum_finish_kernel") > 0) == (at >= 0)
+    assert (eng.launches("modular_finish_kernel") > 0) == (at != 0)
+    assert eng.lib.bsk_sync_check(None) == (_lib.BSK_OK if at < 0 else _lib.BSK_ERR_TIMEOUT)
+    eng.close(p, ts)
