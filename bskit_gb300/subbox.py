@@ -136,6 +136,7 @@ class SubboxBispectrum(object):
         ntri = kmean = None
         if meas_type in ('grid_info', 'full') and tset is not None:
             nt, km = plan.gridinfo(tset)
+            plan.sync_check()
             ntri, kmean = nt.cpu().numpy(), km.cpu().numpy() / units
         fulls = None
         if meas_type in ('unnorm_b_value', 'full') and tset is not None:

@@ -128,3 +128,36 @@ def test_subbox_with_cic_matches_oracle(cuda):
     babs = O.triple_sums(np.abs(f), np.abs(f), np.abs(f), tri) * box ** 6 / n ** 3
     _check(r['B'], bo, babs)
     sb.close()
+
+
+def test_grid_info_of_subboxes_is_checked(monkeypatch):
+    """A contraction that gave up waiting is reported by the measurement that ran it, as in
+    FFTBispectrum.measure_gridinfo_faster."""
+    from bskit_gb300 import subbox
+
+    class GaveUp(Exception):
+        pass
+
+    class Set(object):
+        def close(self):
+            pass
+
+    class FakePlan(object):
+        device = torch.device("cpu")
+
+        def triangles(self, tri):
+            self.T = len(tri)
+            return Set()
+
+        def gridinfo(self, tset):
+            return torch.ones(self.T, dtype=torch.float64), torch.ones((self.T, 3))
+
+        def sync_check(self):
+            raise GaveUp()
+
+    kf = TWO_PI / 50.0
+    sb = subbox.SubboxBispectrum(np.zeros((16, 16, 16), np.float32), 2, BoxSize=100.0, dk=kf,
+                                 kmin=kf, kmax=3 * kf)
+    monkeypatch.setattr(sb.fb, "_plan", lambda edges: FakePlan())
+    with pytest.raises(GaveUp):
+        sb.measure(subboxes=[0], meas_type='grid_info')
