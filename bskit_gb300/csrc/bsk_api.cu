@@ -1307,10 +1307,12 @@ void paint(bsk_plan* p, int slot, const float* mesh, int nmesh_cic, cudaStream_t
   if (nfull) make_r2c_sub(p, nfull);
   cufftHandle h = nfull ? p->r2c_sub : p->r2c;
   const size_t fine_bytes = (size_t)p->N * p->N * (p->N / 2 + 1) * sizeof(cufftComplex);
+  const bool first = !f.spec;
+  if (first) f.spec = (cufftComplex*)dmalloc((size_t)p->Mh * sizeof(cufftComplex));
   // A small mesh's slot keeps the scratch of its transform: allocating it from the stream's pool
   // takes longer than a 64^3 paint, and after a synchronisation, which empties the pool, 60 us
   // more.  Without room, and for large meshes and under a memory budget, it is taken per call.
-  if (!f.spec && !p->mem_budget && fine_bytes <= kKeptFine &&
+  if (first && !p->mem_budget && fine_bytes <= kKeptFine &&
       cudaMalloc(&f.fine, fine_bytes) != cudaSuccess) {
     cudaGetLastError();
     f.fine = nullptr;
@@ -1320,7 +1322,6 @@ void paint(bsk_plan* p, int slot, const float* mesh, int nmesh_cic, cudaStream_t
   cufftComplex* fine = f.fine ? f.fine : (cufftComplex*)fine_t->ptr;
   bind_work(p, h, st);
   BSK_CHECK_CUFFT(cufftExecR2C(h, const_cast<float*>(mesh), fine));
-  if (!f.spec) f.spec = (cufftComplex*)dmalloc((size_t)p->Mh * sizeof(cufftComplex));
   launch_extract(p, fine, f.spec, axis_w, st);
   if (fine_t) fine_t->release();
   f.painted = true;

@@ -66,3 +66,17 @@ def test_gridinfo_does_not_trust_a_contraction_that_gave_up(eng, at):
     assert (eng.launches("modular_finish_kernel") > 0) == (at != 0)
     assert eng.lib.bsk_sync_check(None) == (_lib.BSK_OK if at < 0 else _lib.BSK_ERR_TIMEOUT)
     eng.close(p, ts)
+
+
+def test_a_paint_without_memory_keeps_nothing_it_loses(eng):
+    before = eng.live()
+    edges, _ = binning(100.0, 16, 2.0)
+    p = eng.plan(64, 100.0, edges)
+    # room for the transform's output (1.08 MB), not for the slot's spectrum (0.46 MB) as well
+    eng.lib.fake_set_limit(eng.live() + (1200 << 10))
+    for _ in range(3):
+        assert eng.lib.bsk_paint(p, 0, engine_fake.MESH, None) == _lib.BSK_ERR_OOM
+    eng.lib.fake_set_limit(0)
+    eng.paint(p)
+    eng.close(p)
+    assert eng.live() == before
