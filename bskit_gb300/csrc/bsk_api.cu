@@ -192,35 +192,63 @@ void check_budget(const bsk_plan* p, size_t bytes, const char* what) {
                                  std::to_string(root->mem_budget)};
 }
 
-// Shells per synthesis launch: the FFT batch, or more on a small grid, as long as the workspace
-// stays within kSmallWorkspace (96^3, 15 shells: one launch a pass instead of two that half
-// fill the GPU).  Under a memory budget the batch, whose workspace the budget was sized for.
+// The synthesis workspace: twiddles and the X / Y arrays of a launch, and at its end the shells'
+// |q_a| intervals and radii that the passes mask by.  Shells per launch: the FFT batch, or more
+// on a small grid, as long as the workspace stays within kSmallWorkspace (96^3, 15 shells: one
+// launch a pass instead of two that half fill the GPU).  Under a memory budget the workspace is
+// that of the batch without the intervals, for which budgets are sized; the launches of the
+// largest shells, the only ones that would reach them, are then a shell or so shorter.
 constexpr size_t kSmallWorkspace = (size_t)256 << 20;
 void size_synth(bsk_plan* p, size_t mem_budget) {
+  const size_t q1 = p->qmax + 1;
+  p->range_bytes = ((size_t)p->n * q1 * q1 + p->n) * sizeof(uint32_t);
   p->synth_batch = p->chunk;
   while (!mem_budget && p->synth_batch < p->n &&
          synth_workspace_bytes(p->Ng, p->qmax, p->synth_batch + 1) <= kSmallWorkspace)
     ++p->synth_batch;
   p->synth_ws_bytes = synth_workspace_bytes(p->Ng, p->qmax, p->synth_batch);
+  const size_t tables = p->range_bytes + 256;  // with their alignment
+  if (!mem_budget) p->synth_ws_bytes += tables;
+  else  // one shell and the tables at least
+    p->synth_ws_bytes = std::max(p->synth_ws_bytes,
+                                 synth_workspace_bytes(p->Ng, p->qmax, 1) + tables);
 }
 
-// The synthesis workspace, with the twiddles, and (not counted in the footprint, like the shell
-// edges) the shells' |q_a| intervals and radii that its passes mask by.
+// Bytes of the workspace before the tables at its end.
+size_t synth_room(const bsk_plan* p) { return (p->synth_ws_bytes - p->range_bytes) / 256 * 256; }
+
 void ensure_synth(bsk_plan* p, bool against_budget = true) {
   if (p->synth_ws) return;
   if (against_budget) check_budget(p, p->synth_ws_bytes, "the field-synthesis workspace");
-  const size_t q1 = p->qmax + 1, n_range = (size_t)p->n * q1 * q1;
-  if (!p->range) {
-    p->range = (uint32_t*)dmalloc((n_range + p->n) * sizeof(uint32_t));
-    p->d_radius = (int*)(p->range + n_range);
-    launch_shell_range(p, p->range, nullptr, 0);
-    BSK_CHECK_CUDA(cudaMemcpy(p->d_radius, p->shell_r.data(), (size_t)p->n * sizeof(int),
-                              cudaMemcpyHostToDevice));
-  }
-  p->synth_ws = dmalloc(p->synth_ws_bytes);
-  synth_init_workspace(p->Ng, p->synth_ws);
+  SyncTemp ws(p->synth_ws_bytes);  // the plan's once its tables are there
+  const size_t q1 = p->qmax + 1;
+  p->range = (uint32_t*)((char*)ws.ptr + synth_room(p));
+  p->d_radius = (int*)(p->range + (size_t)p->n * q1 * q1);
+  launch_shell_range(p, p->range, nullptr, 0);
+  BSK_CHECK_CUDA(cudaMemcpy(p->d_radius, p->shell_r.data(), (size_t)p->n * sizeof(int),
+                            cudaMemcpyHostToDevice));
+  synth_init_workspace(p->Ng, ws.ptr);
   // the passes may run on a stream that does not wait for the default one
   BSK_CHECK_CUDA(cudaStreamSynchronize(nullptr));
+  std::swap(p->synth_ws, ws.ptr);
+}
+
+// Synthesis of shells [s0, s1) of a slot's spectrum in as few launches as the workspace allows;
+// the other arguments are launch_synth's.
+void synth_shells(bsk_plan* p, const cufftComplex* spec, int s0, int s1, float* fields,
+                  __nv_bfloat16* split, cudaStream_t st, int out_s0 = 0, int fields_from = 0,
+                  int split_to = 1 << 30) {
+  while (s0 < s1) {
+    int ns = std::min(p->synth_batch, s1 - s0), R = 0;
+    for (;; --ns) {
+      R = 0;
+      for (int k = s0; k < s0 + ns; ++k) R = std::max(R, p->shell_r[k]);
+      if (ns == 1 || synth_workspace_bytes(p->Ng, R, ns) <= synth_room(p)) break;
+    }
+    launch_synth(p->Ng, spec, p->table, p->range, p->d_radius, p->qmax + 1, s0, ns, R, p->synth_ws,
+                 fields, split, p->n_alloc(), st, out_s0, fields_from, split_to);
+    s0 += ns;
+  }
 }
 
 void release_stream(bsk_plan* p) {
@@ -265,21 +293,13 @@ void ensure_fields(bsk_plan* p, int s, cudaStream_t st, bool with_split = false,
   if (p->use_synth) {
     ensure_synth(p);
     if (with_split) alloc_split(p, f);
-    int done = 0;
-    for (int s0 = 0; s0 < need; s0 += p->synth_batch) {
-      const int ns = std::min(p->synth_batch, p->n - s0);
-      int R = 0;
-      for (int k = s0; k < s0 + ns; ++k) R = std::max(R, p->shell_r[k]);
-      launch_synth(p->Ng, f.spec, p->table, p->range, p->d_radius, p->qmax + 1, s0, ns, R, p->synth_ws, f.fields,
-                   with_split ? f.split : nullptr, p->n_alloc(), st);
-      done = s0 + ns;
-    }
+    synth_shells(p, f.spec, 0, need, f.fields, with_split ? f.split : nullptr, st);
     f.fields_ok = true;
-    f.fields_n = done;
+    f.fields_n = need;
     f.fields_from = 0;
     if (with_split) {
       f.split_ok = true;
-      f.split_n = done;
+      f.split_n = need;
       f.split_from = 0;
     }
     return;
@@ -343,14 +363,10 @@ void ensure_level_fields(bsk_plan* q, int s, cudaStream_t st, int nn, int fp_fro
   for (int s0 = first / q->chunk * q->chunk; s0 < nn; s0 += q->synth_batch) {
     // up to nn only: a column-only slot has no FP32 fields, and a shell past nn >= fp_from of a
     // batch cut at the level plan's n (every shell that fits its side) would be written to them
-    const int ns = std::min(q->synth_batch, nn - s0);
-    const bool cols = s0 < col_to && s0 + ns > col_from;
-    if (!cols && s0 + ns <= fp_from) continue;
-    int R = 0;
-    for (int k = s0; k < s0 + ns; ++k) R = std::max(R, q->shell_r[k]);
-    launch_synth(q->Ng, f.spec, q->table, q->range, q->d_radius, q->qmax + 1, s0, ns, R,
-                 q->synth_ws, f.fields, cols ? f.split : nullptr, q->n_alloc(), st, 0, fp_from,
-                 col_to);
+    const int s1 = std::min(s0 + q->synth_batch, nn);
+    const bool cols = s0 < col_to && s1 > col_from;
+    if (!cols && s1 <= fp_from) continue;
+    synth_shells(q, f.spec, s0, s1, f.fields, cols ? f.split : nullptr, st, 0, fp_from, col_to);
   }
   // what this pass wrote replaces what the slot held
   f.fields_ok = fp_from < nn;
@@ -390,7 +406,6 @@ void destroy_plan(bsk_plan* p) {
   p->levels.clear();
   for (auto& s : p->slot) free_slot(s);
   if (p->table) cudaFree(p->table);
-  if (p->range) cudaFree(p->range);
   if (p->d_edges) cudaFree(p->d_edges);
   if (p->chunk_spec) cudaFree(p->chunk_spec);
   if (p->cic_w) cudaFree(p->cic_w);
@@ -544,10 +559,7 @@ void chunk_fields(bsk_plan* p, int slot, int s0, int C, float* dst, cudaStream_t
                                        (size_t)(C - b) * p->K * sizeof(float), st));
         break;
       }
-      int R = 0;
-      for (int k = first; k < first + ns; ++k) R = std::max(R, p->shell_r[k]);
-      launch_synth(p->Ng, f.spec, p->table, p->range, p->d_radius, p->qmax + 1, first, ns, R, p->synth_ws,
-                   dst, nullptr, 0, st, s0);
+      synth_shells(p, f.spec, first, first + ns, dst, nullptr, st, s0);
       if (ns < p->chunk)
         BSK_CHECK_CUDA(cudaMemsetAsync(dst + (size_t)(b + ns) * p->K, 0,
                                        (size_t)(p->chunk - ns) * p->K * sizeof(float), st));

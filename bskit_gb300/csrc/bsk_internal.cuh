@@ -174,7 +174,7 @@ struct bsk_plan {
   int64_t Mh = 0;       // Ng*Ng*(Ng/2+1) half-complex modes
   uint16_t* table = nullptr;  // device [Mh] shell code
   uint32_t* range = nullptr;  // device [n][qmax + 1]^2, the shells' |q_a| intervals, then
-  int* d_radius = nullptr;    // [n], shell_r (same allocation; with the synthesis workspace)
+  int* d_radius = nullptr;    // [n], shell_r (both at the end of the synthesis workspace)
   double* d_edges = nullptr;  // device [2n]
   cufftHandle r2c = 0;        // N^3 R2C
   bool r2c_ok = false;
@@ -201,8 +201,9 @@ struct bsk_plan {
   bool use_synth = false;
   std::vector<int> shell_r;             // largest |q_c| of a mode in each shell
   int synth_batch = 0;                  // shells per synthesis launch (>= chunk)
-  void* synth_ws = nullptr;             // twiddles + X / Y pass intermediates of one batch
-  size_t synth_ws_bytes = 0;
+  void* synth_ws = nullptr;             // twiddles + X / Y pass intermediates of one batch,
+  size_t synth_ws_bytes = 0;            // then `range` and `d_radius`
+  size_t range_bytes = 0;               // of these two
   // grid levels: smaller contraction grids for bins of small shells (owned by the plan);
   // a level's plan has `parent` set, takes its spectra from the parent's slots and holds a
   // prefix of the parent's shells

@@ -80,3 +80,42 @@ def test_a_paint_without_memory_keeps_nothing_it_loses(eng):
     eng.paint(p)
     eng.close(p)
     assert eng.live() == before
+
+
+def _synth_bytes(ng, qmax, shells):
+    nk, cp = min(2 * qmax + 1, ng), (qmax + 16) // 16 * 16
+    return shells * ng * cp * 8 * (nk + ng) + ng * 8
+
+
+def _split_bytes(shells, k):
+    return 2 * 2 * shells * ((k + 127) // 128 * 128)
+
+
+@pytest.mark.parametrize("n,kmax,dk,levels", [(64, 16, 1.0, False), (128, 32, 6.0, False),
+                                              (256, 64, 2.0, True)])
+def test_budgeted_plans_hold_what_they_report(eng, monkeypatch, n, kmax, dk, levels):
+    """Under a memory budget the synthesis' tables cost nothing beyond the workspace, every byte
+    taken is in the footprint, and the figure is enough as the next plan's budget."""
+    if levels:
+        monkeypatch.setenv("BSK_LEVEL_MIN_POINTS", "0.2")
+    edges, tri = binning(100.0, kmax, dk)
+    grid = _lib.GRID_REDUCED if levels else _lib.GRID_REDUCED_SINGLE
+    budget, shells = 1 << 40, len(edges)
+    for _ in range(2):
+        p = eng.plan(n, 100.0, edges, budget=budget, grid=grid)
+        ts = eng.triangles(p, tri)
+        assert (len(eng.levels(ts)) > 1) == levels
+        eng.paint(p)
+        live, fp = eng.live(), eng.footprint(p)
+        eng.measure(p, ts)
+        assert eng.info(p, _lib.INFO_STREAM) == 0
+        assert eng.live() - live == eng.footprint(p) - fp
+        if not levels:
+            ng, alloc, batch = eng.info(p, _lib.INFO_NGRID), -(-shells // 8) * 8, 8
+            if shells < 8:
+                alloc = batch = shells
+            assert eng.footprint(p) - fp == (
+                4 * alloc * ng ** 3 + _split_bytes(alloc, ng ** 3)
+                + _synth_bytes(ng, eng.info(p, _lib.INFO_QMAX), batch))
+        budget = eng.footprint(p)
+        eng.close(p, ts)
