@@ -276,13 +276,13 @@ void alloc_split(bsk_plan* p, FieldSlot& f) {
 // Masked shell fields of `slot` for shells [0, n_need) (every shell by default).  With a
 // grid the field synthesis supports, its pruned FFT passes write the fields (and, when
 // `with_split`, their bf16 hi / lo planes in the same pass) batch by batch; otherwise filter
-// kernel + batched cuFFT C2R for every shell.
-void ensure_fields(bsk_plan* p, int s, cudaStream_t st, bool with_split = false,
+// kernel + batched cuFFT C2R for every shell.  True when it used the plan's workspace.
+bool ensure_fields(bsk_plan* p, int s, cudaStream_t st, bool with_split = false,
                    int n_need = -1) {
   FieldSlot& f = p->slot[s];
   BSK_REQUIRE(f.painted, BSK_ERR_STATE, "field slot " + std::to_string(s) + " was not painted");
   const int need = n_need < 0 ? p->n : std::min(n_need, p->n);
-  if (f.fields_ok && f.fields_n >= need && f.fields_from == 0) return;
+  if (f.fields_ok && f.fields_n >= need && f.fields_from == 0) return false;
   if (!f.fields) {
     check_budget(p, (size_t)p->n_alloc() * p->K * sizeof(float), "the shell fields");
     f.fields = (float*)dmalloc((size_t)p->n_alloc() * p->K * sizeof(float));
@@ -302,7 +302,7 @@ void ensure_fields(bsk_plan* p, int s, cudaStream_t st, bool with_split = false,
       f.split_n = need;
       f.split_from = 0;
     }
-    return;
+    return true;
   }
   bind_work(p, p->c2r, st);
   for (int s0 = 0; s0 < p->n; s0 += p->chunk) {
@@ -318,27 +318,29 @@ void ensure_fields(bsk_plan* p, int s, cudaStream_t st, bool with_split = false,
   f.fields_n = p->n;
   f.fields_from = 0;
   f.split_ok = false;
+  return true;
 }
 
-void ensure_split(bsk_plan* p, int s, cudaStream_t st, int n_need = -1) {
+bool ensure_split(bsk_plan* p, int s, cudaStream_t st, int n_need = -1) {
   FieldSlot& f = p->slot[s];
   const int need = n_need < 0 ? p->n : std::min(n_need, p->n);
-  ensure_fields(p, s, st, true, n_need);
-  if (f.split_ok && f.split_n >= need && f.split_from == 0) return;
+  const bool built = ensure_fields(p, s, st, true, n_need);
+  if (f.split_ok && f.split_n >= need && f.split_from == 0) return built;
   alloc_split(p, f);
   launch_split(f.fields, p->n_alloc(), p->K, f.split, st);  // FP32 valid from shell 0
   f.split_ok = true;
   f.split_n = p->n;
   f.split_from = 0;
+  return built;
 }
 
 // A grid level's slot for shells [0, nn): the FP32 fields of shells >= fp_from (the pair
 // factors of its bins; nn when the slot is not a pair factor) and the bf16 split of shells
 // [col_from, col_to) (its third shells; an empty range when the slot is no column operand), in
-// one synthesis pass per batch; batches that hold neither are skipped.  (On the 512^3 headline
+// one synthesis pass per batch; batches that hold neither are skipped.  True when there was one.  (On the 512^3 headline
 // the 384^3 level's bins use no shell below 16 and the 288^3 level's no third shell above 46:
 // two batches less of 384^3 and a quarter of the 288^3 planes.)
-void ensure_level_fields(bsk_plan* q, int s, cudaStream_t st, int nn, int fp_from, int col_from,
+bool ensure_level_fields(bsk_plan* q, int s, cudaStream_t st, int nn, int fp_from, int col_from,
                          int col_to) {
   FieldSlot& f = q->slot[s];
   BSK_REQUIRE(f.painted, BSK_ERR_STATE, "field slot " + std::to_string(s) + " was not painted");
@@ -349,7 +351,7 @@ void ensure_level_fields(bsk_plan* q, int s, cudaStream_t st, int nn, int fp_fro
                                        f.fields_n >= nn);
   const bool split_ok = !need_split ||
                         (f.split_ok && f.split_from <= col_from && f.split_n >= col_to);
-  if (fp_ok && split_ok) return;
+  if (fp_ok && split_ok) return false;
   if (!f.fields && fp_from < nn) {  // a column-only slot needs no FP32 fields
     check_budget(q, (size_t)q->n_alloc() * q->K * sizeof(float), "the shell fields");
     f.fields = (float*)dmalloc((size_t)q->n_alloc() * q->K * sizeof(float));
@@ -377,6 +379,7 @@ void ensure_level_fields(bsk_plan* q, int s, cudaStream_t st, int nn, int fp_fro
     f.split_from = col_from;
     f.split_n = col_to;
   }
+  return true;
 }
 
 void free_slot(FieldSlot& f) {
@@ -416,6 +419,8 @@ void destroy_plan(bsk_plan* p) {
   if (p->work) cudaFree(p->work);
   if (p->synth_ws) cudaFree(p->synth_ws);
   if (p->tail_scratch) cudaFree(p->tail_scratch);
+  if (p->build_scratch) cudaFree(p->build_scratch);
+  for (void* q : p->kept_scratch) cudaFree(q);
   if (p->tail_done) cudaEventDestroy(p->tail_done);
   release_stream(p);
   delete p;
@@ -434,63 +439,91 @@ void copy_dups(const bsk_triset* set, double* v, cudaStream_t st) {
   BSK_CHECK_CUDA(cudaGetLastError());
 }
 
-// The contraction scratch of one measurement (set->scratch_need).  Eager calls share the plan's,
-// taken with the first that wants it; as calls may come on several streams, each waits for
-// the last one's use of it on another.  A captured call takes its own from the
-// stream's pool (an allocation node of its graph), as graphs replay on any streams.  Without room
-// a set runs without.  The scratch is a triangle set's resource, like its schedule, so the
-// plan's footprint does not count it (callers size budgets from that figure).
+// This thread's allocations while another call, or this one's stream, is being captured.
+struct RelaxedCapture {
+  cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+  RelaxedCapture() { cudaThreadExchangeStreamCaptureMode(&mode); }
+  ~RelaxedCapture() { cudaThreadExchangeStreamCaptureMode(&mode); }
+};
+
+// At least `need` bytes in (ptr, have), or nothing changed.  A block that `keep` names stays
+// allocated until the plan goes: a graph holds its address.
+void grow_scratch(bsk_plan* p, void*& ptr, size_t& have, size_t need, bool keep) {
+  if (have >= need) return;
+  RelaxedCapture relaxed;
+  if (ptr && !keep) {
+    cudaFree(ptr);  // waits for the work that uses it
+    ptr = nullptr;
+    have = 0;
+  }
+  // at least double beside a kept one, so that the kept ones together stay below the last
+  const size_t bytes = std::max(need, 2 * have);
+  void* q = nullptr;
+  if (cudaMalloc(&q, bytes) != cudaSuccess) {
+    cudaGetLastError();
+    return;
+  }
+  if (ptr) {
+    p->kept_scratch.push_back(ptr);
+    p->kept_bytes += have;
+  }
+  ptr = q;
+  have = bytes;
+}
+
+// The contraction scratch of one launch on plan p's fields: `need` bytes, or none without room
+// or under a memory budget (the launch then runs whole items, with the same bits).
+//  - A call that synthesised fields on p (`built`) has used p's synthesis workspace, so nothing
+//    that orders it with the next such call, eager or replayed, is missing for a scratch that
+//    is p's in the same way: build_scratch.
+//  - Eager calls on fields that were there may run beside one another on several streams: each
+//    waits for the last one's use of tail_scratch on another stream.
+//  - A captured call on fields that were there may be replayed beside any other: it has none.
+//    (With an allocation node of its own the graph could not be cloned, nor instantiated twice,
+//    and lack of room would show at its instantiation.)
 struct TailScratch {
   bsk_plan* p;
   cudaStream_t st;
   void* ptr = nullptr;
   size_t bytes = 0;
-  std::unique_ptr<AsyncTemp> own;
-  TailScratch(bsk_plan* plan, const bsk_triset* set, int precision, cudaStream_t s)
+  bool shared = false;
+  TailScratch(bsk_plan* plan, size_t need, int precision, bool built, cudaStream_t s)
       : p(plan), st(s) {
-    const size_t need = set->scratch_need;
     if (!need || (precision != BSK_PREC_BF16X3 && precision != BSK_PREC_BF16)) return;
     cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
     BSK_CHECK_CUDA(cudaStreamIsCapturing(st, &cap));
-    if (cap != cudaStreamCaptureStatusNone) {
-      own.reset(new AsyncTemp(need, st));
-      ptr = own->ptr;
-      bytes = need;
+    const bool capturing = cap != cudaStreamCaptureStatusNone;
+    if (built) {
+      grow_scratch(p, p->build_scratch, p->build_bytes, need, p->build_captured || capturing);
+      p->build_captured = p->build_captured || capturing;
+      ptr = p->build_scratch;
+      bytes = p->build_bytes;
       return;
     }
+    if (capturing) return;
     if (!p->tail_done)
       BSK_CHECK_CUDA(cudaEventCreateWithFlags(&p->tail_done, cudaEventDisableTiming));
-    if (p->tail_bytes < need) {
-      if (p->tail_scratch) cudaFree(p->tail_scratch);  // waits for the work that uses it
-      p->tail_scratch = nullptr;
-      p->tail_bytes = 0;
-      if (cudaMalloc(&p->tail_scratch, need) != cudaSuccess) {
-        cudaGetLastError();
-        p->tail_scratch = nullptr;
-        return;
-      }
-      p->tail_bytes = need;
-    }
+    grow_scratch(p, p->tail_scratch, p->tail_bytes, need, false);
+    if (!p->tail_scratch) return;
     unsigned long long id = 0;  // unlike the handle, never used again
     BSK_CHECK_CUDA(cudaStreamGetId(st, &id));
     if (id != p->tail_stream) BSK_CHECK_CUDA(cudaStreamWaitEvent(st, p->tail_done, 0));
     p->tail_stream = id;
     ptr = p->tail_scratch;
     bytes = p->tail_bytes;
+    shared = true;
   }
-  void release() {  // everything that uses it is enqueued
-    if (own) {
-      own->release();
-    } else if (ptr) {
-      BSK_CHECK_CUDA(cudaEventRecord(p->tail_done, st));
-    }
+  ~TailScratch() {  // what uses it is enqueued, also when an error cut the call short
+    if (shared) cudaEventRecord(p->tail_done, st);
   }
+  TailScratch(const TailScratch&) = delete;
+  TailScratch& operator=(const TailScratch&) = delete;
 };
 
 void contract_dispatch(bsk_plan* p, const bsk_triset* set, const float* f1, const float* f2,
                        const float* f3, const __nv_bfloat16* split, int split_shells,
                        int64_t K, int64_t k0, int64_t k1, int precision, double* out,
-                       cudaStream_t st) {
+                       bool built, cudaStream_t st) {
   BSK_CHECK_CUDA(cudaMemsetAsync(out, 0, (size_t)set->T * sizeof(double), st));
   switch (precision) {
     case BSK_PREC_FP64:
@@ -501,11 +534,10 @@ void contract_dispatch(bsk_plan* p, const bsk_triset* set, const float* f1, cons
       break;
     case BSK_PREC_BF16X3:
     case BSK_PREC_BF16: {
-      TailScratch ts(p, set, precision, st);
+      TailScratch ts(p, set->scratch_need, precision, built, st);
       launch_contract_tc(set->sched, f1, f2, split, split_shells, p->n, K, k0, k1,
                          precision == BSK_PREC_BF16X3 ? 3 : 1, out, p->num_sms, st, 1.0, ts.ptr,
                          ts.bytes);
-      ts.release();
       break;
     }
     default:
@@ -806,15 +838,15 @@ void build_levels(bsk_plan* p, bsk_triset* set) {
   }
 }
 
-// The contraction scratch that a set's resident launches want (levels run one after the other
-// and share it); none under a memory budget.
-size_t scratch_need(const bsk_plan* p, const bsk_triset* set) {
-  if (p->mem_budget) return 0;
-  if (set->levels.empty()) return contract_tc_scratch(set->sched.h_tiles, p->K, p->num_sms);
-  size_t need = 0;
-  for (const GridLevel& lv : set->levels)
-    need = std::max(need, contract_tc_scratch(lv.sched.h_tiles, lv.plan->K, p->num_sms));
-  return need;
+// The contraction scratch that the launches on a set's grids want; none under a memory budget.
+void size_scratch(const bsk_plan* p, bsk_triset* set) {
+  if (p->mem_budget) return;
+  for (GridLevel& lv : set->levels) {
+    lv.scratch_need = contract_tc_scratch(lv.sched.h_tiles, lv.plan->K, p->num_sms);
+    set->scratch_need = std::max(set->scratch_need, lv.scratch_need);
+  }
+  if (set->levels.empty())
+    set->scratch_need = contract_tc_scratch(set->sched.h_tiles, p->K, p->num_sms);
 }
 
 // A point range [k0, k1) of the plan's grid as the matching share of a level's grid
@@ -830,7 +862,6 @@ void measure_levels(bsk_plan* p, const bsk_triset* set, int a, int b, int c, int
                     int64_t k0, int64_t k1, double* out, cudaStream_t st) {
   const bool tc = precision == BSK_PREC_BF16X3 || precision == BSK_PREC_BF16;
   BSK_CHECK_CUDA(cudaMemsetAsync(out, 0, (size_t)set->T * sizeof(double), st));
-  TailScratch ts(p, set, precision, st);
   for (const GridLevel& lv : set->levels) {
     bsk_plan* q = lv.plan;
     const int nn = lv.n_shells;
@@ -842,14 +873,15 @@ void measure_levels(bsk_plan* p, const bsk_triset* set, int a, int b, int c, int
     // tensor-core paths read FP32 fields only as pair factors (shells >= the level's smallest
     // i or j) and the split of slot c; the SIMT paths read FP32 fields of every shell they use
     const int sls[3] = {a, b, c};
+    bool built = false;
     for (int k = 0; k < 3; ++k) {
       const int sl = sls[k];
       if ((k >= 1 && sl == sls[0]) || (k == 2 && sl == sls[1])) continue;  // done already
       const bool factor = sl == a || sl == b;
       const int fp_from = !tc ? std::min(lv.src_min, lv.col_min) : factor ? lv.src_min : nn;
       const bool column = tc && sl == c;
-      ensure_level_fields(q, sl, st, nn, fp_from, column ? lv.col_min : nn,
-                          column ? lv.col_end : nn);
+      built |= ensure_level_fields(q, sl, st, nn, fp_from, column ? lv.col_min : nn,
+                                   column ? lv.col_end : nn);
     }
     BSK_REQUIRE(q->slot[a].fields && q->slot[b].fields &&
                     (tc ? q->slot[c].split != nullptr : q->slot[c].fields != nullptr),
@@ -867,14 +899,15 @@ void measure_levels(bsk_plan* p, const bsk_triset* set, int a, int b, int c, int
         launch_contract_simt_f32(lv.sched, fa, fb, fc, q->n, q->K, q0, q1, out, q->num_sms, st,
                                  scale);
         break;
-      default:
+      default: {
+        TailScratch ts(q, lv.scratch_need, precision, built, st);
         launch_contract_tc(lv.sched, fa, fb, q->slot[c].split, q->n_alloc(), q->n, q->K, q0,
                            q1, precision == BSK_PREC_BF16X3 ? 3 : 1, out, q->num_sms, st,
                            scale, ts.ptr, ts.bytes);
         break;
+      }
     }
   }
-  ts.release();
   copy_dups(set, out, st);
 }
 
@@ -940,17 +973,18 @@ void measure_b(bsk_plan* p, const bsk_triset* set, int a, int b, int c, int prec
     measure_levels(p, set, a, b, c, precision, k0, k1, out, st);
     return;
   }
-  if (tc) ensure_split(p, c, st);  // first, so that a synthesis pass writes the split as well
-  ensure_fields(p, a, st);
-  ensure_fields(p, b, st);
-  ensure_fields(p, c, st);
+  bool built = false;
+  if (tc) built |= ensure_split(p, c, st);  // first: a synthesis pass writes the split as well
+  built |= ensure_fields(p, a, st);
+  built |= ensure_fields(p, b, st);
+  built |= ensure_fields(p, c, st);
   const __nv_bfloat16* split = nullptr;
   if (tc) {
-    ensure_split(p, c, st);
+    built |= ensure_split(p, c, st);
     split = p->slot[c].split;
   }
   contract_dispatch(p, set, p->slot[a].fields, p->slot[b].fields, p->slot[c].fields, split,
-                    p->n_alloc(), p->K, k0, k1, precision, out, st);
+                    p->n_alloc(), p->K, k0, k1, precision, out, built, st);
   const double scale = std::pow(p->L, 6) / (double)p->K;
   launch_scale(out, set->T, scale, st);
 }
@@ -1212,7 +1246,7 @@ int bsk_triset_create(bsk_plan* p, int64_t n_tri, const int32_t* tri, bsk_triset
     }
     build_schedule(s->u_tri, p->n, s->sched, &s->u_idx);
     if (p->use_levels && !s->u_tri.empty()) build_levels(p, s.get());
-    s->scratch_need = scratch_need(p, s.get());
+    size_scratch(p, s.get());
     if (!dups.empty()) {
       s->n_dups = (int)dups.size();
       s->dups = (int2*)dmalloc(dups.size() * sizeof(int2));
@@ -1467,7 +1501,7 @@ int bsk_contract(bsk_plan* p, const bsk_triset* set, const float* f1, const floa
       split = (__nv_bfloat16*)split_t->ptr;
       launch_split(f3, p->n, K, split, st);
     }
-    contract_dispatch(p, set, f1, f2, f3, split, p->n, K, 0, K, precision, out, st);
+    contract_dispatch(p, set, f1, f2, f3, split, p->n, K, 0, K, precision, out, false, st);
     if (split_t) split_t->release();
   });
 }

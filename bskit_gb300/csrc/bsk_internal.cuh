@@ -154,6 +154,7 @@ struct GridLevel {
   int n_shells = 0;       // shells [0, n_shells) the level's bins use
   int src_min = 0;        // smallest shell of the level's bins used as a pair factor (i or j)
   int col_min = 0, col_end = 0;  // the third shells l lie in [col_min, col_end)
+  size_t scratch_need = 0;       // contraction scratch wanted (0: none)
   int64_t bins = 0;
 };
 
@@ -210,11 +211,18 @@ struct bsk_plan {
   bool use_levels = false;
   bsk_plan* parent = nullptr;
   std::vector<bsk_plan*> levels;
-  // scratch of the eager tensor-core contractions, grown when a triangle set wants more
+  // contraction scratch (TailScratch), grown when a triangle set wants more: of the eager calls
+  // on fields that were there, with the event of its last use, on stream tail_stream ...
   void* tail_scratch = nullptr;
   size_t tail_bytes = 0;
-  cudaEvent_t tail_done = nullptr;  // the last use of it (TailScratch), on stream tail_stream
+  cudaEvent_t tail_done = nullptr;
   unsigned long long tail_stream = ~0ull;
+  // ... and of the calls that synthesise, with the smaller ones before it that graphs hold
+  void* build_scratch = nullptr;
+  size_t build_bytes = 0;
+  bool build_captured = false;
+  std::vector<void*> kept_scratch;
+  size_t kept_bytes = 0;
   int n_alloc() const { return (n + chunk - 1) / chunk * chunk; }  // shells rounded to batches
 };
 
@@ -229,7 +237,7 @@ struct bsk_triset {
   std::vector<bsk::HostTriangle> u_tri;  // first occurrences, in order
   std::vector<int> u_idx;                // their positions in the list
   mutable std::map<int, std::vector<bsk::StreamGroup>> groups;  // per streaming chunk size
-  size_t scratch_need = 0;               // contraction scratch wanted (0: none)
+  size_t scratch_need = 0;               // contraction scratch wanted (the most of a level)
   std::vector<bsk::GridLevel> levels;    // the resident path's grids (empty: the plan's only)
 };
 

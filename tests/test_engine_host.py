@@ -119,3 +119,86 @@ def test_budgeted_plans_hold_what_they_report(eng, monkeypatch, n, kmax, dk, lev
                 + _synth_bytes(ng, eng.info(p, _lib.INFO_QMAX), batch))
         budget = eng.footprint(p)
         eng.close(p, ts)
+
+
+def _short_grid(eng, n=128, kmax=32.0, part=None):
+    edges, tri = binning(100.0, kmax, 2.0)
+    p = eng.plan(n, 100.0, edges, grid=_lib.GRID_REDUCED_SINGLE)
+    return p, eng.triangles(p, tri if part is None else tri[tri.max(1) < part]), tri
+
+
+def test_captured_contraction_of_ready_fields_allocates_nothing(eng):
+    """Such a graph may be replayed beside any other call, cloned and instantiated twice: no
+    scratch of the plan, no allocation node, whole items as before the scratch existed."""
+    p, ts, _ = _short_grid(eng)
+    eng.paint(p)
+    eng.measure(p, ts)
+    assert eng.launches("tail_sum_kernel") == 1
+    live = eng.live()
+    eng.lib.fake_reset_counts()
+    with eng.capture():
+        eng.measure(p, ts)
+    assert eng.lib.fake_pool_allocs() == 0 and eng.live() == live
+    assert eng.launches("contract_tc_kernel") == 1 and eng.launches("tail_sum_kernel") == 0
+    eng.close(p, ts)
+
+
+def test_captured_passes_share_the_plans_scratch(eng):
+    """A pass that synthesises uses the plan's workspace, and with it the plan's scratch."""
+    p, ts, _ = _short_grid(eng)
+    for _ in range(2):  # the second pass finds everything there
+        eng.paint(p)
+        eng.measure(p, ts)
+    live = eng.live()
+    eng.lib.fake_reset_counts()
+    for _ in range(3):
+        with eng.capture():
+            eng.paint(p)
+            eng.measure(p, ts)
+    assert eng.lib.fake_pool_allocs() == 0 and eng.live() == live
+    assert eng.launches("tail_sum_kernel") == 3
+    eng.close(p, ts)
+
+
+@pytest.mark.parametrize("captured", [False, True])
+def test_without_room_a_pass_runs_without_scratch(eng, captured):
+    p, ts, tri = _short_grid(eng)
+    eng.paint(p)
+    eng.measure(p, ts, precision=_lib.PREC_FP32)  # fields and workspace, no scratch
+    small = eng.triangles(p, tri[:1])
+    eng.measure(p, small)                         # and the split
+    eng.paint(p)
+    eng.lib.fake_set_limit(eng.live() + (8 << 20))
+    eng.lib.fake_reset_counts()
+    if captured:
+        with eng.capture():
+            eng.paint(p)
+            eng.measure(p, ts)
+    else:
+        eng.measure(p, ts)
+    assert eng.launches("contract_tc_kernel") == 1 and eng.launches("tail_sum_kernel") == 0
+    eng.close(p, ts, small)
+
+
+def test_scratch_that_a_graph_holds_is_kept(eng):
+    before = eng.live()
+    p, small, tri = _short_grid(eng, part=8)
+    large = eng.triangles(p, tri)
+    eng.paint(p)
+    eng.measure(p, small)
+    with eng.capture():
+        eng.paint(p)
+        eng.measure(p, small)
+    live = eng.live()
+    # the larger set's scratch comes beside the one in the graph, whether captured or not
+    with eng.capture():
+        eng.paint(p)
+        eng.measure(p, large)
+    grown = eng.live()
+    assert grown > live
+    eng.lib.fake_reset_counts()
+    eng.paint(p)
+    eng.measure(p, large)
+    assert eng.live() == grown and eng.launches("tail_sum_kernel") == 1
+    eng.close(p, small, large)
+    assert eng.live() == before

@@ -85,3 +85,49 @@ def test_streams_and_graphs_share_no_scratch_unordered(plans):
         torch.cuda.synchronize()
         for got, w, b in zip(outs + eager, want, bound):
             assert torch.all((got - w).abs() <= b)
+
+
+def test_captured_passes_keep_their_scratch(cuda):
+    """Graphs of whole passes (paint, synthesis, contraction in parts) replayed after another set
+    has grown the plan's scratch, and graphs of contractions alone, which have none, beside an
+    eager pass of another plan: each gives what its eager call gave."""
+    kf = 2 * np.pi / 100.0
+    kw = dict(kmin=kf, kmax=32 * kf, dk=2 * kf)
+    edges = B.generate_bin_edge_list(**kw)
+    tri = np.asarray(B.generate_triangle_bin_list(return_indices=True, **kw))
+    g = torch.Generator(device="cuda")
+    g.manual_seed(3)
+    mesh = torch.randn((128,) * 3, generator=g, device="cuda")
+    plan, other = (Plan(128, 100.0, edges, grid="single") for _ in range(2))
+    small, large = plan.triangles(tri[tri.max(1) < 8]), plan.triangles(tri)
+    other.paint(0, mesh)
+
+    def run(ts, paint):
+        if paint:
+            plan.paint(0, mesh)
+        return plan.measure_b(ts)
+
+    want, graphs = [], []
+    for ts, paint in ((small, True), (large, True), (small, False), (large, False)):
+        want.append(run(ts, paint).clone())
+        torch.cuda.synchronize()
+        gr = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(gr):
+            out = run(ts, paint)
+        graphs.append((gr, out))
+    side = torch.cuda.Stream()
+    whole = other.measure_b(other.triangles(tri))
+    for order in ((0, 1, 2, 3), (3, 2, 1, 0), (1, 0, 1, 0)):
+        for k in order:
+            gr, out = graphs[k]
+            out.zero_()
+            torch.cuda.synchronize()
+            gr.replay()
+            with torch.cuda.stream(side):
+                other.paint(0, mesh)
+                beside = other.measure_b(other.triangles(tri))
+            torch.cuda.synchronize()
+            # slices added in FP64 in any order: 54 of them, each below the largest bin
+            for got, ref in ((out, want[k]), (beside, whole)):
+                assert torch.all((got - ref).abs() <= 54 * 2.0 ** -52 * 54 * ref.abs().max())
+    plan.sync_check()
