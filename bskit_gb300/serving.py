@@ -195,9 +195,10 @@ class Scheduler(object):
         # first: the only 512^3 group is not given up for what one of four 256^3 groups frees
         def shared(g):
             return sum(1 for o in self.groups if o.shell_key == g.shell_key) > 1
-        idle.sort(key=lambda g: (pinned_too and not shared(g), self.last_used.get(g, 0.0)))
         while self.used + need > self.mem_budget and idle:
-            g = idle.pop(0)
+            # asked again after each: the last of several is an only one
+            g = min(idle, key=lambda g: (pinned_too and not shared(g), self.last_used.get(g, 0.0)))
+            idle.remove(g)
             self.backend.destroy_group(g)
             self.groups.remove(g)
             self.used -= g.footprint

@@ -130,6 +130,18 @@ def test_a_first_group_takes_the_place_of_one_of_several():
     assert sorted(g.shell_key[0] for g in sch.groups) == [16, 32, 64]
 
 
+def test_a_first_group_leaves_every_set_a_group_while_several_have_more():
+    be = FakeBackend()
+    # two 32^3 groups (640 each) and two 48^3 ones (960) leave 100: the first 64^3 group (1280)
+    # takes one of each, not both of the same set
+    sch = serving.Scheduler(be, mem_budget=3300, max_batch=2, max_groups=2, clock=FakeClock())
+    sch.prepare([_req(0, 32), _req(1, 48)])
+    assert be.created == [(32, 2), (32, 2), (48, 2), (48, 2)]
+    sch.prepare([_req(2, 64)], groups=1)
+    assert sorted(be.destroyed) == [32, 48]
+    assert sorted(g.shell_key[0] for g in sch.groups) == [32, 48, 64]
+
+
 def test_no_eviction_for_a_group_that_cannot_fit_and_smaller_groups_tried_first():
     be = FakeBackend()
     # a 64^3 group of 4 (2560) cannot fit a 2000 budget even in an empty server; a group of
