@@ -44,6 +44,7 @@ SIGNATURES = [
                                ctypes.POINTER(_VP)]),
     ("bsk_plan_destroy", _INT, [_VP]),
     ("bsk_plan_query", _INT, [_VP, _VP]),
+    ("bsk_plan_scratch_bytes", _I64, [_VP]),
     ("bsk_shell_mode_counts", _INT, [_VP, _VP]),
     ("bsk_triset_create", _INT, [_VP, _I64, _VP, ctypes.POINTER(_VP)]),
     ("bsk_triset_destroy", _INT, [_VP]),

@@ -180,6 +180,14 @@ int64_t footprint(const bsk_plan* p) {
   return fp;
 }
 
+// Device bytes that a plan without a budget keeps beyond its footprint: of plan p alone.
+int64_t own_scratch(const bsk_plan* p) {
+  int64_t b = (int64_t)(p->tail_bytes + p->build_bytes + p->kept_bytes);
+  for (const auto& s : p->slot)
+    if (s.fine) b += (int64_t)p->N * p->N * (p->N / 2 + 1) * (int64_t)sizeof(cufftComplex);
+  return b;
+}
+
 // Refuse an allocation of `bytes` that would take the plan (with its grid levels: the
 // budget is the root plan's) above its budget.
 void check_budget(const bsk_plan* p, size_t bytes, const char* what) {
@@ -1197,6 +1205,13 @@ int bsk_plan_query(const bsk_plan* p, int64_t* info) {
     info[BSK_INFO_DEVICE] = p->device;
     info[BSK_INFO_STREAM] = p->last_stream_C;
   });
+}
+
+int64_t bsk_plan_scratch_bytes(const bsk_plan* p) {
+  if (!p) return -1;
+  int64_t b = own_scratch(p);
+  for (const bsk_plan* q : p->levels) b += own_scratch(q);
+  return b;
 }
 
 int bsk_shell_mode_counts(const bsk_plan* p, int64_t* counts) {

@@ -115,6 +115,10 @@ class Plan:
         _lib.call("bsk_plan_query", self.handle, info)
         return int(info[_lib.INFO_FOOTPRINT])
 
+    def scratch_bytes(self):
+        """Device bytes kept beyond the footprint (none under a memory budget)."""
+        return int(_lib.load().bsk_plan_scratch_bytes(self.handle))
+
     def stream_chunk(self):
         """Shells per chunk of the last measurement's shell streaming (0 = fields resident)."""
         info = (ctypes.c_int64 * _lib.INFO_COUNT)()

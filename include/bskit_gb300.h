@@ -105,8 +105,16 @@ int bsk_plan_create(int nmesh, double box_size, int n_shells, const double* shel
 int bsk_plan_destroy(bsk_plan* plan);
 
 /* info[BSK_INFO_COUNT] <- N, Ng, n, qmax, footprint bytes, shell chunk, device,
- * streaming chunk of the last measurement. */
+ * streaming chunk of the last measurement.  The footprint is what the plan and its
+ * grid levels hold and a memory budget is held against. */
 int bsk_plan_query(const bsk_plan* plan, int64_t* info);
+/* Device bytes that a plan without a memory budget keeps beyond its footprint, to
+ * be faster: the transform scratch of small painted meshes (up to 80 MB a slot) and
+ * the contraction scratch of short grids (up to 128 MB, once for passes that
+ * synthesise and once for contractions of fields that are there; those that
+ * captured graphs hold stay when a larger one is taken).  Grows when they are first
+ * wanted; 0 under a budget; -1 for NULL. */
+int64_t bsk_plan_scratch_bytes(const bsk_plan* plan);
 
 /*
  * counts[n] <- number of full-grid Fourier modes in each shell (exact int64).

@@ -202,3 +202,35 @@ def test_scratch_that_a_graph_holds_is_kept(eng):
     assert eng.live() == grown and eng.launches("tail_sum_kernel") == 1
     eng.close(p, small, large)
     assert eng.live() == before
+
+
+@pytest.mark.parametrize("n,levels", [(128, False), (256, True), (70, False)])
+def test_plans_report_every_byte_they_keep(eng, monkeypatch, n, levels):
+    """Footprint and scratch together are what a plan has taken, after eager and captured
+    passes, contractions of ready fields on several streams, and a larger set."""
+    if levels:
+        monkeypatch.setenv("BSK_LEVEL_MIN_POINTS", "0.01")
+    edges, tri = binning(100.0, 32, 2.0)
+    p = eng.plan(n, 100.0, edges, grid=_lib.GRID_REDUCED if levels else _lib.GRID_REDUCED_SINGLE)
+    sets = [eng.triangles(p, tri[tri.max(1) < 8]), eng.triangles(p, tri)]
+
+    def reported():
+        return eng.footprint(p) + eng.lib.bsk_plan_scratch_bytes(p)
+
+    live, rep = eng.live(), reported()
+    assert eng.lib.bsk_plan_scratch_bytes(p) == 0
+    for ts in sets:
+        for slots in ((0, 0, 0), (0, 0, 1)):
+            eng.paint(p, 0)
+            eng.paint(p, 1)
+            eng.measure(p, ts, slots)
+            for stream in (1, 2):
+                eng.measure(p, ts, slots, stream=ctypes.c_void_p(stream))
+            with eng.capture():
+                eng.paint(p, 0)
+                eng.paint(p, 1)
+                eng.measure(p, ts, slots)
+            assert eng.live() - live == reported() - rep
+    assert eng.lib.bsk_plan_scratch_bytes(p) > 0
+    eng.close(p, *sets)
+    assert eng.lib.bsk_plan_scratch_bytes(None) == -1

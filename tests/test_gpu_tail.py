@@ -131,3 +131,42 @@ def test_captured_passes_keep_their_scratch(cuda):
             for got, ref in ((out, want[k]), (beside, whole)):
                 assert torch.all((got - ref).abs() <= 54 * 2.0 ** -52 * 54 * ref.abs().max())
     plan.sync_check()
+
+
+def test_plans_report_the_memory_they_keep(cuda):
+    """Footprint and scratch against the device's own count, after an eager pass, one on fields
+    that were there, and a captured one.  64 MiB cover the schedules, the FFT library's tables and
+    the granularity of a few dozen allocations; the scratch alone is above that."""
+    kf = 2 * np.pi / 100.0
+    kw = dict(kmin=kf, kmax=32 * kf, dk=2 * kf)
+    edges = B.generate_bin_edge_list(**kw)
+    tri = B.generate_triangle_bin_list(return_indices=True, **kw)
+    mesh = torch.randn((128,) * 3, device="cuda")
+    out = torch.empty(len(tri), dtype=torch.float64, device="cuda")
+
+    def passes():
+        plan = Plan(128, 100.0, edges, grid="single")
+        ts = plan.triangles(tri)
+        plan.paint(0, mesh)
+        for _ in range(2):
+            plan.measure_b(ts, out=out)
+        torch.cuda.synchronize()
+        gr = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(gr):
+            plan.paint(0, mesh)
+            plan.measure_b(ts, out=out)
+        gr.replay()
+        torch.cuda.synchronize()
+        return plan, gr
+
+    plan, gr = passes()  # loads the kernels
+    del gr
+    plan.close()
+    torch.cuda.synchronize()
+    torch.cuda.empty_cache()
+    free = torch.cuda.mem_get_info()[0]
+    plan, gr = passes()
+    taken = free - torch.cuda.mem_get_info()[0]
+    assert plan.scratch_bytes() > 64 << 20
+    assert abs(taken - plan.footprint() - plan.scratch_bytes()) <= 64 << 20
+    plan.close()
