@@ -128,6 +128,8 @@ class Scheduler(object):
       destroy_group(group)
       launch(group, jobs) -> batch handle (asynchronous)
       poll(batch) -> True when finished (results written into the requests)
+    and may provide:
+      group_bytes(group) -> bytes that the group holds by now
     """
 
     def __init__(self, backend, mem_budget, max_batch=4, max_groups=4, clock=time.perf_counter):
@@ -160,15 +162,20 @@ class Scheduler(object):
             per_shell.setdefault(j.shell_key, []).append(j)
         want = self.max_groups if groups is None else int(groups)
         for key, js in per_shell.items():
+            def capture(g):
+                for j in js:
+                    self.backend.prepare(g, j)
+                self._recount(g)
+
+            for g in self.groups:
+                if g.shell_key == key:
+                    capture(g)
             while sum(1 for g in self.groups if g.shell_key == key) < want:
                 g = self._admit_group(js[0])
                 if g is None:
                     break
                 g.pinned = True  # prepared ahead: never evicted to make room for another group
-            for g in self.groups:
-                if g.shell_key == key:
-                    for j in js:
-                        self.backend.prepare(g, j)
+                capture(g)  # before the next is admitted, with what this one came to hold
         return jobs
 
     def n_pending(self):
@@ -204,6 +211,13 @@ class Scheduler(object):
             self.used -= g.footprint
             self.log.append(("evict", g.shell_key[:2]))
         return self.used + need <= self.mem_budget
+
+    def _recount(self, g):
+        """A group holds more than it was admitted with once a bin set wants more scratch."""
+        held = getattr(self.backend, "group_bytes", lambda _: 0)(g)
+        if held > g.footprint:
+            self.used += held - g.footprint
+            g.footprint = held
 
     def _admit_group(self, job):
         have = sum(1 for g in self.groups if g.shell_key == job.shell_key)
@@ -241,6 +255,8 @@ class Scheduler(object):
                     self.done.append(j.req)
                 del self.busy[g]
                 self.last_used[g] = t
+        if self.used > self.mem_budget:  # groups took more than they were admitted with
+            self._evict_for(0)
         # the shell set whose oldest request waits longest first; a batch takes that set's
         # requests in arrival order, whatever their bin sets
         order = sorted(self.pending.keys(), key=lambda k: self.pending[k][0].req.arrival
@@ -259,6 +275,7 @@ class Scheduler(object):
                     j.req.t_dispatch = t
                 self.log.append(("batch", key[:2], len(jobs), len({j.bin_key for j in jobs})))
                 self.busy[g] = (self.backend.launch(g, jobs), jobs)
+                self._recount(g)
                 self.last_used[g] = t
             if not q:
                 del self.pending[key]
@@ -325,6 +342,8 @@ class EngineBackend(object):
         self.use_graphs = use_graphs
         self.gridinfo = {}      # bin_key -> (ntri, kmean) device tensors
         self.probe = {}         # shell_key -> measured footprint of one instance
+        self.mem_budget = None  # the server's: an instance above it takes lean plans
+        self.lean = set()       # shell_keys whose plans keep no scratch
         self.captures = 0       # graphs captured (prepare + dispatch)
         self.captures_at_dispatch = 0
         self.captures_at_dispatch_by_n = {}
@@ -335,7 +354,10 @@ class EngineBackend(object):
         torch = self.torch
         req = job.req
         inst = _Instance()
-        inst.plan = Plan(req.nmesh, req.box, job.edges, device=self.device)
+        # a plan under a budget, here one that is never reached, keeps nothing beyond its
+        # footprint
+        inst.plan = Plan(req.nmesh, req.box, job.edges, device=self.device,
+                         mem_budget=1 << 60 if job.shell_key in self.lean else 0)
         n = req.nmesh
         inst.dmesh = [torch.empty((n, n, n), dtype=torch.float32, device=self.device)
                       for _ in range(2)]
@@ -368,6 +390,10 @@ class EngineBackend(object):
 
     def group_footprint(self, job, size):
         fp = self.probe.get(job.shell_key)
+        if fp is not None and self.mem_budget is not None and fp > self.mem_budget \
+                and job.shell_key not in self.lean:
+            self.lean.add(job.shell_key)  # slower, rather than never served
+            fp = None
         if fp is None:
             # an instance serves auto and cross requests of its shell set alike: measure it
             # with both field slots built
@@ -378,10 +404,22 @@ class EngineBackend(object):
             inst.plan.measure_b(self._tset(inst, job), slots=(0, 0, 1),
                                 precision=job.req.precision)
             self.torch.cuda.synchronize(self.device)
-            fp = inst.plan.footprint() + 2 * job.req.nmesh ** 3 * 4
+            fp = self._instance_bytes(inst.plan)
             self.probe[job.shell_key] = fp
             inst.plan.close()
+            return self.group_footprint(job, size)
         return fp * size
+
+    @staticmethod
+    def _instance_bytes(plan):
+        """The plan, with the scratch it keeps, and the instance's two meshes."""
+        return plan.footprint() + plan.scratch_bytes() + 2 * plan.nmesh ** 3 * 4
+
+    def group_bytes(self, g):
+        each = [self._instance_bytes(inst.plan) for inst in g.instances]
+        # the shell set's next groups are admitted with what an instance of it came to hold
+        self.probe[g.shell_key] = max(each + [self.probe.get(g.shell_key, 0)])
+        return sum(each)
 
     def create_group(self, job, size):
         torch = self.torch
@@ -509,4 +547,5 @@ def make_server(mem_budget=None, max_batch=4, max_groups=4, device=None, use_gra
     if mem_budget is None:
         free, _ = torch.cuda.mem_get_info(backend.device)
         mem_budget = int(0.8 * free)
+    backend.mem_budget = mem_budget
     return Scheduler(backend, mem_budget, max_batch=max_batch, max_groups=max_groups)

@@ -168,6 +168,43 @@ def test_admission_by_footprint_and_eviction():
     assert max(sizes) <= 2
 
 
+def test_what_groups_take_after_admission_is_counted():
+    class Growing(FakeBackend):
+        """Groups take 100 more per bin set that was prepared or launched on them."""
+
+        def __init__(self):
+            super().__init__()
+            self.seen = {}
+
+        def _see(self, g, *jobs):
+            self.seen.setdefault(g, set()).update(j.req.spec["triangle_type"] for j in jobs)
+
+        def prepare(self, g, job):
+            super().prepare(g, job)
+            self._see(g, job)
+
+        def launch(self, g, jobs):
+            self._see(g, *jobs)
+            return super().launch(g, jobs)
+
+        def group_bytes(self, g):
+            return 10 * g.shell_key[0] * g.size + 100 * len(self.seen.get(g, ()))
+
+    be = Growing()
+    sch = serving.Scheduler(be, mem_budget=1000, max_batch=2, max_groups=2, clock=FakeClock())
+    sch.prepare([_req(0, 16, "all"), _req(1, 16, "equilateral")], groups=1)
+    assert sch.used == 320 + 200
+    # 480 are left for a second group of 320; the third bin set is counted on both when it is
+    # launched, and as that is 40 too much the group that was not prepared goes when it is idle
+    reqs = [_req(2 + i, 16, "squeezed") for i in range(4)]
+    sch.run(reqs, realtime=False)
+    assert all(r.B is not None for r in reqs) and be.created == [(16, 2), (16, 2)]
+    assert be.destroyed == [16]
+    assert sch.used == sum(be.group_bytes(g) for g in sch.groups) == 320 + 300
+    sch.close()
+    assert sch.used == 0
+
+
 def test_group_cap_per_shell_set():
     be = FakeBackend()
     sch = serving.Scheduler(be, mem_budget=10 ** 6, max_batch=2, max_groups=1, clock=FakeClock())
@@ -259,3 +296,56 @@ def test_mixed_stream_equals_each_request_alone(cuda):
         assert np.array_equal(m.N_tri, r.N_tri)
         scale = np.abs(r.B_unnorm).max()
         assert np.abs(m.B_unnorm - r.B_unnorm).max() <= 1e-12 * scale
+
+
+@pytest.mark.gpu
+def test_groups_hold_no_more_than_the_scheduler_counts(cuda):
+    """Every instance's plan (footprint and scratch), after bin sets that the group was not
+    admitted with were captured and served on it, is in the scheduler's count."""
+    from bskit_gb300 import synthetic
+    n, box = 128, 100.0
+    kf = 2 * np.pi / box
+    mesh = synthetic.lognormal_mesh_torch(n, box, seed=1, device=cuda).cpu().numpy()
+    spec = dict(kmin=kf, kmax=32 * kf, dk=2 * kf)
+    reqs = [serving.Request(i, mesh, box, dict(spec, triangle_type=t), second=mesh if c else None)
+            for i, (t, c) in enumerate([("equilateral", False), ("all", False), ("all", True)])]
+    sch = serving.make_server(mem_budget=40 << 30, max_batch=2, max_groups=1)
+    sch.prepare(reqs[:1])
+    sch.run(reqs, realtime=False)
+    assert all(r.B is not None and np.all(np.isfinite(r.B)) for r in reqs)
+    for g in sch.groups:
+        held = [i.plan.footprint() + i.plan.scratch_bytes() + 2 * n ** 3 * 4 for i in g.instances]
+        assert sum(i.plan.scratch_bytes() for i in g.instances) > 0
+        assert sum(held) <= g.footprint
+    assert sch.used == sum(g.footprint for g in sch.groups)
+    sch.close()
+
+
+@pytest.mark.gpu
+def test_a_server_too_small_for_the_scratch_serves_without(cuda):
+    from bskit_gb300 import synthetic
+    from bskit_gb300.engine import Plan
+    n, box = 128, 100.0
+    kf = 2 * np.pi / box
+    mesh = synthetic.lognormal_mesh_torch(n, box, seed=2, device=cuda).cpu().numpy()
+    spec = dict(kmin=kf, kmax=32 * kf, dk=2 * kf, triangle_type="all")
+    edges, tri = serving.bin_lists(spec)
+    plan = Plan(n, box, edges, mem_budget=1 << 60)
+    for s in (0, 1):
+        plan.paint(s, mesh)
+    ts = plan.triangles(tri)
+    want = plan.measure_b(ts).cpu().numpy()
+    plan.measure_b(ts, slots=(0, 0, 1))
+    room = plan.footprint() + 2 * n ** 3 * 4
+    assert plan.scratch_bytes() == 0
+    plan.close()
+    sch = serving.make_server(mem_budget=room, max_batch=2, max_groups=1)
+    r = serving.Request(0, mesh, box, spec)
+    sch.submit(r)
+    for _ in range(10 ** 6):
+        if sch.idle():
+            break
+        sch.step()
+    assert sch.idle() and 0 < sch.used <= room
+    assert np.abs(r.B_unnorm - want).max() <= 1e-12 * np.abs(want).max()
+    sch.close()
