@@ -342,25 +342,43 @@ bool ensure_split(bsk_plan* p, int s, cudaStream_t st, int n_need = -1) {
   return built;
 }
 
+// A range of shells [from, to).
+struct Shells {
+  int from = 0, to = 0;
+  bool empty() const { return from >= to; }
+  // the smallest range that holds both
+  Shells hull(const Shells& o) const {
+    if (empty()) return o;
+    if (o.empty()) return *this;
+    return Shells{std::min(from, o.from), std::max(to, o.to)};
+  }
+  bool has(const Shells& o) const { return o.empty() || (from <= o.from && o.to <= to); }
+  // whether [s0, s1) holds a shell of this range that `have` lacks
+  bool misses(const Shells& have, int s0, int s1) const {
+    const int a = std::max(from, s0), b = std::min(to, s1);
+    return a < b && !have.has(Shells{a, b});
+  }
+};
+
 // A grid level's slot for shells [0, nn): the FP32 fields of shells >= fp_from (the pair
 // factors of its bins; nn when the slot is not a pair factor) and the bf16 split of shells
 // [col_from, col_to) (its third shells; an empty range when the slot is no column operand), in
-// one synthesis pass per batch; batches that hold neither are skipped.  True when there was one.  (On the 512^3 headline
+// one synthesis pass per batch; batches that hold neither are skipped.  (On the 512^3 headline
 // the 384^3 level's bins use no shell below 16 and the 288^3 level's no third shell above 46:
-// two batches less of 384^3 and a quarter of the 288^3 planes.)
+// two batches less of 384^3 and a quarter of the 288^3 planes.)  What the slot holds is kept:
+// its ranges grow to the hull of what it holds and what is needed, so that sets which use
+// different shells of a mesh do not undo each other's fields.  True when there was a pass.
 bool ensure_level_fields(bsk_plan* q, int s, cudaStream_t st, int nn, int fp_from, int col_from,
                          int col_to) {
   FieldSlot& f = q->slot[s];
   BSK_REQUIRE(f.painted, BSK_ERR_STATE, "field slot " + std::to_string(s) + " was not painted");
   nn = std::min(nn, q->n);
-  fp_from = std::min(fp_from, nn);
-  const bool need_split = col_from < col_to;
-  const bool fp_ok = fp_from >= nn || (f.fields_ok && f.fields_from <= fp_from &&
-                                       f.fields_n >= nn);
-  const bool split_ok = !need_split ||
-                        (f.split_ok && f.split_from <= col_from && f.split_n >= col_to);
-  if (fp_ok && split_ok) return false;
-  if (!f.fields && fp_from < nn) {  // a column-only slot needs no FP32 fields
+  const Shells have = f.fields_ok ? Shells{f.fields_from, f.fields_n} : Shells{};
+  const Shells have_split = f.split_ok ? Shells{f.split_from, f.split_n} : Shells{};
+  const Shells need{std::min(fp_from, nn), nn}, need_split{col_from, col_to};
+  if (have.has(need) && have_split.has(need_split)) return false;
+  const Shells want = have.hull(need), want_split = have_split.hull(need_split);
+  if (!f.fields && !want.empty()) {  // a column-only slot needs no FP32 fields
     check_budget(q, (size_t)q->n_alloc() * q->K * sizeof(float), "the shell fields");
     f.fields = (float*)dmalloc((size_t)q->n_alloc() * q->K * sizeof(float));
     const size_t pad = (size_t)(q->n_alloc() - q->n) * q->K;
@@ -368,25 +386,28 @@ bool ensure_level_fields(bsk_plan* q, int s, cudaStream_t st, int nn, int fp_fro
       BSK_CHECK_CUDA(cudaMemset(f.fields + (size_t)q->n * q->K, 0, pad * sizeof(float)));
   }
   ensure_synth(q);
-  if (need_split) alloc_split(q, f);
-  const int first = need_split ? std::min(fp_from, col_from) : fp_from;
-  for (int s0 = first / q->chunk * q->chunk; s0 < nn; s0 += q->synth_batch) {
-    // up to nn only: a column-only slot has no FP32 fields, and a shell past nn >= fp_from of a
-    // batch cut at the level plan's n (every shell that fits its side) would be written to them
-    const int s1 = std::min(s0 + q->synth_batch, nn);
-    const bool cols = s0 < col_to && s1 > col_from;
-    if (!cols && s1 <= fp_from) continue;
-    synth_shells(q, f.spec, s0, s1, f.fields, cols ? f.split : nullptr, st, 0, fp_from, col_to);
+  if (!want_split.empty()) alloc_split(q, f);
+  // batches from the first missing shell to the last, and no further: a column-only slot has no
+  // FP32 fields, and a shell past them would be written to them
+  int first = q->n, last = -1;
+  for (int k = 0; k < q->n; ++k)
+    if (want.misses(have, k, k + 1) || want_split.misses(have_split, k, k + 1)) {
+      first = std::min(first, k);
+      last = k;
+    }
+  for (int s0 = first / q->chunk * q->chunk; s0 <= last; s0 += q->synth_batch) {
+    const int s1 = std::min(s0 + q->synth_batch, last + 1);
+    const bool fp32 = want.misses(have, s0, s1), cols = want_split.misses(have_split, s0, s1);
+    if (!fp32 && !cols) continue;
+    synth_shells(q, f.spec, s0, s1, f.fields, cols ? f.split : nullptr, st, 0,
+                 fp32 ? want.from : s1, want_split.to);
   }
-  // what this pass wrote replaces what the slot held
-  f.fields_ok = fp_from < nn;
-  f.fields_from = fp_from;
-  f.fields_n = nn;
-  if (need_split) {
-    f.split_ok = true;
-    f.split_from = col_from;
-    f.split_n = col_to;
-  }
+  f.fields_ok = !want.empty();
+  f.fields_from = want.from;
+  f.fields_n = want.to;
+  f.split_ok = !want_split.empty();
+  f.split_from = want_split.from;
+  f.split_n = want_split.to;
   return true;
 }
 

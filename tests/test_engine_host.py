@@ -234,3 +234,34 @@ def test_plans_report_every_byte_they_keep(eng, monkeypatch, n, levels):
     assert eng.lib.bsk_plan_scratch_bytes(p) > 0
     eng.close(p, *sets)
     assert eng.lib.bsk_plan_scratch_bytes(None) == -1
+
+
+@pytest.mark.parametrize("precision", [_lib.PREC_BF16X3, _lib.PREC_FP32])
+def test_sets_of_other_shells_do_not_undo_each_other(eng, monkeypatch, precision):
+    """Sets that use different shells of one painted mesh on one level: each is synthesised once,
+    and measured again without a synthesis, in any order; no shell twice for the split alone."""
+    monkeypatch.setenv("BSK_LEVEL_MIN_POINTS", "0.9")  # one level: the plan's grid
+    edges, tri = binning(500.0, 64, 2.0)
+    p = eng.plan(256, 500.0, edges)
+    parts = [tri[tri.max(1) < 9], tri[tri.min(1) >= 20], tri[(tri.max(1) < 20)], tri]
+    sets = [eng.triangles(p, t) for t in parts]
+    assert all(len(eng.levels(ts)) == 1 for ts in sets)
+    for order in ((0, 1, 2, 3), (1, 0, 3, 2), (3, 0, 1, 2), (2, 1, 0, 3)):
+        eng.paint(p, 0)
+        eng.paint(p, 1)
+        for k in order:
+            for slots in ((0, 0, 0), (0, 0, 1), (1, 0, 1)):
+                eng.measure(p, sets[k], slots, precision)
+        eng.lib.fake_reset_counts()
+        for k in order[::-1] + order:
+            for slots in ((1, 0, 1), (0, 0, 0), (0, 0, 1)):
+                eng.measure(p, sets[k], slots, precision)
+        assert eng.launches("x_kernel") == 0, order
+        assert eng.launches("contract") == 8 * 3
+    # a set whose shells are there but for one batch: that batch alone
+    eng.paint(p, 0)
+    eng.measure(p, sets[2], precision=precision)
+    eng.lib.fake_reset_counts()
+    eng.measure(p, sets[3], precision=precision)
+    assert eng.launches("x_kernel") == 2  # shells 16 .. 31: two batches of eight
+    eng.close(p, *sets)

@@ -81,3 +81,42 @@ def test_column_slot_without_fields(cuda, monkeypatch, low):
         p.sync_check()
         p.close()
     assert torch.all((got[0] - got[1]).abs() <= 4096 * 2.0 ** -53 * got[1].abs().max())
+
+
+@pytest.mark.parametrize("precision", ["bf16x3", "fp32"])
+def test_ranges_that_grow_over_a_gap(cuda, monkeypatch, precision):
+    """Low and high shells of one level, as pair factors, columns or both, in turn: the slot's
+    ranges grow to hulls, whose middle is synthesised with the second set."""
+    monkeypatch.setenv("BSK_LEVEL_MIN_POINTS", "0.9")  # one level
+    n, box = 256, 500.0
+    kf = 2 * np.pi / box
+    kw = dict(kmin=kf, kmax=64 * kf, dk=2 * kf)
+    edges = B.generate_bin_edge_list(**kw)
+    tri = B.generate_triangle_bin_list(return_indices=True, **kw)
+    sets = [tri[tri.max(1) < 9], tri[tri.min(1) >= 20],
+            tri[(tri.max(1) < 20) & (tri.min(1) >= 9)]]
+    d = synthetic.lognormal_mesh_torch(n, box, seed=5, device=cuda).contiguous()
+    e = (1.5 * d + 0.3 * torch.randn_like(d)).contiguous()
+    slots = ((0, 0, 1), (0, 0, 0), (1, 0, 1))
+
+    def plan():
+        p = Plan(n, box, edges)
+        p.paint(0, d)
+        p.paint(1, e)
+        return p, [p.triangles(t) for t in sets]
+
+    want = {}
+    for k in range(3):
+        for sl in slots:
+            p, made = plan()
+            want[k, sl] = p.measure_b(made[k], slots=sl, precision=precision)
+            p.close()
+    for order in itertools.permutations(range(3)):
+        p, made = plan()
+        for k in order + order:
+            for sl in slots:
+                got = p.measure_b(made[k], slots=sl, precision=precision)
+                assert torch.all((got - want[k, sl]).abs() <=
+                                 4096 * 2.0 ** -53 * want[k, sl].abs().max()), (order, k, sl)
+        p.sync_check()
+        p.close()
