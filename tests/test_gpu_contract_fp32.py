@@ -81,3 +81,55 @@ def test_shards_off_16_bytes(cuda, cut):
     parts = sum(plan.measure_b_range(ts, a, b, precision="fp32") for a, b in ((0, cut), (cut, k)))
     whole = plan.measure_b(ts, precision="fp64")
     assert torch.all((parts - whole).abs() <= (SLICE + 2) * 2.0 ** -24 * top)
+
+
+# three different source arrays; more than 64 shells, where a tile's two factor ranges start at
+# different shells even of one array
+@pytest.mark.parametrize("shells,distinct", [(5, 3), (15, 3), (24, 2), (80, 3), (80, 1)])
+@pytest.mark.parametrize("k", [8, 40, SLICE + 24, "long"])
+def test_chain_of_two_sources(cuda, shells, distinct, k):
+    kf = 2 * np.pi / 100.0
+    edges = np.array([[q, q + 1.0] for q in range(1, shells + 1)]) * kf
+    rng = np.random.default_rng(shells + distinct)
+    tri = np.unique(rng.integers(0, shells, (700, 3)), axis=0)
+    plan = Plan(2 * (shells + 4), 100.0, edges, grid="native")
+    g = torch.Generator(device="cuda")
+    g.manual_seed(shells * 10 + distinct)
+    points = SLICE if k == "long" else k
+    f = [torch.randn((shells, points), generator=g, device="cuda") for _ in range(distinct)]
+    f = {1: [0, 0, 0], 2: [0, 1, 0], 3: [0, 1, 2]}[distinct], f
+    f = [f[1][i] for i in f[0]]
+    want, top = _chain(f, tri)
+    # enough slices for the tiles of long grids (four items an SM), points repeated
+    repeat = 700 if k == "long" else 1
+    if repeat > 1:
+        wide = {id(v): v.repeat(1, repeat) for v in f}
+        f = [wide[id(v)] for v in f]
+    got = plan.contract(plan.triangles(tri), *f, precision="fp32")
+    tol = 4 * 2.0 ** -24 * top + repeat * 2.0 ** -52 * top
+    assert torch.all((got - repeat * want).abs() <= repeat * tol)
+    plan.close()
+
+
+@pytest.mark.parametrize("cut", [1, 4099, 50001])
+@pytest.mark.parametrize("n,kmax", [(64, 16), (256, 64)])
+def test_shards_of_three_fields_off_16_bytes(cuda, cut, n, kmax):
+    """As above for <ABC>, on a short grid and on one of whole-tile items."""
+    box = 100.0
+    kf = 2 * np.pi / box
+    kw = dict(kmin=kf, kmax=kmax * kf, dk=kmax * kf / 8)
+    edges = B.generate_bin_edge_list(**kw)
+    tri = B.generate_triangle_bin_list(num_fields=3, return_indices=True, **kw)
+    plan = Plan(n, box, edges, grid="single")
+    g = torch.Generator(device="cuda").manual_seed(cut + n)
+    for s in range(3):
+        plan.paint(s, torch.randn((n, n, n), generator=g, device="cuda"))
+    ts, k = plan.triangles(tri), plan.ngrid ** 3
+    f = [torch.stack([plan.field(s, i).reshape(-1) for i in range(len(edges))]).abs()
+         for s in range(3)]
+    top = plan.contract(ts, *f, precision="fp64") * box ** 6 / k
+    parts = sum(plan.measure_b_range(ts, a, b, slots=(0, 1, 2), precision="fp32")
+                for a, b in ((0, cut), (cut, k)))
+    whole = plan.measure_b(ts, slots=(0, 1, 2), precision="fp64")
+    assert torch.all((parts - whole).abs() <= (SLICE + 2) * 2.0 ** -24 * top)
+    plan.close()

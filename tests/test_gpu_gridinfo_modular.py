@@ -35,3 +35,25 @@ def test_residues_equal_enumeration(cuda, n, box, kmax, dk, fields):
     ok = nt0 > 0
     assert torch.all(torch.isnan(km[~ok])) and torch.any(ok)
     assert torch.all((km[ok] - km0[ok]).abs() <= 4096 * 2.0 ** -52 * km0[ok])
+
+
+# the upper half of the route's range: the headline's 127, sides of more than 192 points along
+# z (135), blocks of 64 pairs (150, 159), and the first value past it (both plans enumerate).
+# Thin shells keep the enumeration short: fewer than 4096 batches, as above.
+@pytest.mark.parametrize("q", [127, 135, 150, 159, 160])
+def test_large_q_equal_enumeration(cuda, q):
+    n, box = 512, 900.0
+    edges = np.array([[1.0, 3.0], [0.6 * q, 0.6 * q + 2.2], [q - 4.1, q + 0.4]])
+    edges *= 2 * np.pi / box
+    tri = np.array([(a, b, c) for a in range(3) for b in range(a + 1) for c in range(b + 1)])
+    free = Plan(n, box, edges, grid="single")
+    assert free.qmax == q
+    tight = Plan(n, box, edges, grid="single", mem_budget=free.footprint() + (1 << 20))
+    (nt, km), (nt0, km0) = (p.gridinfo(p.triangles(tri)) for p in (free, tight))
+    free.sync_check()
+    assert torch.equal(nt, nt0) and torch.any(nt0 > 0) and torch.any(nt0 == 0)
+    ok = nt0 > 0
+    assert torch.all(torch.isnan(km[~ok]))
+    assert torch.all((km[ok] - km0[ok]).abs() <= 4096 * 2.0 ** -52 * km0[ok])
+    free.close()
+    tight.close()
