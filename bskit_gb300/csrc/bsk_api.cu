@@ -5,6 +5,7 @@
 #include <cstring>
 #include <map>
 #include <memory>
+#include <mutex>
 
 #include "bsk_internal.cuh"
 
@@ -180,9 +181,63 @@ int64_t footprint(const bsk_plan* p) {
   return fp;
 }
 
+// This thread's allocations while another call, or this one's stream, is being captured.
+struct RelaxedCapture {
+  cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+  RelaxedCapture() { cudaThreadExchangeStreamCaptureMode(&mode); }
+  ~RelaxedCapture() { cudaThreadExchangeStreamCaptureMode(&mode); }
+};
+
+}  // namespace
+
+// The blocks that captured graphs hold.  A block that came back may still be in use by the last
+// replay of its graph: it is freed, which waits for that, by the plan's next call, not handed out.
+struct LeasedScratch {
+  struct Block {
+    size_t bytes;
+    bool back;
+  };
+  mutable std::mutex m;  // graphs go on other threads
+  std::map<void*, Block> blocks;
+  void add(void* q, size_t bytes) {
+    std::lock_guard<std::mutex> lock(m);
+    blocks[q] = Block{bytes, false};
+  }
+  void give_back(void* q) {
+    std::lock_guard<std::mutex> lock(m);
+    auto it = blocks.find(q);
+    if (it != blocks.end()) it->second.back = true;  // else its plan has gone before it
+  }
+  size_t bytes() const {
+    std::lock_guard<std::mutex> lock(m);
+    size_t b = 0;
+    for (const auto& kv : blocks) b += kv.second.bytes;
+    return b;
+  }
+  void sweep(bool all = false) {
+    std::vector<void*> gone;
+    {
+      std::lock_guard<std::mutex> lock(m);
+      for (auto it = blocks.begin(); it != blocks.end();)
+        if (all || it->second.back) {
+          gone.push_back(it->first);
+          it = blocks.erase(it);
+        } else {
+          ++it;
+        }
+    }
+    if (gone.empty()) return;
+    RelaxedCapture relaxed;
+    for (void* q : gone) cudaFree(q);
+  }
+};
+
+namespace {
+
 // Device bytes that a plan without a budget keeps beyond its footprint: of plan p alone.
 int64_t own_scratch(const bsk_plan* p) {
   int64_t b = (int64_t)(p->tail_bytes + p->build_bytes + p->kept_bytes);
+  if (p->leased) b += (int64_t)p->leased->bytes();
   for (const auto& s : p->slot)
     if (s.fine) b += (int64_t)p->N * p->N * (p->N / 2 + 1) * (int64_t)sizeof(cufftComplex);
   return b;
@@ -450,6 +505,7 @@ void destroy_plan(bsk_plan* p) {
   if (p->tail_scratch) cudaFree(p->tail_scratch);
   if (p->build_scratch) cudaFree(p->build_scratch);
   for (void* q : p->kept_scratch) cudaFree(q);
+  if (p->leased) p->leased->sweep(true);
   if (p->tail_done) cudaEventDestroy(p->tail_done);
   release_stream(p);
   delete p;
@@ -467,13 +523,6 @@ void copy_dups(const bsk_triset* set, double* v, cudaStream_t st) {
   copy_dups_kernel<<<(n + 255) / 256, 256, 0, st>>>(n, set->dups, v);
   BSK_CHECK_CUDA(cudaGetLastError());
 }
-
-// This thread's allocations while another call, or this one's stream, is being captured.
-struct RelaxedCapture {
-  cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
-  RelaxedCapture() { cudaThreadExchangeStreamCaptureMode(&mode); }
-  ~RelaxedCapture() { cudaThreadExchangeStreamCaptureMode(&mode); }
-};
 
 // At least `need` bytes in (ptr, have), or nothing changed.  A block that `keep` names stays
 // allocated until the plan goes: a graph holds its address.
@@ -500,6 +549,53 @@ void grow_scratch(bsk_plan* p, void*& ptr, size_t& have, size_t need, bool keep)
   have = bytes;
 }
 
+// A block of `need` bytes for the call that `st` is capturing, or none: at most kMaxLeased of
+// them, and only with room.  The graph, its copies and their instances hold it as a user
+// object; when the last is gone it goes back.
+constexpr size_t kMaxLeased = (size_t)512 << 20;
+void* lease_scratch(bsk_plan* p, size_t need, cudaStream_t st) {
+  cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+  cudaGraph_t graph = nullptr;
+  BSK_CHECK_CUDA(cudaStreamGetCaptureInfo(st, &cap, nullptr, &graph, nullptr, nullptr, nullptr));
+  if (cap != cudaStreamCaptureStatusActive || !graph) return nullptr;
+  if (!p->leased) p->leased = std::make_shared<LeasedScratch>();
+  p->leased->sweep();
+  if (p->leased->bytes() + need > kMaxLeased) return nullptr;
+  void* q = nullptr;
+  {
+    RelaxedCapture relaxed;
+    if (cudaMalloc(&q, need) != cudaSuccess) {
+      cudaGetLastError();
+      return nullptr;
+    }
+  }
+  p->leased->add(q, need);
+  struct Lease {
+    std::shared_ptr<LeasedScratch> from;
+    void* block;
+  };
+  std::unique_ptr<Lease> lease(new Lease{p->leased, q});
+  cudaUserObject_t obj;
+  // runs on a thread of CUDA's: no CUDA call in it
+  const auto back = [](void* v) {
+    std::unique_ptr<Lease> l((Lease*)v);
+    l->from->give_back(l->block);
+  };
+  if (cudaUserObjectCreate(&obj, lease.get(), back, 1, cudaUserObjectNoDestructorSync) !=
+      cudaSuccess) {
+    cudaGetLastError();
+    p->leased->give_back(q);
+    return nullptr;
+  }
+  lease.release();  // the user object's
+  if (cudaGraphRetainUserObject(graph, obj, 1, cudaGraphUserObjectMove) != cudaSuccess) {
+    cudaGetLastError();
+    cudaUserObjectRelease(obj, 1);
+    return nullptr;
+  }
+  return q;
+}
+
 // The contraction scratch of one launch on plan p's fields: `need` bytes, or none without room
 // or under a memory budget (the launch then runs whole items, with the same bits).
 //  - A call that synthesised fields on p (`built`) has used p's synthesis workspace, so nothing
@@ -507,9 +603,10 @@ void grow_scratch(bsk_plan* p, void*& ptr, size_t& have, size_t need, bool keep)
 //    is p's in the same way: build_scratch.
 //  - Eager calls on fields that were there may run beside one another on several streams: each
 //    waits for the last one's use of tail_scratch on another stream.
-//  - A captured call on fields that were there may be replayed beside any other: it has none.
-//    (With an allocation node of its own the graph could not be cloned, nor instantiated twice,
-//    and lack of room would show at its instantiation.)
+//  - A captured call on fields that were there may be replayed beside any other: a block of its
+//    own, for as long as its graph lives (lease_scratch).  (With an allocation node the graph
+//    could not be cloned, nor instantiated twice, and lack of room would show at its
+//    instantiation.)
 struct TailScratch {
   bsk_plan* p;
   cudaStream_t st;
@@ -529,7 +626,12 @@ struct TailScratch {
       bytes = p->build_bytes;
       return;
     }
-    if (capturing) return;
+    if (capturing) {
+      ptr = lease_scratch(p, need, st);
+      bytes = ptr ? need : 0;
+      return;
+    }
+    if (p->leased) p->leased->sweep();
     if (!p->tail_done)
       BSK_CHECK_CUDA(cudaEventCreateWithFlags(&p->tail_done, cudaEventDisableTiming));
     grow_scratch(p, p->tail_scratch, p->tail_bytes, need, false);

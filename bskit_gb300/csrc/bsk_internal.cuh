@@ -6,6 +6,7 @@
 #include <cuda_bf16.h>
 #include <stdint.h>
 #include <map>
+#include <memory>
 #include <string>
 #include <vector>
 
@@ -14,6 +15,7 @@
 struct bsk_plan;
 
 namespace bsk {
+struct LeasedScratch;
 
 // ---------------------------------------------------------------- errors
 void set_error(const std::string& msg);
@@ -223,6 +225,8 @@ struct bsk_plan {
   bool build_captured = false;
   std::vector<void*> kept_scratch;
   size_t kept_bytes = 0;
+  // ... and of captured calls on fields that were there
+  std::shared_ptr<bsk::LeasedScratch> leased;
   int n_alloc() const { return (n + chunk - 1) / chunk * chunk; }  // shells rounded to batches
 };
 

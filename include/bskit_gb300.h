@@ -110,10 +110,12 @@ int bsk_plan_destroy(bsk_plan* plan);
 int bsk_plan_query(const bsk_plan* plan, int64_t* info);
 /* Device bytes that a plan without a memory budget keeps beyond its footprint, to
  * be faster: the transform scratch of small painted meshes (up to 80 MB a slot) and
- * the contraction scratch of short grids (up to 128 MB, once for passes that
- * synthesise and once for contractions of fields that are there; those that
- * captured graphs hold stay when a larger one is taken).  Grows when they are first
- * wanted; 0 under a budget; -1 for NULL. */
+ * the contraction scratch of short grids, up to 128 MB each: one for passes that
+ * synthesise (with smaller ones before it that captured graphs hold), one for
+ * contractions of fields that are there, and one for each captured graph of such a
+ * contraction while the graph lives (512 MB of them at most; a graph beyond that,
+ * or without room, runs without).  Grows when they are first wanted; 0 under a
+ * budget; -1 for NULL. */
 int64_t bsk_plan_scratch_bytes(const bsk_plan* plan);
 
 /*

@@ -11,6 +11,8 @@
 #include <cstring>
 #include <map>
 #include <string>
+#include <utility>
+#include <vector>
 
 namespace {
 struct Block {
@@ -27,6 +29,7 @@ size_t g_live = 0, g_limit = 0;
 int g_capturing = 0, g_capture_broken = 0, g_symbol = 0, g_symbol_at = -1, g_symbol_reads = 0;
 int g_pool_allocs = 0, g_launched = 0;
 cudaStreamCaptureMode g_mode = cudaStreamCaptureModeGlobal;
+std::vector<std::pair<cudaHostFn_t, void*>> g_user_objects;
 
 // calls that a capture in global mode does not allow
 cudaError_t unsafe_call() {
@@ -71,6 +74,12 @@ void fake_set_capturing(int on) {
   g_capture_broken = 0;
 }
 int fake_capture_broken() { return g_capture_broken; }
+// every captured graph goes, and the user objects they held with them
+void fake_destroy_graphs() {
+  std::vector<std::pair<cudaHostFn_t, void*>> objects;
+  objects.swap(g_user_objects);
+  for (auto& o : objects) o.first(o.second);
+}
 // device variables read as `value`, from their `at`-th read on
 void fake_set_symbol(int value, int at) {
   g_symbol = value;
@@ -199,6 +208,21 @@ cudaError_t cudaStreamIsCapturing(cudaStream_t, cudaStreamCaptureStatus* s) {
   *s = g_capturing ? cudaStreamCaptureStatusActive : cudaStreamCaptureStatusNone;
   return cudaSuccess;
 }
+cudaError_t cudaStreamGetCaptureInfo(cudaStream_t, cudaStreamCaptureStatus* s,
+                                     unsigned long long*, cudaGraph_t* g, const cudaGraphNode_t**,
+                                     const cudaGraphEdgeData**, size_t*) {
+  if (g) *g = (cudaGraph_t)1;
+  return cudaStreamIsCapturing(nullptr, s);
+}
+cudaError_t cudaUserObjectCreate(cudaUserObject_t* o, void* p, cudaHostFn_t f, unsigned, unsigned) {
+  g_user_objects.emplace_back(f, p);
+  *o = (cudaUserObject_t)1;
+  return cudaSuccess;
+}
+cudaError_t cudaGraphRetainUserObject(cudaGraph_t, cudaUserObject_t, unsigned, unsigned) {
+  return cudaSuccess;
+}
+cudaError_t cudaUserObjectRelease(cudaUserObject_t, unsigned) { return cudaSuccess; }
 cudaError_t cudaThreadExchangeStreamCaptureMode(cudaStreamCaptureMode* m) {
   std::swap(*m, g_mode);
   return cudaSuccess;

@@ -127,19 +127,17 @@ def _short_grid(eng, n=128, kmax=32.0, part=None):
     return p, eng.triangles(p, tri if part is None else tri[tri.max(1) < part]), tri
 
 
-def test_captured_contraction_of_ready_fields_allocates_nothing(eng):
-    """Such a graph may be replayed beside any other call, cloned and instantiated twice: no
-    scratch of the plan, no allocation node, whole items as before the scratch existed."""
+def test_captured_contraction_of_ready_fields_has_no_allocation_node(eng):
+    """Such a graph may be replayed beside any other call, cloned and instantiated twice."""
     p, ts, _ = _short_grid(eng)
     eng.paint(p)
     eng.measure(p, ts)
     assert eng.launches("tail_sum_kernel") == 1
-    live = eng.live()
     eng.lib.fake_reset_counts()
     with eng.capture():
         eng.measure(p, ts)
-    assert eng.lib.fake_pool_allocs() == 0 and eng.live() == live
-    assert eng.launches("contract_tc_kernel") == 1 and eng.launches("tail_sum_kernel") == 0
+    assert eng.lib.fake_pool_allocs() == 0
+    assert eng.launches("contract_tc_kernel") == 1
     eng.close(p, ts)
 
 
@@ -265,3 +263,44 @@ def test_sets_of_other_shells_do_not_undo_each_other(eng, monkeypatch, precision
     eng.measure(p, sets[3], precision=precision)
     assert eng.launches("x_kernel") == 2  # shells 16 .. 31: two batches of eight
     eng.close(p, *sets)
+
+
+def test_graphs_of_ready_fields_lease_scratch(eng):
+    """A captured contraction of ready fields has scratch of its own, owned by the plan and
+    handed back when the last copy of its graph goes: no allocation node, a bounded number of
+    them, and whole items where there is no room."""
+    before = eng.live()
+    p, ts, _ = _short_grid(eng)
+    eng.paint(p)
+    eng.measure(p, ts)
+    live, scratch = eng.live(), eng.lib.bsk_plan_scratch_bytes(p)
+    eng.lib.fake_reset_counts()
+    sizes = []
+    for k in range(8):
+        with eng.capture():
+            eng.measure(p, ts)
+        sizes.append(eng.live() - live)
+        assert eng.lib.bsk_plan_scratch_bytes(p) - scratch == sizes[-1]
+    assert eng.lib.fake_pool_allocs() == 0
+    # 113 MB each, up to 512 MB of them
+    assert sizes[0] > 100 << 20 and sizes[3:] == [4 * sizes[0]] * 5
+    assert eng.launches("tail_sum_kernel") == 4 and eng.launches("contract_tc_kernel") == 8
+    # graphs that went make room; an eager call gives the memory back as well
+    eng.lib.fake_destroy_graphs()
+    with eng.capture():
+        eng.measure(p, ts)
+    assert eng.live() - live == sizes[0] and eng.launches("tail_sum_kernel") == 5
+    eng.lib.fake_destroy_graphs()
+    eng.measure(p, ts)
+    assert eng.live() - live == sizes[0]  # the eager call's own
+    eng.lib.fake_set_limit(eng.live() + (1 << 20))
+    with eng.capture():
+        eng.measure(p, ts)
+    assert eng.launches("tail_sum_kernel") == 6 and eng.launches("contract_tc_kernel") == 11
+    eng.lib.fake_set_limit(0)
+    with eng.capture():
+        eng.measure(p, ts)
+    eng.close(p, ts)
+    assert eng.live() == before
+    eng.lib.fake_destroy_graphs()  # after its plan
+    assert eng.live() == before

@@ -170,3 +170,54 @@ def test_plans_report_the_memory_they_keep(cuda):
     assert plan.scratch_bytes() > 64 << 20
     assert abs(taken - plan.footprint() - plan.scratch_bytes()) <= 64 << 20
     plan.close()
+
+
+def test_graphs_of_ready_fields(cuda):
+    """A graph of a contraction of ready fields: instantiated twice, replayed beside the eager
+    call on another stream, and its scratch goes back to the plan with it."""
+    import time
+    kf = 2 * np.pi / 100.0
+    kw = dict(kmin=kf, kmax=32 * kf, dk=2 * kf)
+    edges = B.generate_bin_edge_list(**kw)
+    tri = np.asarray(B.generate_triangle_bin_list(return_indices=True, **kw))
+    plan = Plan(128, 100.0, edges, grid="single")
+    ts = plan.triangles(tri)
+    plan.paint(0, torch.randn((128,) * 3, device="cuda"))
+    for _ in range(2):  # the second finds the fields ready
+        want = plan.measure_b(ts).clone()
+    torch.cuda.synchronize()
+    kept = plan.scratch_bytes()
+    out = torch.zeros_like(want)
+    gr = torch.cuda.CUDAGraph(keep_graph=True)
+    with torch.cuda.graph(gr):
+        plan.measure_b(ts, out=out)
+    assert plan.scratch_bytes() > kept
+    runtime = ctypes.CDLL("libcudart.so.13")
+    execs = [ctypes.c_void_p() for _ in range(2)]
+    for e in execs:
+        assert runtime.cudaGraphInstantiate(ctypes.byref(e), ctypes.c_void_p(gr.raw_cuda_graph()),
+                                            ctypes.c_ulonglong(0)) == 0
+    side = torch.cuda.Stream()
+    tol = 54 * 2.0 ** -52 * 54 * want.abs().max()  # as above
+    for e in execs + execs:
+        out.zero_()
+        torch.cuda.synchronize()
+        stream = ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)
+        assert runtime.cudaGraphLaunch(e, stream) == 0
+        with torch.cuda.stream(side):
+            beside = plan.measure_b(ts)
+        torch.cuda.synchronize()
+        for got in (out, beside):
+            assert torch.all((got - want).abs() <= tol)
+    for e in execs:
+        assert runtime.cudaGraphExecDestroy(e) == 0
+    assert plan.scratch_bytes() > kept  # the graph itself has it still
+    del gr
+    for _ in range(100):  # the runtime's own thread hands it back
+        plan.measure_b(ts)
+        if plan.scratch_bytes() == kept:
+            break
+        time.sleep(0.05)
+    assert plan.scratch_bytes() == kept
+    plan.sync_check()
+    plan.close()
