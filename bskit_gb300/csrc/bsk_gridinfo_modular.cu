@@ -36,6 +36,12 @@ namespace gmod {
 constexpr int kMaxPrimes = 16;
 constexpr int kFrac = 44;       // fractional bits of w, as in the enumeration
 constexpr int kMinQ = 40, kMaxQ = 159;  // kMaxQ: shared memory of the transforms
+// Below kFewQ the enumeration is the faster one for plans of few modes too (us, enumeration /
+// residues): one shell of 21 000 modes at 41 956 / 1094, of 31 000 at 50 1391 / 1522, but of
+// 250 000 at 41 2511 / 1444 and of 41 000 at 57 1850 / 1747; two shells of 12 000 at 40 893 / 1077,
+// of 20 000 1294 / 1096; six of 4600 1026 / 1072, of 15 000 1246 / 1089.
+constexpr int kFewQ = 53;
+inline int64_t few_modes(int n_shells) { return n_shells == 1 ? 80000 : 24000 / n_shells; }
 constexpr int kRun = 32;        // products added between reductions
 
 struct Prime {
@@ -43,6 +49,12 @@ struct Prime {
   int np;               // (x, y) pairs, h (h + 1) / 2
   int64_t K;            // np hz rounded up to 128
   int inv_n3;           // N^-3 mod p
+  void size() {
+    h = N / 2 + 1;
+    hz = (h + 1) & ~1;
+    np = h * (h + 1) / 2;
+    K = ((int64_t)np * hz + 127) / 128 * 128;
+  }
 };
 
 struct Garner {         // inv[j][k] = p_j^-1 mod p_k (j < k)
@@ -89,10 +101,7 @@ std::vector<Prime> choose_primes(int qmax, double bits) {
   for (Prime q : all) {
     if (have > bits) break;
     if ((int)out.size() == kMaxPrimes) return {};
-    q.h = q.N / 2 + 1;
-    q.hz = (q.h + 1) & ~1;
-    q.np = q.h * (q.h + 1) / 2;
-    q.K = ((int64_t)q.np * q.hz + 127) / 128 * 128;
+    q.size();
     q.inv_n3 = pow_mod(pow_mod(q.N, 3, q.p), q.p - 2, q.p);
     have += std::log2((double)q.p);
     out.push_back(q);
@@ -503,6 +512,18 @@ bool gridinfo_modular(bsk_plan* p, const std::vector<HostTriangle>& tri, double*
   const int n = p->n, q1 = p->qmax + 1;
   const int64_t T = (int64_t)tri.size();
   if (T > (int64_t)1 << 28) return false;
+  int64_t modes = 0;
+  for (int64_t c : p->counts) modes += c;
+  if (p->qmax < kFewQ && modes <= few_modes(n)) return false;
+  const int cp = (q1 + 3) / 4 * 4;
+  if (p->mem_budget) {  // the least that any primes need, before the 130 us of choosing them
+    Prime q{};
+    q.N = 3 * p->qmax + 1;
+    q.size();
+    const size_t least = (size_t)n * (q.np * (size_t)cp + q.K) * sizeof(float) +
+                         split_elems(n, q.K) * sizeof(__nv_bfloat16);
+    if (device_bytes(p) + (int64_t)least > (int64_t)p->mem_budget) return false;
+  }
 
   // distinct counts (shells sorted) and distinct |k| sums (pair (y >= z), the weighted shell x)
   std::vector<HostTriangle> ec, es;
@@ -539,7 +560,6 @@ bool gridinfo_modular(bsk_plan* p, const std::vector<HostTriangle>& tri, double*
   int n_cnt = 0;
   double have = 0;
   while (n_cnt < n_pr && have <= std::log2(bound) + 1.0) have += std::log2((double)primes[n_cnt++].p);
-  const int cp = (q1 + 3) / 4 * 4;
   int64_t max_k = 0, max_np = 0;
   for (const Prime& q : primes) {
     if (q.hz > 256 || z_smem(q, q1, cp, 64) > kMaxSmem) return false;

@@ -54,9 +54,9 @@ def test_everything_is_given_back(eng):
 # the route's own launches (second and later reads)
 @pytest.mark.parametrize("at", [-1, 0, 1])
 def test_gridinfo_does_not_trust_a_contraction_that_gave_up(eng, at):
-    edges, tri = binning(100.0, 45, 5.0)
+    edges, tri = binning(100.0, 60, 5.0)
     p = eng.plan(192, 100.0, edges, grid=_lib.GRID_REDUCED_SINGLE)
-    assert eng.info(p, _lib.INFO_QMAX) >= 40
+    assert eng.info(p, _lib.INFO_QMAX) >= 53
     ts = eng.triangles(p, tri)
     eng.lib.fake_reset_counts()
     eng.lib.fake_set_symbol(1, at)
@@ -304,3 +304,18 @@ def test_graphs_of_ready_fields_lease_scratch(eng):
     assert eng.live() == before
     eng.lib.fake_destroy_graphs()  # after its plan
     assert eng.live() == before
+
+
+# residues from |q| = 53 on (up to 159); below, not for plans of few modes (the fake's have none)
+@pytest.mark.parametrize("q,residues", [(39, False), (41, False), (52, False), (53, True),
+                                        (159, True), (160, False)])
+def test_route_of_the_grid_information(eng, q, residues):
+    edges = np.array([[0.5 * q, 0.7 * q], [q - 1.0, q + 0.5]]) * TWO_PI / 100.0
+    p = eng.plan(2 * (3 * q // 2 + 4), 100.0, edges, grid=_lib.GRID_REDUCED_SINGLE)
+    assert eng.info(p, _lib.INFO_QMAX) == q
+    ts = eng.triangles(p, [[1, 1, 0]])
+    eng.lib.fake_reset_counts()
+    eng.ok(eng.lib.bsk_gridinfo(p, ts, engine_fake.OUT, engine_fake.OUT, None))
+    assert (eng.launches("modular_finish_kernel") > 0) == residues
+    assert (eng.launches("enum_finish_kernel") > 0) != residues
+    eng.close(p, ts)
