@@ -157,11 +157,15 @@ __global__ void __launch_bounds__(THREADS) contract_simt_kernel(
 // warps an SM (168 or 200 of them spill: +60%).  256^3 (31 shells, 3 tiles): 4.15 ms, where a
 // block of four warps a tile took 6.5.
 //
-// Short grids (TR = 4: 32 rows x up to 16 columns).  A slice is a chain of 8192 dependent
-// multiply-adds an entry, so with few items the chain's pace is the time (48^3, 14 items: 144
-// cycles a point with four warps and three barriers a chunk, 623 us): more, smaller items, and
-// copies three chunks ahead (250 us).  Forming the next chunk's products before the current
-// chunk's multiply-adds, to save a barrier, was 7% slower.
+// Short grids and sparse sets (TR = 4: 32 rows x up to 16 columns).  A slice is a chain of 8192
+// dependent multiply-adds an entry, so with few items the chain's pace is the time (48^3, 14
+// items: 144 cycles a point with four warps and three barriers a chunk, 623 us): more, smaller
+// items, and copies three chunks ahead (250 us).  Forming the next chunk's products before the
+// current chunk's multiply-adds, to save a barrier, was 7% slower.  The items are the parts of the
+// tiles that hold bins, listed with the schedule (f32_parts), each with its own source shells, so
+// that sparse sets do no work for the rest of their tiles: 60 equilateral bins on 192^3 take
+// 1.6 ms, as whole tiles 4.4, and 3.4 where a block of four warps a tile skipped what held no
+// bin.  (Skipping empty parts in this kernel saved nothing: a block met the full ones every round.)
 namespace f32 {
 constexpr int ROWS = 128, COLS = 32, SRC = 64;
 constexpr int64_t SLICE = 8192;
@@ -321,38 +325,42 @@ __device__ __forceinline__ void run_item(float* sm, int src, const TileDesc& td,
     }
 }
 
-// Item = (slice, sub-tile of 32 columns, part of the sub-tile): `parts` of them, rows in 128 / (8
-// TR) parts and, for short grids, columns in two.
-template <class C>
-constexpr int parts() { return C::TR == 16 ? 1 : 2 * ROWS / (8 * C::TR); }
-
+// Item = (slice, sub-tile of 32 columns) on long grids, (slice, part) on short ones.
 template <class C>
 __global__ void __launch_bounds__(32)
     contract_f32_kernel(const TileDesc* __restrict__ tiles, const int2* __restrict__ subs,
-                        int n_sub, const int16_t* __restrict__ row_i,
-                        const int16_t* __restrict__ row_j, const int32_t* __restrict__ map,
-                        const float* __restrict__ f1, const float* __restrict__ f2,
-                        const float* __restrict__ f3, int n_shells, int64_t K, int64_t k_begin,
-                        int64_t k_end, int64_t n_slices, int src, double* __restrict__ out,
-                        double scale) {
+                        const F32Part* __restrict__ parts, int per_slice,
+                        const int16_t* __restrict__ row_i, const int16_t* __restrict__ row_j,
+                        const int32_t* __restrict__ map, const float* __restrict__ f1,
+                        const float* __restrict__ f2, const float* __restrict__ f3, int n_shells,
+                        int64_t K, int64_t k_begin, int64_t k_end, int64_t n_slices, int src,
+                        double* __restrict__ out, double scale) {
   extern __shared__ __align__(16) float f32_smem[];
   float* sm = f32_smem;
-  constexpr int P = parts<C>();
-  for (int64_t item = blockIdx.x; item < n_slices * n_sub * P; item += gridDim.x) {
-    const int64_t sl = item / (n_sub * P);
-    const int in_slice = (int)(item - sl * (n_sub * P));
-    const int part = in_slice % P;
-    const int2 sub = subs[in_slice / P];
-    const TileDesc td = tiles[sub.x];
-    // the tile's columns in as many equal runs, multiples of 8, as it has 32-column sub-tiles
-    const int runs = (td.nc + COLS - 1) / COLS, width = ((td.nc + runs - 1) / runs + 7) / 8 * 8;
-    int c0 = sub.y / COLS * width, nc = min(width, td.nc - c0), r0 = 0;
-    if (P > 1) {
-      const int half = (nc + 15) / 16 * 8;  // columns [c0, c0 + half) and the rest
-      r0 = (part >> 1) * 8 * C::TR;
-      c0 += part & 1 ? half : 0;
-      nc = part & 1 ? nc - half : half;
-      if (nc <= 0 || r0 >= td.nrows) continue;
+  constexpr bool kParts = C::TR != 16;
+  for (int64_t item = blockIdx.x; item < n_slices * per_slice; item += gridDim.x) {
+    const int64_t sl = item / per_slice;
+    const int in_slice = (int)(item - sl * per_slice);
+    TileDesc td;
+    int r0 = 0, c0, nc;
+    if constexpr (kParts) {
+      const F32Part p = parts[in_slice];
+      td = tiles[p.tile];
+      td.i0 = p.i0;
+      td.ni = p.ni;
+      td.j0 = p.j0;
+      td.nj = p.nj;
+      r0 = p.r0;
+      c0 = p.c0;
+      nc = p.nc;
+    } else {
+      const int2 sub = subs[in_slice];
+      td = tiles[sub.x];
+      // the tile's columns in as many equal runs, multiples of 8, as it has 32-column sub-tiles
+      const int runs = (td.nc + COLS - 1) / COLS;
+      const int width = ((td.nc + runs - 1) / runs + 7) / 8 * 8;
+      c0 = sub.y / COLS * width;
+      nc = min(width, td.nc - c0);
     }
     const bool one_src = !C::kTwoSrc || (f1 == f2 && td.i0 == td.j0);
     const int64_t x_begin = k_begin + sl * SLICE;
@@ -361,7 +369,7 @@ __global__ void __launch_bounds__(32)
       run_item<C, 2>(sm, src, td, r0, c0, row_i, row_j, map, f1, f2, f3, n_shells, K, x_begin, x_end, one_src, out, scale);
     else if (nc <= 16)
       run_item<C, 4>(sm, src, td, r0, c0, row_i, row_j, map, f1, f2, f3, n_shells, K, x_begin, x_end, one_src, out, scale);
-    else if constexpr (P == 1) {
+    else if constexpr (!kParts) {
       if (nc <= 24)
         run_item<C, 6>(sm, src, td, r0, c0, row_i, row_j, map, f1, f2, f3, n_shells, K, x_begin, x_end, one_src, out, scale);
       else
@@ -370,13 +378,26 @@ __global__ void __launch_bounds__(32)
   }
 }
 
+// Parts of one column block as long as the SMs hold them all at once, twice the items with half
+// the chain: then of two.  Both sides measured, us, pairs / single blocks, at that many single
+// blocks an SM: one source range 2: 369 / 273, 7.1: 468 / 339, 10.1: 482 / 420, 13.2: 479 / 540 and
+// 551 / 852; two ranges or arrays 7.1: 532 / 421, 8.1: 521 / 706, 11.0: 602 / 867.
+template <class C>
+constexpr int64_t kNarrowPerSm = C::kTwoSrc ? 8 : 11;
+
 template <class C>
 void launch(const DeviceSchedule& s, const float* f1, const float* f2, const float* f3,
             int n_shells, int64_t K, int64_t k_begin, int64_t k_end, double* out, int num_sms,
             cudaStream_t st, double scale) {
   const int64_t n_slices = (k_end - k_begin + SLICE - 1) / SLICE;
-  int src = 8;
-  for (const TileDesc& d : s.h_tiles) src = std::max(src, std::max(d.ni, d.nj));
+  constexpr bool kParts = C::TR != 16;
+  int src = kParts ? s.part_src : 8;
+  if (!kParts)
+    for (const TileDesc& d : s.h_tiles) src = std::max(src, std::max(d.ni, d.nj));
+  const int list = n_slices * s.n_parts[kNarrowParts] <= kNarrowPerSm<C> * num_sms ? kNarrowParts
+                                                                               : kWideParts;
+  const F32Part* parts = s.parts + (list == kNarrowParts ? s.n_parts[kWideParts] : 0);
+  const int per_slice = kParts ? s.n_parts[list] : s.n_sub;
   const size_t smem = C::smem(src);
   auto kern = contract_f32_kernel<C>;
   BSK_CHECK_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
@@ -384,9 +405,10 @@ void launch(const DeviceSchedule& s, const float* f1, const float* f2, const flo
   int per_sm = 0;
   BSK_CHECK_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, 32, smem));
   const int64_t grid =
-      std::min<int64_t>((int64_t)num_sms * std::max(per_sm, 1), n_slices * s.n_sub * parts<C>());
-  kern<<<(unsigned)grid, 32, smem, st>>>(s.tiles, s.subs, s.n_sub, s.row_i, s.row_j, s.map, f1, f2,
-                                         f3, n_shells, K, k_begin, k_end, n_slices, src, out, scale);
+      std::min<int64_t>((int64_t)num_sms * std::max(per_sm, 1), n_slices * per_slice);
+  kern<<<(unsigned)grid, 32, smem, st>>>(s.tiles, s.subs, parts, per_slice, s.row_i, s.row_j,
+                                         s.map, f1, f2, f3, n_shells, K, k_begin, k_end, n_slices,
+                                         src, out, scale);
   BSK_CHECK_CUDA(cudaGetLastError());
 }
 }  // namespace f32
@@ -415,9 +437,15 @@ void launch_simt(const DeviceSchedule& s, const Tin* f1, const Tin* f2, const Ti
 
 }  // namespace
 
-// Whole-tile items from four an SM on (both sides measured, us): 335 items 848 short / 845 long,
-// 670 items 1522 .. 1917 / 1613 .. 1727, 824 items 2218 / 1610; 211 items 682 / 1180.
+// Whole-tile items from four an SM on (both sides measured, us, parts / whole tiles; one array,
+// different arrays): 500 items 1122 / 1132, 1323 / 1334; 730 items 1714 / 1947, 2511 / 2013; 864
+// items 1884 / 1682, 2096 / 1927; 2916 items 5794 / 3948, 7104 / 4739 ...
 constexpr int64_t kLongItemsPerSm = 4;
+// ... unless the parts have few columns between them: with 1.9 times the tiles' columns
+// 110 400 / 103 500 (every seventh bin of 90 shells, 216^3), with 2.4 times 108 000 / 97 200 (all
+// of them), but with no more than the tiles' (equilateral and squeezed sets: only the diagonal of
+// a tile holds bins) 837 / 2002 (30 shells, 192^3), 1570 / 4382 (60), 5217 / 12 840 (60, 288^3).
+constexpr double kLongDensity = 1.75;
 
 // FP32 products and tile sums (8192-point slices), FP64 cross-slice sum.
 void launch_contract_simt_f32(const DeviceSchedule& s, const float* f1, const float* f2,
@@ -426,9 +454,11 @@ void launch_contract_simt_f32(const DeviceSchedule& s, const float* f1, const fl
                               double scale) {
   if (s.n_tiles == 0 || k_end <= k_begin) return;
   const int64_t n_slices = (k_end - k_begin + f32::SLICE - 1) / f32::SLICE;
-  const bool is_long = n_slices * s.n_sub >= kLongItemsPerSm * num_sms;
-  bool two_src = f1 != f2;
-  for (const TileDesc& d : s.h_tiles) two_src = two_src || d.i0 != d.j0;
+  const bool is_long = n_slices * s.n_sub >= kLongItemsPerSm * num_sms &&
+                       s.part_cols >= kLongDensity * s.sum_nc;
+  bool two_src = f1 != f2 || (!is_long && s.part_two);
+  if (is_long)
+    for (const TileDesc& d : s.h_tiles) two_src = two_src || d.i0 != d.j0;
   const bool aligned = k_begin % 4 == 0 && K % 4 == 0 &&
                        ((uintptr_t)f1 | (uintptr_t)f2 | (uintptr_t)f3) % 16 == 0;
   const auto pick = [&](auto two, auto al) {

@@ -63,6 +63,15 @@ struct TileDesc {
   int pad;
 };
 
+// An item of the plain FP32 contraction on short grids and of sparse sets: 32 rows from r0 and
+// nc (8 or 16) columns from c0 of a tile, with at least one bin among them, and the shells that
+// its rows' pair factors come from (one range for both when i0 == j0).
+enum { kWideParts, kNarrowParts, kPartLists };
+struct F32Part {
+  int tile, r0, c0, nc;
+  int i0, ni, j0, nj;
+};
+
 struct DeviceSchedule {
   int n_tiles = 0;
   int sum_nc = 0;
@@ -72,6 +81,11 @@ struct DeviceSchedule {
   int32_t* map = nullptr;      // device, triangle index or -1
   int2* subs = nullptr;        // device, SIMT sub-tiles (tile, first column), 32 columns each
   int n_sub = 0;
+  F32Part* parts = nullptr;    // device, in the allocation of subs: the lists, one after another
+  int n_parts[kPartLists] = {};
+  int part_cols = 0;              // columns of a list's parts
+  int part_src = 8;               // the widest ni or nj
+  bool part_two = false;          // a part has two ranges
   std::vector<TileDesc> h_tiles;
   void release();
 };

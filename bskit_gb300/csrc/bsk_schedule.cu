@@ -27,6 +27,7 @@ void DeviceSchedule::release() {
   if (map) cudaFree(map);
   if (subs) cudaFree(subs);
   subs = nullptr;
+  parts = nullptr;
   n_sub = 0;
   tiles = nullptr;
   row_i = row_j = nullptr;
@@ -239,6 +240,52 @@ std::vector<int> choose_level_sides(const std::vector<HostTriangle>& tri,
   return lev;
 }
 
+// The parts of the tiles' rows and columns that hold bins, in blocks of 32 rows and of 8 columns.
+// A run of neighbouring column blocks is cut into pairs (kWideParts) or single blocks.
+static void f32_parts(const HostSchedule& hs, std::vector<F32Part> (&out)[kPartLists]) {
+  for (int u = 0; u < (int)hs.tiles.size(); ++u) {
+    const TileDesc& d = hs.tiles[u];
+    for (int r0 = 0; r0 < d.nrows; r0 += 32) {
+      const int r1 = std::min(r0 + 32, d.nrows);
+      int lo[2] = {1 << 30, 1 << 30}, hi[2] = {-1, -1};
+      for (int r = r0; r < r1; ++r) {
+        const int s[2] = {hs.ri[d.row_off + r], hs.rj[d.row_off + r]};
+        for (int k = 0; k < 2; ++k) {
+          lo[k] = std::min(lo[k], s[k]);
+          hi[k] = std::max(hi[k], s[k]);
+        }
+      }
+      F32Part p{u, r0, 0, 0, lo[0], round_up(hi[0] - lo[0] + 1, 8),
+                lo[1], round_up(hi[1] - lo[1] + 1, 8)};
+      const int all0 = std::min(lo[0], lo[1]);
+      const int all = round_up(std::max(hi[0], hi[1]) - all0 + 1, 8);
+      // one range unless two save 16 shells or more: the kernel for two is the slower one
+      if (all <= kMaxSrcRows && all < p.ni + p.nj + 16) {
+        p.i0 = p.j0 = all0;
+        p.ni = p.nj = all;
+      }
+      auto used = [&](int block) {
+        for (int c = 8 * block; c < 8 * block + 8; ++c)
+          for (int r = r0; r < r1; ++r)
+            if (hs.map[d.map_off + (size_t)c * kTileRows + r] >= 0) return true;
+        return false;
+      };
+      auto add = [&](int list, int block, int blocks) {
+        p.c0 = 8 * block;
+        p.nc = 8 * blocks;
+        out[list].push_back(p);
+      };
+      for (int b = 0; b < d.nc / 8;) {
+        int e = b;
+        while (e < d.nc / 8 && used(e)) ++e;
+        for (int k = b; k < e; k += 2) add(kWideParts, k, std::min(2, e - k));
+        for (int k = b; k < e; ++k) add(kNarrowParts, k, 1);
+        b = e + 1;  // block e holds no bin, or lies past the tile
+      }
+    }
+  }
+}
+
 void build_schedule(const std::vector<HostTriangle>& tri, int n_shells, DeviceSchedule& out,
                     const std::vector<int>* map_index) {
   out.release();
@@ -268,9 +315,26 @@ void build_schedule(const std::vector<HostTriangle>& tri, int n_shells, DeviceSc
   for (int u = 0; u < (int)tiles.size(); ++u)
     for (int c = 0; c < tiles[u].nc; c += 32) subs.push_back(make_int2(u, c));
   out.n_sub = (int)subs.size();
-  BSK_CHECK_CUDA(cudaMalloc(&out.subs, subs.size() * sizeof(int2)));
-  BSK_CHECK_CUDA(cudaMemcpy(out.subs, subs.data(), subs.size() * sizeof(int2),
-                            cudaMemcpyHostToDevice));
+  std::vector<F32Part> lists[kPartLists];
+  f32_parts(hs, lists);
+  out.part_cols = 0;
+  out.part_src = 8;
+  out.part_two = false;
+  for (const F32Part& p : lists[kWideParts]) {
+    out.part_cols += p.nc;
+    out.part_src = std::max(out.part_src, std::max(p.ni, p.nj));
+    out.part_two = out.part_two || p.i0 != p.j0;
+  }
+  // the parts lie after the sub-tiles, list after list
+  std::vector<char> both((const char*)subs.data(), (const char*)(subs.data() + subs.size()));
+  for (int k = 0; k < kPartLists; ++k) {
+    out.n_parts[k] = (int)lists[k].size();
+    both.insert(both.end(), (const char*)lists[k].data(),
+                (const char*)(lists[k].data() + lists[k].size()));
+  }
+  BSK_CHECK_CUDA(cudaMalloc(&out.subs, both.size()));
+  out.parts = (F32Part*)(out.subs + subs.size());
+  BSK_CHECK_CUDA(cudaMemcpy(out.subs, both.data(), both.size(), cudaMemcpyHostToDevice));
 }
 
 }  // namespace bsk

@@ -101,6 +101,12 @@ int main(int argc, char** argv) {
     rows = d.row_off + bsk::kTileRows;
     maps = d.map_off + (size_t)d.nc * bsk::kTileRows;
   }
+  const bsk::F32Part* p = s.parts;
+  for (int k = 0; k < bsk::kPartLists; ++k)
+    for (int n = 0; n < s.n_parts[k]; ++n, ++p)
+      printf("part %d %d %d %d %d %d %d %d %d\n", k, p->tile, p->r0, p->c0, p->nc, p->i0, p->ni,
+             p->j0, p->nj);
+  printf("parts %d %d %d\n", s.part_cols, s.part_src, (int)s.part_two);
   for (size_t r = 0; r < rows; ++r) printf("r %d %d\n", s.row_i[r], s.row_j[r]);
   for (size_t m = 0; m < maps; ++m) printf("m %d\n", s.map[m]);
   return 0;

@@ -133,3 +133,44 @@ def test_shards_of_three_fields_off_16_bytes(cuda, cut, n, kmax):
     whole = plan.measure_b(ts, slots=(0, 1, 2), precision="fp64")
     assert torch.all((parts - whole).abs() <= (SLICE + 2) * 2.0 ** -24 * top)
     plan.close()
+
+
+# sparse sets, whose items of a short grid partly hold no bin: the diagonal, one far corner, a band
+@pytest.mark.parametrize("shells", [9, 24, 40, 64, 90])
+@pytest.mark.parametrize("kind", ["diagonal", "corner", "band"])
+@pytest.mark.parametrize("k", [40, SLICE + 24])
+def test_chain_of_sparse_sets(cuda, shells, kind, k):
+    kf = 2 * np.pi / 100.0
+    edges = np.array([[q, q + 1.0] for q in range(1, shells + 1)]) * kf
+    s = np.arange(shells)
+    tri = {"diagonal": np.stack([s, s, s], 1),
+           "corner": np.array([[0, 0, 0], [shells - 1, shells - 2, shells - 1]]),
+           "band": np.stack([s, s // 2, np.maximum(s - 3, 0)], 1)}[kind]
+    plan = Plan(2 * (shells + 4), 100.0, edges, grid="native")
+    g = torch.Generator(device="cuda")
+    g.manual_seed(shells + k)
+    f = [torch.randn((shells, k), generator=g, device="cuda")] * 3
+    want, top = _chain(f, tri)
+    got = plan.contract(plan.triangles(tri), *f, precision="fp32")
+    assert torch.all((got - want).abs() <= 4 * 2.0 ** -24 * top + 2.0 ** -52 * top)
+    plan.close()
+
+
+# the same on long grids, where dense sets take whole tiles and sparse ones their parts
+@pytest.mark.parametrize("shells,distinct", [(40, 1), (64, 2)])
+def test_chain_of_sparse_sets_on_long_grids(cuda, shells, distinct):
+    kf = 2 * np.pi / 100.0
+    edges = np.array([[q, q + 1.0] for q in range(1, shells + 1)]) * kf
+    s = np.arange(shells)
+    tri = np.stack([s, s // 2, s], 1)
+    plan = Plan(2 * (shells + 4), 100.0, edges, grid="native")
+    g = torch.Generator(device="cuda")
+    g.manual_seed(shells)
+    f = [torch.randn((shells, SLICE), generator=g, device="cuda") for _ in range(distinct)]
+    want, top = _chain([f[0], f[-1], f[0]], tri)
+    repeat = 800
+    wide = [v.repeat(1, repeat) for v in f]
+    got = plan.contract(plan.triangles(tri), wide[0], wide[-1], wide[0], precision="fp32")
+    tol = 4 * 2.0 ** -24 * top + repeat * 2.0 ** -52 * top
+    assert torch.all((got - repeat * want).abs() <= repeat * tol)
+    plan.close()

@@ -153,3 +153,45 @@ def test_grid_level_sides_exact_and_cheapest(harness, tmp_path, case):
     best = min(_chain_cost(cost, list(sub) + [len(sides) - 1])
                for k in range(len(sides)) for sub in itertools.combinations(range(len(sides) - 1), k))
     assert _chain_cost(cost, chosen) <= best * (1 + 1e-12)
+
+
+@pytest.mark.parametrize("shells,kind", [(5, "all"), (9, "equi"), (20, "all"), (40, "equi"),
+                                         (40, "squeezed"), (64, "all"), (90, "sparse"),
+                                         (126, "band"), (200, "corner")])
+def test_parts_of_the_fp32_contraction(harness, tmp_path, shells, kind):
+    """In each list every bin lies in exactly one part; a part holds at least one, lies inside its
+    tile, and its source ranges hold its rows' shells, one range for both factors or two."""
+    s = np.arange(shells)
+    every = np.array([(a, b, c) for a in range(shells) for b in range(a + 1) for c in range(b + 1)
+                      if a <= b + c + 1]) if kind in ("all", "sparse") else None
+    tri = {"all": lambda: every, "sparse": lambda: every[::7],
+           "equi": lambda: np.stack([s, s, s], 1), "squeezed": lambda: np.stack([0 * s, s, s], 1),
+           "band": lambda: np.stack([s, s // 2, np.maximum(s - 3, 0)], 1),
+           "corner": lambda: np.array([[0, shells - 1, 3], [shells - 1, 0, shells - 1]])}[kind]()
+    tiles = schedule(harness, tmp_path, shells, tri)
+    out = subprocess.run([harness, str(tmp_path / "tri.txt")], check=True, capture_output=True,
+                         text=True).stdout.splitlines()
+    parts = [tuple(map(int, line.split()[1:])) for line in out if line.startswith("part ")]
+    cols, src, two = next(map(int, line.split()[1:]) for line in out if line.startswith("parts "))
+    rows = np.array([line.split()[1:] for line in out if line.startswith("r ")], dtype=int)
+    cmap = np.array([line.split()[1] for line in out if line.startswith("m ")], dtype=int)
+    blocks = []
+    for which in range(2):
+        mine = [p[1:] for p in parts if p[0] == which]
+        seen = np.zeros(len(tri), dtype=int)
+        for u, r0, c0, nc, i0, ni, j0, nj in mine:
+            d = tiles[u]
+            assert r0 % 32 == 0 and r0 < d["nrows"] and nc == 8 or nc == 16 and which == 0
+            assert c0 % 8 == 0 and c0 + nc <= d["nc"]
+            assert 8 <= ni <= 64 and 8 <= nj <= 64 and (i0 != j0 or ni == nj)
+            for i, j in rows[d["row_off"] + r0:d["row_off"] + min(r0 + 32, d["nrows"])]:
+                assert i0 <= i < i0 + ni and j0 <= j < j0 + nj
+            block = cmap[d["map_off"]:][:d["nc"] * 128].reshape(-1, 128)[c0:c0 + nc, r0:r0 + 32]
+            assert all(np.any(block[k:k + 8] >= 0) for k in range(0, nc, 8))
+            seen[block[block >= 0]] += 1
+        assert np.all(seen == 1)
+        assert cols == sum(p[3] for p in mine) and two == any(p[4] != p[6] for p in mine)
+        assert src == max([8] + [max(p[5], p[7]) for p in mine])
+        blocks.append(sorted((u, r0, c0 + k) for u, r0, c0, nc, *_ in mine
+                             for k in range(0, nc, 8)))
+    assert blocks[0] == blocks[1]
