@@ -235,34 +235,50 @@ class ClockSampler(object):
                 "reasons": sorted(reasons), "samples_in_region": n_inside}
 
 
-def kernel_launches_per_step(plan, ts, slots=(0, 0, 0)):
-    """Kernels of libbskit_gb300 launched by one step (cuFFT's R2C kernels excluded): the
-    spectrum extraction of each painted slot; per grid level the level's spectrum (levels
-    below the plan's grid), the field synthesis (X, Y, Z passes per batch of 8 shells from the
-    first that the level's bins use, the bf16 split written by the Z pass) and one
-    contraction; the normalisation.  (The sums of a contraction's last wave, on some sizes,
-    are one launch more.)"""
+def synthesis_batch(ngrid, qmax, n_shells):
+    """Shells per launch of a plan's field synthesis: a batch of 8, or more on small grids (as
+    long as the two intermediate arrays stay within 256 MiB)."""
+    rows, cols = min(2 * qmax + 1, ngrid), (qmax + 16) // 16 * 16
+    batch = min(n_shells, 8)
+    while batch < n_shells and \
+            (batch + 1) * ngrid * (rows + ngrid) * cols * 8 + 8 * ngrid <= 256 << 20:
+        batch += 1
+    return batch
+
+
+def kernel_launches_per_step(plan, ts):
+    """Kernels of libbskit_gb300 launched by one step of an auto bispectrum (cuFFT's R2C kernels
+    excluded): the spectrum extraction; per grid level the level's spectrum (levels below the
+    plan's grid), the field synthesis (X, Y, Z passes per batch of shells that the level's
+    bins use) and one contraction; the normalisation.  (The sums of a contraction's last wave,
+    on some sizes, are one launch more.)"""
     import numpy as np
-    nslot = len(set(slots))
     levels = ts.levels()
-    n = nslot
-    if levels:
-        # a level holds the bins that fit its side and no smaller level's; batches below its
-        # bins' first shell are not synthesised
-        kf = 2 * np.pi / plan.box_size
-        r = np.floor(np.asarray(plan.shell_edges).reshape(-1, 2)[:, 1] / kf * (1 + 1e-9))
-        tri = ts.indices
-        need = np.maximum(r[tri].sum(1), 2 * r[tri].max(1))
-        done = np.zeros(len(tri), bool)
-        for lv in levels:
-            if lv["ngrid"] != plan.ngrid:
-                n += nslot
-            mine = ~done & ((need < lv["ngrid"]) | (lv is levels[-1]))
-            done |= mine
-            first = int(tri[mine].min()) // 8 if mine.any() else 0
-            n += 3 * ((lv["shells"] + 7) // 8 - first) * nslot + 1
-    else:
-        n += 3 * ((plan.n_shells + 7) // 8) * nslot + 1 + 1  # synthesis, contraction, scale
+    kf = 2 * np.pi / plan.box_size
+    r = np.floor(np.asarray(plan.shell_edges).reshape(-1, 2)[:, 1] / kf * (1 + 1e-9)).astype(int)
+    if not levels:  # every shell; contraction and scale
+        batch = synthesis_batch(plan.ngrid, plan.qmax, plan.n_shells)
+        return 1 + 3 * -(-plan.n_shells // batch) + 2 + 1
+    n = 1
+    # a level holds the bins that fit its side and no smaller level's; its plan holds every shell
+    # that fits the side
+    tri = np.unique(ts.indices, axis=0)
+    need = np.maximum(r[tri].sum(1), 2 * r[tri].max(1))
+    done = np.zeros(len(tri), bool)
+    for lv in levels:
+        own = lv["ngrid"] == plan.ngrid
+        shells = plan.n_shells if own else int(np.sum(2 * r < lv["ngrid"]))
+        batch = synthesis_batch(lv["ngrid"], int(r[:shells].max()), shells)
+        mine = ~done & ((need < lv["ngrid"]) | own)
+        done |= mine
+        t = tri[mine]
+        factor, low, high = t[:, :2].min(), t[:, 2].min(), t[:, 2].max() + 1
+        first = min(factor, low) // min(shells, 8) * min(shells, 8)
+        for s0 in range(first, lv["shells"], batch):
+            s1 = min(s0 + batch, lv["shells"])
+            if s1 > factor or (s0 < high and s1 > low):
+                n += 3
+        n += 1 + (not own)
     return n + 1
 
 

@@ -319,3 +319,40 @@ def test_route_of_the_grid_information(eng, q, residues):
     assert (eng.launches("modular_finish_kernel") > 0) == residues
     assert (eng.launches("enum_finish_kernel") > 0) != residues
     eng.close(p, ts)
+
+
+@pytest.mark.parametrize("n,box,kmax,dk,levels", [
+    (64, 100.0, 16, 2.0, None), (128, 100.0, 32, 2.0, None), (256, 500.0, 64, 2.0, None),
+    (256, 500.0, 64, 2.0, "0.2"), (512, 1000.0, 128, 2.0, None), (512, 1000.0, 128, 2.0, "1"),
+    (128, 100.0, 32, 2.0, "single")])
+def test_launches_that_the_benchmark_states(eng, monkeypatch, n, box, kmax, dk, levels):
+    import bench
+    grid = _lib.GRID_REDUCED
+    if levels == "single":
+        grid = _lib.GRID_REDUCED_SINGLE
+    elif levels:
+        monkeypatch.setenv("BSK_LEVEL_MIN_POINTS", levels)
+    edges, tri = binning(box, kmax, dk)
+    p = eng.plan(n, box, edges, grid=grid)
+    ts = eng.triangles(p, tri)
+
+    class Shim(object):
+        box_size, shell_edges, n_shells = box, edges, len(edges)
+        ngrid, qmax = eng.info(p, _lib.INFO_NGRID), eng.info(p, _lib.INFO_QMAX)
+        indices = tri
+
+        @staticmethod
+        def levels():
+            out = (ctypes.c_int64 * 60)()
+            k = eng.lib.bsk_triset_levels(ts, out, 10)
+            return [dict(ngrid=int(out[6 * i]), shells=int(out[6 * i + 5])) for i in range(k)]
+
+    for _ in range(2):  # the second step has no tables to make
+        eng.lib.fake_reset_counts()
+        eng.paint(p)
+        eng.measure(p, ts)
+        eng.ok(eng.lib.bsk_normalize(len(tri), engine_fake.OUT, engine_fake.OUT, engine_fake.OUT,
+                                     None))
+    assert (bench.kernel_launches_per_step(Shim, Shim)
+            == eng.launches() - eng.launches("tail_sum_kernel"))
+    eng.close(p, ts)
