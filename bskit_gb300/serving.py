@@ -213,7 +213,7 @@ class Scheduler(object):
         return self.used + need <= self.mem_budget
 
     def _recount(self, g):
-        """A group holds more than it was admitted with once a bin set wants more scratch."""
+        """A group keeps more than it was admitted with once a bin set wants more scratch."""
         held = getattr(self.backend, "group_bytes", lambda _: 0)(g)
         if held > g.footprint:
             self.used += held - g.footprint
@@ -341,7 +341,7 @@ class EngineBackend(object):
                                    else torch.device(device).index or 0)
         self.use_graphs = use_graphs
         self.gridinfo = {}      # bin_key -> (ntri, kmean) device tensors
-        self.probe = {}         # shell_key -> measured footprint of one instance
+        self.probe = {}         # shell_key -> one instance: (footprint and meshes, scratch)
         self.mem_budget = None  # the server's: an instance above it takes lean plans
         self.lean = set()       # shell_keys whose plans keep no scratch
         self.captures = 0       # graphs captured (prepare + dispatch)
@@ -390,7 +390,7 @@ class EngineBackend(object):
 
     def group_footprint(self, job, size):
         fp = self.probe.get(job.shell_key)
-        if fp is not None and self.mem_budget is not None and fp > self.mem_budget \
+        if fp is not None and self.mem_budget is not None and sum(fp) > self.mem_budget \
                 and job.shell_key not in self.lean:
             self.lean.add(job.shell_key)  # slower, rather than never served
             fp = None
@@ -404,22 +404,19 @@ class EngineBackend(object):
             inst.plan.measure_b(self._tset(inst, job), slots=(0, 0, 1),
                                 precision=job.req.precision)
             self.torch.cuda.synchronize(self.device)
-            fp = self._instance_bytes(inst.plan)
-            self.probe[job.shell_key] = fp
+            self.probe[job.shell_key] = (inst.plan.footprint() + 2 * job.req.nmesh ** 3 * 4,
+                                         inst.plan.scratch_bytes())
             inst.plan.close()
             return self.group_footprint(job, size)
-        return fp * size
-
-    @staticmethod
-    def _instance_bytes(plan):
-        """The plan, with the scratch it keeps, and the instance's two meshes."""
-        return plan.footprint() + plan.scratch_bytes() + 2 * plan.nmesh ** 3 * 4
+        return sum(fp) * size
 
     def group_bytes(self, g):
-        each = [self._instance_bytes(inst.plan) for inst in g.instances]
-        # the shell set's next groups are admitted with what an instance of it came to hold
-        self.probe[g.shell_key] = max(each + [self.probe.get(g.shell_key, 0)])
-        return sum(each)
+        """What the group was measured at, with the scratch that its plans keep by now."""
+        fp, most = self.probe[g.shell_key]
+        scratch = [inst.plan.scratch_bytes() for inst in g.instances]
+        # the shell set's next groups are admitted with what an instance of it came to keep
+        self.probe[g.shell_key] = (fp, max([most] + scratch))
+        return fp * g.size + sum(scratch)
 
     def create_group(self, job, size):
         torch = self.torch
