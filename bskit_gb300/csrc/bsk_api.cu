@@ -397,6 +397,12 @@ bool ensure_split(bsk_plan* p, int s, cudaStream_t st, int n_need = -1) {
   return built;
 }
 
+bool is_capturing(cudaStream_t st) {
+  cudaStreamCaptureStatus s = cudaStreamCaptureStatusNone;
+  BSK_CHECK_CUDA(cudaStreamIsCapturing(st, &s));
+  return s != cudaStreamCaptureStatusNone;
+}
+
 // A range of shells [from, to).
 struct Shells {
   int from = 0, to = 0;
@@ -428,10 +434,12 @@ bool ensure_level_fields(bsk_plan* q, int s, cudaStream_t st, int nn, int fp_fro
   FieldSlot& f = q->slot[s];
   BSK_REQUIRE(f.painted, BSK_ERR_STATE, "field slot " + std::to_string(s) + " was not painted");
   nn = std::min(nn, q->n);
-  const Shells have = f.fields_ok ? Shells{f.fields_from, f.fields_n} : Shells{};
-  const Shells have_split = f.split_ok ? Shells{f.split_from, f.split_n} : Shells{};
+  Shells have = f.fields_ok ? Shells{f.fields_from, f.fields_n} : Shells{};
+  Shells have_split = f.split_ok ? Shells{f.split_from, f.split_n} : Shells{};
   const Shells need{std::min(fp_from, nn), nn}, need_split{col_from, col_to};
   if (have.has(need) && have_split.has(need_split)) return false;
+  // a graph makes all that its set needs: by its replay the slot may hold another mesh's
+  if (is_capturing(st)) have = have_split = Shells{};
   const Shells want = have.hull(need), want_split = have_split.hull(need_split);
   if (!f.fields && !want.empty()) {  // a column-only slot needs no FP32 fields
     check_budget(q, (size_t)q->n_alloc() * q->K * sizeof(float), "the shell fields");
@@ -616,9 +624,7 @@ struct TailScratch {
   TailScratch(bsk_plan* plan, size_t need, int precision, bool built, cudaStream_t s)
       : p(plan), st(s) {
     if (!need || (precision != BSK_PREC_BF16X3 && precision != BSK_PREC_BF16)) return;
-    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
-    BSK_CHECK_CUDA(cudaStreamIsCapturing(st, &cap));
-    const bool capturing = cap != cudaStreamCaptureStatusNone;
+    const bool capturing = is_capturing(st);
     if (built) {
       grow_scratch(p, p->build_scratch, p->build_bytes, need, p->build_captured || capturing);
       p->build_captured = p->build_captured || capturing;

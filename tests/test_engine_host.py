@@ -356,3 +356,23 @@ def test_launches_that_the_benchmark_states(eng, monkeypatch, n, box, kmax, dk, 
     assert (bench.kernel_launches_per_step(Shim, Shim)
             == eng.launches() - eng.launches("tail_sum_kernel"))
     eng.close(p, ts)
+
+
+def test_a_captured_synthesis_depends_on_no_earlier_one(eng, monkeypatch):
+    """A graph that synthesises makes every shell its set needs: it may be replayed after another
+    paint, when what an eager call had made is of the mesh before."""
+    monkeypatch.setenv("BSK_LEVEL_MIN_POINTS", "0.9")
+    edges, tri = binning(500.0, 64, 2.0)
+    p = eng.plan(256, 500.0, edges)
+    low, every = eng.triangles(p, tri[tri.max(1) < 9]), eng.triangles(p, tri)
+    eng.paint(p)
+    eng.lib.fake_reset_counts()
+    eng.measure(p, every)
+    whole = eng.launches("x_kernel")
+    eng.paint(p)
+    eng.measure(p, low)
+    eng.lib.fake_reset_counts()
+    with eng.capture():
+        eng.measure(p, every)
+    assert eng.launches("x_kernel") == whole == 4
+    eng.close(p, low, every)
