@@ -542,8 +542,8 @@ void grow_scratch(bsk_plan* p, void*& ptr, size_t& have, size_t need, bool keep)
     ptr = nullptr;
     have = 0;
   }
-  // at least double beside a kept one, so that the kept ones together stay below the last
-  const size_t bytes = std::max(need, 2 * have);
+  // double beside a kept one, so that there are few of them
+  const size_t bytes = std::max(need, std::min(2 * have, kMaxContractScratch));
   void* q = nullptr;
   if (cudaMalloc(&q, bytes) != cudaSuccess) {
     cudaGetLastError();

@@ -977,9 +977,8 @@ void make_split_map(CUtensorMap* m, const __nv_bfloat16* split, int S, int64_t K
 // (~8 units, launch included) and for writing and reading their scratch (~4 units a megabyte
 // over ~5 TB/s: 0.5 unit).  Taken when that saves 3%: the 7 items of 48^3 (110 -> 15 us with
 // the sum kernel) and the 54 of 96^3 do; a last wave that is more than about half full
-// does not.  Scratch above kMaxTailBytes is not considered.
+// does not.  Scratch above kMaxContractScratch is not considered.
 constexpr double kTailSumStages = 8.0, kTailStagesPerMB = 0.5;
-constexpr size_t kMaxTailBytes = (size_t)128 << 20;
 
 struct Split {
   int64_t slice = kSliceShort;
@@ -1004,7 +1003,7 @@ Split make_split(const std::vector<TileDesc>& tiles, int64_t points, int num_sms
   for (const TileDesc& d : tiles) nc = std::max(nc, d.nc);
   const size_t bytes =
       (size_t)rem * (sp.slice / KCH) * 2 * nc * kTileRows * sizeof(float);
-  if (bytes > kMaxTailBytes || bytes > scratch_have) return sp;
+  if (bytes > kMaxContractScratch || bytes > scratch_have) return sp;
   const double extra = kTailSumStages + kTailStagesPerMB * bytes / 1e6;
   int best_ps = 0;
   double best = 0.97 * stages;  // the last wave as it is
@@ -1031,7 +1030,7 @@ Split make_split(const std::vector<TileDesc>& tiles, int64_t points, int num_sms
 
 size_t contract_tc_scratch(const std::vector<TileDesc>& tiles, int64_t points, int num_sms) {
   if (tiles.empty() || points <= 0) return 0;
-  return tc::make_split(tiles, points, num_sms, tc::kMaxTailBytes).scratch_bytes;
+  return tc::make_split(tiles, points, num_sms, kMaxContractScratch).scratch_bytes;
 }
 
 void launch_contract_tc(const DeviceSchedule& s, const float* f1, const float* f2,

@@ -354,6 +354,7 @@ void launch_contract_tc(const DeviceSchedule& s, const float* f1, const float* f
                         void* scratch = nullptr, size_t scratch_bytes = 0);
 // Scratch with which launch_contract_tc spreads the last wave of a schedule's items over all
 // SMs (0: it has no use for any; with less than this it runs without, with the same result).
+constexpr size_t kMaxContractScratch = (size_t)128 << 20;
 size_t contract_tc_scratch(const std::vector<TileDesc>& tiles, int64_t points, int num_sms);
 
 // The contraction modulo a prime p < kModMaxPrime: out[t] += the sum over K of f[i] f[j] f3[l],
