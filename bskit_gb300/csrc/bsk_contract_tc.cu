@@ -975,7 +975,7 @@ void make_split_map(CUtensorMap* m, const __nv_bfloat16* split, int S, int64_t K
 // the launch takes ceil(items / SMs) x the stages of a slice.  With one, the last wave's items
 // go out in parts of `ps` stages, in ceil(parts / SMs) rounds, then pay for tail_sum_kernel
 // (~8 units, launch included) and for writing and reading their scratch (~4 units a megabyte
-// over ~5 TB/s: 0.5 unit).  Taken when that saves 3%: the 7 items of 48^3 (110 -> 15 us with
+// over ~5 TB/s: 0.5 unit).  Taken when that saves 3%: the 7 items of 48^3 (110 -> 17 us with
 // the sum kernel) and the 54 of 96^3 do; a last wave that is more than about half full
 // does not.  Scratch above kMaxContractScratch is not considered.
 constexpr double kTailSumStages = 8.0, kTailStagesPerMB = 0.5;

@@ -265,9 +265,12 @@ namespace bsk {
 // become resident while its predecessor in the stream drains, so its first statement that
 // touches what earlier kernels wrote, or writes what they read, comes after pdl_wait(), which
 // returns when the predecessor has completed and its writes are visible.  pdl_trigger() lets
-// the successor come: called at the start.  Measured: 128^3 <AAB> (96^3) 232 -> 216 us, eight
-// 128^3 sub-boxes 1197 -> 1138; but 256^3 (192^3) 1621 -> 1663 us and 512^3 cross 11.8 -> 13.0 ms,
-// where early blocks hold an SM in the predecessor's shared-memory split for their whole run.
+// the successor come: called at the start.  Measured, without / with: 48^3 61 / 52 us a pass, 96^3
+// 153 / 146, 108^3 191 / 181, 120^3 222 / 217 (128^3 <AAB>, 96^3, 232 / 216; eight 128^3 sub-boxes
+// 1197 / 1138); above it depends on the binning: 144^3 295 / 287 (8 shells) and 360 / 358 (15),
+// 160^3 396 / 399 and 491 / 477, 192^3 1621 / 1663 (31), 512^3 cross 11.8 / 13.0 ms, where early
+// blocks hold an SM in the predecessor's shared-memory split for their whole run.  Replays of a
+// captured pass, which have no launch gaps, move by less than 3% either way.
 constexpr int kPdlSide = 128;
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void pdl_trigger() {
