@@ -325,43 +325,25 @@ __device__ __forceinline__ void run_item(float* sm, int src, const TileDesc& td,
     }
 }
 
-// Item = (slice, sub-tile of 32 columns) on long grids, (slice, part) on short ones.
+// Long grids: item = (slice, sub-tile of 32 columns).
 template <class C>
 __global__ void __launch_bounds__(32)
     contract_f32_kernel(const TileDesc* __restrict__ tiles, const int2* __restrict__ subs,
-                        const F32Part* __restrict__ parts, int per_slice,
-                        const int16_t* __restrict__ row_i, const int16_t* __restrict__ row_j,
-                        const int32_t* __restrict__ map, const float* __restrict__ f1,
-                        const float* __restrict__ f2, const float* __restrict__ f3, int n_shells,
-                        int64_t K, int64_t k_begin, int64_t k_end, int64_t n_slices, int src,
-                        double* __restrict__ out, double scale) {
+                        int n_sub, const int16_t* __restrict__ row_i,
+                        const int16_t* __restrict__ row_j, const int32_t* __restrict__ map,
+                        const float* __restrict__ f1, const float* __restrict__ f2,
+                        const float* __restrict__ f3, int n_shells, int64_t K, int64_t k_begin,
+                        int64_t k_end, int64_t n_slices, int src, double* __restrict__ out,
+                        double scale) {
   extern __shared__ __align__(16) float f32_smem[];
   float* sm = f32_smem;
-  constexpr bool kParts = C::TR != 16;
-  for (int64_t item = blockIdx.x; item < n_slices * per_slice; item += gridDim.x) {
-    const int64_t sl = item / per_slice;
-    const int in_slice = (int)(item - sl * per_slice);
-    TileDesc td;
-    int r0 = 0, c0, nc;
-    if constexpr (kParts) {
-      const F32Part p = parts[in_slice];
-      td = tiles[p.tile];
-      td.i0 = p.i0;
-      td.ni = p.ni;
-      td.j0 = p.j0;
-      td.nj = p.nj;
-      r0 = p.r0;
-      c0 = p.c0;
-      nc = p.nc;
-    } else {
-      const int2 sub = subs[in_slice];
-      td = tiles[sub.x];
-      // the tile's columns in as many equal runs, multiples of 8, as it has 32-column sub-tiles
-      const int runs = (td.nc + COLS - 1) / COLS;
-      const int width = ((td.nc + runs - 1) / runs + 7) / 8 * 8;
-      c0 = sub.y / COLS * width;
-      nc = min(width, td.nc - c0);
-    }
+  for (int64_t item = blockIdx.x; item < n_slices * n_sub; item += gridDim.x) {
+    const int64_t sl = item / n_sub;
+    const int2 sub = subs[(int)(item - sl * n_sub)];
+    const TileDesc td = tiles[sub.x];
+    // the tile's columns in as many equal runs, multiples of 8, as it has 32-column sub-tiles
+    const int runs = (td.nc + COLS - 1) / COLS, width = ((td.nc + runs - 1) / runs + 7) / 8 * 8;
+    const int c0 = sub.y / COLS * width, nc = min(width, td.nc - c0), r0 = 0;
     const bool one_src = !C::kTwoSrc || (f1 == f2 && td.i0 == td.j0);
     const int64_t x_begin = k_begin + sl * SLICE;
     const int64_t x_end = min(k_end, x_begin + SLICE);
@@ -369,12 +351,41 @@ __global__ void __launch_bounds__(32)
       run_item<C, 2>(sm, src, td, r0, c0, row_i, row_j, map, f1, f2, f3, n_shells, K, x_begin, x_end, one_src, out, scale);
     else if (nc <= 16)
       run_item<C, 4>(sm, src, td, r0, c0, row_i, row_j, map, f1, f2, f3, n_shells, K, x_begin, x_end, one_src, out, scale);
-    else if constexpr (!kParts) {
-      if (nc <= 24)
-        run_item<C, 6>(sm, src, td, r0, c0, row_i, row_j, map, f1, f2, f3, n_shells, K, x_begin, x_end, one_src, out, scale);
-      else
-        run_item<C, 8>(sm, src, td, r0, c0, row_i, row_j, map, f1, f2, f3, n_shells, K, x_begin, x_end, one_src, out, scale);
-    }
+    else if (nc <= 24)
+      run_item<C, 6>(sm, src, td, r0, c0, row_i, row_j, map, f1, f2, f3, n_shells, K, x_begin, x_end, one_src, out, scale);
+    else
+      run_item<C, 8>(sm, src, td, r0, c0, row_i, row_j, map, f1, f2, f3, n_shells, K, x_begin, x_end, one_src, out, scale);
+  }
+}
+
+// Short grids and sparse sets: item = (slice, part).
+template <class C>
+__global__ void __launch_bounds__(32)
+    contract_f32_parts_kernel(const TileDesc* __restrict__ tiles,
+                              const F32Part* __restrict__ parts, int n_parts,
+                              const int16_t* __restrict__ row_i,
+                              const int16_t* __restrict__ row_j, const int32_t* __restrict__ map,
+                              const float* __restrict__ f1, const float* __restrict__ f2,
+                              const float* __restrict__ f3, int n_shells, int64_t K,
+                              int64_t k_begin, int64_t k_end, int64_t n_slices, int src,
+                              double* __restrict__ out, double scale) {
+  extern __shared__ __align__(16) float f32_smem[];
+  float* sm = f32_smem;
+  for (int64_t item = blockIdx.x; item < n_slices * n_parts; item += gridDim.x) {
+    const int64_t sl = item / n_parts;
+    const F32Part p = parts[(int)(item - sl * n_parts)];
+    TileDesc td = tiles[p.tile];
+    td.i0 = p.i0;
+    td.ni = p.ni;
+    td.j0 = p.j0;
+    td.nj = p.nj;
+    const bool one_src = !C::kTwoSrc || (f1 == f2 && td.i0 == td.j0);
+    const int64_t x_begin = k_begin + sl * SLICE;
+    const int64_t x_end = min(k_end, x_begin + SLICE);
+    if (p.nc <= 8)
+      run_item<C, 2>(sm, src, td, p.r0, p.c0, row_i, row_j, map, f1, f2, f3, n_shells, K, x_begin, x_end, one_src, out, scale);
+    else
+      run_item<C, 4>(sm, src, td, p.r0, p.c0, row_i, row_j, map, f1, f2, f3, n_shells, K, x_begin, x_end, one_src, out, scale);
   }
 }
 
@@ -385,30 +396,38 @@ __global__ void __launch_bounds__(32)
 template <class C>
 constexpr int64_t kNarrowPerSm = C::kTwoSrc ? 8 : 11;
 
+template <class Kern>
+unsigned blocks(Kern kern, size_t smem, size_t most_smem, int64_t items, int num_sms) {
+  BSK_CHECK_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                      (int)most_smem));
+  int per_sm = 0;
+  BSK_CHECK_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, 32, smem));
+  return (unsigned)std::min<int64_t>((int64_t)num_sms * std::max(per_sm, 1), items);
+}
+
 template <class C>
 void launch(const DeviceSchedule& s, const float* f1, const float* f2, const float* f3,
             int n_shells, int64_t K, int64_t k_begin, int64_t k_end, double* out, int num_sms,
             cudaStream_t st, double scale) {
   const int64_t n_slices = (k_end - k_begin + SLICE - 1) / SLICE;
-  constexpr bool kParts = C::TR != 16;
-  int src = kParts ? s.part_src : 8;
-  if (!kParts)
+  if constexpr (C::TR == 16) {
+    int src = 8;
     for (const TileDesc& d : s.h_tiles) src = std::max(src, std::max(d.ni, d.nj));
-  const int list = n_slices * s.n_parts[kNarrowParts] <= kNarrowPerSm<C> * num_sms ? kNarrowParts
-                                                                               : kWideParts;
-  const F32Part* parts = s.parts + (list == kNarrowParts ? s.n_parts[kWideParts] : 0);
-  const int per_slice = kParts ? s.n_parts[list] : s.n_sub;
-  const size_t smem = C::smem(src);
-  auto kern = contract_f32_kernel<C>;
-  BSK_CHECK_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                      (int)C::smem(SRC)));
-  int per_sm = 0;
-  BSK_CHECK_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, 32, smem));
-  const int64_t grid =
-      std::min<int64_t>((int64_t)num_sms * std::max(per_sm, 1), n_slices * per_slice);
-  kern<<<(unsigned)grid, 32, smem, st>>>(s.tiles, s.subs, parts, per_slice, s.row_i, s.row_j,
-                                         s.map, f1, f2, f3, n_shells, K, k_begin, k_end, n_slices,
-                                         src, out, scale);
+    auto kern = contract_f32_kernel<C>;
+    const size_t smem = C::smem(src);
+    kern<<<blocks(kern, smem, C::smem(SRC), n_slices * s.n_sub, num_sms), 32, smem, st>>>(
+        s.tiles, s.subs, s.n_sub, s.row_i, s.row_j, s.map, f1, f2, f3, n_shells, K, k_begin, k_end,
+        n_slices, src, out, scale);
+  } else {
+    const int list = n_slices * s.n_parts[kNarrowParts] <= kNarrowPerSm<C> * num_sms ? kNarrowParts
+                                                                                 : kWideParts;
+    const F32Part* parts = s.parts + (list == kNarrowParts ? s.n_parts[kWideParts] : 0);
+    auto kern = contract_f32_parts_kernel<C>;
+    const size_t smem = C::smem(s.part_src);
+    kern<<<blocks(kern, smem, C::smem(SRC), n_slices * s.n_parts[list], num_sms), 32, smem, st>>>(
+        s.tiles, parts, s.n_parts[list], s.row_i, s.row_j, s.map, f1, f2, f3, n_shells, K, k_begin,
+        k_end, n_slices, s.part_src, out, scale);
+  }
   BSK_CHECK_CUDA(cudaGetLastError());
 }
 }  // namespace f32
