@@ -853,8 +853,8 @@ void measure_b_stream(bsk_plan* p, const bsk_triset* set, int a, int b, int c, i
 // cost proportional to Ng^3 per point, with the shells they use synthesised on those grids.
 
 // The grid-level plan of side Ng of p (made on first use, holding every shell of p that
-// fits the side, at least shells [0, n)).  Its spectra come from p's slots (launch_subgrid); it has no transforms of
-// its own besides the field synthesis.
+// fits the side, at least shells [0, n)).  Its spectra come from p's slots (launch_subgrid);
+// it has no transforms of its own besides the field synthesis.
 bsk_plan* level_plan(bsk_plan* p, int Ng, int n) {
   for (bsk_plan* q : p->levels)
     if (q->Ng == Ng) {

@@ -348,13 +348,17 @@ __global__ void __launch_bounds__(32)
     const int64_t x_begin = k_begin + sl * SLICE;
     const int64_t x_end = min(k_end, x_begin + SLICE);
     if (nc <= 8)
-      run_item<C, 2>(sm, src, td, r0, c0, row_i, row_j, map, f1, f2, f3, n_shells, K, x_begin, x_end, one_src, out, scale);
+      run_item<C, 2>(sm, src, td, r0, c0, row_i, row_j, map, f1, f2, f3, n_shells, K, x_begin,
+                     x_end, one_src, out, scale);
     else if (nc <= 16)
-      run_item<C, 4>(sm, src, td, r0, c0, row_i, row_j, map, f1, f2, f3, n_shells, K, x_begin, x_end, one_src, out, scale);
+      run_item<C, 4>(sm, src, td, r0, c0, row_i, row_j, map, f1, f2, f3, n_shells, K, x_begin,
+                     x_end, one_src, out, scale);
     else if (nc <= 24)
-      run_item<C, 6>(sm, src, td, r0, c0, row_i, row_j, map, f1, f2, f3, n_shells, K, x_begin, x_end, one_src, out, scale);
+      run_item<C, 6>(sm, src, td, r0, c0, row_i, row_j, map, f1, f2, f3, n_shells, K, x_begin,
+                     x_end, one_src, out, scale);
     else
-      run_item<C, 8>(sm, src, td, r0, c0, row_i, row_j, map, f1, f2, f3, n_shells, K, x_begin, x_end, one_src, out, scale);
+      run_item<C, 8>(sm, src, td, r0, c0, row_i, row_j, map, f1, f2, f3, n_shells, K, x_begin,
+                     x_end, one_src, out, scale);
   }
 }
 
@@ -383,9 +387,11 @@ __global__ void __launch_bounds__(32)
     const int64_t x_begin = k_begin + sl * SLICE;
     const int64_t x_end = min(k_end, x_begin + SLICE);
     if (p.nc <= 8)
-      run_item<C, 2>(sm, src, td, p.r0, p.c0, row_i, row_j, map, f1, f2, f3, n_shells, K, x_begin, x_end, one_src, out, scale);
+      run_item<C, 2>(sm, src, td, p.r0, p.c0, row_i, row_j, map, f1, f2, f3, n_shells, K, x_begin,
+                     x_end, one_src, out, scale);
     else
-      run_item<C, 4>(sm, src, td, p.r0, p.c0, row_i, row_j, map, f1, f2, f3, n_shells, K, x_begin, x_end, one_src, out, scale);
+      run_item<C, 4>(sm, src, td, p.r0, p.c0, row_i, row_j, map, f1, f2, f3, n_shells, K, x_begin,
+                     x_end, one_src, out, scale);
   }
 }
 

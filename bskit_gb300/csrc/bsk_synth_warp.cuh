@@ -244,9 +244,10 @@ __device__ __forceinline__ void fill_twiddles(float2* t, const float2* __restric
   }
 }
 
-// L lines: load(line, r, j, v) -> v[r] = input j + RB r of the line for every r; store(line, k, v):
-// outputs k + RA q in v[q]; mid() runs between the stages, when every input has been read.  Each lane's butterflies are numbered with the line fastest or
-// slowest (the layout of the global arrays decides which coalesces).
+// L lines: load(line, j, v) -> v[r] = input j + RB r of the line for every r; store(on, line, k,
+// v): outputs k + RA q in v[q], of no line unless `on`; mid() runs between the stages, when every
+// input has been read.  Each lane's butterflies are numbered with the line fastest or slowest
+// (the layout of the global arrays decides which coalesces).
 template <int N, int L, bool kLineFast, class Load, class Mid, class Store>
 __device__ __forceinline__ void warp_fft(float2* __restrict__ buf, const float2* __restrict__ tw,
                                          const FftPlan& pl, Load load, Mid mid, Store store) {

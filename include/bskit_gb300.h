@@ -232,8 +232,10 @@ int bsk_measure_b_range(bsk_plan* plan, const bsk_triset* set, int slot_a, int s
  * three times the largest |q_c| of a shell mode: every reduced plan) and the
  * plan has at most 64 shells, the sums over the lattice triangles q1 + q2 + q3
  * = 0 are evaluated exactly (integer counts, fixed-point |q| sums): from
- * residues modulo small primes when 40 <= qmax <= 159 and the temporary memory
- * (3.4 GB for 63 shells at 512^3) fits, else by enumeration; otherwise from FP64 indicator / |k| fields and an FP64 contraction
+ * residues modulo small primes when 40 <= qmax <= 159 (below 53 not for plans of
+ * few modes) and the temporary memory (3.4 GB for 63 shells at 512^3) fits, else
+ * by enumeration, which also takes over when a bounded wait expired on the way.
+ * Otherwise they come from FP64 indicator / |k| fields and an FP64 contraction
  * (counts are the rounded FP64 sums).  The exact routes synchronise `stream`.
  * Replaces: FFTBispectrum.measure_gridinfo_faster, bskit/main.py:1941-2132,
  *           compute_Nbin / compute_k_means_on_grid, main.py:431-567.
